@@ -6,10 +6,9 @@
 //   r = b - A x0; z = M r; r_z = <r,z>; p = z
 //   loop: Ap = A p; alpha = r_z/<Ap,p>; x += alpha p; r -= alpha Ap; test;
 //         z = M r; beta = (1/r_z) * <r,z>; r_z = <r,z>; p = z + beta p
-// Three kernels per iteration: SpMV with the fused <Ap,p>, the x/r update with the fused
-// norms and the convergence test, and the p update.  Scalars and the done flag stay on
-// the device; kernels of iterations after the stop return at once, so the host polls
-// only every few iterations, replaying a CUDA graph of a fixed chunk of iterations.
+// One cooperative launch runs many iterations (k_pcg64): SpMV with <Ap,p>, the x/r update
+// with the norms and the convergence test, and the p update, a grid barrier after each.
+// Scalars stay on the device; the host polls after each launch.
 //
 // Mixed path: CG on an FP32 copy of the matrix with FP32 vectors, with "reliable updates"
 // in FP64: whenever the recursive FP32 residual has dropped by a factor delta (default 0.1)
@@ -20,15 +19,17 @@
 // the direction keeps the iteration count close to the FP64 CG's, where restarting an inner
 // solve per refinement step would lose the Krylov space each time.  With Jacobi the FP32
 // segments run CG on D^-1/2 A D^-1/2 (the same iterates in exact arithmetic, no diagonal
-// read per iteration) in two kernels per iteration (see k_update32s).
+// read per iteration) in two steps per iteration (see k_pcg32).
 //
 // Inner products.  GB300 runs FP64 FMA and FP32<->FP64 conversion at about 0.5 Tera-op/s,
 // some 70x below FP32.  FP64-path dots accumulate in FP64.  FP32-path dots form each
 // product exactly as an FP32 pair (p = a*b, e = fma(a,b,-p)) and accumulate it with a
-// compensated (double-float) sum; each thread's sum is converted once and the block and
-// grid totals are added in FP64.  Reductions are deterministic: fixed grid, fixed
-// per-thread index sets, block partials summed in index order by the last block.
+// compensated (double-float) sum; blocks add their threads' pairs in float-float and the grid
+// total is formed in FP64.  Reductions are deterministic: fixed grid, fixed per-thread index
+// sets, block partials summed in a fixed order.
+#include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -43,7 +44,8 @@ enum { S_RZ = 0, S_ALPHA, S_BETA, S_ERR, S_TOL, S_APP, S_RNRMM, S_BNRM, S_R0NRM,
        S_RRH, S_COUNT = 16 };
 // I_PEND: a segment end decided by the last x/r/p update, taken at the next iteration;
 // I_SKIPP: this iteration's update keeps p (the segment ends after it)
-enum { I_ITER = 0, I_DONE, I_CONV, I_MAXIT, I_FLAG, I_PEND, I_SKIPP, I_COUNT = 8 };
+// I_ABORT: a grid barrier of the CG kernels ran out of time
+enum { I_ITER = 0, I_DONE, I_CONV, I_MAXIT, I_FLAG, I_PEND, I_SKIPP, I_ABORT, I_COUNT = 8 };
 // FLAG_BREAK: the FP32 recurrence broke down (non-finite or non-positive r_z, residual grown
 // 1e4-fold): the segment's correction is dropped and the solve finishes in FP64
 enum { FLAG_NONE = 0, FLAG_UPDATE = 1, FLAG_CHECK = 2, FLAG_MAXIT = 3, FLAG_BREAK = 4 };
@@ -85,14 +87,11 @@ struct AccPlain {
   __device__ __forceinline__ double value() const { return (double)s; }
 };
 
-// <q,q> of the fused mixed SpMV: compensated (1) or plain per-thread FP32 sums (0).  Measured
-// on GB300 at 128^3 Q2: plain sums 1097 iterations and 0.853 ms per iteration, compensated
-// 1106 and 0.863 ms (a thread sums ~80 positive terms; the grid total is formed in FP64).
-#ifndef FG_MIXED_QQ_COMPENSATED
-#define FG_MIXED_QQ_COMPENSATED 0
-#endif
-// the fused update sums the unscaled residual norm (the stop estimate) every
-// FG_MIXED_EXACT_EVERY iterations (a divisor of the graph chunk); 8 vs 4: -2 us per iteration
+// (<q,q> of the mixed iteration.  Measured on GB300 at 128^3 Q2: plain sums 1097 iterations,
+// compensated 1106: a thread sums ~80 positive terms, the grid total is formed in FP64.)
+
+// the mixed update sums the unscaled residual norm (the stop estimate) every
+// FG_MIXED_EXACT_EVERY iterations; 8 vs 4: -2 us per iteration at 128^3 Q2
 #ifndef FG_MIXED_EXACT_EVERY
 #define FG_MIXED_EXACT_EVERY 8
 #endif
@@ -164,121 +163,7 @@ __device__ __forceinline__ void ld4(const double* p, double (&v)[4]) {
 // ---------------------------------------------------------------------------
 // Mixed path, FP32 segments on the scaled system A^ = S A S, S = D^-1/2 (D = diag A): Jacobi
 // PCG on A is CG on A^ with x = S x^ and r = S^-1 r^, so no diagonal is streamed per
-// iteration.  Two kernels per iteration:
-//   SpMV (MODE 3): q = A^ p, <p,q>, <q,q>; then alpha = |r|^2/<p,q> and, by the recurrence
-//     |r - alpha q|^2 = alpha^2 |q|^2 - |r|^2 (as <r,q> = <p,q> in CG), beta = |r_new|^2/|r|^2;
-//   update: x += alpha p; r -= alpha q; p = r + beta p; the exact |r_new|^2 for the next alpha,
-//     and on every fourth iteration sum r^2 D (the unscaled residual, for the stop estimate).
-// A segment end (reliable update, stop check, breakdown, iteration limit) found by an update
-// is taken one iteration later: that iteration's update keeps p, so the host can fold x and
-// restart the recursion from the true residual with the direction kept.
-__device__ __forceinline__ void mixed_alpha_beta(double pap, double qq, double* S, int* I) {
-  const double rr = S[S_RRH];
-  int skip = I[I_PEND] != FLAG_NONE;
-  double a = 0.0, b = 0.0;
-  if (!(pap > 0.0 && pap <= 1e300) || !(qq <= 1e300)) {
-    I[I_PEND] = FLAG_BREAK;  // alpha = 0: the update leaves x and r as they are
-    skip = 1;
-  } else {
-    a = rr / pap;
-    const double rrn = a * a * qq - rr;
-    b = rrn / rr;
-    if (!(rrn > 0.0)) {  // the recurrence lost its digits: end the segment here
-      skip = 1;
-      if (I[I_PEND] == FLAG_NONE) I[I_PEND] = FLAG_UPDATE;
-    }
-  }
-  S[S_ALPHA] = a;
-  S[S_BETA] = b;
-  I[I_SKIPP] = skip;
-}
-
-template <bool EXACT>
-__global__ void __launch_bounds__(RB)
-    k_update32s(int64_t n, float* __restrict__ x, float* __restrict__ r, float* __restrict__ p,
-                const float* __restrict__ q, const float* __restrict__ idiag, RedBuf rb, double* S, int* I) {
-  if (I[I_DONE]) return;
-  const float a = (float)S[S_ALPHA], b = (float)S[S_BETA];
-  const bool keep_p = I[I_SKIPP] != 0;
-  Acc<float> rr, rt;
-  const int64_t t0 = blockIdx.x * (int64_t)RB + threadIdx.x, stride = (int64_t)gridDim.x * RB;
-  const int64_t n4 = n >> 2;
-  {
-    float4* x4 = reinterpret_cast<float4*>(x);
-    float4* r4 = reinterpret_cast<float4*>(r);
-    float4* p4 = reinterpret_cast<float4*>(p);
-    const float4* q4 = reinterpret_cast<const float4*>(q);
-    const float4* d4 = reinterpret_cast<const float4*>(idiag);
-    for (int64_t i = t0; i < n4; i += stride) {
-      float4 xi = x4[i], ri = r4[i], pi = p4[i];
-      const float4 qi = q4[i];
-      xi.x = fmaf(a, pi.x, xi.x);
-      xi.y = fmaf(a, pi.y, xi.y);
-      xi.z = fmaf(a, pi.z, xi.z);
-      xi.w = fmaf(a, pi.w, xi.w);
-      ri.x = fmaf(-a, qi.x, ri.x);
-      ri.y = fmaf(-a, qi.y, ri.y);
-      ri.z = fmaf(-a, qi.z, ri.z);
-      ri.w = fmaf(-a, qi.w, ri.w);
-      x4[i] = xi;
-      r4[i] = ri;
-      if (!keep_p) {
-        pi.x = fmaf(b, pi.x, ri.x);
-        pi.y = fmaf(b, pi.y, ri.y);
-        pi.z = fmaf(b, pi.z, ri.z);
-        pi.w = fmaf(b, pi.w, ri.w);
-        p4[i] = pi;
-      }
-      rr.add(ri.x, ri.x);
-      rr.add(ri.y, ri.y);
-      rr.add(ri.z, ri.z);
-      rr.add(ri.w, ri.w);
-      if (EXACT) {
-        const float4 di = idiag ? d4[i] : make_float4(1.f, 1.f, 1.f, 1.f);
-        // unscaled residual entry r^ sqrt(d): r^2 d = r^2 / (1/d); slots that are not free
-        // dofs hold r = 0 and 1/d = 0: skipped
-        rt.add(ri.x, di.x != 0.f ? ri.x / di.x : 0.f);
-        rt.add(ri.y, di.y != 0.f ? ri.y / di.y : 0.f);
-        rt.add(ri.z, di.z != 0.f ? ri.z / di.z : 0.f);
-        rt.add(ri.w, di.w != 0.f ? ri.w / di.w : 0.f);
-      }
-    }
-  }
-  for (int64_t i = (n4 << 2) + t0; i < n; i += stride) {
-    x[i] = fmaf(a, p[i], x[i]);
-    const float ri = fmaf(-a, q[i], r[i]);
-    r[i] = ri;
-    if (!keep_p) p[i] = fmaf(b, p[i], ri);
-    rr.add(ri, ri);
-    if (EXACT) {
-      const float di = idiag ? idiag[i] : 1.f;
-      rt.add(ri, di != 0.f ? ri / di : 0.f);
-    }
-  }
-  double v[2] = {rr.value(), rt.value()}, tot[2];
-  if (block_reduce_last<2>(v, rb, tot) && threadIdx.x == 0) {
-    const int it = I[I_ITER] + 1;
-    I[I_ITER] = it;
-    if (keep_p) {
-      // the segment ends: |r|^2 of the new residual for the record; the old one stays in
-      // S_RRH for the direction the host keeps
-      S[S_APP] = tot[0];
-      I[I_FLAG] = I[I_PEND] != FLAG_NONE ? I[I_PEND] : FLAG_UPDATE;
-      I[I_DONE] = 1;
-      return;
-    }
-    S[S_RRH] = tot[0];
-    const double rn = sqrt(tot[0]);
-    int pend = FLAG_NONE;
-    if (!(rn <= 1e4 * S[S_RMAX])) pend = FLAG_BREAK;  // NaN fails too
-    else if (EXACT && sqrt(tot[1]) * S[S_SIGMA] <= S[S_TOL]) pend = FLAG_CHECK;
-    else if (rn < S[S_DELTA] * S[S_RMAX]) pend = FLAG_UPDATE;
-    else if (it + 1 >= I[I_MAXIT]) pend = FLAG_MAXIT;
-    if (rn > S[S_RMAX]) S[S_RMAX] = rn;
-    S[S_RNSCALED] = rn;
-    I[I_PEND] = pend;
-  }
-}
+// iteration (k_pcg32).  Around a segment: fold the correction, refresh the residual.
 
 // x64 += sigma * s x^32; x^32 = 0 (s = D^-1/2 per slot; null: 1)
 __global__ void k_fold_scaled(int64_t n, double sigma, const double* __restrict__ sd, float* __restrict__ x32,
@@ -381,23 +266,16 @@ __global__ void __launch_bounds__(RB)
 
 // ---------------------------------------------------------------------------
 // SELL SpMV, warp per slice, lane per row, slices strided over a fixed grid.
-// MODE 0: y = A x.  MODE 1: y = A x, <y,x> reduced, alpha = r_z/<Ap,p>.
-// MODE 2: y = b - A x (b FP64), <y,y> reduced into S_ERR as a norm.
+// MODE 0: y = A x.  MODE 2: y = b - A x (b FP64), <y,y> reduced into S_ERR as a norm.
 template <typename T, int MODE>
 __global__ void __launch_bounds__(RB)
     k_sell_spmv(int64_t nslices, int64_t n, const int64_t* __restrict__ sptr, const int32_t* __restrict__ scol,
                 const T* __restrict__ sval, const T* __restrict__ x, T* __restrict__ y, const double* __restrict__ b,
                 RedBuf rb, double* S, const int* I) {
-  if ((MODE == 1 || MODE == 3) && I[I_DONE]) return;
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * RB + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * RB) >> 5;
   Acc<T> dot;
-#if FG_MIXED_QQ_COMPENSATED
-  Acc<T> dot2;
-#else
-  AccPlain dot2;
-#endif
   for (int64_t s = warp; s < nslices; s += nwarps) {
     const int64_t base = sptr[s];
     const int w4 = (int)((sptr[s + 1] - base) >> 7);  // groups of 4 entries per lane
@@ -425,26 +303,12 @@ __global__ void __launch_bounds__(RB)
         dot.add(rr, rr);
       } else {
         y[slot] = acc;
-        if (MODE == 1 || MODE == 3) dot.add(acc, x[slot]);
-        if (MODE == 3) dot2.add(acc, acc);
       }
     }
   }
   if (MODE == 0) return;
-  if (MODE == 3) {
-    double v2[2] = {dot.value(), dot2.value()}, tot2[2];
-    if (block_reduce_last<2>(v2, rb, tot2) && threadIdx.x == 0) mixed_alpha_beta(tot2[0], tot2[1], S, const_cast<int*>(I));
-    return;
-  }
   double v[1] = {dot.value()}, tot[1];
-  if (block_reduce_last<1>(v, rb, tot) && threadIdx.x == 0) {
-    if (MODE == 1) {
-      S[S_APP] = tot[0];
-      S[S_ALPHA] = tot[0] != 0.0 ? S[S_RZ] / tot[0] : 0.0;
-    } else {
-      S[S_ERR] = sqrt(tot[0]);
-    }
-  }
+  if (block_reduce_last<1>(v, rb, tot) && threadIdx.x == 0) S[S_ERR] = sqrt(tot[0]);
 }
 
 // FP64 path start: r = b - r (r holds A x0) or r = b; z = M r; p = z; <r,r>, <r,z>, <b,b>, <b,Mb>.
@@ -489,86 +353,24 @@ __global__ void __launch_bounds__(RB)
   }
 }
 
-// FP64 path: x += alpha p; r -= alpha Ap; the reference's convergence test; beta, r_z.
-template <bool PRECOND, bool NEED_PP>
+// p = r + beta p, four entries per thread and load (the vectors are 16-byte aligned)
 __global__ void __launch_bounds__(RB)
-    k_update64(int64_t n, double* __restrict__ x, double* __restrict__ r, const double* __restrict__ p,
-               const double* __restrict__ Ap, const double* __restrict__ idiag, int criterion, double rtol,
-               double atol, RedBuf rb, double* S, int* I) {
-  if (I[I_DONE]) return;
-  const double a = S[S_ALPHA];
-  Acc<double> rr, rz, pp;
-  for (int64_t i = blockIdx.x * (int64_t)RB + threadIdx.x; i < n; i += (int64_t)gridDim.x * RB) {
-    const double pi = p[i];
-    x[i] = fma(a, pi, x[i]);
-    const double ri = fma(-a, Ap[i], r[i]);
-    r[i] = ri;
-    rr.add(ri, ri);
-    if (PRECOND) rz.add(ri, idiag[i] * ri);
-    if (NEED_PP) pp.add(pi, pi);
-  }
-  double v[3] = {rr.value(), PRECOND ? rz.value() : rr.value(), pp.value()}, tot[3];
-  if (block_reduce_last<3>(v, rb, tot) && threadIdx.x == 0) {
-    const int it = I[I_ITER] + 1;
-    I[I_ITER] = it;
-    double err = S[S_ERR];
-    if (it == 1 && (criterion == FG_DELTA_RHS || criterion == FG_DELTA_DELTA)) {
-      err = a * sqrt(tot[2]);
-      if (criterion == FG_DELTA_DELTA) S[S_TOL] = rtol * err + atol;
-    }
-    switch (criterion) {
-      case FG_RES_RES: case FG_RES_RHS: err = sqrt(tot[0]); break;
-      case FG_DELTA_RHS: case FG_DELTA_DELTA: if (it != 1) err = a * sqrt(tot[2]); break;
-      default: err = S[S_RNRMM]; break;
-    }
-    S[S_ERR] = err;
-    const bool conv = err <= S[S_TOL];
-    if (conv || it >= I[I_MAXIT]) {
-      I[I_DONE] = 1;
-      I[I_CONV] = conv ? 1 : 0;
-    } else {
-      double beta = 1.0 / S[S_RZ];
-      S[S_RZ] = tot[1];
-      beta = beta * tot[1];
-      S[S_BETA] = beta;
-      S[S_RNRMM] = sqrt(tot[1]);
-    }
-  }
-}
-
-// p = z + beta p (FP32: four entries per thread and load; the vectors are 16-byte aligned)
-template <typename T, bool PRECOND>
-__global__ void __launch_bounds__(RB)
-    k_pupdate(int64_t n, T* __restrict__ p, const T* __restrict__ r, const T* __restrict__ idiag, const double* S,
-              const int* I) {
-  if (I[I_DONE]) return;
-  const T beta = (T)S[S_BETA];
+    k_pupdate(int64_t n, float* __restrict__ p, const float* __restrict__ r, const double* S) {
+  const float b = (float)S[S_BETA];
   const int64_t t0 = blockIdx.x * (int64_t)RB + threadIdx.x, stride = (int64_t)gridDim.x * RB;
-  int64_t head = 0;
-  if (sizeof(T) == 4) {
-    const int64_t n4 = n >> 2;
-    head = n4 << 2;
-    float4* p4 = reinterpret_cast<float4*>(p);
-    const float4* r4 = reinterpret_cast<const float4*>(r);
-    const float4* d4 = reinterpret_cast<const float4*>(idiag);
-    const float b = (float)beta;
-    for (int64_t i = t0; i < n4; i += stride) {
-      const float4 ri = r4[i];
-      float4 pi = p4[i];
-      float4 di = make_float4(1.f, 1.f, 1.f, 1.f);
-      if (PRECOND) di = d4[i];
-      pi.x = fmaf(b, pi.x, PRECOND ? di.x * ri.x : ri.x);
-      pi.y = fmaf(b, pi.y, PRECOND ? di.y * ri.y : ri.y);
-      pi.z = fmaf(b, pi.z, PRECOND ? di.z * ri.z : ri.z);
-      pi.w = fmaf(b, pi.w, PRECOND ? di.w * ri.w : ri.w);
-      p4[i] = pi;
-    }
+  const int64_t n4 = n >> 2;
+  float4* p4 = reinterpret_cast<float4*>(p);
+  const float4* r4 = reinterpret_cast<const float4*>(r);
+  for (int64_t i = t0; i < n4; i += stride) {
+    const float4 ri = r4[i];
+    float4 pi = p4[i];
+    pi.x = fmaf(b, pi.x, ri.x);
+    pi.y = fmaf(b, pi.y, ri.y);
+    pi.z = fmaf(b, pi.z, ri.z);
+    pi.w = fmaf(b, pi.w, ri.w);
+    p4[i] = pi;
   }
-  for (int64_t i = head + t0; i < n; i += stride) {
-    const T ri = r[i];
-    const T zi = PRECOND ? idiag[i] * ri : ri;
-    p[i] = fmaT(beta, p[i], zi);
-  }
+  for (int64_t i = (n4 << 2) + t0; i < n; i += stride) p[i] = fmaf(b, p[i], r[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -592,16 +394,10 @@ __global__ void __launch_bounds__(RB)
                    const int32_t* __restrict__ st_row, const T* __restrict__ tval,
                    int ncomp, const T* __restrict__ x, T* __restrict__ y, const double* __restrict__ b, RedBuf rb,
                    double* S, const int* I) {
-  if ((MODE == 1 || MODE == 3) && I[I_DONE]) return;
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * RB + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * RB) >> 5;
   Acc<T> dot;
-#if FG_MIXED_QQ_COMPENSATED
-  Acc<T> dot2;
-#else
-  AccPlain dot2;
-#endif
   for (int64_t s = warp; s < nslices; s += nwarps) {
     const int k = scls[s];
     const int64_t vb = voff[s];
@@ -642,24 +438,697 @@ __global__ void __launch_bounds__(RB)
         dot.add(rr, rr);
       } else {
         y[vec] = acc;
-        if (MODE == 1 || MODE == 3) dot.add(acc, x[vec]);
-        if (MODE == 3) dot2.add(acc, acc);
       }
     }
   }
   if (MODE == 0) return;
-  if (MODE == 3) {
-    double v2[2] = {dot.value(), dot2.value()}, tot2[2];
-    if (block_reduce_last<2>(v2, rb, tot2) && threadIdx.x == 0) mixed_alpha_beta(tot2[0], tot2[1], S, const_cast<int*>(I));
-    return;
-  }
   double v[1] = {dot.value()}, tot[1];
-  if (block_reduce_last<1>(v, rb, tot) && threadIdx.x == 0) {
-    if (MODE == 1) {
-      S[S_APP] = tot[0];
-      S[S_ALPHA] = tot[0] != 0.0 ? S[S_RZ] / tot[0] : 0.0;
+  if (block_reduce_last<1>(v, rb, tot) && threadIdx.x == 0) S[S_ERR] = sqrt(tot[0]);
+}
+
+// ---------------------------------------------------------------------------
+// The CG loop as one cooperative launch.  A launch runs up to max_launch iterations; its
+// blocks are co-resident and meet at grid barriers (one per inner product, and one before
+// the next SpMV gathers the new p; ~1.4 us each), so an iteration costs two or three barriers
+// instead of two or three kernels.  As separate kernels (a CUDA graph of them) each reduction
+// cost 12-18 us whatever the size: 912-1216 blocks took a ticket on one counter, each warp
+// butterflied its sums on the FP64 pipe (16 cycles per warp instruction), and the last block
+// started from cold.  Solve, before -> after: 8^3 Q1 FP64 1.48 -> 0.28 ms, 32^3 Q1 FP64 3.54 ->
+// 1.42 ms, 24^3 Q2 mixed 10.9 -> 4.9 ms, 23 x 17 x 21 Q3 FP64 65.8 -> 48.1 ms, 384^2 Q2 FP64
+// 253 -> 227 ms, 96^3 Q2 mixed 374 -> 364 ms.  Bound by barriers and FP64 latency where the
+// matrix is small, by the SpMV (FP64 pipe; HBM in FP32) where it is large.
+//
+// Rows: warp w of block b owns the slices w nb + b + k (warps nb), k = 0.. (an SM then holds
+// slices of every width).  R > 0: a lane keeps its R rows' x, r, p and 1/d in registers
+// (small and medium systems: at most R slices per warp); only p goes through memory.  R = 0:
+// any size, vectors streamed.
+
+struct GridSync {
+  double* part;     // [2 buffers][3 values][blocks] partial sums
+  unsigned* count;  // arrivals of this launch (zero at launch)
+  int* abort;       // set by a wait that ran out
+  unsigned long long limit_ns;  // a wait gives up after this long
+  int drop;         // test switch (FG_PCG_TEST_DROP_ARRIVAL): block 0 skips its first arrival
+};
+
+template <typename T>
+struct MatArgs {
+  int64_t nslices, n;  // slices; rows (SELL: the vector length)
+  const T* val;
+  // lattice-implicit
+  const uint8_t* scls;
+  const int64_t* voff;
+  const StencilClass* cls;
+  const int32_t* soff;
+  const int32_t* st_row;
+  int ncomp;
+  int noff;            // entries of soff
+  // explicit columns
+  const int64_t* sptr;
+  const int32_t* scol;
+};
+
+// One arrival of the calling block (its other threads have met at a block barrier) and the
+// bounded wait for all blocks; called by one thread.  False: the wait ran out or another
+// block's did.
+__device__ __forceinline__ bool grid_wait(const GridSync& g, unsigned target) {
+  __threadfence();
+  if (!(g.drop && blockIdx.x == 0 && target == gridDim.x)) atomicAdd(g.count, 1u);
+  unsigned spins = 0;
+  unsigned long long t0 = 0;
+  for (;;) {
+    unsigned c;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(g.count) : "memory");
+    if (c >= target) break;
+    if ((++spins & 255u) == 0) {
+      unsigned long long t;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+      if (t0 == 0) t0 = t;
+      if (*(volatile int*)g.abort || t - t0 > g.limit_ns) {
+        *(volatile int*)g.abort = 1;
+        __threadfence();
+        return false;
+      }
+    }
+  }
+  __threadfence();  // what the other blocks wrote before arriving is visible to this block
+  return true;
+}
+
+// sum of the lanes' float-float values
+__device__ __forceinline__ void ff_acc(float& h, float& l, float h2, float l2) {
+  const float s = __fadd_rn(h, h2);
+  const float bb = __fsub_rn(s, h);
+  const float e = __fadd_rn(__fsub_rn(h, __fsub_rn(s, bb)), __fsub_rn(h2, bb));
+  l = __fadd_rn(l, __fadd_rn(l2, e));
+  h = s;
+}
+
+// Block and grid sums of NV accumulators, then f(totals) on lane 0 of warp 0 (the step's
+// scalars, in shared memory); every thread returns after f.  Threads leave their sums in
+// shared memory and warp 0 alone adds them (NT/32 + 5 additions per value instead of 5 in
+// every warp: the FP64 pipe takes 16 cycles per warp instruction).  FP32 accumulators are
+// added as float-float pairs and become FP64 once per block.  Sums in fixed order:
+// deterministic.  False: the grid barrier gave up.
+template <typename T>
+struct RedShared;
+template <>
+struct RedShared<double> {
+  double v[3][1024];
+};
+template <>
+struct RedShared<float> {
+  float2 v[2][1024];
+};
+
+template <int NV, typename F>
+__device__ __forceinline__ bool grid_reduce(RedShared<double>& sh, const double (&v)[NV], const GridSync& g, int buf,
+                                            unsigned& target, int* s_ok, F&& f) {
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) sh.v[k][t] = v[k];
+  __syncthreads();
+  target += gridDim.x;
+  if (t < 32) {
+    double s[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      s[k] = 0.0;
+      for (int i = t; i < (int)blockDim.x; i += 32) s[k] += sh.v[k][i];
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) s[k] += __shfl_down_sync(0xffffffffu, s[k], off);
+    }
+    bool ok = true;
+    if (gridDim.x > 1) {
+      const int nb = gridDim.x;
+      double* part = g.part + (size_t)buf * 3 * nb;
+      if (t == 0) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) part[k * nb + blockIdx.x] = s[k];
+        ok = grid_wait(g, target);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        s[k] = 0.0;
+        for (int i = t; i < nb; i += 32) s[k] += __ldcg(part + k * nb + i);
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) s[k] += __shfl_down_sync(0xffffffffu, s[k], off);
+      }
+    }
+    if (t == 0) {
+      *s_ok = ok ? 1 : 0;
+      if (ok) f(s);
+    }
+  }
+  __syncthreads();
+  return *s_ok != 0;
+}
+
+template <int NV, typename F>
+__device__ __forceinline__ bool grid_reduce(RedShared<float>& sh, const float2 (&v)[NV], const GridSync& g, int buf,
+                                            unsigned& target, int* s_ok, F&& f) {
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) sh.v[k][t] = v[k];
+  __syncthreads();
+  target += gridDim.x;
+  if (t < 32) {
+    double s[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      float h = 0.f, l = 0.f;
+      for (int i = t; i < (int)blockDim.x; i += 32) {
+        const float2 w = sh.v[k][i];
+        ff_acc(h, l, w.x, w.y);
+      }
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+        const float h2 = __shfl_down_sync(0xffffffffu, h, off), l2 = __shfl_down_sync(0xffffffffu, l, off);
+        ff_acc(h, l, h2, l2);
+      }
+      s[k] = (double)h + (double)l;
+    }
+    bool ok = true;
+    if (gridDim.x > 1) {
+      const int nb = gridDim.x;
+      double* part = g.part + (size_t)buf * 3 * nb;
+      if (t == 0) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) part[k * nb + blockIdx.x] = s[k];
+        ok = grid_wait(g, target);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        s[k] = 0.0;
+        for (int i = t; i < nb; i += 32) s[k] += __ldcg(part + k * nb + i);
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) s[k] += __shfl_down_sync(0xffffffffu, s[k], off);
+      }
+    }
+    if (t == 0) {
+      *s_ok = ok ? 1 : 0;
+      if (ok) f(s);
+    }
+  }
+  __syncthreads();
+  return *s_ok != 0;
+}
+
+// barrier without a sum
+__device__ __forceinline__ bool grid_barrier(const GridSync& g, unsigned& target, int* s_ok) {
+  __syncthreads();
+  target += gridDim.x;
+  if (gridDim.x == 1) return true;
+  if (threadIdx.x == 0) *s_ok = grid_wait(g, target) ? 1 : 0;
+  __syncthreads();
+  return *s_ok != 0;
+}
+
+// matrix values of one group: cached (R > 0: the matrix of such a system mostly stays in L2
+// from one iteration to the next) or streamed
+template <bool KEEP>
+__device__ __forceinline__ void ld4k(const float* p, float (&v)[4]) {
+  if (!KEEP) { ld4(p, v); return; }
+  const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+  v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+}
+template <bool KEEP>
+__device__ __forceinline__ void ld4k(const double* p, double (&v)[4]) {
+  if (!KEEP) { ld4(p, v); return; }
+  asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+}
+
+// One slice of the matrix as one lane sees it.
+template <typename T, bool STENCIL>
+struct SliceRef {
+  const T* vp;         // the lane's first value
+  const int32_t* cp;   // lattice-implicit: offsets of the class; explicit: the lane's first column
+  int w4;              // groups of 4 entries
+  int32_t base, vec;   // gather base; the row's vector index (-1: no row)
+  __device__ __forceinline__ void load(const MatArgs<T>& m, int64_t s, int lane, const int32_t* s_off) {
+    if (STENCIL) {
+      const int k = m.scls[s];
+      const StencilClass& C = m.cls[k];
+      int32_t st = m.st_row[s * 32 + lane];
+      const bool valid = st >= 0;
+      if (!valid) st = ~st;
+      base = m.ncomp == 1 ? st : st - st % m.ncomp;
+      vec = valid ? (int32_t)(st + C.ownoff) : -1;
+      w4 = C.Bp >> 2;
+      vp = m.val + m.voff[s] + 4 * lane;
+      cp = s_off + C.offbase;
     } else {
-      S[S_ERR] = sqrt(tot[0]);
+      const int64_t b = m.sptr[s];
+      w4 = (int)((m.sptr[s + 1] - b) >> 7);
+      vp = m.val + b + 4 * lane;
+      cp = m.scol + b + 4 * lane;
+      const int64_t slot = s * 32 + lane;
+      base = 0;
+      vec = slot < m.n ? (int32_t)slot : -1;
+    }
+  }
+  // the row's products with x; x changes during the launch, so it is read with plain loads
+  // (coherent after a grid barrier), never through the read-only path
+  template <bool KEEP, int UNROLL>
+  __device__ __forceinline__ T dot(const T* x) const {
+    T acc = 0;
+    const T* v0 = vp;
+    const int32_t* c0 = cp;
+    const T* xb = x + base;
+#pragma unroll UNROLL
+    for (int j = 0; j < w4; ++j) {
+      if (!KEEP && STENCIL && sizeof(T) == 4 && j + kPrefetch < w4)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(v0 + kPrefetch * 128));
+      T v[4];
+      ld4k<KEEP>(v0, v);
+      int4 o;
+      if (STENCIL) o = reinterpret_cast<const int4*>(c0)[j];
+      else if (KEEP) o = __ldg(reinterpret_cast<const int4*>(c0));
+      else o = __ldcs(reinterpret_cast<const int4*>(c0));
+      const T x0 = xb[o.x], x1 = xb[o.y], x2 = xb[o.z], x3 = xb[o.w];
+      acc = fmaT(v[0], x0, acc);
+      acc = fmaT(v[1], x1, acc);
+      acc = fmaT(v[2], x2, acc);
+      acc = fmaT(v[3], x3, acc);
+      v0 += 128;
+      if (!STENCIL) c0 += 128;
+    }
+    return acc;
+  }
+};
+
+// the class offsets in shared memory (lattice-implicit layout)
+template <typename T, bool STENCIL>
+__device__ __forceinline__ const int32_t* stage_offsets(const MatArgs<T>& m, int32_t* s_off) {
+  if (!STENCIL) return nullptr;
+  for (int i = threadIdx.x; i < m.noff; i += blockDim.x) s_off[i] = m.soff[i];
+  __syncthreads();
+  return s_off;
+}
+
+static constexpr int pcg_threads(int R) { return R > 0 ? 1024 : 768; }
+static constexpr int pcg_blocks(int R) { return R > 0 ? 1 : 2; }
+
+// FP64 CG, the sequence and stopping tests of the reference (cg.f90:101-238, 279-407).
+// idiag null: no preconditioner.  chunk: the polling interval the caller asked for (a
+// non-finite iteration is reported at its end, if the iteration limit lies beyond it).
+template <bool STENCIL, int R>
+__global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
+    k_pcg64(MatArgs<double> m, int64_t nvec, double* x, double* r, double* p, double* Ap,
+            const double* __restrict__ idiag, int criterion, double rtol, double atol, int max_launch, int chunk,
+            GridSync g, double* S, int* I) {
+  extern __shared__ __align__(16) int32_t s_off_buf[];
+  __shared__ RedShared<double> sh;
+  __shared__ double sc[8];  // alpha, beta, rz, err, tol, rnrmm
+  __shared__ int si[4];     // stop (1 done, 2 non-finite), converged, ok
+  if (I[I_DONE]) return;
+  constexpr int RR = R > 0 ? R : 1;
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  const int64_t nwarps = (int64_t)(blockDim.x >> 5) * gridDim.x;
+  const bool need_pp = criterion == FG_DELTA_RHS || criterion == FG_DELTA_DELTA;
+  const int32_t* s_off = stage_offsets<double, STENCIL>(m, s_off_buf);
+  const int it0 = I[I_ITER], maxit = I[I_MAXIT];
+  if (threadIdx.x == 0) {
+    sc[2] = S[S_RZ];
+    sc[3] = S[S_ERR];
+    sc[4] = S[S_TOL];
+    sc[5] = S[S_RNRMM];
+    si[0] = si[1] = 0;
+  }
+  SliceRef<double, STENCIL> ref[RR];
+  double rx[RR], rr_[RR], rp[RR], rd[RR], ra[RR];
+  if (R > 0) {
+#pragma unroll
+    for (int k = 0; k < RR; ++k) {
+      const int64_t s = warp + k * nwarps;
+      rx[k] = rr_[k] = rp[k] = rd[k] = 0.0;
+      ref[k].vec = -1;
+      ref[k].w4 = 0;
+      if (s < m.nslices) {
+        ref[k].load(m, s, lane, s_off);
+        const int32_t v = ref[k].vec;
+        if (v >= 0) {
+          rx[k] = x[v];
+          rr_[k] = r[v];
+          rp[k] = p[v];
+          rd[k] = idiag ? idiag[v] : 1.0;
+        }
+      }
+    }
+  }
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  unsigned target = 0;
+  int it = it0;
+  for (int n = 0; n < max_launch; ++n) {
+    // Ap = A p, <Ap,p>
+    Acc<double> dot;
+    if (R > 0) {
+#pragma unroll
+      for (int k = 0; k < RR; ++k) {
+        ra[k] = ref[k].template dot<true, 2>(p);
+        if (ref[k].vec >= 0) dot.add(ra[k], rp[k]);
+      }
+    } else {
+      for (int64_t s = warp; s < m.nslices; s += nwarps) {
+        SliceRef<double, STENCIL> q;
+        q.load(m, s, lane, s_off);
+        const double a = q.template dot<false, kUnroll>(p);
+        if (q.vec >= 0) {
+          Ap[q.vec] = a;
+          dot.add(a, p[q.vec]);
+        }
+      }
+    }
+    double v1[1] = {dot.value()};
+    if (!grid_reduce<1>(sh, v1, g, 0, target, &si[2], [&](double (&t)[1]) { sc[0] = t[0] != 0.0 ? sc[2] / t[0] : 0.0; }))
+      return;
+    // x += alpha p; r -= alpha Ap; the convergence test; beta
+    const double a = sc[0];
+    Acc<double> rr, rz, pp;
+    if (R > 0) {
+#pragma unroll
+      for (int k = 0; k < RR; ++k) {
+        rx[k] = fma(a, rp[k], rx[k]);
+        if (ref[k].vec >= 0) rr_[k] = fma(-a, ra[k], rr_[k]);
+        rr.add(rr_[k], rr_[k]);
+        if (idiag) rz.add(rr_[k], rd[k] * rr_[k]);
+        if (need_pp) pp.add(rp[k], rp[k]);
+      }
+    } else {
+      for (int64_t i = t0; i < nvec; i += stride) {
+        const double pi = p[i];
+        x[i] = fma(a, pi, x[i]);
+        const double ri = fma(-a, Ap[i], r[i]);
+        r[i] = ri;
+        rr.add(ri, ri);
+        if (idiag) rz.add(ri, idiag[i] * ri);
+        if (need_pp) pp.add(pi, pi);
+      }
+    }
+    ++it;
+    auto test = [&](double trr, double trz, double tpp) {
+      double err = sc[3];
+      if (it == 1 && need_pp) {
+        err = a * sqrt(tpp);
+        if (criterion == FG_DELTA_DELTA) sc[4] = rtol * err + atol;
+      }
+      switch (criterion) {
+        case FG_RES_RES: case FG_RES_RHS: err = sqrt(trr); break;
+        case FG_DELTA_RHS: case FG_DELTA_DELTA: if (it != 1) err = a * sqrt(tpp); break;
+        default: err = sc[5]; break;
+      }
+      sc[3] = err;
+      const bool conv = err <= sc[4];
+      if (conv || it >= maxit) {
+        si[0] = 1;
+        si[1] = conv ? 1 : 0;
+        return;
+      }
+      double beta = 1.0 / sc[2];
+      sc[2] = trz;
+      beta = beta * trz;
+      sc[1] = beta;
+      sc[5] = sqrt(trz);
+      if (!(isfinite(a) && isfinite(trz)) && (it + chunk - 1) / chunk * chunk < maxit) si[0] = 2;
+    };
+    bool ok;
+    if (need_pp) {
+      double v3[3] = {rr.value(), idiag ? rz.value() : rr.value(), pp.value()};
+      ok = grid_reduce<3>(sh, v3, g, 1, target, &si[2], [&](double (&t)[3]) { test(t[0], t[1], t[2]); });
+    } else if (idiag) {
+      double v2[2] = {rr.value(), rz.value()};
+      ok = grid_reduce<2>(sh, v2, g, 1, target, &si[2], [&](double (&t)[2]) { test(t[0], t[1], 0.0); });
+    } else {
+      double v2[1] = {rr.value()};
+      ok = grid_reduce<1>(sh, v2, g, 1, target, &si[2], [&](double (&t)[1]) { test(t[0], t[0], 0.0); });
+    }
+    if (!ok) return;
+    if (si[0]) break;
+    // p = z + beta p
+    const double beta = sc[1];
+    if (R > 0) {
+#pragma unroll
+      for (int k = 0; k < RR; ++k) {
+        rp[k] = fma(beta, rp[k], rd[k] * rr_[k]);
+        if (ref[k].vec >= 0) p[ref[k].vec] = rp[k];
+      }
+    } else {
+      for (int64_t i = t0; i < nvec; i += stride) {
+        const double ri = r[i];
+        p[i] = fma(beta, p[i], idiag ? idiag[i] * ri : ri);
+      }
+    }
+    if (n + 1 < max_launch && !grid_barrier(g, target, &si[2])) return;
+  }
+  if (R > 0) {
+#pragma unroll
+    for (int k = 0; k < RR; ++k)
+      if (ref[k].vec >= 0) {
+        x[ref[k].vec] = rx[k];
+        r[ref[k].vec] = rr_[k];
+      }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    S[S_ALPHA] = sc[0];
+    S[S_BETA] = sc[1];
+    S[S_RZ] = sc[2];
+    S[S_ERR] = sc[3];
+    S[S_TOL] = sc[4];
+    S[S_RNRMM] = sc[5];
+    I[I_ITER] = it;
+    I[I_DONE] = si[0] == 1;
+    I[I_CONV] = si[1];
+  }
+}
+
+// FP32 segment of the mixed path on A^ = S A S (or A): two grid barriers per iteration.
+//   q = A^ p, <p,q>, <q,q>; then alpha = |r|^2/<p,q> and, by the recurrence
+//   |r - alpha q|^2 = alpha^2 |q|^2 - |r|^2 (as <r,q> = <p,q> in CG), beta = |r_new|^2/|r|^2;
+//   x += alpha p; r -= alpha q; p = r + beta p; the exact |r_new|^2 for the next alpha, and on
+//   every FG_MIXED_EXACT_EVERY-th iteration sum r^2 D (the unscaled residual, for the stop
+//   estimate).
+// A segment end (reliable update, stop check, breakdown, iteration limit) found by an update
+// is taken one iteration later: that iteration's update keeps p, so the host can fold x and
+// restart the recursion from the true residual with the direction kept.
+template <bool STENCIL, int R>
+__global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
+    k_pcg32(MatArgs<float> m, int64_t nvec, float* x, float* r, float* p, float* q, const float* __restrict__ idiag,
+            int max_launch, GridSync g, double* S, int* I) {
+  extern __shared__ __align__(16) int32_t s_off_buf[];
+  __shared__ RedShared<float> sh;
+  __shared__ double sd[8];  // rr, rmax, delta, sigma, tol, app
+  __shared__ float sf[2];   // alpha, beta
+  __shared__ int si[8];     // pend, skip, done flag, ok
+  if (I[I_DONE]) return;
+  constexpr int RR = R > 0 ? R : 1;
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  const int64_t nwarps = (int64_t)(blockDim.x >> 5) * gridDim.x;
+  const int32_t* s_off = stage_offsets<float, STENCIL>(m, s_off_buf);
+  const int maxit = I[I_MAXIT];
+  int it = I[I_ITER];
+  if (threadIdx.x == 0) {
+    sd[0] = S[S_RRH];
+    sd[1] = S[S_RMAX];
+    sd[2] = S[S_DELTA];
+    sd[3] = S[S_SIGMA];
+    sd[4] = S[S_TOL];
+    sd[5] = S[S_APP];
+    si[0] = I[I_PEND];
+    si[1] = I[I_SKIPP];
+    si[2] = FLAG_NONE;
+  }
+  SliceRef<float, STENCIL> ref[RR];
+  float rx[RR], rr_[RR], rp[RR], rq[RR];
+  if (R > 0) {
+#pragma unroll
+    for (int k = 0; k < RR; ++k) {
+      const int64_t s = warp + k * nwarps;
+      rx[k] = rr_[k] = rp[k] = 0.f;
+      ref[k].vec = -1;
+      ref[k].w4 = 0;
+      if (s < m.nslices) {
+        ref[k].load(m, s, lane, s_off);
+        const int32_t v = ref[k].vec;
+        if (v >= 0) {
+          rx[k] = x[v];
+          rr_[k] = r[v];
+          rp[k] = p[v];
+        }
+      }
+    }
+  }
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  unsigned target = 0;
+  for (int n = 0; n < max_launch; ++n) {
+    Acc<float> pq;
+    AccPlain qq;
+    if (R > 0) {
+#pragma unroll
+      for (int k = 0; k < RR; ++k) {
+        rq[k] = ref[k].template dot<true, R == 1 ? 4 : 2>(p);
+        if (ref[k].vec >= 0) {
+          pq.add(rq[k], rp[k]);
+          qq.add(rq[k], rq[k]);
+        }
+      }
+    } else {
+      for (int64_t s = warp; s < m.nslices; s += nwarps) {
+        SliceRef<float, STENCIL> w;
+        w.load(m, s, lane, s_off);
+        const float a = w.template dot<false, kUnroll>(p);
+        if (w.vec >= 0) {
+          q[w.vec] = a;
+          pq.add(a, p[w.vec]);
+          qq.add(a, a);
+        }
+      }
+    }
+    const float2 v2[2] = {make_float2(pq.hi, pq.lo), make_float2(qq.s, 0.f)};
+    if (!grid_reduce<2>(sh, v2, g, 0, target, &si[3], [&](double (&t)[2]) {
+          const double pap = t[0], nq = t[1], rr = sd[0];
+          int skip = si[0] != FLAG_NONE;
+          double a = 0.0, b = 0.0;
+          if (!(pap > 0.0 && pap <= 1e300) || !(nq <= 1e300)) {
+            si[0] = FLAG_BREAK;  // alpha = 0: the update leaves x and r as they are
+            skip = 1;
+          } else {
+            a = rr / pap;
+            const double rrn = a * a * nq - rr;
+            b = rrn / rr;
+            if (!(rrn > 0.0)) {  // the recurrence lost its digits: end the segment here
+              skip = 1;
+              if (si[0] == FLAG_NONE) si[0] = FLAG_UPDATE;
+            }
+          }
+          sf[0] = (float)a;
+          sf[1] = (float)b;
+          sd[6] = a;
+          sd[7] = b;
+          si[1] = skip;
+        }))
+      return;
+    const float a = sf[0], b = sf[1];
+    const bool keep_p = si[1] != 0;
+    const bool exact = n % FG_MIXED_EXACT_EVERY == FG_MIXED_EXACT_EVERY - 1 || n == max_launch - 1;
+    Acc<float> rr, rt;
+    // unscaled residual entry r^ sqrt(d): r^2 d = r^2 / (1/d); slots that are not free dofs hold
+    // r = 0 and 1/d = 0: skipped
+    auto unscaled = [&](float ri, float di) { rt.add(ri, di != 0.f ? ri / di : 0.f); };
+    if (R > 0) {
+#pragma unroll
+      for (int k = 0; k < RR; ++k) {
+        if (ref[k].vec < 0) continue;
+        rx[k] = fmaf(a, rp[k], rx[k]);
+        rr_[k] = fmaf(-a, rq[k], rr_[k]);
+        if (!keep_p) {
+          rp[k] = fmaf(b, rp[k], rr_[k]);
+          p[ref[k].vec] = rp[k];
+        }
+        rr.add(rr_[k], rr_[k]);
+        if (exact) unscaled(rr_[k], idiag ? idiag[ref[k].vec] : 1.f);
+      }
+    } else {
+      const int64_t n4 = nvec >> 2;
+      float4* x4 = reinterpret_cast<float4*>(x);
+      float4* r4 = reinterpret_cast<float4*>(r);
+      float4* p4 = reinterpret_cast<float4*>(p);
+      const float4* q4 = reinterpret_cast<const float4*>(q);
+      const float4* d4 = reinterpret_cast<const float4*>(idiag);
+      for (int64_t i = t0; i < n4; i += stride) {
+        float4 xi = x4[i], ri = r4[i], pi = p4[i];
+        const float4 qi = q4[i];
+        xi.x = fmaf(a, pi.x, xi.x);
+        xi.y = fmaf(a, pi.y, xi.y);
+        xi.z = fmaf(a, pi.z, xi.z);
+        xi.w = fmaf(a, pi.w, xi.w);
+        ri.x = fmaf(-a, qi.x, ri.x);
+        ri.y = fmaf(-a, qi.y, ri.y);
+        ri.z = fmaf(-a, qi.z, ri.z);
+        ri.w = fmaf(-a, qi.w, ri.w);
+        x4[i] = xi;
+        r4[i] = ri;
+        if (!keep_p) {
+          pi.x = fmaf(b, pi.x, ri.x);
+          pi.y = fmaf(b, pi.y, ri.y);
+          pi.z = fmaf(b, pi.z, ri.z);
+          pi.w = fmaf(b, pi.w, ri.w);
+          p4[i] = pi;
+        }
+        rr.add(ri.x, ri.x);
+        rr.add(ri.y, ri.y);
+        rr.add(ri.z, ri.z);
+        rr.add(ri.w, ri.w);
+        if (exact) {
+          const float4 di = idiag ? d4[i] : make_float4(1.f, 1.f, 1.f, 1.f);
+          unscaled(ri.x, di.x);
+          unscaled(ri.y, di.y);
+          unscaled(ri.z, di.z);
+          unscaled(ri.w, di.w);
+        }
+      }
+      for (int64_t i = (n4 << 2) + t0; i < nvec; i += stride) {
+        x[i] = fmaf(a, p[i], x[i]);
+        const float ri = fmaf(-a, q[i], r[i]);
+        r[i] = ri;
+        if (!keep_p) p[i] = fmaf(b, p[i], ri);
+        rr.add(ri, ri);
+        if (exact) unscaled(ri, idiag ? idiag[i] : 1.f);
+      }
+    }
+    ++it;
+    auto decide = [&](double trr, double trt) {
+      if (keep_p) {
+        // the segment ends: |r|^2 of the new residual for the record; the old one stays in
+        // S_RRH for the direction the host keeps
+        sd[5] = trr;
+        si[2] = si[0] != FLAG_NONE ? si[0] : FLAG_UPDATE;
+        return;
+      }
+      sd[0] = trr;
+      const double rn = sqrt(trr);
+      int pend = FLAG_NONE;
+      if (!(rn <= 1e4 * sd[1])) pend = FLAG_BREAK;  // NaN fails too
+      else if (exact && sqrt(trt) * sd[3] <= sd[4]) pend = FLAG_CHECK;
+      else if (rn < sd[2] * sd[1]) pend = FLAG_UPDATE;
+      else if (it + 1 >= maxit) pend = FLAG_MAXIT;
+      if (rn > sd[1]) sd[1] = rn;
+      si[0] = pend;
+    };
+    bool ok;
+    if (exact) {
+      const float2 v[2] = {make_float2(rr.hi, rr.lo), make_float2(rt.hi, rt.lo)};
+      ok = grid_reduce<2>(sh, v, g, 1, target, &si[3], [&](double (&t)[2]) { decide(t[0], t[1]); });
+    } else {
+      const float2 v[1] = {make_float2(rr.hi, rr.lo)};
+      ok = grid_reduce<1>(sh, v, g, 1, target, &si[3], [&](double (&t)[1]) { decide(t[0], 0.0); });
+    }
+    if (!ok) return;
+    if (si[2] != FLAG_NONE) break;
+  }
+  if (R > 0) {
+#pragma unroll
+    for (int k = 0; k < RR; ++k)
+      if (ref[k].vec >= 0) {
+        x[ref[k].vec] = rx[k];
+        r[ref[k].vec] = rr_[k];
+      }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    S[S_ALPHA] = sd[6];
+    S[S_BETA] = sd[7];
+    S[S_RRH] = sd[0];
+    S[S_RMAX] = sd[1];
+    S[S_APP] = sd[5];
+    I[I_ITER] = it;
+    I[I_PEND] = si[0];
+    I[I_SKIPP] = si[1];
+    if (si[2] != FLAG_NONE) {
+      I[I_FLAG] = si[2];
+      I[I_DONE] = 1;
     }
   }
 }
@@ -738,6 +1207,13 @@ template <typename... KA, typename... A>
 static inline void launch_k(void (*k)(KA...), const Work& w, cudaStream_t st, A... args) {
   k<<<grid_for((const void*)k, w.sms), RB, 0, st>>>(args...);
 }
+// the same for `threads` threads of work: no more blocks than they fill (a reducing kernel's
+// blocks each take a ticket, 15 us of them at 1216 blocks)
+template <typename... KA, typename... A>
+static inline void launch_kn(void (*k)(KA...), const Work& w, cudaStream_t st, int64_t threads, A... args) {
+  const unsigned need = (unsigned)std::max<int64_t>(1, (threads + RB - 1) / RB);
+  k<<<std::min(grid_for((const void*)k, w.sms), need), RB, 0, st>>>(args...);
+}
 
 static fg_status ensure_work(fg_system* sys, Work& w) {
   fg_space* sp = sys->space;
@@ -797,34 +1273,18 @@ static void spmv_k(fg_system* sys, const Work& w, const T* x, T* y, const double
   void spmv_k<T, MODE>(fg_system * sys, const Work& w, const T* x, T* y, const double* b, cudaStream_t st) {       \
     fg_space* sp = sys->space;                                                                                      \
     if (sp->layout == FG_LAYOUT_STENCIL)                                                                            \
-      launch_k(k_stencil_spmv<T, MODE>, w, st, sp->st_nslices, (const uint8_t*)sp->d_st_scls,                       \
+      launch_kn(k_stencil_spmv<T, MODE>, w, st, sp->st_nslices * 32, sp->st_nslices, (const uint8_t*)sp->d_st_scls,                       \
                (const int64_t*)sp->d_st_voff, (const StencilClass*)sp->d_st_cls, (const int32_t*)sp->d_st_off, (const int32_t*)sp->d_st_row,       \
                (const T*)sys->TVALS, sp->ncomp, x, y, b, w.rb, w.S, (const int*)w.I);                               \
     else                                                                                                            \
-      launch_k(k_sell_spmv<T, MODE>, w, st, sp->nslices, sp->nfree, (const int64_t*)sp->d_sptr,                     \
+      launch_kn(k_sell_spmv<T, MODE>, w, st, sp->nslices * 32, sp->nslices, sp->nfree, (const int64_t*)sp->d_sptr,                     \
                (const int32_t*)sp->d_scol, (const T*)sys->VALS, x, y, b, w.rb, w.S, (const int*)w.I);              \
     sp->mesh->ctx->launches += 1;                                                                                   \
   }
 FG_SPMV_IMPL(double, 0, d_sval, d_tval)
-FG_SPMV_IMPL(double, 1, d_sval, d_tval)
 FG_SPMV_IMPL(double, 2, d_sval, d_tval)
 FG_SPMV_IMPL(float, 0, d_sval32, d_tval32)
-FG_SPMV_IMPL(float, 1, d_sval32, d_tval32)
 #undef FG_SPMV_IMPL
-
-// FP32 SpMV of the fused mixed iteration on the given values (the scaled copy with Jacobi,
-// the plain FP32 copy without a preconditioner)
-static void spmv_fused32(fg_system* sys, const Work& w, const float* vals, const float* x, float* y, cudaStream_t st) {
-  fg_space* sp = sys->space;
-  if (sp->layout == FG_LAYOUT_STENCIL)
-    launch_k(k_stencil_spmv<float, 3>, w, st, sp->st_nslices, (const uint8_t*)sp->d_st_scls,
-             (const int64_t*)sp->d_st_voff, (const StencilClass*)sp->d_st_cls, (const int32_t*)sp->d_st_off, (const int32_t*)sp->d_st_row, vals,
-             sp->ncomp, x, y, (const double*)nullptr, w.rb, w.S, (const int*)w.I);
-  else
-    launch_k(k_sell_spmv<float, 3>, w, st, sp->nslices, sp->nfree, (const int64_t*)sp->d_sptr,
-             (const int32_t*)sp->d_scol, vals, x, y, (const double*)nullptr, w.rb, w.S, (const int*)w.I);
-  sp->mesh->ctx->launches += 1;
-}
 
 // D^-1/2 and the FP32 copy of D^-1/2 A D^-1/2 (once per numeric assembly)
 static fg_status ensure_scaled(fg_system* sys, const Work& w) {
@@ -905,63 +1365,148 @@ fg_status system_spmv_layout_noalloc(fg_system* sys, int precision, const void* 
   return FG_OK;
 }
 
-// Launch one FP64 CG iteration (3 kernels).
-static void iter64(fg_system* sys, const Work& w, int precond, bool need_pp, int criterion, double rtol, double atol,
-                   cudaStream_t st) {
-  fg_space* sp = sys->space;
-  const int64_t n = sp->nvec;
-  spmv_k<double, 1>(sys, w, w.p, w.Ap, nullptr, st);
-#define FG_UPD(P, Q) \
-  launch_k(k_update64<P, Q>, w, st, n, w.x, w.r, (const double*)w.p, (const double*)w.Ap, (const double*)sys->d_idiag, criterion, rtol, atol, w.rb, w.S, w.I)
-  if (precond) { if (need_pp) FG_UPD(true, true); else FG_UPD(true, false); }
-  else { if (need_pp) FG_UPD(false, true); else FG_UPD(false, false); }
-#undef FG_UPD
-  if (precond) launch_k(k_pupdate<double, true>, w, st, n, w.p, (const double*)w.r, (const double*)sys->d_idiag, (const double*)w.S, (const int*)w.I);
-  else launch_k(k_pupdate<double, false>, w, st, n, w.p, (const double*)w.r, (const double*)sys->d_idiag, (const double*)w.S, (const int*)w.I);
+// matrix arguments of the CG kernels
+template <typename T>
+static MatArgs<T> mat_args(const fg_space* sp, const T* vals) {
+  MatArgs<T> m;
+  const bool stencil = sp->layout == FG_LAYOUT_STENCIL;
+  m.nslices = stencil ? sp->st_nslices : sp->nslices;
+  m.n = sp->nfree;
+  m.val = vals;
+  m.scls = sp->d_st_scls;
+  m.voff = sp->d_st_voff;
+  m.cls = sp->d_st_cls;
+  m.soff = sp->d_st_off;
+  m.st_row = sp->d_st_row;
+  m.ncomp = sp->ncomp;
+  m.noff = 0;
+  if (stencil)
+    for (const StencilClass& C : sp->h_st_cls) m.noff += C.Bp;
+  m.sptr = sp->d_sptr;
+  m.scol = sp->d_scol;
+  return m;
 }
 
-// Launch one fused FP32 iteration of the mixed path (2 kernels); `exact`: this update also
-// sums the unscaled residual norm for the stop estimate.
-static void iter32s(fg_system* sys, const Work& w, const float* vals, const float* idiag32, bool exact, cudaStream_t st) {
-  const int64_t n = sys->space->nvec;
-  spmv_fused32(sys, w, vals, w.p32, w.Ap32, st);
-  if (exact) launch_k(k_update32s<true>, w, st, n, w.x32, w.r32, w.p32, (const float*)w.Ap32, idiag32, w.rb, w.S, w.I);
-  else launch_k(k_update32s<false>, w, st, n, w.x32, w.r32, w.p32, (const float*)w.Ap32, idiag32, w.rb, w.S, w.I);
+// Launch shape of the CG kernels.  One block per SM, a slice per warp while the warps suffice
+// (32 per SM): its lanes' vector entries stay in registers.  Up to 16 slices fit one block,
+// whose barriers are block barriers (8^3 Q1: 8.7 us per iteration, 11.4 with 4 blocks, 12.9
+// with 11).  Twice the slices take two per warp (23 x 17 x 21 Q3 in FP64: 85 us per iteration
+// against 103 streaming; four per warp 120).  Beyond that two blocks per SM, 48 warps, stream
+// the vectors: four slices per warp were slower there too (unstructured 40^3 Q2, 15.4 k
+// slices: 136-144 us against 92).
+struct PcgShape {
+  int R;
+  unsigned blocks, threads;
+};
+static PcgShape pcg_shape(int64_t nslices, int sms) {
+  const int64_t cap = (int64_t)sms * 32;
+  if (nslices > 2 * cap) return PcgShape{0, (unsigned)(2 * sms), (unsigned)pcg_threads(0)};
+  const int R = nslices <= cap ? 1 : 2;
+  const int64_t warps = std::max<int64_t>(1, (nslices + R - 1) / R);
+  const int64_t blocks = warps <= 16 ? 1 : std::min<int64_t>(sms, warps);
+  return PcgShape{R, (unsigned)blocks, (unsigned)(32 * ((warps + blocks - 1) / blocks))};
 }
 
-// Capture `chunk` iterations into a graph and replay it until the device done flag is set.
-template <typename F>
-static fg_status run_chunks(fg_ctx* ctx, const Work& w, int chunk, F launch_iter, int* h_I, double* h_S) {
-  cudaStream_t st = ctx->stream;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  FG_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-  for (int k = 0; k < chunk; ++k) launch_iter();
-  cudaError_t e = cudaStreamEndCapture(st, &graph);
-  if (e != cudaSuccess) { set_error("graph capture: %s", cudaGetErrorString(e)); return FG_ERR_CUDA; }
-  e = cudaGraphInstantiate(&exec, graph, 0);
-  if (e != cudaSuccess) {
-    cudaGraphDestroy(graph);
-    set_error("graph instantiate: %s", cudaGetErrorString(e));
-    return FG_ERR_CUDA;
+template <typename... KA>
+static fg_status launch_pcg(void (*k)(KA...), const PcgShape& sh, const Work& w, int noff, cudaStream_t st, void** args) {
+  const size_t smem = sizeof(int32_t) * (size_t)noff;
+  if (smem > 16 * 1024)  // static and dynamic shared memory together pass 48 KB
+    FG_CUDA_TRY(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  FG_CUDA_TRY(cudaMemsetAsync(w.rb.ticket + 1, 0, sizeof(unsigned), st));
+  FG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k, dim3(sh.blocks), dim3(sh.threads), args, smem, st));
+  return FG_OK;
+}
+
+// Iterations of one launch: about 5 ms (contexts on other threads get the GPU in between),
+// or the caller's polling interval.
+static int pcg_iters(const fg_solver_params* prm, int64_t entries, int64_t nvec, int width) {
+  if (prm->check_every > 0) return prm->check_every;
+  const double us = 8.0 + ((double)entries + 10.0 * (double)nvec) * width / 5.5e6;
+  const int n = (int)(5000.0 / us) & ~7;
+  return std::min(1024, std::max(16, n));
+}
+
+// scalars and flags of the solve, copied to the host in one piece
+struct SolveState {
+  double S[S_COUNT];
+  int I[I_COUNT];
+};
+static fg_status read_state(const Work& w, SolveState& h, cudaStream_t st) {
+  static_assert(sizeof(SolveState) == sizeof(double) * S_COUNT + sizeof(int) * I_COUNT, "the device keeps I after S");
+  FG_CUDA_TRY(cudaMemcpyAsync(&h, w.S, sizeof(h), cudaMemcpyDeviceToHost, st));
+  FG_CUDA_TRY(cudaStreamSynchronize(st));
+  if (h.I[I_ABORT]) {
+    set_error("the CG kernel's grid barrier ran out of time");
+    return FG_ERR_TIMEOUT;
   }
-  fg_status out = FG_OK;
+  return FG_OK;
+}
+
+// grid barriers of the CG kernels: bounded at 10 s (FG_PCG_BARRIER_TIMEOUT_MS; read per solve)
+static GridSync grid_sync(const Work& w) {
+  const char* ms = getenv("FG_PCG_BARRIER_TIMEOUT_MS");
+  const char* drop = getenv("FG_PCG_TEST_DROP_ARRIVAL");
+  return GridSync{w.rb.part, w.rb.ticket + 1, w.I + I_ABORT, (ms ? (unsigned long long)atoll(ms) : 10000ull) * 1000000ull,
+                  drop ? atoi(drop) : 0};
+}
+
+static int64_t solver_entries(const fg_space* sp) {
+  return sp->layout == FG_LAYOUT_STENCIL ? sp->st_nvals : sp->sell_nnz;
+}
+
+// FP64 CG from the state k_init64 left, until it is done.
+static fg_status run_pcg64(fg_system* sys, const Work& w, const fg_solver_params* prm, int criterion, double rtol,
+                           double atol, int chunk, SolveState& h, cudaStream_t st) {
+  fg_space* sp = sys->space;
+  const bool stencil = sp->layout == FG_LAYOUT_STENCIL;
+  MatArgs<double> m = mat_args<double>(sp, stencil ? sys->d_tval : sys->d_sval);
+  const PcgShape sh = pcg_shape(m.nslices, w.sms);
+  int64_t nvec = sp->nvec;
+  double *x = w.x, *r = w.r, *p = w.p, *Ap = w.Ap;
+  const double* idiag = prm->precond == FG_PREC_JACOBI ? sys->d_idiag : nullptr;
+  int iters = pcg_iters(prm, solver_entries(sp), nvec, 8);
+  GridSync g = grid_sync(w);
+  double* S = w.S;
+  int* I = w.I;
+  void* args[] = {&m, &nvec, &x, &r, &p, &Ap, &idiag, &criterion, &rtol, &atol, &iters, &chunk, &g, &S, &I};
   for (;;) {
-    e = cudaGraphLaunch(exec, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_I, w.I, sizeof(int) * I_COUNT, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_S, w.S, sizeof(double) * S_COUNT, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) { set_error("cg loop: %s", cudaGetErrorString(e)); out = FG_ERR_CUDA; break; }
-    if (h_I[I_DONE]) break;
-    if (!std::isfinite(h_S[S_ALPHA]) || !std::isfinite(h_S[S_RZ])) {
-      out = FG_ERR_NUMERIC;
+#define FG_PCG64(L) \
+  (sh.R == 1 ? k_pcg64<L, 1> : sh.R == 2 ? k_pcg64<L, 2> : k_pcg64<L, 0>)
+    FG_TRY(launch_pcg(stencil ? FG_PCG64(true) : FG_PCG64(false), sh, w, m.noff, st, args));
+#undef FG_PCG64
+    sp->mesh->ctx->launches += 1;
+    FG_TRY(read_state(w, h, st));
+    if (h.I[I_DONE]) return FG_OK;
+    if (!std::isfinite(h.S[S_ALPHA]) || !std::isfinite(h.S[S_RZ])) {
       set_error("non-finite CG scalars");
-      break;
+      return FG_ERR_NUMERIC;
     }
   }
-  cudaGraphExecDestroy(exec);
-  cudaGraphDestroy(graph);
-  return out;
+}
+
+// FP32 iterations of the mixed path until the segment ends.
+static fg_status run_pcg32(fg_system* sys, const Work& w, const fg_solver_params* prm, const float* vals,
+                           const float* idiag, SolveState& h, cudaStream_t st) {
+  fg_space* sp = sys->space;
+  const bool stencil = sp->layout == FG_LAYOUT_STENCIL;
+  MatArgs<float> m = mat_args<float>(sp, vals);
+  const PcgShape sh = pcg_shape(m.nslices, w.sms);
+  int64_t nvec = sp->nvec;
+  float *x = w.x32, *r = w.r32, *p = w.p32, *q = w.Ap32;
+  int iters = pcg_iters(prm, solver_entries(sp), nvec, 4);
+  GridSync g = grid_sync(w);
+  double* S = w.S;
+  int* I = w.I;
+  void* args[] = {&m, &nvec, &x, &r, &p, &q, &idiag, &iters, &g, &S, &I};
+  do {
+#define FG_PCG32(L) \
+  (sh.R == 1 ? k_pcg32<L, 1> : sh.R == 2 ? k_pcg32<L, 2> : k_pcg32<L, 0>)
+    FG_TRY(launch_pcg(stencil ? FG_PCG32(true) : FG_PCG32(false), sh, w, m.noff, st, args));
+#undef FG_PCG32
+    sp->mesh->ctx->launches += 1;
+    FG_TRY(read_state(w, h, st));
+  } while (!h.I[I_DONE]);
+  return FG_OK;
 }
 
 fg_status system_solve(fg_system* sys, const fg_solver_params* prm, const double* d_b, const double* d_x0,
@@ -983,8 +1528,8 @@ fg_status system_solve(fg_system* sys, const fg_solver_params* prm, const double
   const double* b_row = d_b ? d_b : sys->d_rhs;
   const int precond = prm->precond == FG_PREC_JACOBI ? 1 : 0;
   const int chunk = prm->check_every > 0 ? prm->check_every : (n < 200000 ? 64 : 16);
-  int h_I[I_COUNT];
-  double h_S[S_COUNT];
+  SolveState h;
+  std::memset(&h, 0, sizeof(h));
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -997,35 +1542,31 @@ fg_status system_solve(fg_system* sys, const fg_solver_params* prm, const double
   else k_fill<double><<<nblk(nv, RB), RB, 0, st>>>(nv, w.x, 0.0);
   ctx->launches += 2;
   FG_CUDA_TRY(cudaGetLastError());
+  FG_CUDA_TRY(cudaMemsetAsync(w.I, 0, sizeof(int) * I_COUNT, st));
   if (prm->precision == FG_FP64) {
     if (d_x0) spmv_k<double, 0>(sys, w, w.x, w.r, nullptr, st);
-    launch_k(k_init64, w, st, nv, (const double*)w.b, d_x0 ? 1 : 0, w.r, w.p, (const double*)sys->d_idiag, precond,
-             prm->criterion, prm->rtol, prm->atol, prm->max_iters, w.rb, w.S, w.I);
+    launch_kn(k_init64, w, st, nv, nv, (const double*)w.b, d_x0 ? 1 : 0, w.r, w.p, (const double*)sys->d_idiag, precond,
+              prm->criterion, prm->rtol, prm->atol, prm->max_iters, w.rb, w.S, w.I);
     ctx->launches += 1;
     FG_CUDA_TRY(cudaGetLastError());
-    const bool need_pp = prm->criterion == FG_DELTA_RHS || prm->criterion == FG_DELTA_DELTA;
-    status = run_chunks(ctx, w, chunk,
-                        [&]() { iter64(sys, w, precond, need_pp, prm->criterion, prm->rtol, prm->atol, st); }, h_I, h_S);
-    ctx->launches += (int64_t)3 * chunk * (((int64_t)h_I[I_ITER] + chunk - 1) / chunk + 0);
-    out.iterations = h_I[I_ITER];
-    out.converged = h_I[I_CONV];
-    out.error_estimate = h_S[S_ERR];
-    out.tolerance = h_S[S_TOL];
+    status = run_pcg64(sys, w, prm, prm->criterion, prm->rtol, prm->atol, chunk, h, st);
+    out.iterations = h.I[I_ITER];
+    out.converged = h.I[I_CONV];
+    out.error_estimate = h.S[S_ERR];
+    out.tolerance = h.S[S_TOL];
   } else {
     const double delta = prm->inner_rtol > 0 ? prm->inner_rtol : 0.1;
     // true residual of the initial guess and the tolerance
     spmv_k<double, 2>(sys, w, w.x, w.r, w.b, st);
-    FG_CUDA_TRY(cudaMemcpyAsync(h_S, w.S, sizeof(double) * S_COUNT, cudaMemcpyDeviceToHost, st));
-    FG_CUDA_TRY(cudaStreamSynchronize(st));
-    double rn = h_S[S_ERR];
+    FG_TRY(read_state(w, h, st));
+    double rn = h.S[S_ERR];
     double tol;
     if (prm->criterion == FG_RES_RHS) {
-      launch_k(k_init64, w, st, nv, (const double*)w.b, 0, w.t, w.Ap, (const double*)sys->d_idiag, 0, (int)FG_RES_RHS,
-               prm->rtol, prm->atol, 1, w.rb, w.S, w.I);
+      launch_kn(k_init64, w, st, nv, nv, (const double*)w.b, 0, w.t, w.Ap, (const double*)sys->d_idiag, 0,
+                (int)FG_RES_RHS, prm->rtol, prm->atol, 1, w.rb, w.S, w.I);
       ctx->launches += 1;
-      FG_CUDA_TRY(cudaMemcpyAsync(h_S, w.S, sizeof(double) * S_COUNT, cudaMemcpyDeviceToHost, st));
-      FG_CUDA_TRY(cudaStreamSynchronize(st));
-      tol = prm->rtol * h_S[S_BNRM] + prm->atol;
+      FG_TRY(read_state(w, h, st));
+      tol = prm->rtol * h.S[S_BNRM] + prm->atol;
       spmv_k<double, 2>(sys, w, w.x, w.r, w.b, st);
     } else {
       tol = prm->rtol * rn + prm->atol;
@@ -1033,7 +1574,6 @@ fg_status system_solve(fg_system* sys, const fg_solver_params* prm, const double
     int outer = 0, stalls = 0, polish_its = 0;
     bool polish = false;
     double rn_prev = rn;
-    int64_t graph_launches = 0;
     if (!std::isfinite(rn)) {
       status = FG_ERR_NUMERIC;
       set_error("non-finite initial residual");
@@ -1049,7 +1589,7 @@ fg_status system_solve(fg_system* sys, const fg_solver_params* prm, const double
       int hI0[I_COUNT] = {0};
       hI0[I_MAXIT] = prm->max_iters;
       FG_CUDA_TRY(cudaMemcpyAsync(w.I, hI0, sizeof(hI0), cudaMemcpyHostToDevice, st));
-      // FP32 segments on D^-1/2 A D^-1/2 (Jacobi) or A (no preconditioner), fused iterations
+      // FP32 segments on D^-1/2 A D^-1/2 (Jacobi) or A (no preconditioner)
       const double* sd = nullptr;
       const float* vals32 = sp->layout == FG_LAYOUT_STENCIL ? sys->d_tval32 : sys->d_sval32;
       const float* id32 = nullptr;
@@ -1060,49 +1600,29 @@ fg_status system_solve(fg_system* sys, const fg_solver_params* prm, const double
         id32 = sys->d_idiag32;
       }
       auto refresh = [&](int first) {
-        launch_k(k_refresh_scaled, w, st, nv, (const double*)w.r, sd, w.r32, first, w.rb, w.S, w.I);
-        launch_k(k_pupdate<float, false>, w, st, nv, w.p32, (const float*)w.r32, (const float*)nullptr,
-                 (const double*)w.S, (const int*)w.I);
+        launch_kn(k_refresh_scaled, w, st, nv, nv, (const double*)w.r, sd, w.r32, first, w.rb, w.S, w.I);
+        launch_kn(k_pupdate, w, st, (nv + 3) / 4, nv, w.p32, (const float*)w.r32, (const double*)w.S);
         ctx->launches += 2;
       };
       refresh(1);
       FG_CUDA_TRY(cudaGetLastError());
-      // graph of `chunk` FP32 iterations, replayed; reliable updates on the host's cue
-      cudaGraph_t graph = nullptr;
-      cudaGraphExec_t exec = nullptr;
-      FG_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      for (int k = 0; k < chunk; ++k)  // at least the last iteration of a chunk sums the stop estimate
-        iter32s(sys, w, vals32, id32, k % FG_MIXED_EXACT_EVERY == FG_MIXED_EXACT_EVERY - 1 || k == chunk - 1, st);
-      cudaError_t e = cudaStreamEndCapture(st, &graph);
-      if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
-      if (e != cudaSuccess) {
-        if (graph) cudaGraphDestroy(graph);
-        set_error("graph: %s", cudaGetErrorString(e));
-        return FG_ERR_CUDA;
-      }
+      // FP32 segments; reliable updates on the host's cue
       for (;;) {
-        e = cudaGraphLaunch(exec, st);
-        ++graph_launches;
-        if (e == cudaSuccess) e = cudaMemcpyAsync(h_I, w.I, sizeof(int) * I_COUNT, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) { set_error("mixed loop: %s", cudaGetErrorString(e)); status = FG_ERR_CUDA; break; }
-        if (!h_I[I_DONE]) continue;
+        status = run_pcg32(sys, w, prm, vals32, id32, h, st);
+        if (status != FG_OK) break;
         // reliable update: fold the FP32 correction into x64 and recompute the true residual
         // (after a breakdown the segment's correction is dropped instead)
-        FG_CUDA_TRY(cudaMemcpyAsync(h_S, w.S, sizeof(double) * S_COUNT, cudaMemcpyDeviceToHost, st));
-        FG_CUDA_TRY(cudaStreamSynchronize(st));
-        const bool broke = h_I[I_FLAG] == FLAG_BREAK;
+        const bool broke = h.I[I_FLAG] == FLAG_BREAK;
         if (broke) k_fill<float><<<nblk(nv, RB), RB, 0, st>>>(nv, w.x32, 0.0f);
-        else launch_k(k_fold_scaled, w, st, nv, h_S[S_SIGMA], sd, w.x32, w.x);
+        else launch_kn(k_fold_scaled, w, st, nv, nv, h.S[S_SIGMA], sd, w.x32, w.x);
         ctx->launches += 1;
         spmv_k<double, 2>(sys, w, w.x, w.r, w.b, st);
         ++outer;
-        FG_CUDA_TRY(cudaMemcpyAsync(h_S, w.S, sizeof(double) * S_COUNT, cudaMemcpyDeviceToHost, st));
-        FG_CUDA_TRY(cudaStreamSynchronize(st));
-        rn = h_S[S_ERR];
+        FG_TRY(read_state(w, h, st));
+        rn = h.S[S_ERR];
         if (!std::isfinite(rn)) { status = FG_ERR_NUMERIC; set_error("non-finite residual"); break; }
         if (rn <= tol) { out.converged = 1; break; }
-        if (h_I[I_ITER] >= prm->max_iters) break;
+        if (h.I[I_ITER] >= prm->max_iters) break;
         // FP32 segments aim at a 10x reduction of the true residual; a breakdown, or two
         // segments in a row that gain less than 2x (FP32 rounding of an ill-conditioned
         // matrix near a tight tolerance), hand the rest of the solve to the FP64 PCG
@@ -1112,29 +1632,22 @@ fg_status system_solve(fg_system* sys, const fg_solver_params* prm, const double
         refresh(0);
         FG_CUDA_TRY(cudaGetLastError());
       }
-      cudaGraphExecDestroy(exec);
-      cudaGraphDestroy(graph);
-      FG_CUDA_TRY(cudaMemcpyAsync(h_I, w.I, sizeof(int) * I_COUNT, cudaMemcpyDeviceToHost, st));
-      FG_CUDA_TRY(cudaStreamSynchronize(st));
-      ctx->launches += graph_launches * 2 * chunk;
       if (polish && status == FG_OK) {
         // FP64 PCG from x64 to the same absolute tolerance, with the iterations left
-        const int mixed_its = h_I[I_ITER];
+        const int mixed_its = h.I[I_ITER];
         spmv_k<double, 0>(sys, w, w.x, w.r, nullptr, st);
-        launch_k(k_init64, w, st, nv, (const double*)w.b, 1, w.r, w.p, (const double*)sys->d_idiag, precond,
-                 (int)FG_RES_RES, 0.0, tol, std::max(prm->max_iters - mixed_its, 1), w.rb, w.S, w.I);
+        launch_kn(k_init64, w, st, nv, nv, (const double*)w.b, 1, w.r, w.p, (const double*)sys->d_idiag, precond,
+                  (int)FG_RES_RES, 0.0, tol, std::max(prm->max_iters - mixed_its, 1), w.rb, w.S, w.I);
         ctx->launches += 1;
         FG_CUDA_TRY(cudaGetLastError());
-        status = run_chunks(ctx, w, chunk,
-                            [&]() { iter64(sys, w, precond, false, (int)FG_RES_RES, 0.0, tol, st); }, h_I, h_S);
-        ctx->launches += (int64_t)3 * chunk * (((int64_t)h_I[I_ITER] + chunk - 1) / chunk);
-        polish_its = h_I[I_ITER];
-        out.converged = h_I[I_CONV];
-        rn = h_S[S_ERR];
-        h_I[I_ITER] = mixed_its;
+        status = run_pcg64(sys, w, prm, (int)FG_RES_RES, 0.0, tol, chunk, h, st);
+        polish_its = h.I[I_ITER];
+        out.converged = h.I[I_CONV];
+        rn = h.S[S_ERR];
+        h.I[I_ITER] = mixed_its;
       }
     }
-    out.iterations = h_I[I_ITER] + polish_its;
+    out.iterations = h.I[I_ITER] + polish_its;
     out.outer_iterations = outer;
     out.error_estimate = rn;
     out.tolerance = tol;
