@@ -24,26 +24,36 @@
 //     dropped (|error| <~ K 2^-57 max_l |x_il| max_l |y_jl|).  The cut keeps 54 bits below
 //     the row maximum, so a value far below it loses its low bits: overall the product is
 //     within ~K 2^-52 max|x_i.| max|y_j.| of the exact one (about the FP64 dot-product bound);
-//   * the epilogue converts the 8 class sums to integers, combines them exactly in int64,
-//     turns the chunk's sum into FP64 with one rounding (two exact conversions by bit
-//     arithmetic, one addition), adds the K chunks in FP64, applies the power of two
-//     2^(e_i + f_j - 16) through the exponent field and updates C: about two FP64
-//     operations per output element and chunk instead of 128.  (A rounding by integer
-//     arithmetic alone measured slower: 421 vs 330 us at 4096 x 4096 x 128.)
+//   * the epilogue converts the 8 class sums to integers, combines them exactly (H 2^-24 +
+//     L 2^-56), turns the chunk's sum into FP64 with one rounding (two exact bit patterns, one
+//     addition), adds the K chunks in FP64, applies the power of two 2^(e_i + f_j - 16) through
+//     the exponent field and updates C: about two FP64 operations per output element and chunk
+//     instead of 128.
 //
 // Digit layout in HBM: per operand, blocks of 128 rows x 16 columns (one MMA K step) per
 // digit, 4 KB each, ordered [row tile][K step][digit]; inside a block the rows are in the
 // canonical K-major, non-swizzled UMMA layout: core matrices of 8 rows x 16 bytes, the two
 // 8-column halves 128 B apart (LBO), row groups 256 B apart (SBO).  An operand B tile of 64
-// rows is half a block (2 KB), of 32 rows a quarter.  A CTA computes 128 x 64 (or 128 x 32)
-// output tiles: warp 0's lane 0 streams the digit blocks into shared memory with
-// cp.async.bulk (5 or 6 stages, mbarrier
-// transaction counts) and issues the MMAs; warps 1-8 read the accumulators (tcgen05.ld, two
-// warps per TMEM lane quarter, 32 columns each) and write C.  CTAs are persistent (one per SM, tiles round robin):
-// the epilogue releases the accumulators before its FP64 writes, which then overlap the next
-// tile's MMAs, and the stages of the next tile are loaded meanwhile.  Every wait is bounded: after ~1 s the CTA records
-// FG_ERR_TIMEOUT, stops, waits (bounded) for its copies and MMAs in flight, frees its tensor
-// memory and returns.
+// rows is half a block (2 KB).  A CTA computes 128 x 64 output tiles: warp 17's lane 0 streams
+// the digit blocks into shared memory with cp.async.bulk (5 stages, mbarrier transaction
+// counts), warp 0 issues the MMAs, warps 1-16 read the accumulators (tcgen05.ld, four warps per
+// TMEM lane quarter, 16 columns each) and write C.  CTAs are persistent (one per SM, tiles
+// round robin).  Every wait is bounded: after ~1 s the CTA records FG_ERR_TIMEOUT, stops, waits
+// (bounded) for its copies and MMAs in flight, frees its tensor memory and returns.
+//
+// What bounds it (4096^3: 13.1 us per chunk of 10 K steps and tile): the MMAs, ~60 cycles each
+// where a 128 x 64 x 16 one runs 32, then ~4.7 k cycles in which the epilogue takes the class
+// sums out of the accumulators (they fill the tensor memory, so the next tile's MMAs wait); the
+// conversion and the update of C (10 k cycles) run beside the next tile's MMAs.  What it took,
+// TFLOP/s at 4096^3 and 8192 x 8192 x 128:
+//     13.7 / 13.0  eight epilogue warps converting before they release the accumulators, MMAs
+//                  issued by the lane that also feeds the copies
+//     16.8 / 15.2  release first, sixteen warps
+//     26.0 / 23.0  a copy warp, and MMAs issued from warp-uniform code (descriptors in uniform
+//                  registers): 139 -> 78 cycles per MMA
+//     30.5 / 25.6  each A digit block read from shared memory once per K step and held in the
+//                  collector buffer for its run of MMAs: 78 -> 60
+// 128 x 32 tiles with two accumulator sets: 25.9 / 22.9.
 
 #include <cuda_runtime.h>
 
@@ -66,24 +76,25 @@ constexpr uint32_t OZ_BLOCK = OZ_BM * OZ_BK * 2;           // one digit block: 4
 constexpr uint32_t OZ_A_BYTES = OZ_S * OZ_BLOCK;           // 28672 B per K step
 constexpr uint32_t OZ_TMEM_COLS = 512;                     // all of it
 constexpr long long OZ_WAIT_CYCLES = 1ll << 31;            // ~1 s at 2 GHz
-constexpr int OZ_THREADS = 32 + 8 * 32;                    // MMA warp + 8 epilogue warps
+constexpr int OZ_EPI_WARPS = 16;                           // epilogue warps: 4 per TMEM lane quarter
+constexpr int OZ_THREADS = (OZ_EPI_WARPS + 2) * 32;        // with the MMA warp (0) and the copy warp (17)
 
-// Output tiles of 128 x BN.  BN = 64: the 8 accumulators fill the tensor memory (one set);
-// BN = 32: two sets, so one tile's MMAs run while the epilogue reads the previous tile.
+// Output tiles of 128 x BN: the 8 accumulators of BN = 64 columns fill the tensor memory.
+constexpr int OZ_BN = 64;
 template <int BN>
 struct OzT {
   static constexpr int NSET = (int)OZ_TMEM_COLS / (OZ_NACC * BN);
-  static constexpr int EPI = BN / 2;                          // columns per epilogue thread
+  static constexpr int EPI = BN * 4 / OZ_EPI_WARPS;           // columns per epilogue thread
   static constexpr int QB = OZ_BM / BN;                       // B tiles per 128-row digit block
   static constexpr uint32_t B_DIGIT = BN * OZ_BK * 2;         // one digit of a B tile per K step
   static constexpr uint32_t STAGE = OZ_A_BYTES + OZ_S * B_DIGIT;
-  static constexpr int NBUF = BN == 64 ? 5 : 6;               // stages: 215040 B either way
+  static constexpr int NBUF = 5;                              // stages: 215040 B
   static constexpr uint32_t SMEM = NBUF * STAGE;
   // kind::f16: FP32 accumulator, bf16 A and B, both K-major, N = BN, M = 128
   static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
                                     ((uint32_t)(OZ_BM >> 4) << 24);
 };
-constexpr int OZ_MAXBUF = 6;
+constexpr int OZ_MAXBUF = 5;
 
 // ---- PTX wrappers -------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -114,17 +125,32 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
                "l"(src), "r"(bytes), "r"(mbar)
                : "memory");
 }
+// one lane of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, 128 x 64 x 16, bf16 -> FP32
+// D[tmem] (+)= A[smem] * B[smem]^T, 128 x BN x 16, bf16 -> FP32.  A run of MMAs on the same A
+// block reads it from shared memory once: the first fills the A collector buffer, the others
+// use it, the last one gives it up.
+enum { COLL_FILL = 0, COLL_USE = 1, COLL_LAST = 2 };
+template <int COLL>
 __device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-      "l"(a), "l"(b), "r"(idesc), "r"(acc)
-      : "memory");
+#define FG_TC_MMA(C)                                                                   \
+  asm volatile(                                                                        \
+      "{\n\t.reg .pred p;\n\t"                                                         \
+      "setp.ne.b32 p, %4, 0;\n\t"                                                      \
+      "tcgen05.mma.cta_group::1.kind::f16.collector::a::" C " [%0], %1, %2, %3, p;\n\t}" \
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc)                                   \
+      : "memory")
+  if (COLL == COLL_FILL) FG_TC_MMA("fill");
+  else if (COLL == COLL_USE) FG_TC_MMA("use");
+  else FG_TC_MMA("lastuse");
+#undef FG_TC_MMA
 }
 // arrive on the mbarrier once every tcgen05 operation issued so far by this thread is done
 __device__ __forceinline__ void tc_commit(uint32_t mbar) {
@@ -206,37 +232,43 @@ __device__ __forceinline__ OzSplit split_of(const OzSplitArgs& a, int rtile) {
 // Row exponents: e_r with max_l |x_rl| < 2^(e_r - 2), from the largest biased exponent of
 // the row (an all-zero or padding row gets 0).  Blocks (digit row tile, part of 32).  Rows
 // with consecutive elements (cs == 1): a warp per row, lanes along it, part p taking rows
-// 4p .. 4p + 3; otherwise part 0 takes the tile, a thread per row (consecutive rows are
-// consecutive in memory).
+// 4p .. 4p + 3.  Otherwise part p < 4 takes rows 32p .. 32p + 31 (consecutive rows are
+// consecutive in memory), a warp per quarter of the columns: one thread per row walking the
+// 128 columns of a Cholesky panel alone took 56 us of load latency.
 __global__ void __launch_bounds__(OZ_BM) k_oz_rowexp(OzSplitArgs a) {
+  __shared__ unsigned long long s_mx[OZ_BM / 32][32];
   const int rtile = blockIdx.x;
   const OzSplit it = split_of(a, rtile);
-  if (it.cs != 1 && blockIdx.y != 0) return;
+  if (it.cs != 1 && blockIdx.y >= OZ_BM / 32) return;
   const int64_t r0 = (int64_t)(rtile - it.rtile0) * OZ_BM;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   auto finish = [&](int local, unsigned long long mx) {
     const int E = (int)(mx >> 52);  // biased exponent of the largest |x| (0: zero/subnormal)
     a.ex[(int64_t)rtile * OZ_BM + local] = mx == 0 ? 0 : (E == 0 ? 1 : E) - 1020;
   };
+  auto bits = [&](int64_t r, int64_t l) {
+    return (unsigned long long)__double_as_longlong(it.x[r * it.rs + l * it.cs]) & 0x7FFFFFFFFFFFFFFFull;
+  };
+  unsigned long long mx = 0;
   if (it.cs == 1) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    {
-      const int local = blockIdx.y * (OZ_BM / 32) + warp;
-      const int64_t r = r0 + local;
-      unsigned long long mx = 0;
-      if (r < it.rows)
-        for (int64_t l = lane; l < it.k; l += 32)
-          mx = max(mx, (unsigned long long)__double_as_longlong(it.x[r * it.rs + l]) & 0x7FFFFFFFFFFFFFFFull);
-#pragma unroll
-      for (int o = 16; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      if (lane == 0) finish(local, mx);
-    }
-  } else {
-    const int64_t r = r0 + threadIdx.x;
-    unsigned long long mx = 0;
+    const int local = blockIdx.y * (OZ_BM / 32) + warp;
+    const int64_t r = r0 + local;
     if (r < it.rows)
-      for (int64_t l = 0; l < it.k; ++l)
-        mx = max(mx, (unsigned long long)__double_as_longlong(it.x[r * it.rs + l * it.cs]) & 0x7FFFFFFFFFFFFFFFull);
-    finish(threadIdx.x, mx);
+      for (int64_t l = lane; l < it.k; l += 32) mx = max(mx, bits(r, l));
+#pragma unroll
+    for (int o = 16; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane == 0) finish(local, mx);
+  } else {
+    const int local = blockIdx.y * 32 + lane;
+    const int64_t r = r0 + local;
+    if (r < it.rows) {
+      const int64_t q = (it.k + 3) / 4, l1 = min((int64_t)it.k, q * (warp + 1));
+#pragma unroll 8
+      for (int64_t l = q * warp; l < l1; ++l) mx = max(mx, bits(r, l));
+    }
+    s_mx[warp][lane] = mx;
+    __syncthreads();
+    if (warp == 0) finish(local, max(max(mx, s_mx[1][lane]), max(s_mx[2][lane], s_mx[3][lane])));
   }
 }
 
@@ -300,6 +332,17 @@ struct OzItem {
   int arow0, brow0;
   int tiles_n;
   int tile0;
+  int tiles_m;  // > 0: tiles numbered down the columns (tiles_m row tiles each)
+  __device__ __forceinline__ void locate(int t, int& rt, int& ct) const {
+    const int lt = t - tile0;
+    if (tiles_m > 0) {
+      ct = lt / tiles_m;
+      rt = lt - ct * tiles_m;
+    } else {
+      rt = lt / tiles_n;
+      ct = lt - rt * tiles_n;
+    }
+  }
 };
 
 struct OzGemmArgs {
@@ -328,21 +371,15 @@ __device__ __forceinline__ OzItem item_of(const OzGemmArgs& g, int t) {
   return g.items[lo];
 }
 
-// x 2^off as FP64, for |x| < 2^53 (exact), by integer operations on the bit pattern (no
-// FP64 operation); false if the result would leave the normal FP64 range.
-__device__ __forceinline__ bool i64_to_f64(long long x, int off, double& d) {
-  if (x == 0) {
-    d = 0.0;
-    return true;
-  }
+// x 2^off as FP64, for |x| < 2^53 (exact) and an exponent that stays normal, by integer
+// operations on the bit pattern (no FP64 operation)
+__device__ __forceinline__ double i64_to_f64(long long x, int off) {
+  if (x == 0) return 0.0;
   const unsigned long long sgn = x < 0 ? (1ull << 63) : 0ull;
   const unsigned long long a = x < 0 ? (unsigned long long)(-x) : (unsigned long long)x;
   const int lz = __clzll((long long)a);
-  const int be = (63 - lz) + 1023 + off;
-  if (be < 1 || be > 2046) return false;
   const unsigned long long mant = (a << (lz + 1)) >> 12;  // the bits after the leading one
-  d = __longlong_as_double((long long)(sgn | ((unsigned long long)be << 52) | mant));
-  return true;
+  return __longlong_as_double((long long)(sgn | ((unsigned long long)(63 - lz + 1023 + off) << 52) | mant));
 }
 
 // d 2^off by adding off to the exponent field; false if d or the result is not a normal
@@ -376,12 +413,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ntiles = g.ntiles;
-  // tile t of item it: local tile lt = t - tile0, row tile lt / tiles_n, column tile lt % tiles_n
   auto valid = [&](int t) {
     if (!g.lower) return true;
     const OzItem it = item_of(g, t);
-    const int lt = t - it.tile0;
-    return (lt % it.tiles_n) * BN <= (lt / it.tiles_n) * OZ_BM + OZ_BM - 1;
+    int rt, ct;
+    it.locate(t, rt, ct);
+    return ct * BN <= rt * OZ_BM + OZ_BM - 1;
   };
   auto next_tile = [&](int t) {
     for (t += gridDim.x; t < ntiles && !valid(t); t += gridDim.x) {
@@ -403,7 +440,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
       }
       for (int z = 0; z < 2; ++z) {
         mbar_init(smem_u32(&bar_acc_full[z]), 1);
-        mbar_init(smem_u32(&bar_acc_empty[z]), OZ_THREADS - 32);
+        mbar_init(smem_u32(&bar_acc_empty[z]), OZ_EPI_WARPS * 32);
       }
       abort_flag = 0;
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -416,93 +453,97 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
   const int KS = g.ksteps;
   const int nchunks = (KS + g.chunk - 1) / g.chunk;
 
+  const uint32_t sbase = smem_u32(oz_smem);
   if (warp == 0) {
-    if (lane == 0) {
-      const uint32_t sbase = smem_u32(oz_smem);
-      // producer cursor: tile pt (its digit rows pa, pb and half), K step pks, stage counter pgs
-      int pt = first, pks = 0, pgs = 0;
-      const uint8_t *pa = nullptr, *pb = nullptr;
-      auto locate = [&]() {
-        if (pt >= ntiles) return;
-        const OzItem it = item_of(g, pt);
-        const int lt = pt - it.tile0, rt = lt / it.tiles_n, ct = lt % it.tiles_n;
-        pa = g.dig + (size_t)(it.arow0 + rt) * KS * OZ_A_BYTES;
-        pb = g.dig + (size_t)(it.brow0 + ct / T::QB) * KS * OZ_A_BYTES + (size_t)(ct % T::QB) * T::B_DIGIT;
-      };
-      locate();
-      auto produce = [&]() -> bool {
-        if (pt >= ntiles) return true;
-        const int buf = pgs % OZ_NBUF;
-        if (pgs >= OZ_NBUF && !mbar_wait(smem_u32(&bar_empty[buf]), ((pgs / OZ_NBUF) - 1) & 1, &abort_flag, g.err))
-          return false;
-        const uint32_t full = smem_u32(&bar_full[buf]);
-        const uint32_t dst = sbase + buf * T::STAGE;
-        mbar_expect_tx(full, T::STAGE);
-        if (!(blockIdx.x == 0 && pgs == g.drop_stage)) {
-          bulk_g2s(dst, pa + (size_t)pks * OZ_A_BYTES, OZ_A_BYTES, full);
-          for (int t = 0; t < OZ_S; ++t)
-            bulk_g2s(dst + OZ_A_BYTES + t * T::B_DIGIT, pb + ((size_t)pks * OZ_S + t) * OZ_BLOCK, T::B_DIGIT, full);
-        }
-        ++pgs;
-        if (++pks == KS) {
-          pks = 0;
-          pt = next_tile(pt);
-          locate();
-        }
-        return true;
-      };
-      bool ok = true;
-      for (int p = 0; p < OZ_NBUF - 1 && ok; ++p) ok = produce();
-      int gs = 0, gc = 0;
-      for (int t = first; t < ntiles && ok; t = next_tile(t)) {
-        for (int ks = 0; ks < KS && ok; ++ks) {
-          const int kin = ks % g.chunk;
-          const int buf = gs % OZ_NBUF;
-          const int z = gc % T::NSET;  // accumulator set of this chunk
-          if (kin == 0 && gc >= T::NSET &&
-              !mbar_wait(smem_u32(&bar_acc_empty[z]), ((gc / T::NSET) - 1) & 1, &abort_flag, g.err)) {
-            ok = false;
-            break;
-          }
-          if (!mbar_wait(smem_u32(&bar_full[buf]), (gs / OZ_NBUF) & 1, &abort_flag, g.err)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t sa = sbase + buf * T::STAGE, sb = sa + OZ_A_BYTES;
-          const uint64_t da = smem_desc(sa), db = smem_desc(sb);
-          const uint32_t tacc = tmem + z * (OZ_NACC * BN);
+    // MMA warp.  The whole warp runs the loop and one elected lane issues: the descriptors then
+    // stay in uniform registers.  (Issued from a branch on lane == 0, an MMA cost ~80 cycles
+    // of moves to the uniform registers, more than the 32 it runs.)
+    bool ok = true;
+    int gs = 0, gc = 0;
+    for (int t = first; t < ntiles && ok; t = next_tile(t)) {
+      for (int ks = 0; ks < KS; ++ks) {
+        const int kin = ks % g.chunk;
+        const int buf = gs % OZ_NBUF;
+        const int z = gc % T::NSET;  // accumulator set of this chunk
+        if (kin == 0 && gc >= T::NSET)
+          ok = mbar_wait(smem_u32(&bar_acc_empty[z]), ((gc / T::NSET) - 1) & 1, &abort_flag, g.err);
+        ok = ok && mbar_wait(smem_u32(&bar_full[buf]), (gs / OZ_NBUF) & 1, &abort_flag, g.err);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t sa = sbase + buf * T::STAGE, sb = sa + OZ_A_BYTES;
+        const uint64_t da = smem_desc(sa), db = smem_desc(sb);
+        const uint32_t tacc = tmem + z * (OZ_NACC * BN);
+        const bool last = kin == g.chunk - 1 || ks == KS - 1;
+        if (elect_one()) {
+          // A digit by A digit: the digit stays in the collector buffer for its run; the first
+          // pair of a class starts the chunk's sum
 #pragma unroll
-          for (int kk = 0; kk < OZ_NACC; ++kk)
+          for (int s = 0; s < OZ_S; ++s)
 #pragma unroll
-            for (int s = (kk > OZ_S - 1 ? kk - (OZ_S - 1) : 0); s <= (kk < OZ_S - 1 ? kk : OZ_S - 1); ++s)
-              // start-address field in 16-byte units; the first pair of a class starts the chunk's sum
-              tc_mma(tacc + kk * BN, da + (uint64_t)(s * (OZ_BLOCK >> 4)),
-                     db + (uint64_t)((kk - s) * (T::B_DIGIT >> 4)), T::IDESC,
-                     (kin > 0 || s > (kk > OZ_S - 1 ? kk - (OZ_S - 1) : 0)) ? 1u : 0u);
+            for (int kk = s; kk < OZ_NACC && kk - s < OZ_S; ++kk) {
+              const bool end = kk + 1 == OZ_NACC || kk + 1 - s == OZ_S;
+              // start-address field in 16-byte units
+              const uint32_t d = tacc + kk * BN;
+              const uint64_t ad = da + (uint64_t)(s * (OZ_BLOCK >> 4)), bd = db + (uint64_t)((kk - s) * (T::B_DIGIT >> 4));
+              const uint32_t acc = (kin > 0 || s > (kk > OZ_S - 1 ? kk - (OZ_S - 1) : 0)) ? 1u : 0u;
+              if (kk == s) tc_mma<COLL_FILL>(d, ad, bd, T::IDESC, acc);
+              else if (!end) tc_mma<COLL_USE>(d, ad, bd, T::IDESC, acc);
+              else tc_mma<COLL_LAST>(d, ad, bd, T::IDESC, acc);
+            }
           tc_commit(smem_u32(&bar_empty[buf]));
-          if (kin == g.chunk - 1 || ks == KS - 1) {
-            tc_commit(smem_u32(&bar_acc_full[z]));
-            ++gc;
+          if (last) tc_commit(smem_u32(&bar_acc_full[z]));
+        }
+        __syncwarp();
+        if (last) ++gc;
+        ++gs;
+      }
+    }
+    // after an abort: every MMA issued
+    if (!ok && gs > 0) mbar_drain(smem_u32(&bar_empty[(gs - 1) % OZ_NBUF]), ((gs - 1) / OZ_NBUF) & 1);
+    __syncwarp();
+  } else if (warp == OZ_EPI_WARPS + 1) {
+    // copy warp: lane 0 streams the stages
+    if (lane == 0) {
+      bool ok = true;
+      int gs = 0;
+      for (int t = first; t < ntiles && ok; t = next_tile(t)) {
+        const OzItem it = item_of(g, t);
+        int rt, ct;
+        it.locate(t, rt, ct);
+        const uint8_t* pa = g.dig + (size_t)(it.arow0 + rt) * KS * OZ_A_BYTES;
+        const uint8_t* pb =
+            g.dig + (size_t)(it.brow0 + ct / T::QB) * KS * OZ_A_BYTES + (size_t)(ct % T::QB) * T::B_DIGIT;
+        for (int ks = 0; ks < KS; ++ks, ++gs) {
+          const int buf = gs % OZ_NBUF;
+          if (gs >= OZ_NBUF && !mbar_wait(smem_u32(&bar_empty[buf]), ((gs / OZ_NBUF) - 1) & 1, &abort_flag, g.err)) {
+            ok = false;
+            break;
           }
-          ++gs;
-          ok = produce();
+          const uint32_t full = smem_u32(&bar_full[buf]);
+          const uint32_t dst = sbase + buf * T::STAGE;
+          mbar_expect_tx(full, T::STAGE);
+          if (blockIdx.x == 0 && gs == g.drop_stage) continue;
+          bulk_g2s(dst, pa + (size_t)ks * OZ_A_BYTES, OZ_A_BYTES, full);
+          for (int d = 0; d < OZ_S; ++d)
+            bulk_g2s(dst + OZ_A_BYTES + d * T::B_DIGIT, pb + ((size_t)ks * OZ_S + d) * OZ_BLOCK, T::B_DIGIT, full);
         }
       }
-      if (!ok) {
-        // drain: the stages whose copies were issued but not consumed, then every MMA issued
-        for (int q = gs; q < pgs; ++q) mbar_drain(smem_u32(&bar_full[q % OZ_NBUF]), (q / OZ_NBUF) & 1);
-        if (gs > 0) mbar_drain(smem_u32(&bar_empty[(gs - 1) % OZ_NBUF]), ((gs - 1) / OZ_NBUF) & 1);
-      }
+      // nothing may land in this CTA's shared memory after it is gone (an abort elsewhere leaves
+      // copies nobody waits for): wait for the last one into each stage
+      for (int q = gs > OZ_NBUF ? gs - OZ_NBUF : 0; q < gs; ++q)
+        mbar_drain(smem_u32(&bar_full[q % OZ_NBUF]), (q / OZ_NBUF) & 1);
     }
     __syncwarp();
   } else {
-    // epilogue: warps 1-8; warp w reads TMEM lanes 32 (w % 4) .. +31 (tile rows), columns
-    // EPI h .. EPI h + EPI - 1 with h = (w - 1) / 4
+    // epilogue: warps 1-16; warp w reads TMEM lanes 32 (w % 4) .. +31 (tile rows), columns
+    // EPI h .. EPI h + EPI - 1 with h = (w - 1) / 4.  The next tile's MMAs need the
+    // accumulators, so a warp first takes all its class sums as integers (hi, lo per column)
+    // and releases them; the conversion to FP64 and the update of C run beside those MMAs.
     constexpr int OZ_EPI_COLS = T::EPI;
-    const int quarter = warp & 3, half = (warp - 1) >> 2;
+    const int quarter = warp & 3, part4 = (warp - 1) >> 2;
     const int row = quarter * 32 + lane;
-    const uint32_t trow0 = tmem + ((uint32_t)(quarter * 32) << 16) + half * OZ_EPI_COLS;
+    const uint32_t trow0 = tmem + ((uint32_t)(quarter * 32) << 16) + part4 * OZ_EPI_COLS;
     // alpha, beta cases as integers, decided once (an FP64 compare per element would cost as
     // much as the element's arithmetic)
     const int amode = g.alpha == -1.0 ? 0 : (g.alpha == 1.0 ? 1 : 2);
@@ -511,8 +552,6 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
     for (int t = first; t < ntiles; t = next_tile(t)) {
       // per column: sum over K chunks of the chunk's product / 2^(e_i + f_j - 16), in FP64
       double acc[OZ_EPI_COLS];
-#pragma unroll
-      for (int j = 0; j < OZ_EPI_COLS; ++j) acc[j] = 0.0;
       bool ok = true;
       for (int chunk = 0; chunk < nchunks; ++chunk, ++gc) {
         const int z = gc % T::NSET;
@@ -522,12 +561,12 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
         }
         tc_fence_after();
         const uint32_t trow = trow0 + z * (OZ_NACC * BN);
+        // sum_k v_k 2^(-8k) = H 2^-24 + L 2^-56 exactly (every v_k is an integer below 2^24 held
+        // in FP32): |H| < 2^50 and 0 <= L < 2^32, three registers per column
+        long long H[OZ_EPI_COLS];
+        uint32_t L[OZ_EPI_COLS];
 #pragma unroll
         for (int cb = 0; cb < OZ_EPI_COLS / 8; ++cb) {
-          // sum_k v_k 2^(-8k) exactly: every v_k is an integer below 2^24 held in FP32; hi in
-          // units of 2^-16 (classes 0-2), lo in units of 2^-56 (classes 3-7), loaded four
-          // classes at a time
-          long long hi[8], lo[8];
 #pragma unroll
           for (int part = 0; part < 2; ++part) {
             uint32_t v[OZ_NACC / 2][8];
@@ -540,36 +579,40 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
 #pragma unroll
               for (int q = 0; q < OZ_NACC / 2; ++q) a[q] = __float2int_rn(__uint_as_float(v[q][j]));
               if (part == 0) {
-                hi[j] = (long long)a[0] * 65536 + (long long)a[1] * 256 + a[2];
-                lo[j] = (long long)a[3] * 4294967296ll;
+                // |a0| < 2^19.5, |a1| < 2^21.5, |a2| < 2^22.5, |a3| < 2^23: each pair fits 32 bits
+                H[cb * 8 + j] = (long long)(a[0] * 256 + a[1]) * 65536 + (a[2] * 256 + a[3]);
               } else {
-                lo[j] += (long long)a[0] * 16777216 + (long long)a[1] * 65536 + (long long)a[2] * 256 + a[3];
+                const long long x = ((long long)a[0] * 256 + a[1]) * 65536 + ((long long)a[2] * 256 + a[3]);
+                H[cb * 8 + j] += x >> 32;
+                L[cb * 8 + j] = (uint32_t)x;
               }
             }
-          }
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            // |hi| < 2^42 and |lo| < 2^57: move lo's bits above 2^40 into hi, then both
-            // convert exactly (bit arithmetic); one FP64 rounding for the chunk
-            const long long carry = lo[j] >> 40;
-            double xh, xl;
-            i64_to_f64(hi[j] + carry, -16, xh);
-            i64_to_f64(lo[j] - carry * 1099511627776ll, -56, xl);
-            acc[cb * 8 + j] = chunk == 0 ? xh + xl : acc[cb * 8 + j] + (xh + xl);
           }
         }
         tc_fence_before();
         mbar_arrive(smem_u32(&bar_acc_empty[z]));  // accumulators free: the next MMAs may start
+        // keeps the conversion below the release (volatile statements stay in order)
+#pragma unroll
+        for (int j = 0; j < OZ_EPI_COLS; ++j) asm volatile("" : "+l"(H[j]), "+r"(L[j]));
+#pragma unroll
+        for (int j = 0; j < OZ_EPI_COLS; ++j) {
+          // xl = 2^-4 + L 2^-56 is a bit pattern (the ulp of 2^-4 is 2^-56); xh takes the 2^-4
+          // (2^20 units of 2^-24) away again, exactly: one FP64 rounding for the chunk
+          const double xl = __hiloint2double(0x3FB00000, (int)L[j]);
+          const double xh = i64_to_f64(H[j] - (1ll << 20), -24);
+          acc[j] = chunk == 0 ? xh + xl : acc[j] + (xh + xl);
+        }
       }
       if (!ok) break;
       const OzItem it = item_of(g, t);
-      const int lt = t - it.tile0, rt = lt / it.tiles_n, ct = lt % it.tiles_n;
+      int rt, ct;
+      it.locate(t, rt, ct);
       const int i = rt * OZ_BM + row;
       const bool row_ok = i < it.m;
       const int ei = g.ex[(int64_t)(it.arow0 + rt) * OZ_BM + row];
-      const int c0 = ct * BN + half * OZ_EPI_COLS;
+      const int c0 = ct * BN + part4 * OZ_EPI_COLS;
       // lane j < EPI holds the exponent of column c0 + j (padding rows of the exponents are 0)
-      const int ecol = g.ex[(int64_t)(it.brow0 + ct / T::QB) * OZ_BM + (ct % T::QB) * BN + half * OZ_EPI_COLS +
+      const int ecol = g.ex[(int64_t)(it.brow0 + ct / T::QB) * OZ_BM + (ct % T::QB) * BN + part4 * OZ_EPI_COLS +
                             (lane < OZ_EPI_COLS ? lane : 0)];
       double* crow = it.c + (int64_t)i * it.c_rs;
 #pragma unroll
@@ -629,15 +672,6 @@ size_t ozaki_workspace_bytes(int64_t m, int64_t n, int64_t k, bool same) {
   return (size_t)rt * ks * OZ_A_BYTES + (size_t)rt * OZ_BM * sizeof(int32_t) + 256;
 }
 
-// output tile width: 64 (default) or 32 (FG_OZ_BN=32: two accumulator sets)
-static int oz_bn() {
-  static const int bn = [] {
-    const char* e = std::getenv("FG_OZ_BN");
-    return (e && std::atoi(e) == 32) ? 32 : 64;
-  }();
-  return bn;
-}
-
 template <int BN>
 static fg_status oz_gemm_launch(fg_ctx* ctx, cudaStream_t st, OzGemmArgs& g, int64_t ntiles) {
   FG_CUDA_TRY(cudaFuncSetAttribute((const void*)k_oz_gemm<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -656,7 +690,7 @@ static fg_status oz_launch(fg_ctx* ctx, cudaStream_t st, OzSplitArgs& sa, int64_
   g.drop_stage = drop ? std::atoi(drop) : -1;
   k_oz_rowexp<<<dim3((unsigned)rtiles, 32), OZ_BM, 0, st>>>(sa);
   k_oz_split<<<dim3((unsigned)rtiles, (unsigned)sa.ksteps), OZ_BM, 0, st>>>(sa);
-  FG_TRY(oz_bn() == 32 ? oz_gemm_launch<32>(ctx, st, g, ntiles) : oz_gemm_launch<64>(ctx, st, g, ntiles));
+  FG_TRY(oz_gemm_launch<OZ_BN>(ctx, st, g, ntiles));
   ctx->launches += 3;
   FG_CUDA_TRY(cudaGetLastError());
   return FG_OK;
@@ -676,9 +710,21 @@ fg_status ozaki_gemm_nt(fg_ctx* ctx, cudaStream_t st, int64_t m, int64_t n, int6
     return FG_OK;
   }
   const bool same = B == nullptr;
+  // The epilogue's lanes are consecutive rows of a tile: a row-major C is computed as its
+  // transpose B A^T, so that a warp's store is 256 contiguous bytes instead of 32 sectors (the
+  // digit sums are exact integers: the same results bit for bit).
+  if (c_cs == 1 && c_rs != 1 && !lower) {
+    if (!same) {
+      std::swap(A, B);
+      std::swap(a_rs, b_rs);
+      std::swap(a_cs, b_cs);
+    }
+    std::swap(m, n);
+    std::swap(c_rs, c_cs);
+  }
   const int64_t ksteps = (k + OZ_BK - 1) / OZ_BK;
   const int64_t rta = rtiles_of(m), rtb = same ? 0 : rtiles_of(n);
-  const int64_t tiles_n = (n + oz_bn() - 1) / oz_bn();
+  const int64_t tiles_n = (n + OZ_BN - 1) / OZ_BN;
   if (rta * tiles_n > (1ll << 31) - 1 || rta + rtb > (1ll << 31) - 1 || ksteps > 65535) {
     set_error("ozaki_gemm_nt: %lld x %lld x %lld is too large", (long long)m, (long long)n, (long long)k);
     return FG_ERR_UNSUPPORTED;
@@ -697,7 +743,10 @@ fg_status ozaki_gemm_nt(fg_ctx* ctx, cudaStream_t st, int64_t m, int64_t n, int6
   g.ex = sa.ex;
   g.items = nullptr;
   g.nitems = 1;
-  g.one = OzItem{C, c_rs, c_cs, (int)m, (int)n, 0, same ? 0 : (int)rta, (int)tiles_n, 0};
+  // consecutive CTAs walk the shorter side of the tile grid: the longer operand's digits are
+  // read from HBM once and shared through L2
+  g.one = OzItem{C, c_rs, c_cs, (int)m, (int)n, 0, same ? 0 : (int)rta, (int)tiles_n, 0,
+                 !lower && rta < tiles_n ? (int)rta : 0};
   g.ntiles = (int)(rta * tiles_n);
   g.ksteps = (int)ksteps;
   g.chunk = k <= OZ_KEXACT ? (int)ksteps : OZ_CHUNK_STEPS;
@@ -727,9 +776,9 @@ fg_status ozaki_syrk_batch(fg_ctx* ctx, cudaStream_t st, const std::vector<OzSyr
       set_error("ozaki_syrk_batch: k = %d > 128", x.k);
       return FG_ERR_UNSUPPORTED;
     }
-    const int64_t tn = (x.m + oz_bn() - 1) / oz_bn();
+    const int64_t tn = (x.m + OZ_BN - 1) / OZ_BN;
     hs.push_back(OzSplit{x.p, 1, x.ld, x.m, x.k, (int)rt});
-    hi.push_back(OzItem{x.c, 1, x.ld, x.m, x.m, (int)rt, (int)rt, (int)tn, (int)tiles});
+    hi.push_back(OzItem{x.c, 1, x.ld, x.m, x.m, (int)rt, (int)rt, (int)tn, (int)tiles, 0});
     rt += rtiles_of(x.m);
     tiles += rtiles_of(x.m) * tn;
   }
