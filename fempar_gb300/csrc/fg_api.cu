@@ -374,6 +374,8 @@ static void space_free(fg_space* sp) {
   dev_free(ctx, sp->d_st_slot2row);
   dev_free(ctx, sp->d_tcT);
   dev_free(ctx, sp->d_tcff);
+  dev_free(ctx, sp->d_tcA);
+  dev_free(ctx, sp->d_tcgeo);
   delete sp;
 }
 

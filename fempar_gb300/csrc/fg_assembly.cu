@@ -71,25 +71,18 @@ struct SourceSpec {
   const double* qp;  // per-qp values
 };
 
-// tutorial_01 source f = -lap(atan(alpha(|x-c|-r))) (tutorial modules :395-458)
+// tutorial_01 source f = -lap(atan(alpha(|x-c|-r))) (tutorial modules :395-458).  The three
+// second derivatives there add up to 2 alpha/(rho A) - 2 alpha^3 (rho - r)/A^2, rho = |x-c|,
+// A = 1 + alpha^2 (rho - r)^2: one square root and one division instead of a pow and nine (FP64 is
+// the scarce pipe; 32^3 Q1 spent 0.63 ms of 0.86 ms assembly here).
 __device__ double sharp_wave_source(const double* prm, const double* x) {
-  double alpha = prm[0], r = prm[1];
-  double alpha_2 = alpha * alpha, alpha_3 = alpha_2 * alpha;
-  double x_minus_xc_2 = (x[0] - prm[2]) * (x[0] - prm[2]);
-  double y_minus_yc_2 = (x[1] - prm[3]) * (x[1] - prm[3]);
-  double z_minus_zc_2 = (x[2] - prm[4]) * (x[2] - prm[4]);
-  double term1 = x_minus_xc_2 + y_minus_yc_2 + z_minus_zc_2;
-  double sqrt_term1 = sqrt(term1);
-  double term2 = sqrt_term1 - r;
-  double term2_2 = term2 * term2;
-  double a2t = alpha_2 * term2_2 + 1.0;
-  double denom1 = sqrt_term1 * a2t;
-  double denom2 = pow(term1, 1.5) * a2t;
-  double denom3 = term1 * a2t * a2t;
-  double dx2 = alpha / denom1 - (alpha * x_minus_xc_2) / denom2 - (2.0 * alpha_3 * x_minus_xc_2 * term2) / denom3;
-  double dy2 = alpha / denom1 - (alpha * y_minus_yc_2) / denom2 - (2.0 * alpha_3 * y_minus_yc_2 * term2) / denom3;
-  double dz2 = alpha / denom1 - (alpha * z_minus_zc_2) / denom2 - (2.0 * alpha_3 * z_minus_zc_2 * term2) / denom3;
-  return -dx2 - dy2 - dz2;
+  const double alpha = prm[0], r = prm[1];
+  const double dx = x[0] - prm[2], dy = x[1] - prm[3], dz = x[2] - prm[4];
+  const double rho = sqrt(dx * dx + dy * dy + dz * dz);
+  const double t = rho - r;
+  const double A = fma(alpha * alpha * t, t, 1.0);
+  // 2 alpha (alpha^2 t rho - A) / (rho A^2)
+  return 2.0 * alpha * (alpha * alpha * t * rho - A) / (rho * A * A);
 }
 
 __device__ double boundary_value(int fn, const double* prm, const double* x) {
@@ -524,55 +517,176 @@ template <int P>
 struct PoissonTC {
   using S = PoissonShape<P>;
   static constexpr int NQ = S::NQ, ND = S::ND, NPAIR = S::NPAIR, K = 6 * NQ;
-  static constexpr int WARPS = 8;
-  static constexpr int SM_DOUBLES = S::SM_XV + S::SM_INVJ + S::SM_FAC + S::SM_XQ + S::SM_F;
-  static constexpr size_t SM_BYTES_WARP = ((size_t)SM_DOUBLES * 8 + ND * 4 + 15) / 16 * 16;
+};
+
+// Cell geometry of the tensor-core path, GL lanes per cell (Q1: four cells per warp).  A column
+// J(:, d) = dx/dxi_d of the trilinear map depends on the two other coordinates only, so it is
+// evaluated once per line of Gauss points -- half the four edge differences along d, weighted
+// bilinearly: 4 FMAs for each of 9 (p+1)^2 values where summing 8 vertices at every point takes
+// 72 per point.  FP64 instructions are what the kernels below are bound by (a warp instruction
+// holds the SM's FP64 pipe for 16 cycles).
+template <int P>
+struct CellGeo {
+  static constexpr int NP1 = P + 1, NC2 = NP1 * NP1, NQ = NC2 * NP1;
+  static constexpr int GL = P == 1 ? 8 : 32;
+  static constexpr int WARPS = 8, CELLS = WARPS * 32 / GL;  // per block
+  // block: edge weights, 1D shape values, quadrature weights
+  static constexpr int TAB = NC2 * 4 + NC2 + NQ;
+  // cell: vertices, edge differences, J per line, two arrays over the Gauss points
+  static constexpr int CELL = 24 + 36 + 9 * NC2 + 2 * NQ;
+  static constexpr size_t SMEM = sizeof(double) * (TAB + (size_t)CELLS * CELL);
 };
 
 template <int P>
-__global__ void __launch_bounds__(PoissonTC<P>::WARPS * 32)
-    k_poisson_geom(AsmGeom g, int64_t ncells, const double* __restrict__ coords, DevTables tb,
-                   const int32_t* __restrict__ latdof, const double* __restrict__ coef, double coef_const,
-                   SourceSpec src, double* __restrict__ G, double* __restrict__ EV) {
-  using T = PoissonTC<P>;
-  constexpr int NQ = T::NQ, ND = T::ND, K = T::K;
-  extern __shared__ double smem[];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  double* xv = smem + (size_t)wib * (T::SM_BYTES_WARP / 8);
-  double* invj = xv + T::S::SM_XV;
-  double* fac = invj + T::S::SM_INVJ;
-  double* xq = fac + T::S::SM_FAC;
-  double* fsrc = xq + T::S::SM_XQ;
-  int32_t* gid = (int32_t*)(fsrc + T::S::SM_F);
-  const int64_t c = (int64_t)blockIdx.x * T::WARPS + wib;
-  if (c >= ncells) return;
+__device__ __forceinline__ void geo_stage_tables(const double* __restrict__ geo, double* tab) {
+  for (int i = threadIdx.x; i < CellGeo<P>::TAB; i += blockDim.x) tab[i] = geo[i];
+  __syncthreads();
+}
+
+template <int P>
+__device__ __forceinline__ void geo_lines(const AsmGeom& g, int64_t c, const double* __restrict__ coords,
+                                          const double* ew, int gl, double* xv, double* D, double* Jt) {
+  using T = CellGeo<P>;
   const int ci = (int)(c % g.n[0]);
   const int cj = (int)((c / g.n[0]) % g.n[1]);
   const int ck = (int)(c / ((int64_t)g.n[0] * g.n[1]));
-  const double kc = coef ? coef[c] : coef_const;
-  poisson_cell_geometry<P>(g, c, ci, cj, ck, coords, tb, latdof, src, lane, xv, invj, fac, xq, fsrc, gid);
-  // per Gauss point: |det J| w k (into xq, free unless the source read it) and |det J| w f
-  double* fk = xq;
-  for (int q = lane; q < NQ; q += 32) {
-    const double fq = fac[q];
-    fk[q] = fq * kc;
-    fsrc[q] = fq * fsrc[q];
+  for (int t = gl; t < 24; t += T::GL) xv[t] = coords[asm_vertex(g, c, ci, cj, ck, t / 3) * 3 + t % 3];
+  __syncwarp();
+  for (int t = gl; t < 36; t += T::GL) {
+    const int d = t / 12, e = (t / 3) & 3, l = t % 3;
+    const int d1 = d == 0 ? 1 : 0, d2 = d == 2 ? 1 : 2;
+    const int lo = ((e & 1) << d1) | ((e >> 1) << d2);
+    D[t] = xv[(lo | (1 << d)) * 3 + l] - xv[lo * 3 + l];
   }
   __syncwarp();
-  // M_jk = |det J| w k sum_l B[j + 3l] B[k + 3l], B = J^-1 as stored by invmtx; order 00 11 22 01 02 12
-  for (int e = lane; e < K; e += 32) {
-    const int q = e / 6, m = e - 6 * q;
-    const int j = m < 3 ? m : (m == 5 ? 1 : 0), k = m < 3 ? m : (m == 3 ? 1 : 2);
-    const double* b = invj + q * 9;
-    G[c * K + e] = fk[q] * (b[j] * b[k] + b[j + 3] * b[k + 3] + b[j + 6] * b[k + 6]);
+  for (int t = gl; t < 9 * T::NC2; t += T::GL) {
+    const int d = t / (3 * T::NC2), line = (t / 3) % T::NC2, l = t % 3;
+    double v = 0.0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v = fma(ew[line * 4 + e], D[d * 12 + e * 3 + l], v);
+    Jt[t] = v;
   }
-  // element vector, source part (the lifting follows the product); the same products and
-  // order as k_integrate_poisson's (fac f) phi
-  for (int a = lane; a < ND; a += 32) {
-    double ev = 0.0;
-    for (int q = 0; q < NQ; ++q) ev = ev + fsrc[q] * tb.shp[(size_t)a * NQ + q];
-    EV[c * ND + a] = ev;
+  __syncwarp();
+}
+
+// J, its cofactors (C[k + 3i] = det dxi_k/dx_i, the invmtx order) and determinant at point q
+template <int P>
+__device__ __forceinline__ double geo_cofactors(const double* Jt, int q, double (&J)[9], double (&C)[9]) {
+  using T = CellGeo<P>;
+  const int i = q % T::NP1, j = (q / T::NP1) % T::NP1, k = q / T::NC2;
+  const int line[3] = {j + T::NP1 * k, i + T::NP1 * k, i + T::NP1 * j};
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+#pragma unroll
+    for (int l = 0; l < 3; ++l) J[l + 3 * d] = Jt[(d * T::NC2 + line[d]) * 3 + l];
+  C[0] = J[4] * J[8] - J[5] * J[7];
+  C[1] = J[2] * J[7] - J[1] * J[8];
+  C[2] = J[1] * J[5] - J[2] * J[4];
+  C[3] = J[5] * J[6] - J[3] * J[8];
+  C[4] = J[0] * J[8] - J[2] * J[6];
+  C[5] = J[3] * J[2] - J[0] * J[5];
+  C[6] = J[3] * J[7] - J[4] * J[6];
+  C[7] = J[1] * J[6] - J[0] * J[7];
+  C[8] = J[0] * J[4] - J[1] * J[3];
+  return J[0] * C[0] + J[3] * C[1] + J[6] * C[2];
+}
+
+// sum_q shp_a(x_q) f_q for every node a, one direction at a time; f is destroyed, out may be
+// global memory
+template <int P>
+__device__ __forceinline__ void geo_load_vector(const double* L1, int gl, double* f, double* t, bool valid,
+                                                double* __restrict__ out) {
+  using T = CellGeo<P>;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double* in = d == 1 ? t : f;
+    const int st = d == 0 ? 1 : (d == 1 ? T::NP1 : T::NC2);
+    for (int o = gl; o < T::NQ; o += T::GL) {
+      const int a = (o / st) % T::NP1, b = o - a * st;
+      double v = 0.0;
+#pragma unroll
+      for (int q = 0; q < T::NP1; ++q) v = fma(L1[a * T::NP1 + q], in[b + q * st], v);
+      if (d == 0) t[o] = v;
+      else if (d == 1) f[o] = v;
+      else if (valid) out[o] = v;
+    }
+    __syncwarp();
   }
+}
+
+// Geometric factors G_c[6q + m] = (|det J| w k J^-1 J^-T)_m at every Gauss point (m: 00 11 22 01 02
+// 12), from the cofactors C: w k/|det J| C C^T, and the source part of the element vector.
+// FP64-bound; 64^3 Q2: 2.33 -> 1.20 ms with J per line, cofactors in place of J^-1 and the
+// element vector by sum factorisation.
+template <int P>
+__global__ void __launch_bounds__(CellGeo<P>::WARPS * 32)
+    k_poisson_geom(AsmGeom g, int64_t ncells, const double* __restrict__ coords, DevTables tb,
+                   const double* __restrict__ geo, const double* __restrict__ coef, double coef_const, SourceSpec src,
+                   double* __restrict__ G, double* __restrict__ EV) {
+  using T = CellGeo<P>;
+  constexpr int NQ = T::NQ, ND = PoissonTC<P>::ND, K = PoissonTC<P>::K;
+  extern __shared__ double smem[];
+  geo_stage_tables<P>(geo, smem);
+  const double *ew = smem, *L1 = ew + T::NC2 * 4, *qw = L1 + T::NC2;
+  const int lane = threadIdx.x & 31, gl = lane % T::GL, sub = threadIdx.x / T::GL;
+  double* xv = smem + T::TAB + (size_t)sub * T::CELL;
+  double* D = xv + 24;
+  double* Jt = D + 36;
+  double* f = Jt + 9 * T::NC2;
+  double* t = f + NQ;
+  int64_t c = (int64_t)blockIdx.x * T::CELLS + sub;
+  if ((int64_t)blockIdx.x * T::CELLS + (threadIdx.x / 32) * (32 / T::GL) >= ncells) return;  // the whole warp
+  const bool valid = c < ncells;  // a warp's spare cells repeat the last one and store nothing
+  if (!valid) c = ncells - 1;
+  const double kc = coef ? coef[c] : coef_const;
+  geo_lines<P>(g, c, coords, ew, gl, xv, D, Jt);
+  bool neg = false;
+  for (int q0 = 0; q0 < NQ; q0 += T::GL) {
+    const bool act = q0 + gl < NQ;
+    const int q = act ? q0 + gl : NQ - 1;
+    double J[9], C[9];
+    const double det = geo_cofactors<P>(Jt, q, J, C);
+    // |det| everywhere if the first one is negative (lane 0 of the cell holds point 0)
+    if (q0 == 0) neg = __shfl_sync(0xffffffffu, det, lane - gl) < 0.0;
+    if (!act) continue;
+    const double d = neg ? fabs(det) : det, w = qw[q];
+    if (src.fn != FG_FN_ZERO) {
+      double fq = src.prm[0];
+      if (src.fn == FG_FN_QP_VALUES) fq = src.qp[c * NQ + q];
+      else if (src.fn == FG_FN_SHARP_WAVE) {
+        double x[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const double a = tb.gshp[k * NQ + q];
+#pragma unroll
+          for (int l = 0; l < 3; ++l) x[l] = x[l] + a * xv[k * 3 + l];
+        }
+        fq = sharp_wave_source(src.prm, x);
+      }
+      f[q] = d * w * fq;
+    }
+    const double s = w * kc / d;
+    double2* o = reinterpret_cast<double2*>(G + c * K + 6 * q);
+    const double m0 = s * (C[0] * C[0] + C[3] * C[3] + C[6] * C[6]);
+    const double m1 = s * (C[1] * C[1] + C[4] * C[4] + C[7] * C[7]);
+    const double m2 = s * (C[2] * C[2] + C[5] * C[5] + C[8] * C[8]);
+    const double m3 = s * (C[0] * C[1] + C[3] * C[4] + C[6] * C[7]);
+    const double m4 = s * (C[0] * C[2] + C[3] * C[5] + C[6] * C[8]);
+    const double m5 = s * (C[1] * C[2] + C[4] * C[5] + C[7] * C[8]);
+    if (valid) {
+      o[0] = make_double2(m0, m1);
+      o[1] = make_double2(m2, m3);
+      o[2] = make_double2(m4, m5);
+    }
+  }
+  __syncwarp();
+  // element vector, source part (the lifting follows the product)
+  if (src.fn == FG_FN_ZERO) {
+    for (int a = gl; a < ND; a += T::GL)
+      if (valid) EV[c * ND + a] = 0.0;
+    return;
+  }
+  geo_load_vector<P>(L1, gl, f, t, valid, EV + c * ND);
 }
 
 // The same in float-float (FP32 pairs, ~2^-44 relative), for fast-integration requests: the
@@ -1079,36 +1193,71 @@ static int tc_integration_mode() {
 // the product's workspace and its error flag, 256-byte aligned pieces
 static size_t tc_align(size_t b) { return (b + 255) / 256 * 256; }
 
+// tables of CellGeo: edge weights 1/8 (1 +- x)(1 +- y) per line of Gauss points, 1D shape values,
+// quadrature weights
+template <int P>
+static fg_status ensure_geo_table(fg_space* sp) {
+  using T = CellGeo<P>;
+  if (sp->d_tcgeo) return FG_OK;
+  fg_ctx* ctx = sp->mesh->ctx;
+  double x[FG_MAX_ORDER + 1], w[FG_MAX_ORDER + 1];
+  gl_rule(T::NP1, x, w);
+  std::vector<double> h(T::TAB);
+  for (int l = 0; l < T::NC2; ++l)
+    for (int e = 0; e < 4; ++e) {
+      const double a = x[l % T::NP1], b = x[l / T::NP1];
+      h[l * 4 + e] = 0.125 * ((e & 1) ? 1.0 + a : 1.0 - a) * ((e & 2) ? 1.0 + b : 1.0 - b);
+    }
+  for (int a = 0; a < T::NP1; ++a)
+    for (int q = 0; q < T::NP1; ++q) {
+      double v, dv;
+      lagrange_1d(P, a, x[q], v, dv);
+      h[T::NC2 * 4 + a * T::NP1 + q] = v;
+    }
+  for (int q = 0; q < T::NQ; ++q) h[T::NC2 * 5 + q] = sp->tab.qw[q];
+  FG_TRY(dev_alloc(ctx, (void**)&sp->d_tcgeo, sizeof(double) * h.size()));
+  FG_CUDA_TRY(cudaMemcpyAsync(sp->d_tcgeo, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, ctx->stream));
+  FG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  return FG_OK;
+}
+
+// T[p][6q + m] for the row-packed upper pairs p = (a, b), b >= a
+template <int P>
+static fg_status ensure_pair_table(fg_space* sp) {
+  constexpr int NQ = PoissonTC<P>::NQ, NN = PoissonTC<P>::ND, NPAIR = PoissonTC<P>::NPAIR, K = PoissonTC<P>::K;
+  if (sp->d_tcT) return FG_OK;
+  fg_ctx* ctx = sp->mesh->ctx;
+  std::vector<double> hT((size_t)NPAIR * K);
+  const std::vector<double>& r = sp->tab.shg;  // (a NQ + q) 3 + j
+  size_t p = 0;
+  for (int a = 0; a < NN; ++a)
+    for (int b = a; b < NN; ++b, ++p)
+      for (int q = 0; q < NQ; ++q) {
+        const double* ra = &r[((size_t)a * NQ + q) * 3];
+        const double* rb = &r[((size_t)b * NQ + q) * 3];
+        double* t = &hT[p * K + 6 * q];
+        t[0] = ra[0] * rb[0];
+        t[1] = ra[1] * rb[1];
+        t[2] = ra[2] * rb[2];
+        t[3] = ra[0] * rb[1] + ra[1] * rb[0];
+        t[4] = ra[0] * rb[2] + ra[2] * rb[0];
+        t[5] = ra[1] * rb[2] + ra[2] * rb[1];
+      }
+  FG_TRY(dev_alloc(ctx, (void**)&sp->d_tcT, sizeof(double) * hT.size()));
+  FG_CUDA_TRY(cudaMemcpyAsync(sp->d_tcT, hT.data(), sizeof(double) * hT.size(), cudaMemcpyHostToDevice, ctx->stream));
+  FG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  return FG_OK;
+}
+
 template <int P>
 static fg_status launch_poisson_tc(fg_system* sys) {
   using T = PoissonTC<P>;
-  constexpr int NQ = T::NQ, ND = T::ND, NPAIR = T::NPAIR, K = T::K;
+  constexpr int NQ = T::NQ, NPAIR = T::NPAIR, K = T::K;
   fg_space* sp = sys->space;
   fg_ctx* ctx = sp->mesh->ctx;
   cudaStream_t st = ctx->stream;
   const int64_t ncells = sp->mesh->ncells;
-  if (!sp->d_tcT) {
-    // T[p][6q + m] for the row-packed upper pairs p = (a, b), b >= a
-    std::vector<double> hT((size_t)NPAIR * K);
-    const std::vector<double>& r = sp->tab.shg;  // (a NQ + q) 3 + j
-    size_t p = 0;
-    for (int a = 0; a < ND; ++a)
-      for (int b = a; b < ND; ++b, ++p)
-        for (int q = 0; q < NQ; ++q) {
-          const double* ra = &r[((size_t)a * NQ + q) * 3];
-          const double* rb = &r[((size_t)b * NQ + q) * 3];
-          double* t = &hT[p * K + 6 * q];
-          t[0] = ra[0] * rb[0];
-          t[1] = ra[1] * rb[1];
-          t[2] = ra[2] * rb[2];
-          t[3] = ra[0] * rb[1] + ra[1] * rb[0];
-          t[4] = ra[0] * rb[2] + ra[2] * rb[0];
-          t[5] = ra[1] * rb[2] + ra[2] * rb[1];
-        }
-    FG_TRY(dev_alloc(ctx, (void**)&sp->d_tcT, sizeof(double) * hT.size()));
-    FG_CUDA_TRY(cudaMemcpyAsync(sp->d_tcT, hT.data(), sizeof(double) * hT.size(), cudaMemcpyHostToDevice, st));
-    FG_CUDA_TRY(cudaStreamSynchronize(st));
-  }
+  FG_TRY(ensure_pair_table<P>(sp));
   const size_t gbytes = tc_align(sizeof(double) * ncells * K), cbytes = tc_align(sizeof(double) * ncells * NPAIR);
   const size_t wbytes = tc_align(ozaki_workspace_bytes(ncells, NPAIR, K, false));
   const size_t need = gbytes + cbytes + wbytes + 256;
@@ -1155,12 +1304,12 @@ static fg_status launch_poisson_tc(fg_system* sys) {
     k_poisson_geom_ff<P><<<nblk(ncells, F::WARPS), F::WARPS * 32, smem, st>>>(
         g, ncells, sp->mesh->d_coords, sp->dtab, sp->d_tcff, sys->d_coef, sys->integ.coef_const, src, G, sys->d_elvec);
   } else {
-    const size_t smem = T::SM_BYTES_WARP * T::WARPS;
+    using Geo = CellGeo<P>;
+    FG_TRY(ensure_geo_table<P>(sp));
     FG_CUDA_TRY(cudaFuncSetAttribute((const void*)k_poisson_geom<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
-    k_poisson_geom<P><<<nblk(ncells, T::WARPS), T::WARPS * 32, smem, st>>>(g, ncells, sp->mesh->d_coords, sp->dtab,
-                                                                         sp->d_latdof, sys->d_coef,
-                                                                         sys->integ.coef_const, src, G, sys->d_elvec);
+                                     (int)Geo::SMEM));
+    k_poisson_geom<P><<<nblk(ncells, Geo::CELLS), Geo::WARPS * 32, Geo::SMEM, st>>>(
+        g, ncells, sp->mesh->d_coords, sp->dtab, sp->d_tcgeo, sys->d_coef, sys->integ.coef_const, src, G, sys->d_elvec);
   }
   FG_CUDA_TRY(cudaGetLastError());
   FG_CUDA_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), st));
@@ -1184,9 +1333,13 @@ static fg_status launch_poisson(fg_system* sys) {
   using S = PoissonShape<P>;
   fg_space* sp = sys->space;
   fg_ctx* ctx = sp->mesh->ctx;
-  const bool ff = (sys->integ.flags & FG_FAST_INTEGRATION) != 0;
+  bool ff = (sys->integ.flags & FG_FAST_INTEGRATION) != 0;
   const int tcm = tc_integration_mode();
-  if (!sp->dg && sp->mesh->ncells > 0 && (ff ? tcm == 2 : tcm >= 1)) {
+  // Small Q1 meshes: the one FP64 kernel takes less than the five of the tensor-core path (86 vs
+  // 130 us per assembly at 8^3, 135 vs 135 at 16^3, 179 vs 148 at 20^3; Q2 is even up to 512 cells,
+  // Q3 slower from the first).  It serves fast requests too: it is the more accurate of the two.
+  const bool small = P == 1 && sp->mesh->ncells <= 4096;
+  if (!sp->dg && sp->mesh->ncells > 0 && !(small && tcm == 2) && (ff ? tcm == 2 : tcm >= 1)) {
     // the tensor-core path needs scratch (G, packed triangles, digits: ~7 KB per Q2 cell);
     // where the context's HBM budget has no room for it, the direct kernels run instead
     const fg_status s = launch_poisson_tc<P>(sys);
@@ -1199,6 +1352,7 @@ static fg_status launch_poisson(fg_system* sys) {
   for (int i = 0; i < 8; ++i) src.prm[i] = sys->integ.fn_param[i];
   src.qp = sys->d_qpsrc;
   using SF = typename PoissonShapeSel<P, true>::type;
+  if (small && tcm == 2) ff = false;
   const int warps = ff ? SF::WARPS : S::WARPS;
   const size_t smem = ff ? SF::SM_BYTES_WARP * SF::WARPS : S::SM_BYTES_WARP * S::WARPS;
   auto kern = ff ? k_integrate_poisson<P, true> : k_integrate_poisson<P, false>;
@@ -1413,6 +1567,268 @@ __global__ void __launch_bounds__(ElastShape<P>::WARPS * 32)
   }
 }
 
+// ---------------------------------------------------------------------------
+// Elasticity element matrices on the tensor cores.  With B = J^-1, f = |det J| w and r_a the
+// reference gradients, A_ab = sum_q f (B^T r_a)(B^T r_b)^T (3 x 3 per node pair) and the block of
+// the pair is lambda A + mu A^T + mu tr(A) I.  Its symmetric and antisymmetric parts are
+//   A_ij + A_ji = sum_q sum_{k<=l} T_kl(ab) f (B_ki B_lj + B_kj B_li)
+//   A_ij - A_ji = sum_q sum_{k<l} (r_ak r_bl - r_al r_bk) f (B_ki B_lj - B_kj B_li)
+// with T the table of the Poisson form, so the blocks of all cells are two products with tables
+// that every cell shares: six rows of 6 NQ factors per cell against T (K = 162 for Q2: one exact
+// chunk) and three rows of 3 NQ against the antisymmetric table.  The 2 x 2 minors of B are
+// entries of J over det J, so the second kind of factor is +-w J_nm.  lambda and mu are folded
+// into the factors; unpacking a block entry is at most one addition.  0.92 MFLOP per Q2 cell at
+// the products' ~25 TFLOP/s against 0.18 MFLOP on the FP64 pipe's 1.05 (and the warp-per-cell
+// kernel that did that holds 73 KB of shared memory: three warps per SM).
+// 32^3 Q2 element matrices: 10.9 ms -> 2.9 ms (geometry 0.43, digits 0.28, products 1.15, unpacking 1.0).
+template <int P>
+struct ElastTC {
+  static constexpr int NQ = ElastShape<P>::NQ, NN = ElastShape<P>::NN, ND = ElastShape<P>::ND;
+  static constexpr int NPAIR = ElastShape<P>::NPAIR, KS = 6 * NQ, KA = 3 * NQ;
+};
+
+template <int P>
+__global__ void __launch_bounds__(CellGeo<P>::WARPS * 32)
+    k_elasticity_geom(AsmGeom g, int64_t cell0, int64_t ncells, const double* __restrict__ coords,
+                      const double* __restrict__ geo, const double* __restrict__ coef, double coef_const, double nu,
+                      SourceSpec src, double* __restrict__ GS, double* __restrict__ GA, double* __restrict__ EV) {
+  using T = CellGeo<P>;
+  constexpr int NQ = T::NQ, NN = ElastTC<P>::NN, KS = ElastTC<P>::KS, KA = ElastTC<P>::KA;
+  extern __shared__ double smem[];
+  geo_stage_tables<P>(geo, smem);
+  const double *ew = smem, *L1 = ew + T::NC2 * 4, *qw = L1 + T::NC2;
+  const int lane = threadIdx.x & 31, gl = lane % T::GL, sub = threadIdx.x / T::GL;
+  double* xv = smem + T::TAB + (size_t)sub * T::CELL;
+  double* D = xv + 24;
+  double* Jt = D + 36;
+  double* f = Jt + 9 * T::NC2;
+  double* t = f + NQ;
+  int64_t cl = (int64_t)blockIdx.x * T::CELLS + sub;
+  if ((int64_t)blockIdx.x * T::CELLS + (threadIdx.x / 32) * (32 / T::GL) >= ncells) return;  // the whole warp
+  const bool valid = cl < ncells;
+  if (!valid) cl = ncells - 1;
+  const int64_t c = cell0 + cl;
+  const double Ev = coef ? coef[c] : coef_const;
+  const double lambda = (nu * Ev) / ((1.0 + nu) * (1.0 - 2.0 * nu));
+  const double mu = Ev / (2.0 * (1.0 + nu));
+  geo_lines<P>(g, c, coords, ew, gl, xv, D, Jt);
+  bool neg = false;
+  for (int q0 = 0; q0 < NQ; q0 += T::GL) {
+    const bool act = q0 + gl < NQ;
+    const int q = act ? q0 + gl : NQ - 1;
+    double J[9], C[9];
+    const double det = geo_cofactors<P>(Jt, q, J, C);
+    if (q0 == 0) neg = __shfl_sync(0xffffffffu, det, lane - gl) < 0.0;
+    if (!act) continue;
+    const double d = neg ? fabs(det) : det, w = qw[q];
+    f[q] = d * w;
+    const double s = w / d;  // f / det^2
+    const double hs = 0.5 * (lambda + mu) * s;
+    // symmetric rows: (i, i) with the trace term, then (0,1), (0,2), (1,2)
+    const int kk[6] = {0, 1, 2, 0, 0, 1}, ll[6] = {0, 1, 2, 1, 2, 2};
+    double tr[6], di[3][6];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) di[i][m] = C[kk[m] + 3 * i] * C[ll[m] + 3 * i];
+      tr[m] = (mu * s) * (di[0][m] + di[1][m] + di[2][m]);
+    }
+    double* o = GS + (size_t)cl * 6 * KS + 6 * q;
+#pragma unroll
+    for (int e = 0; e < 6; ++e) {
+      double v[6];
+#pragma unroll
+      for (int m = 0; m < 6; ++m) {
+        if (e < 3) {
+          v[m] = fma(2.0 * hs, di[e][m], tr[m]);
+        } else {
+          const int i = e == 5 ? 1 : 0, j = e == 3 ? 1 : 2;
+          v[m] = hs * (C[kk[m] + 3 * i] * C[ll[m] + 3 * j] + C[kk[m] + 3 * j] * C[ll[m] + 3 * i]);
+        }
+      }
+      if (valid) {
+        double2* oe = reinterpret_cast<double2*>(o + (size_t)e * KS);
+        oe[0] = make_double2(v[0], v[1]);
+        oe[1] = make_double2(v[2], v[3]);
+        oe[2] = make_double2(v[4], v[5]);
+      }
+    }
+    // antisymmetric rows (i, j): f (B_ki B_lj - B_kj B_li) = (-1)^(i+j+k+l) (f / det) J(n, m), n and m
+    // the indices that are not in (i, j) and (k, l)
+    const double ha = 0.5 * (lambda - mu) * (neg && det < 0.0 ? -w : w);
+    double* oa = GA + (size_t)cl * 3 * KA + 3 * q;
+#pragma unroll
+    for (int e = 0; e < 3; ++e)
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        const double v = ((e + m) & 1) ? -ha * J[(2 - e) + 3 * (2 - m)] : ha * J[(2 - e) + 3 * (2 - m)];
+        if (valid) oa[(size_t)e * KA + m] = v;
+      }
+  }
+  __syncwarp();
+  // element vector, source part
+  for (int comp = 0; comp < 3; ++comp) {
+    const bool zero = src.fn == FG_FN_ZERO || (src.fn == FG_FN_CONST && src.prm[comp] == 0.0) ||
+                      (src.fn != FG_FN_CONST && src.fn != FG_FN_QP_VALUES);
+    double* out = EV + (c * 3 + comp) * NN;
+    if (zero) {
+      for (int a = gl; a < NN; a += T::GL)
+        if (valid) out[a] = 0.0;
+      continue;
+    }
+    // the sum destroys its input: weighted source values into the cell's line buffer
+    double* fs = D;  // D and Jt (36 + 9 NC2 >= NQ doubles) are spent
+    for (int q = gl; q < NQ; q += T::GL)
+      fs[q] = f[q] * (src.fn == FG_FN_QP_VALUES ? src.qp[(c * NQ + q) * 3 + comp] : src.prm[comp]);
+    __syncwarp();
+    geo_load_vector<P>(L1, gl, fs, t, valid, out);
+  }
+}
+
+// products -> staged element matrices (Dirichlet columns zero) and the strong-Dirichlet lifting
+// in column order; a block per cell
+template <int P>
+__global__ void __launch_bounds__(256)
+    k_elasticity_unpack(AsmGeom g, int64_t cell0, const int32_t* __restrict__ latdof, const double* __restrict__ gvals,
+                        const double* __restrict__ CS, const double* __restrict__ CA, double* __restrict__ E,
+                        double* __restrict__ EV) {
+  using T = ElastTC<P>;
+  constexpr int NN = T::NN, ND = T::ND, NPAIR = T::NPAIR;
+  __shared__ int32_t gid[ND];
+  const int64_t c = cell0 + blockIdx.x;
+  const int ci = (int)(c % g.n[0]);
+  const int cj = (int)((c / g.n[0]) % g.n[1]);
+  const int ck = (int)(c / ((int64_t)g.n[0] * g.n[1]));
+  bool dir = false;
+  for (int s = threadIdx.x; s < ND; s += blockDim.x) {
+    gid[s] = latdof[asm_node<P>(g, c, ci, cj, ck, s % NN) * 3 + s / NN];
+    dir |= gid[s] < 0;
+  }
+  const bool any_dir = __syncthreads_or(dir) != 0;
+  const double* cs = CS + (size_t)blockIdx.x * 6 * NPAIR;
+  const double* ca = CA + (size_t)blockIdx.x * 3 * NPAIR;
+  auto entry = [&](int a, int u, int b, int v) {
+    if (a > b) {
+      const int ta = a, tu = u;
+      a = b; u = v;
+      b = ta; v = tu;
+    }
+    const int p = a * NN - a * (a - 1) / 2 + (b - a);
+    if (u == v) return cs[u * NPAIR + p];
+    const int e = u + v - 1;  // (0,1) (0,2) (1,2)
+    const double x = cs[(3 + e) * NPAIR + p], y = ca[e * NPAIR + p];
+    return u < v ? x + y : x - y;
+  };
+  double* Ec = E + (size_t)c * ND * ND;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int i = w; i < ND; i += 8) {
+    const int a = i % NN, u = i / NN;
+    for (int j = lane; j < ND; j += 32) Ec[(size_t)i * ND + j] = gid[j] < 0 ? 0.0 : entry(a, u, j % NN, j / NN);
+  }
+  if (!any_dir) return;
+  for (int i = threadIdx.x; i < ND; i += blockDim.x) {
+    double ev = EV[c * ND + i];
+    for (int j = 0; j < ND; ++j) {
+      const int32_t gj = gid[j];
+      if (gj < 0) ev = ev - entry(i % NN, i / NN, j % NN, j / NN) * gvals[-gj - 1];
+    }
+    EV[c * ND + i] = ev;
+  }
+}
+
+// scratch of the elasticity products per cell, and the cells of one chunk: the scratch stays
+// within kElastScratch bytes
+static constexpr size_t kElastScratch = (size_t)2 << 30;
+template <int P>
+static size_t elast_cell_bytes() {
+  using T = ElastTC<P>;
+  const size_t ks = (T::KS + 15) / 16 * 16, ka = (T::KA + 15) / 16 * 16;
+  return sizeof(double) * (6 * T::KS + 3 * T::KA + 9 * T::NPAIR) + 16 * std::max(6 * ks, 3 * ka) + 64;
+}
+size_t elasticity_tc_scratch(int order, int64_t ncells) {
+  if (order < 2) return 0;
+  const size_t per = order == 2 ? elast_cell_bytes<2>() : elast_cell_bytes<3>();
+  return std::min(per * (size_t)ncells, kElastScratch) + (16u << 20);
+}
+
+template <int P>
+static fg_status elasticity_element_matrices_tc(fg_system* sys) {
+  using T = ElastTC<P>;
+  using Geo = CellGeo<P>;
+  fg_space* sp = sys->space;
+  fg_ctx* ctx = sp->mesh->ctx;
+  cudaStream_t st = ctx->stream;
+  const int64_t ncells = sp->mesh->ncells;
+  FG_TRY(ensure_pair_table<P>(sp));
+  FG_TRY(ensure_geo_table<P>(sp));
+  if (!sp->d_tcA) {
+    std::vector<double> h((size_t)T::NPAIR * T::KA);
+    const std::vector<double>& r = sp->tab.shg;  // (a NQ + q) 3 + j, the scalar shapes
+    size_t p = 0;
+    for (int a = 0; a < T::NN; ++a)
+      for (int b = a; b < T::NN; ++b, ++p)
+        for (int q = 0; q < T::NQ; ++q) {
+          const double* ra = &r[((size_t)a * T::NQ + q) * 3];
+          const double* rb = &r[((size_t)b * T::NQ + q) * 3];
+          double* t = &h[p * T::KA + 3 * q];
+          t[0] = ra[0] * rb[1] - ra[1] * rb[0];
+          t[1] = ra[0] * rb[2] - ra[2] * rb[0];
+          t[2] = ra[1] * rb[2] - ra[2] * rb[1];
+        }
+    FG_TRY(dev_alloc(ctx, (void**)&sp->d_tcA, sizeof(double) * h.size()));
+    FG_CUDA_TRY(cudaMemcpyAsync(sp->d_tcA, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, st));
+    FG_CUDA_TRY(cudaStreamSynchronize(st));
+  }
+  const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>(ncells, (int64_t)(kElastScratch / elast_cell_bytes<P>())));
+  const size_t gs = tc_align(sizeof(double) * chunk * 6 * T::KS), ga = tc_align(sizeof(double) * chunk * 3 * T::KA);
+  const size_t cs = tc_align(sizeof(double) * chunk * 6 * T::NPAIR), ca = tc_align(sizeof(double) * chunk * 3 * T::NPAIR);
+  const size_t wb = tc_align(std::max(ozaki_workspace_bytes(chunk * 6, T::NPAIR, T::KS, false, 8),
+                                      ozaki_workspace_bytes(chunk * 3, T::NPAIR, T::KA, false, 8)));
+  const size_t need = gs + ga + cs + ca + wb + 256;
+  if (!sys->d_tcbuf || sys->tcbuf_bytes < need) {
+    dev_free(ctx, sys->d_tcbuf);
+    sys->d_tcbuf = nullptr;
+    sys->tcbuf_bytes = 0;
+    FG_TRY(dev_alloc(ctx, &sys->d_tcbuf, need));
+    sys->tcbuf_bytes = need;
+  }
+  uint8_t* buf = (uint8_t*)sys->d_tcbuf;
+  double *GS = (double*)buf, *GA = (double*)(buf + gs), *CS = (double*)(buf + gs + ga), *CA = (double*)(buf + gs + ga + cs);
+  void* work = buf + gs + ga + cs + ca;
+  int* d_err = (int*)((uint8_t*)work + wb);
+  AsmGeom g = make_geom(sp);
+  SourceSpec src;
+  src.fn = sys->integ.source_fn;
+  for (int i = 0; i < 8; ++i) src.prm[i] = sys->integ.fn_param[i];
+  src.qp = sys->d_qpsrc;
+  FG_CUDA_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), st));
+  FG_CUDA_TRY(cudaFuncSetAttribute((const void*)k_elasticity_geom<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)Geo::SMEM));
+  for (int64_t c0 = 0; c0 < ncells; c0 += chunk) {
+    const int64_t nc = std::min(chunk, ncells - c0);
+    k_elasticity_geom<P><<<nblk(nc, Geo::CELLS), Geo::WARPS * 32, Geo::SMEM, st>>>(
+        g, c0, nc, sp->mesh->d_coords, sp->d_tcgeo, sys->d_coef, sys->integ.coef_const, sys->integ.nu, src, GS, GA,
+        sys->d_elvec);
+    FG_CUDA_TRY(cudaGetLastError());
+    FG_TRY(ozaki_gemm_nt(ctx, st, nc * 6, T::NPAIR, T::KS, 1.0, GS, T::KS, 1, sp->d_tcT, T::KS, 1, 0.0, CS, T::NPAIR, 1,
+                         false, work, d_err, 8));
+    FG_TRY(ozaki_gemm_nt(ctx, st, nc * 3, T::NPAIR, T::KA, 1.0, GA, T::KA, 1, sp->d_tcA, T::KA, 1, 0.0, CA, T::NPAIR, 1,
+                         false, work, d_err, 8));
+    k_elasticity_unpack<P><<<(unsigned)nc, 256, 0, st>>>(g, c0, sp->d_latdof, sys->d_gvals, CS, CA, sys->d_elmat,
+                                                         sys->d_elvec);
+    FG_CUDA_TRY(cudaGetLastError());
+    ctx->launches += 2;
+  }
+  int h_err = 0;
+  FG_CUDA_TRY(cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+  FG_CUDA_TRY(cudaStreamSynchronize(st));
+  if (h_err) {
+    set_error("element matrices on the tensor cores: a bounded device wait ran out");
+    return (fg_status)h_err;
+  }
+  return FG_OK;
+}
+
 template <int P>
 static fg_status launch_elasticity(fg_system* sys) {
   using S = ElastShape<P>;
@@ -1424,14 +1840,28 @@ static fg_status launch_elasticity(fg_system* sys) {
   src.fn = sys->integ.source_fn;
   for (int i = 0; i < 8; ++i) src.prm[i] = sys->integ.fn_param[i];
   src.qp = sys->d_qpsrc;
-  const size_t smem = S::SM_BYTES_WARP * S::WARPS;
-  // per call: the attribute is per device, and server workers assemble concurrently
-  FG_CUDA_TRY(cudaFuncSetAttribute(k_integrate_elasticity<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  ctx->launches += sp->nfree > 0 ? 2 : 1;
-  k_integrate_elasticity<P><<<nblk(ncells, S::WARPS), S::WARPS * 32, smem, ctx->stream>>>(
-      g, ncells, sp->mesh->d_coords, sp->dtab, sp->d_latdof, sys->d_gvals, sys->d_coef, sys->integ.coef_const,
-      sys->integ.nu, src, sys->d_elmat, sys->d_elvec);
-  FG_CUDA_TRY(cudaGetLastError());
+  // Q2 and Q3 on the tensor cores unless FG_TC_INTEGRATION=0 or the HBM budget has no room for the
+  // scratch.  Per assembly, FP64 pipe against tensor cores: Q2 225 / 173 us for one cell, 0.60 /
+  // 0.31 ms at 10^3, 5.9 / 2.5 ms at 24^3; Q3 1.8 / 0.28 ms, 7.7 / 2.0 ms at 10^3; Q1 102 / 173 us at
+  // 10^3 and 0.47 / 0.51 ms at 24^3: it stays on the FP64 pipe.
+  fg_status tc = FG_ERR_OOM;
+  if constexpr (P >= 2) {
+    if (tc_integration_mode() >= 1 && ncells > 0) {
+      tc = elasticity_element_matrices_tc<P>(sys);
+      if (tc != FG_OK && tc != FG_ERR_OOM) return tc;
+    }
+  }
+  if (tc == FG_ERR_OOM) {
+    const size_t smem = S::SM_BYTES_WARP * S::WARPS;
+    // per call: the attribute is per device, and server workers assemble concurrently
+    FG_CUDA_TRY(cudaFuncSetAttribute(k_integrate_elasticity<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_integrate_elasticity<P><<<nblk(ncells, S::WARPS), S::WARPS * 32, smem, ctx->stream>>>(
+        g, ncells, sp->mesh->d_coords, sp->dtab, sp->d_latdof, sys->d_gvals, sys->d_coef, sys->integ.coef_const,
+        sys->integ.nu, src, sys->d_elmat, sys->d_elvec);
+    FG_CUDA_TRY(cudaGetLastError());
+    ctx->launches += 1;
+  }
+  ctx->launches += sp->nfree > 0 ? 1 : 0;
   const int64_t n = sp->nfree;
   if (sp->explicit_nodes) return usystem_scatter(sys);
   sys->direct = false;

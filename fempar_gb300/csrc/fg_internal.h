@@ -157,6 +157,8 @@ struct fg_space {
   int st_max_bp = 0;              // largest Bp of the classes
   std::vector<fg::StencilClass> h_st_cls;
   double* d_tcT = nullptr;        // Poisson element tensor T (upper pairs x 6 NQ), tensor-core path
+  double* d_tcA = nullptr;        // antisymmetric element tensor (upper pairs x 3 NQ), elasticity
+  double* d_tcgeo = nullptr;      // line weights, 1D shapes and quadrature weights of its geometry kernels
   float* d_tcff = nullptr;        // float-float tables of its fast-integration geometry kernel
   // unstructured mesh: nodes (nlat of them) are vertices, edge, face and cell interior nodes
   int32_t* d_cellnode = nullptr;  // nn*ncells node ids
@@ -230,6 +232,8 @@ fg_status space_export_upper(fg_space* sp, const double* d_val, int one_based, i
 fg_status system_interpolate_dirichlet(fg_system* sys, int boundary_fn, const double* prm);
 fg_status system_assemble(fg_system* sys);
 fg_status space_qp_coords(fg_space* sp, double* d_xyz);
+// device scratch of the elasticity element matrices on the tensor cores (upper bound)
+size_t elasticity_tc_scratch(int order, int64_t ncells);
 
 fg_status scan_i64(fg_ctx* ctx, int64_t* a, int64_t n, int64_t* total);
 fg_status space_count_upper(fg_space* sp);
@@ -281,11 +285,13 @@ fg_status system_solve(fg_system* sys, const fg_solver_params* prm, const double
 
 // Dense FP64 product on the bf16 tensor cores (fg_ozaki.cu): C = alpha A B^T + beta C,
 // B == nullptr means B = A; work holds ozaki_workspace_bytes(m, n, k, B == nullptr) bytes;
-// d_err receives FG_ERR_TIMEOUT if a bounded device wait ran out.
-size_t ozaki_workspace_bytes(int64_t m, int64_t n, int64_t k, bool same);
+// d_err receives FG_ERR_TIMEOUT if a bounded device wait ran out.  digits: 7, or 8 (62 bits below
+// a row's maximum instead of 54).
+size_t ozaki_workspace_bytes(int64_t m, int64_t n, int64_t k, bool same, int digits = 7);
 fg_status ozaki_gemm_nt(fg_ctx* ctx, cudaStream_t st, int64_t m, int64_t n, int64_t k, double alpha,
                         const double* A, int64_t a_rs, int64_t a_cs, const double* B, int64_t b_rs, int64_t b_cs,
-                        double beta, double* C, int64_t c_rs, int64_t c_cs, bool lower, void* work, int* d_err);
+                        double beta, double* C, int64_t c_rs, int64_t c_cs, bool lower, void* work, int* d_err,
+                        int digits = 7);
 // A batch of lower rank-k updates C_b -= P_b P_b^T (k_b <= 128, column-major with leading
 // dimension ld_b), in one launch of each kernel; work holds ozaki_syrk_batch_bytes(b) bytes.
 struct OzSyrk {

@@ -24,6 +24,10 @@
 //     dropped (|error| <~ K 2^-57 max_l |x_il| max_l |y_jl|).  The cut keeps 54 bits below
 //     the row maximum, so a value far below it loses its low bits: overall the product is
 //     within ~K 2^-52 max|x_i.| max|y_j.| of the exact one (about the FP64 dot-product bound);
+//   * with S = 8 digits (the elasticity element matrices) the cut keeps 62 bits below the row
+//     maximum and the error left is that of the dropped pairs, ~50 times smaller than the cut's
+//     at S = 7 (36 pairs instead of 34; a class 7 sum could pass 2^24 by 11 % if every digit were
+//     extreme, and would then round in its last bit, below what the dropped pairs leave out);
 //   * the epilogue converts the 8 class sums to integers, combines them exactly (H 2^-24 +
 //     L 2^-56), turns the chunk's sum into FP64 with one rounding (two exact bit patterns, one
 //     addition), adds the K chunks in FP64, applies the power of two 2^(e_i + f_j - 16) through
@@ -67,13 +71,13 @@ namespace fg {
 
 namespace {
 
-constexpr int OZ_S = 7;                       // digits per value
+constexpr int OZ_S = 7;                       // digits per value (8 where asked for)
 constexpr int OZ_NACC = 8;                    // accumulators: digit weights k = s + t = 0..7
 constexpr int OZ_BM = 128, OZ_BK = 16;
 constexpr int OZ_KEXACT = 170;                // K values one exact accumulation may sum
 constexpr int OZ_CHUNK_STEPS = 10;            // K steps of a chunk when K > OZ_KEXACT (160 values)
 constexpr uint32_t OZ_BLOCK = OZ_BM * OZ_BK * 2;           // one digit block: 4096 B
-constexpr uint32_t OZ_A_BYTES = OZ_S * OZ_BLOCK;           // 28672 B per K step
+constexpr uint32_t oz_a_bytes(int S) { return S * OZ_BLOCK; }  // a row tile's digits per K step
 constexpr uint32_t OZ_TMEM_COLS = 512;                     // all of it
 constexpr long long OZ_WAIT_CYCLES = 1ll << 31;            // ~1 s at 2 GHz
 constexpr int OZ_EPI_WARPS = 16;                           // epilogue warps: 4 per TMEM lane quarter
@@ -81,14 +85,15 @@ constexpr int OZ_THREADS = (OZ_EPI_WARPS + 2) * 32;        // with the MMA warp 
 
 // Output tiles of 128 x BN: the 8 accumulators of BN = 64 columns fill the tensor memory.
 constexpr int OZ_BN = 64;
-template <int BN>
+template <int BN, int S>
 struct OzT {
   static constexpr int NSET = (int)OZ_TMEM_COLS / (OZ_NACC * BN);
   static constexpr int EPI = BN * 4 / OZ_EPI_WARPS;           // columns per epilogue thread
   static constexpr int QB = OZ_BM / BN;                       // B tiles per 128-row digit block
   static constexpr uint32_t B_DIGIT = BN * OZ_BK * 2;         // one digit of a B tile per K step
-  static constexpr uint32_t STAGE = OZ_A_BYTES + OZ_S * B_DIGIT;
-  static constexpr int NBUF = 5;                              // stages: 215040 B
+  static constexpr uint32_t A_BYTES = oz_a_bytes(S);
+  static constexpr uint32_t STAGE = A_BYTES + S * B_DIGIT;
+  static constexpr int NBUF = S == 7 ? 5 : 4;                 // stages: 215040 or 196608 B
   static constexpr uint32_t SMEM = NBUF * STAGE;
   // kind::f16: FP32 accumulator, bf16 A and B, both K-major, N = BN, M = 128
   static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
@@ -272,18 +277,19 @@ __global__ void __launch_bounds__(OZ_BM) k_oz_rowexp(OzSplitArgs a) {
   }
 }
 
-// Digits: block (digit row tile, K step), thread per row; 16 values, 7 digits each, written as
-// the 7 digit blocks' 32-byte rows.  Rows past the item and columns >= k are zero.
+// Digits: block (digit row tile, K step), thread per row; 16 values, S digits each, written as
+// the S digit blocks' 32-byte rows.  Rows past the item and columns >= k are zero.
+template <int S>
 __global__ void __launch_bounds__(OZ_BM) k_oz_split(OzSplitArgs a) {
   const int tid = threadIdx.x;
   const int rtile = blockIdx.x, ks = blockIdx.y;
   const OzSplit it = split_of(a, rtile);
   const int64_t r = (int64_t)(rtile - it.rtile0) * OZ_BM + tid;
   const int er = a.ex[(int64_t)rtile * OZ_BM + tid];
-  uint32_t w[OZ_S][8];
+  uint32_t w[S][8];
 #pragma unroll
   for (int c = 0; c < OZ_BK; c += 2) {
-    int32_t d[2][OZ_S];
+    int32_t d[2][S];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int64_t l = (int64_t)ks * OZ_BK + c + h;
@@ -291,31 +297,31 @@ __global__ void __launch_bounds__(OZ_BM) k_oz_split(OzSplitArgs a) {
       const unsigned long long b = (unsigned long long)__double_as_longlong(v);
       const int E = (int)((b >> 52) & 0x7FF);
       const long long mant = (long long)(b & 0xFFFFFFFFFFFFFull) | (E ? (1ll << 52) : 0ll);
-      // F = |v| 2^(56 - e_r) as an integer: v = mant 2^(max(E,1) - 1075)
-      const int sh = (E ? E : 1) - 1019 - er;  // <= 1 by the choice of e_r: F < 2^54
+      // F = |v| 2^(8 S - e_r) as an integer: v = mant 2^(max(E,1) - 1075)
+      const int sh = (E ? E : 1) - 1075 + 8 * S - er;  // F < 2^(8 S - 2) by the choice of e_r
       long long F = sh >= 0 ? (mant << sh) : (sh > -64 ? (mant >> -sh) : 0ll);
       if (b >> 63) F = -F;
 #pragma unroll
-      for (int s = 0; s < OZ_S - 1; ++s) {
-        const int q = 48 - 8 * s;
+      for (int s = 0; s < S - 1; ++s) {
+        const int q = 8 * (S - 1 - s);
         const long long dg = (F + (1ll << (q - 1))) >> q;  // nearest digit, in [-128, 128] ([-64, 64] for s = 0)
         F -= dg << q;
         d[h][s] = (int32_t)dg;
       }
-      d[h][OZ_S - 1] = (int32_t)F;  // |F| <= 128 after six digits
+      d[h][S - 1] = (int32_t)F;  // |F| <= 128 after the others
     }
 #pragma unroll
-    for (int s = 0; s < OZ_S; ++s) {
+    for (int s = 0; s < S; ++s) {
       // small integers are exact in bf16: the upper half of their FP32 pattern
       const uint32_t lo = __float_as_uint((float)d[0][s]) >> 16;
       const uint32_t hi = __float_as_uint((float)d[1][s]) >> 16;
       w[s][c / 2] = lo | (hi << 16);
     }
   }
-  const size_t blk = ((size_t)rtile * a.ksteps + ks) * OZ_S;
+  const size_t blk = ((size_t)rtile * a.ksteps + ks) * S;
   const int g = tid >> 3, r8 = tid & 7;
 #pragma unroll
-  for (int s = 0; s < OZ_S; ++s) {
+  for (int s = 0; s < S; ++s) {
     uint4* p = a.dig + (blk + s) * (OZ_BLOCK / 16);
     p[g * 16 + r8] = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);      // columns 0-7
     p[g * 16 + 8 + r8] = make_uint4(w[s][4], w[s][5], w[s][6], w[s][7]);  // columns 8-15
@@ -402,9 +408,9 @@ __device__ __noinline__ double scale_slow(double d, int off) { return ldexp(d, o
 // Persistent: CTA b takes the output tiles b, b + gridDim.x, ... of all items (tiles above
 // the diagonal skipped when lower).  The accumulators are released as soon as the epilogue
 // has read them, so the next tile's MMAs run while the epilogue writes C.
-template <int BN>
+template <int BN, int S>
 __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
-  using T = OzT<BN>;
+  using T = OzT<BN, S>;
   constexpr int OZ_NBUF = T::NBUF;
   extern __shared__ __align__(1024) uint8_t oz_smem[];
   __shared__ __align__(8) uint64_t bar_full[OZ_MAXBUF], bar_empty[OZ_MAXBUF], bar_acc_full[2], bar_acc_empty[2];
@@ -471,7 +477,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t sa = sbase + buf * T::STAGE, sb = sa + OZ_A_BYTES;
+        const uint32_t sa = sbase + buf * T::STAGE, sb = sa + T::A_BYTES;
         const uint64_t da = smem_desc(sa), db = smem_desc(sb);
         const uint32_t tacc = tmem + z * (OZ_NACC * BN);
         const bool last = kin == g.chunk - 1 || ks == KS - 1;
@@ -479,14 +485,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
           // A digit by A digit: the digit stays in the collector buffer for its run; the first
           // pair of a class starts the chunk's sum
 #pragma unroll
-          for (int s = 0; s < OZ_S; ++s)
+          for (int s = 0; s < S; ++s)
 #pragma unroll
-            for (int kk = s; kk < OZ_NACC && kk - s < OZ_S; ++kk) {
-              const bool end = kk + 1 == OZ_NACC || kk + 1 - s == OZ_S;
+            for (int kk = s; kk < OZ_NACC && kk - s < S; ++kk) {
+              const bool end = kk + 1 == OZ_NACC || kk + 1 - s == S;
               // start-address field in 16-byte units
               const uint32_t d = tacc + kk * BN;
               const uint64_t ad = da + (uint64_t)(s * (OZ_BLOCK >> 4)), bd = db + (uint64_t)((kk - s) * (T::B_DIGIT >> 4));
-              const uint32_t acc = (kin > 0 || s > (kk > OZ_S - 1 ? kk - (OZ_S - 1) : 0)) ? 1u : 0u;
+              const uint32_t acc = (kin > 0 || s > (kk > S - 1 ? kk - (S - 1) : 0)) ? 1u : 0u;
               if (kk == s) tc_mma<COLL_FILL>(d, ad, bd, T::IDESC, acc);
               else if (!end) tc_mma<COLL_USE>(d, ad, bd, T::IDESC, acc);
               else tc_mma<COLL_LAST>(d, ad, bd, T::IDESC, acc);
@@ -511,9 +517,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
         const OzItem it = item_of(g, t);
         int rt, ct;
         it.locate(t, rt, ct);
-        const uint8_t* pa = g.dig + (size_t)(it.arow0 + rt) * KS * OZ_A_BYTES;
+        const uint8_t* pa = g.dig + (size_t)(it.arow0 + rt) * KS * T::A_BYTES;
         const uint8_t* pb =
-            g.dig + (size_t)(it.brow0 + ct / T::QB) * KS * OZ_A_BYTES + (size_t)(ct % T::QB) * T::B_DIGIT;
+            g.dig + (size_t)(it.brow0 + ct / T::QB) * KS * T::A_BYTES + (size_t)(ct % T::QB) * T::B_DIGIT;
         for (int ks = 0; ks < KS; ++ks, ++gs) {
           const int buf = gs % OZ_NBUF;
           if (gs >= OZ_NBUF && !mbar_wait(smem_u32(&bar_empty[buf]), ((gs / OZ_NBUF) - 1) & 1, &abort_flag, g.err)) {
@@ -524,9 +530,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
           const uint32_t dst = sbase + buf * T::STAGE;
           mbar_expect_tx(full, T::STAGE);
           if (blockIdx.x == 0 && gs == g.drop_stage) continue;
-          bulk_g2s(dst, pa + (size_t)ks * OZ_A_BYTES, OZ_A_BYTES, full);
-          for (int d = 0; d < OZ_S; ++d)
-            bulk_g2s(dst + OZ_A_BYTES + d * T::B_DIGIT, pb + ((size_t)ks * OZ_S + d) * OZ_BLOCK, T::B_DIGIT, full);
+          bulk_g2s(dst, pa + (size_t)ks * T::A_BYTES, T::A_BYTES, full);
+          for (int d = 0; d < S; ++d)
+            bulk_g2s(dst + T::A_BYTES + d * T::B_DIGIT, pb + ((size_t)ks * S + d) * OZ_BLOCK, T::B_DIGIT, full);
         }
       }
       // nothing may land in this CTA's shared memory after it is gone (an abort elsewhere leaves
@@ -666,22 +672,23 @@ __global__ void k_oz_scale(int64_t m, int64_t n, double beta, double* c, int64_t
 
 static int64_t rtiles_of(int64_t rows) { return (rows + OZ_BM - 1) / OZ_BM; }
 
-size_t ozaki_workspace_bytes(int64_t m, int64_t n, int64_t k, bool same) {
+size_t ozaki_workspace_bytes(int64_t m, int64_t n, int64_t k, bool same, int digits) {
   const int64_t rt = rtiles_of(m) + (same ? 0 : rtiles_of(n));
   const int64_t ks = std::max<int64_t>(1, (k + OZ_BK - 1) / OZ_BK);
-  return (size_t)rt * ks * OZ_A_BYTES + (size_t)rt * OZ_BM * sizeof(int32_t) + 256;
+  return (size_t)rt * ks * oz_a_bytes(digits) + (size_t)rt * OZ_BM * sizeof(int32_t) + 256;
 }
 
-template <int BN>
+template <int BN, int S>
 static fg_status oz_gemm_launch(fg_ctx* ctx, cudaStream_t st, OzGemmArgs& g, int64_t ntiles) {
-  FG_CUDA_TRY(cudaFuncSetAttribute((const void*)k_oz_gemm<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)OzT<BN>::SMEM));
+  FG_CUDA_TRY(cudaFuncSetAttribute((const void*)k_oz_gemm<BN, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)OzT<BN, S>::SMEM));
   // persistent: one CTA per SM (the shared memory allows no second), at most one per tile
-  k_oz_gemm<BN><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ntiles, ctx->sm_count)), OZ_THREADS,
-                  OzT<BN>::SMEM, st>>>(g);
+  k_oz_gemm<BN, S><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ntiles, ctx->sm_count)), OZ_THREADS,
+                  OzT<BN, S>::SMEM, st>>>(g);
   return FG_OK;
 }
 
+template <int S>
 static fg_status oz_launch(fg_ctx* ctx, cudaStream_t st, OzSplitArgs& sa, int64_t rtiles, OzGemmArgs& g,
                            int64_t ntiles) {
   // test switch for the failure-detection test: a stage whose copies never arrive makes the
@@ -689,8 +696,8 @@ static fg_status oz_launch(fg_ctx* ctx, cudaStream_t st, OzSplitArgs& sa, int64_
   const char* drop = std::getenv("FG_OZ_TEST_DROP_STAGE");
   g.drop_stage = drop ? std::atoi(drop) : -1;
   k_oz_rowexp<<<dim3((unsigned)rtiles, 32), OZ_BM, 0, st>>>(sa);
-  k_oz_split<<<dim3((unsigned)rtiles, (unsigned)sa.ksteps), OZ_BM, 0, st>>>(sa);
-  FG_TRY(oz_gemm_launch<OZ_BN>(ctx, st, g, ntiles));
+  k_oz_split<S><<<dim3((unsigned)rtiles, (unsigned)sa.ksteps), OZ_BM, 0, st>>>(sa);
+  FG_TRY((oz_gemm_launch<OZ_BN, S>(ctx, st, g, ntiles)));
   ctx->launches += 3;
   FG_CUDA_TRY(cudaGetLastError());
   return FG_OK;
@@ -699,7 +706,8 @@ static fg_status oz_launch(fg_ctx* ctx, cudaStream_t st, OzSplitArgs& sa, int64_
 // C = alpha A B^T + beta C (lower: only i >= j).  B == nullptr: B = A (same strides).
 fg_status ozaki_gemm_nt(fg_ctx* ctx, cudaStream_t st, int64_t m, int64_t n, int64_t k, double alpha,
                         const double* A, int64_t a_rs, int64_t a_cs, const double* B, int64_t b_rs, int64_t b_cs,
-                        double beta, double* C, int64_t c_rs, int64_t c_cs, bool lower, void* work, int* d_err) {
+                        double beta, double* C, int64_t c_rs, int64_t c_cs, bool lower, void* work, int* d_err,
+                        int digits) {
   if (m <= 0 || n <= 0) return FG_OK;
   if (k <= 0) {
     if (beta != 1.0) {
@@ -737,7 +745,7 @@ fg_status ozaki_gemm_nt(fg_ctx* ctx, cudaStream_t st, int64_t m, int64_t n, int6
   sa.none = same ? 1 : 2;
   sa.ksteps = (int)ksteps;
   sa.dig = (uint4*)work;
-  sa.ex = (int32_t*)((uint8_t*)work + (size_t)(rta + rtb) * ksteps * OZ_A_BYTES);
+  sa.ex = (int32_t*)((uint8_t*)work + (size_t)(rta + rtb) * ksteps * oz_a_bytes(digits));
   OzGemmArgs g;
   g.dig = (const uint8_t*)work;
   g.ex = sa.ex;
@@ -754,14 +762,15 @@ fg_status ozaki_gemm_nt(fg_ctx* ctx, cudaStream_t st, int64_t m, int64_t n, int6
   g.beta = beta;
   g.lower = lower ? 1 : 0;
   g.err = d_err;
-  return oz_launch(ctx, st, sa, rta + rtb, g, rta * tiles_n);
+  return digits == 8 ? oz_launch<8>(ctx, st, sa, rta + rtb, g, rta * tiles_n)
+                     : oz_launch<OZ_S>(ctx, st, sa, rta + rtb, g, rta * tiles_n);
 }
 
 // Batch of lower updates C_b -= P_b P_b^T, P_b m_b x k_b (k_b <= 128), all column-major.
 size_t ozaki_syrk_batch_bytes(const std::vector<OzSyrk>& b) {
   int64_t rt = 0;
   for (const auto& x : b) rt += rtiles_of(x.m);
-  return (size_t)rt * (128 / OZ_BK) * OZ_A_BYTES + (size_t)rt * OZ_BM * sizeof(int32_t) +
+  return (size_t)rt * (128 / OZ_BK) * oz_a_bytes(OZ_S) + (size_t)rt * OZ_BM * sizeof(int32_t) +
          b.size() * (sizeof(OzSplit) + sizeof(OzItem)) + 512;
 }
 
@@ -789,7 +798,7 @@ fg_status ozaki_syrk_batch(fg_ctx* ctx, cudaStream_t st, const std::vector<OzSyr
   }
   const int ksteps = 128 / OZ_BK;
   uint8_t* w = (uint8_t*)work;
-  const size_t dig_bytes = (size_t)rt * ksteps * OZ_A_BYTES;
+  const size_t dig_bytes = (size_t)rt * ksteps * oz_a_bytes(OZ_S);
   int32_t* ex = (int32_t*)(w + dig_bytes);
   uint8_t* tail = (uint8_t*)ex + (size_t)rt * OZ_BM * sizeof(int32_t);
   tail = (uint8_t*)(((uintptr_t)tail + 255) & ~(uintptr_t)255);
@@ -816,7 +825,7 @@ fg_status ozaki_syrk_batch(fg_ctx* ctx, cudaStream_t st, const std::vector<OzSyr
   g.beta = 1.0;
   g.lower = 1;
   g.err = d_err;
-  return oz_launch(ctx, st, sa, rt, g, tiles);
+  return oz_launch<OZ_S>(ctx, st, sa, rt, g, tiles);
 }
 
 }  // namespace fg

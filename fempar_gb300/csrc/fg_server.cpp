@@ -127,6 +127,8 @@ static fg_status footprint(const fg_request* q, uint64_t* bytes, int64_t* nfree_
     // packed upper triangles and the digit workspace (7 bf16 digits, K padded to 16)
     const double K = 6.0 * t.nq, npair = nd * (nd + 1) / 2;
     elm += ncells * (K * 8 + npair * 8 + std::ceil(K / 16.0) * 16 * 7 * 2) + npair * K * 8;
+  } else {
+    elm += (double)elasticity_tc_scratch(p, (int64_t)ncells);  // factors, products and digits of a chunk of cells
   }
   const double csr = nnz * (4 + 8) + nfree * 8.0;             // CSR pattern + FP64 values + row pointers
   const double lay = nnz * 1.15 * (8 + 4);                    // solver layout FP64 + FP32 (padding)

@@ -155,3 +155,37 @@ def test_budget_without_room_for_the_product_falls_back(fg, ctx, monkeypatch):
     got = matrix_rhs(opb.compute())
     assert np.array_equal(got[2], ref[2]) and np.array_equal(got[3], ref[3])
     assert cb.memory()[0] <= used_direct + (2 << 20)
+
+
+def elasticity(fg, ctx, n, order, seed=0, unstructured=False):
+    coef = np.exp(np.random.default_rng(seed + 1).normal(0.0, 1.0, size=int(np.prod(n))))
+    if unstructured:
+        import gidmesh
+        m = gidmesh.box_mesh(n, seed=seed, perturb=0.2)
+        tri = fg.SerialTriangulation.from_arrays(ctx, m["coords"], m["cells"], m["bvef_ptr"], m["bvef_verts"],
+                                                 m["bvef_set"])
+        ids = [1]
+    else:
+        tri = fg.SerialTriangulation(ctx, n, vertex_xyz=perturbed(n, 0.15, seed))
+        ids = [1, 3, 5, 7, 13, 15, 17, 19, 25]
+    sp = fg.SerialFESpace(tri, order=order, ncomp=3, dirichlet_ids=ids)
+    rng = np.random.default_rng(seed + 2)
+    integ = fg.ElasticityIntegration(cell_coef=coef, nu=0.3, source_fn=fg.FG_FN_QP_VALUES,
+                                     qp_source=rng.standard_normal(sp.num_cells * sp.qp_per_cell * 3),
+                                     dirichlet_values=rng.standard_normal(sp.num_dirichlet_dofs))
+    return tri, sp, fg.FEAffineOperator(sp, integ)
+
+
+@pytest.mark.parametrize("unstructured", [False, True])
+@pytest.mark.parametrize("n,order", [((1, 1, 1), 2), ((7, 6, 5), 2), ((4, 3, 3), 3)])
+def test_elasticity_element_matrices_match_fp64_pipe(fg, ctx, monkeypatch, n, order, unstructured):
+    """Two products, K = 6 NQ and 3 NQ per entry: the FP64 dot-product bound of 9 NQ terms (with
+    boundary data that the lifting uses; Q1 stays on the FP64 pipe)."""
+    if unstructured and n == (1, 1, 1):
+        pytest.skip("every dof of a one-cell mesh file's box is on its boundary")
+    tri, sp, op = elasticity(fg, ctx, n, order, seed=3, unstructured=unstructured)
+    monkeypatch.setenv("FG_TC_INTEGRATION", "0")
+    ref = matrix_rhs(op.compute())
+    monkeypatch.delenv("FG_TC_INTEGRATION")
+    tc = matrix_rhs(op.compute())
+    assert_close(tc, ref, 9 * (order + 1) ** 3 * 2.0 ** -52)
