@@ -26,6 +26,8 @@
 // contributions of one cell at a time; the column position comes from a binary search
 // in the row's sorted columns staged in shared memory.  No atomics: the result is
 // identical run to run.  The FP32 copy of the values is written in the same pass.
+#include <algorithm>
+
 #include "fg_internal.h"
 
 namespace fg {
@@ -951,109 +953,129 @@ __global__ void __launch_bounds__(W * 32)
 }
 
 // Row gather straight into the lattice-implicit layout: one block per slice (32 rows of one
-// class).  Each warp assembles rows of the slice in shared memory, in box-position order
-// (the column of position k is fixed by the class, so no search): the row's node sits in at
-// most 8 cells, visited in increasing cell index, and every position sums its contributions
-// in that order -- the reference's duplicate-summation order, so the values equal
-// k_scatter_rows' CSR values bit for bit.  A lane loads its column of every cell first
-// (streaming loads: each element-matrix entry is read once), then the sums run cell by cell.
-// Dirichlet columns of the element matrices are stored as zeros by the integration kernels,
-// so they add exact zeros to positions that stay zero.  The slice's 32 x Bp
-// block is then written out with consecutive threads on consecutive addresses, FP64 and
-// FP32, padding included: no clearing pass and no CSR in between.
+// class).  Each warp assembles four rows of the slice in shared memory, in box-position order:
+// the column of position k is fixed by the class, and so are a cell's place around the row's
+// node, the row's local node in that cell and the positions its columns go to, so a contribution
+// costs one add to a row base.  The row's node sits in at most 8 cells, visited in increasing
+// cell index, and every position sums its contributions in that order -- the reference's
+// duplicate-summation order, so the values equal k_scatter_rows' CSR values bit for bit.
+// Dirichlet columns of the element matrices are stored as zeros by the integration kernels, so
+// they add exact zeros to positions that stay zero.  The slice's 32 x Bp block is then written
+// out, FP64 and FP32, padding included: no clearing pass and no CSR in between.
+//
+// Bound by load latency and HBM: every element-matrix entry is read once, 216-byte rows for Q2.
+// So eight (row, cell) pairs are loaded before any is summed whatever the class (1, 2, 4 or 8
+// cells per row: 4, 4, 2 or 1 rows at once) and the slice's row ids come in one load at the
+// block's start.  64^3 Q2 1.80 -> 1.15 ms (2.8 GB read, 1.6 written), 32^3 elasticity Q2 2.78 ->
+// 1.46 ms, 23 x 17 x 21 Q3 0.285 -> 0.245 ms.  Walking the classes together along the mesh, so that
+// a cell's rows share their lines in L2, gained 3 % on the first and lost 1-7 % on the others.
 template <int P, int NC, int W, int MINB>
 __global__ void __launch_bounds__(W * 32, MINB)
     k_scatter_stencil(AsmGeom g, const uint8_t* __restrict__ scls, const int64_t* __restrict__ voff,
                       const StencilClass* __restrict__ cls,
                       const int32_t* __restrict__ slot2row, const int32_t* __restrict__ free2lat,
-                      const int32_t* __restrict__ latdof, const double* __restrict__ E, const double* __restrict__ EV,
+                      const double* __restrict__ E, const double* __restrict__ EV,
                       double* __restrict__ tval, float* __restrict__ tval32, double* __restrict__ rhs) {
-  constexpr int NP1 = P + 1, NN = NP1 * NP1 * NP1;
-  extern __shared__ double s_slice[];
-  const int64_t sl = blockIdx.x;
-  const StencilClass C = cls[scls[sl]];
-  const int Bp = C.Bp, stride = C.Bp + 4;  // +4 doubles: rows of the buffer start on shifted banks
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  for (int k = threadIdx.x; k < 32 * stride; k += W * 32) s_slice[k] = 0.0;
-  __syncthreads();
-  constexpr int ncomp = NC, ND = NN * NC;
+  constexpr int NP1 = P + 1, NN = NP1 * NP1 * NP1, ND = NN * NC, RW = 32 / W;
   constexpr int BCH = (ND + 31) / 32;  // column chunks per lane and cell
-  for (int rl = wib; rl < 32; rl += W) {
-    const int32_t r = slot2row[sl * 32 + rl];
-    if (r < 0) continue;  // padding row of the class's last slice: zeros
-    double* acc = s_slice + rl * stride;
-    const int32_t slot = free2lat[r];
-    const int64_t L = slot / ncomp;
-    const int comp = slot % ncomp;
-    const int I = (int)(L % g.Ln[0]);
-    const int J = (int)((L / g.Ln[0]) % g.Ln[1]);
-    const int K = (int)(L / ((int64_t)g.Ln[0] * g.Ln[1]));
-    int clo[3], chi[3];
-    const int IJK[3] = {I, J, K};
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const int cc = IJK[d] / P;
-      clo[d] = (IJK[d] % P == 0) ? cc - 1 : cc;
-      chi[d] = cc;
-      if (clo[d] < 0) clo[d] = 0;
-      if (chi[d] > g.n[d] - 1) chi[d] = g.n[d] - 1;
+  extern __shared__ __align__(16) double s_slice[];
+  __shared__ int4 s_row[32];  // row (-1: padding), component, first cell's x, y
+  __shared__ int s_cz[32];
+  const int64_t sl = blockIdx.x;
+  const StencilClass& C = cls[scls[sl]];
+  // cells per direction around a node of the class (2 on vertex planes) and the node's residue
+  const int Bp = C.Bp, stride = Bp + 2;  // +2 doubles: 16-byte reads of 8 rows cover all banks
+  const int w0 = C.w[0], w1 = C.w[1];
+  const int d0 = w0 == 2 * P + 1, d1 = w1 == 2 * P + 1, d2 = C.w[2] == 2 * P + 1;
+  const int ri = d0 ? 0 : -C.lo[0], rj = d1 ? 0 : -C.lo[1], rk = d2 ? 0 : -C.lo[2];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  if (threadIdx.x < 32) {
+    const int32_t r = slot2row[sl * 32 + threadIdx.x];
+    int4 m = make_int4(-1, 0, 0, 0);
+    int cz = 0;
+    if (r >= 0) {
+      const int32_t slot = free2lat[r];
+      const int L = slot / NC;
+      const int I = L % g.Ln[0], J = (L / g.Ln[0]) % g.Ln[1], K = L / (g.Ln[0] * g.Ln[1]);
+      m = make_int4(r, slot % NC, I / P - d0, J / P - d1);
+      cz = K / P - d2;
     }
-    const int nci = chi[0] - clo[0] + 1, ncj = chi[1] - clo[1] + 1, nck = chi[2] - clo[2] + 1;
-    const int ncell = nci * ncj * nck;
+    s_row[threadIdx.x] = m;
+    s_cz[threadIdx.x] = cz;
+  }
+  for (int k = threadIdx.x; k < 16 * stride; k += W * 32) reinterpret_cast<double2*>(s_slice)[k] = make_double2(0.0, 0.0);
+  __syncthreads();
+  // position of the lane's columns in the row of a cell at offset (0,0,0)
+  int posb[BCH];
+#pragma unroll
+  for (int h = 0; h < BCH; ++h) {
+    const int b = lane + 32 * h, bn = b % NN;
+    const int x = bn % NP1 - ri - P * d0 - C.lo[0], y = (bn / NP1) % NP1 - rj - P * d1 - C.lo[1],
+              z = bn / (NP1 * NP1) - rk - P * d2 - C.lo[2];
+    posb[h] = b < ND ? b / NN + NC * (x + w0 * (y + w1 * z)) : 0;
+  }
+  const int lx = d0, ly = d1, lz = d2;       // log2 of the cells per direction
+  const int lc = lx + ly + lz;               // log2 of the cells around a row
+  const int rows = RW < (8 >> lc) ? RW : (8 >> lc);  // rows per batch
+  for (int rb = 0; rb < RW; rb += rows) {
     double v[8][BCH];
-    int pos[8][BCH];
-    double evl = 0.0;  // lane q: the element-vector entry of cell q
-    // loads first (up to 8 cells x BCH columns per lane in flight), in increasing cell order
+    double evl = 0.0;  // lane q: the element-vector entry of pair q
+    const int row0 = wib * RW + rb;
+    // loads first, eight (row, cell) pairs
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
 #pragma unroll
-      for (int h = 0; h < BCH; ++h) pos[q][h] = -1;
-      if (q < ncell) {
-        const int ci = clo[0] + q % nci, cj = clo[1] + (q / nci) % ncj, ck = clo[2] + q / (nci * ncj);
-        const int64_t c = (int64_t)ci + (int64_t)g.n[0] * (cj + (int64_t)g.n[1] * ck);
-        const int a = (I - P * ci) + NP1 * ((J - P * cj) + NP1 * (K - P * ck)) + comp * NN;
-        const double* Erow = E + ((size_t)c * ND + a) * ND;
+      for (int h = 0; h < BCH; ++h) v[q][h] = 0.0;
+      const int rl = q >> lc, j = q & ((1 << lc) - 1);
+      if (rl < rows) {
+        const int4 m = s_row[row0 + rl];
+        const int ox = j & ((1 << lx) - 1), oy = (j >> lx) & ((1 << ly) - 1), oz = j >> (lx + ly);
+        const int cx = m.z + ox, cy = m.w + oy, cz = s_cz[row0 + rl] + oz;
+        if (m.x >= 0 && (unsigned)cx < (unsigned)g.n[0] && (unsigned)cy < (unsigned)g.n[1] && (unsigned)cz < (unsigned)g.n[2]) {
+          const int64_t c = (int64_t)cx + (int64_t)g.n[0] * (cy + (int64_t)g.n[1] * cz);
+          const int a = (ri + P * (d0 - ox)) + NP1 * ((rj + P * (d1 - oy)) + NP1 * (rk + P * (d2 - oz))) + m.y * NN;
+          const double* Erow = E + ((size_t)c * ND + a) * ND;
 #pragma unroll
-        for (int h = 0; h < BCH; ++h) {
-          const int b = lane + 32 * h;
-          if (b < ND) {
-            const int bnode = b % NN, bcomp = b / NN;
-            const int bi = bnode % NP1, bj = (bnode / NP1) % NP1, bk = bnode / (NP1 * NP1);
-            const int Mi = P * ci + bi, Mj = P * cj + bj, Mk = P * ck + bk;
-            // Dirichlet columns hold zeros (the integration stores them so): no lookup needed
-            pos[q][h] = bcomp + ncomp * ((Mi - I - C.lo[0]) + C.w[0] * ((Mj - J - C.lo[1]) + C.w[1] * (Mk - K - C.lo[2])));
-            v[q][h] = __ldcs(Erow + b);
-          }
+          for (int h = 0; h < BCH; ++h)
+            if (lane + 32 * h < ND) v[q][h] = __ldcs(Erow + lane + 32 * h);
+          if (lane == q) evl = EV[c * ND + a];
         }
-        if (lane == q) evl = EV[c * ND + a];
       }
     }
-    double rsum = 0.0;
+    // sums, cell by cell: the columns of one cell are distinct positions, the first cell's are
+    // still zero, and a cell outside the mesh gives zeros at positions of the row's box
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-      if (q < ncell) {
-        // the columns of one cell are distinct positions: lanes never collide within a cell
+      const int rl = q >> lc, j = q & ((1 << lc) - 1);
+      if (rl < rows) {
+        const int ox = j & ((1 << lx) - 1), oy = (j >> lx) & ((1 << ly) - 1), oz = j >> (lx + ly);
+        double* acc = s_slice + (row0 + rl) * stride + NC * P * (ox + w0 * (oy + w1 * oz));
 #pragma unroll
         for (int h = 0; h < BCH; ++h)
-          if (pos[q][h] >= 0) acc[pos[q][h]] = acc[pos[q][h]] + v[q][h];
-        rsum = rsum + __shfl_sync(0xffffffffu, evl, q);
-        __syncwarp();
+          if (lane + 32 * h < ND) acc[posb[h]] = j == 0 ? v[q][h] : acc[posb[h]] + v[q][h];
       }
+      __syncwarp();
     }
-    if (lane == 0) rhs[r] = rsum;
+    // right-hand side: lane = row of the batch, its cells in order
+    double rsum = 0.0;
+    for (int j = 0; j < (1 << lc); ++j) rsum = rsum + __shfl_sync(0xffffffffu, evl, ((lane << lc) + j) & 31);
+    if (lane < rows && s_row[row0 + lane].x >= 0) rhs[s_row[row0 + lane].x] = rsum;
   }
   __syncthreads();
+  // four consecutive entries of a row per thread
   const int64_t vb = voff[sl];
-  for (int k = threadIdx.x; k < 32 * Bp; k += W * 32) {
-    const int grp = k >> 7, w = k & 127;
-    const double x = s_slice[(w >> 2) * stride + grp * 4 + (w & 3)];
-    tval[vb + k] = x;
-    tval32[vb + k] = (float)x;
+  for (int k = threadIdx.x; k < 8 * Bp; k += W * 32) {
+    const double2* q = reinterpret_cast<const double2*>(s_slice + (k & 31) * stride + (k >> 5) * 4);
+    const double2 a = q[0], b = q[1];
+    double2* o = reinterpret_cast<double2*>(tval + vb + 4 * (int64_t)k);
+    o[0] = a;
+    o[1] = b;
+    *reinterpret_cast<float4*>(tval32 + vb + 4 * (int64_t)k) = make_float4((float)a.x, (float)a.y, (float)b.x, (float)b.y);
   }
 }
 
 // shared memory of k_scatter_stencil for the widest class (bytes)
-static size_t scatter_stencil_smem(const fg_space* sp) { return sizeof(double) * 32 * (size_t)(sp->st_max_bp + 4); }
+static size_t scatter_stencil_smem(const fg_space* sp) { return sizeof(double) * 32 * (size_t)(sp->st_max_bp + 2); }
 
 bool stencil_direct_ok(const fg_space* sp) {
   return sp->layout == FG_LAYOUT_STENCIL && !sp->dg && !sp->explicit_nodes && sp->mesh->dim == 3 &&
@@ -1066,17 +1088,15 @@ static fg_status launch_scatter_stencil(fg_system* sys, const AsmGeom& g) {
   fg_ctx* ctx = sp->mesh->ctx;
   constexpr int W = 8;
   const size_t smem = scatter_stencil_smem(sp);
-  // scalar Q1/Q2 rows: four blocks per SM (64 registers, a 4-byte spill; the shared slices
-  // take 4 x 34 KB).  The gather is latency-bound: at 128^3 Q2 the row gather takes ~22.5 ms
-  // at two blocks, 17.9 ms at three, ~14.5 ms at four (identical results: only the register
-  // allocation changes).  Q3 and vector rows would spill heavily.
-  constexpr int MINB = (NC == 1 && P <= 2) ? 4 : 1;
+  // scalar Q1/Q2 rows: six blocks per SM (40 registers, no spill; the shared slices take 6 x 33 KB);
+  // 64^3 Q2: 1.51 ms at four, 1.29 at five, 1.15 at six
+  constexpr int MINB = (NC == 1 && P <= 2) ? 6 : 1;
   auto kern = k_scatter_stencil<P, NC, W, MINB>;
   FG_CUDA_TRY(cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (sp->st_nslices > 0) {
     ctx->launches += 1;
     kern<<<(unsigned)sp->st_nslices, W * 32, smem, ctx->stream>>>(
-        g, sp->d_st_scls, sp->d_st_voff, sp->d_st_cls, sp->d_st_slot2row, sp->d_free2lat, sp->d_latdof, sys->d_elmat, sys->d_elvec,
+        g, sp->d_st_scls, sp->d_st_voff, sp->d_st_cls, sp->d_st_slot2row, sp->d_free2lat, sys->d_elmat, sys->d_elvec,
         sys->d_tval, sys->d_tval32, sys->d_rhs);
     FG_CUDA_TRY(cudaGetLastError());
   }
@@ -1580,7 +1600,7 @@ __global__ void __launch_bounds__(ElastShape<P>::WARPS * 32)
 // into the factors; unpacking a block entry is at most one addition.  0.92 MFLOP per Q2 cell at
 // the products' ~25 TFLOP/s against 0.18 MFLOP on the FP64 pipe's 1.05 (and the warp-per-cell
 // kernel that did that holds 73 KB of shared memory: three warps per SM).
-// 32^3 Q2 element matrices: 10.9 ms -> 2.9 ms (geometry 0.43, digits 0.28, products 1.15, unpacking 1.0).
+// 32^3 Q2 element matrices: 10.9 ms -> 2.5 ms (geometry 0.43, digits 0.30, products 1.15, unpacking 0.64).
 template <int P>
 struct ElastTC {
   static constexpr int NQ = ElastShape<P>::NQ, NN = ElastShape<P>::NN, ND = ElastShape<P>::ND;
@@ -1694,6 +1714,10 @@ __global__ void __launch_bounds__(256)
                         double* __restrict__ EV) {
   using T = ElastTC<P>;
   constexpr int NN = T::NN, ND = T::ND, NPAIR = T::NPAIR;
+  // Q2: the cell's products (27 KB) staged in shared memory by one coalesced pass; the entries of
+  // a row's columns b < a lie a row of the triangle apart
+  constexpr bool STAGED = sizeof(double) * 9 * NPAIR <= 32 * 1024;
+  __shared__ double s_c[STAGED ? 9 * NPAIR : 1];
   __shared__ int32_t gid[ND];
   const int64_t c = cell0 + blockIdx.x;
   const int ci = (int)(c % g.n[0]);
@@ -1704,9 +1728,19 @@ __global__ void __launch_bounds__(256)
     gid[s] = latdof[asm_node<P>(g, c, ci, cj, ck, s % NN) * 3 + s / NN];
     dir |= gid[s] < 0;
   }
-  const bool any_dir = __syncthreads_or(dir) != 0;
   const double* cs = CS + (size_t)blockIdx.x * 6 * NPAIR;
   const double* ca = CA + (size_t)blockIdx.x * 3 * NPAIR;
+  if (STAGED) {
+    for (int i = threadIdx.x; i < 3 * NPAIR; i += blockDim.x) {
+      const double x = __ldcs(cs + 3 * NPAIR + i), y = __ldcs(ca + i);
+      s_c[i] = __ldcs(cs + i);
+      s_c[3 * NPAIR + i] = x + y;  // once per pair, not per entry
+      s_c[6 * NPAIR + i] = x - y;
+    }
+    cs = s_c;
+    ca = s_c + 6 * NPAIR;
+  }
+  const bool any_dir = __syncthreads_or(dir) != 0;
   auto entry = [&](int a, int u, int b, int v) {
     if (a > b) {
       const int ta = a, tu = u;
@@ -1716,6 +1750,7 @@ __global__ void __launch_bounds__(256)
     const int p = a * NN - a * (a - 1) / 2 + (b - a);
     if (u == v) return cs[u * NPAIR + p];
     const int e = u + v - 1;  // (0,1) (0,2) (1,2)
+    if (STAGED) return u < v ? cs[(3 + e) * NPAIR + p] : ca[e * NPAIR + p];
     const double x = cs[(3 + e) * NPAIR + p], y = ca[e * NPAIR + p];
     return u < v ? x + y : x - y;
   };
