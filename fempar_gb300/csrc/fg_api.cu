@@ -365,6 +365,7 @@ static void space_free(fg_space* sp) {
   dev_free(ctx, sp->d_ncl);
   dev_free(ctx, sp->d_dgnbr);
   dev_free(ctx, sp->d_dgnbrface);
+  dev_free(ctx, sp->d_dgtab);
   dev_free(ctx, sp->d_st_cls);
   dev_free(ctx, sp->d_st_off);
   dev_free(ctx, sp->d_st_scls);

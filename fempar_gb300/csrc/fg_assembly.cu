@@ -13,7 +13,7 @@
 // GB300's FP64 rate (about 1 TFLOP/s) makes this stage FP64-bound; the buffer's
 // extra HBM traffic costs a few milliseconds at the 128^3 Q2 size.
 //
-// Stage 1 by default for Poisson (structured and unstructured, not dG): the element
+// Stage 1 by default for Poisson (structured, unstructured and the dG volume terms): the element
 // matrices of all cells as one emulated-FP64 tensor-core product of the cells' geometric
 // factors with a table shared by all cells (k_poisson_geom or k_poisson_geom_ff, then
 // ozaki_gemm_nt, then k_poisson_unpack with the lifting; see the comment at PoissonTC).
@@ -1279,7 +1279,9 @@ static fg_status launch_poisson_tc(fg_system* sys) {
   const int64_t ncells = sp->mesh->ncells;
   FG_TRY(ensure_pair_table<P>(sp));
   const size_t gbytes = tc_align(sizeof(double) * ncells * K), cbytes = tc_align(sizeof(double) * ncells * NPAIR);
-  const size_t wbytes = tc_align(ozaki_workspace_bytes(ncells, NPAIR, K, false));
+  // the dG volume terms were on the FP64 pipe before: eight digits keep its accuracy for Q3 too
+  const int digits = sp->dg ? 8 : 7;
+  const size_t wbytes = tc_align(ozaki_workspace_bytes(ncells, NPAIR, K, false, digits));
   const size_t need = gbytes + cbytes + wbytes + 256;
   if (!sys->d_tcbuf || sys->tcbuf_bytes < need) {
     dev_free(ctx, sys->d_tcbuf);
@@ -1333,7 +1335,8 @@ static fg_status launch_poisson_tc(fg_system* sys) {
   }
   FG_CUDA_TRY(cudaGetLastError());
   FG_CUDA_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), st));
-  FG_TRY(ozaki_gemm_nt(ctx, st, ncells, NPAIR, K, 1.0, G, K, 1, sp->d_tcT, K, 1, 0.0, Cp, NPAIR, 1, false, work, d_err));
+  FG_TRY(ozaki_gemm_nt(ctx, st, ncells, NPAIR, K, 1.0, G, K, 1, sp->d_tcT, K, 1, 0.0, Cp, NPAIR, 1, false, work, d_err,
+                       digits));
   k_poisson_unpack<P><<<nblk(ncells, 8), 256, 0, st>>>(g, ncells, sp->d_latdof, sys->d_gvals, Cp, sys->d_elmat,
                                                        sys->d_elvec);
   FG_CUDA_TRY(cudaGetLastError());
@@ -1359,7 +1362,7 @@ static fg_status launch_poisson(fg_system* sys) {
   // 130 us per assembly at 8^3, 135 vs 135 at 16^3, 179 vs 148 at 20^3; Q2 is even up to 512 cells,
   // Q3 slower from the first).  It serves fast requests too: it is the more accurate of the two.
   const bool small = P == 1 && sp->mesh->ncells <= 4096;
-  if (!sp->dg && sp->mesh->ncells > 0 && !(small && tcm == 2) && (ff ? tcm == 2 : tcm >= 1)) {
+  if (sp->mesh->ncells > 0 && !(small && tcm == 2) && (ff ? tcm == 2 : tcm >= 1)) {
     // the tensor-core path needs scratch (G, packed triangles, digits: ~7 KB per Q2 cell);
     // where the context's HBM budget has no room for it, the direct kernels run instead
     const fg_status s = launch_poisson_tc<P>(sys);

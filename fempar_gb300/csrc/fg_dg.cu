@@ -5,8 +5,8 @@
 // c*nn + a + 1); boundary data enter weakly, so there are no strong Dirichlet dofs.  The row
 // of dof (c, a) holds the dofs of c and of its face neighbours, blocks in increasing cell id.
 //
-// Numeric phase: the volume integrals come from the continuous path's cell kernel (identity
-// node table, no lifting).  Then one warp per cell owns the cell's rows: it starts from the
+// Numeric phase: the volume integrals come from the continuous path's element matrices (identity
+// node table, no lifting).  Then one block per cell owns the cell's rows: it starts from the
 // cell's element matrix and, face by face, integrates the facet terms that land in its rows
 //   interior facet, cell side I, other side J (n_1 = n, n_2 = -n, n outward of the smaller
 //   cell id, as the reference's first cell around the facet):
@@ -17,13 +17,12 @@
 //                    b(i) += w|J_F| ( -g (grad phi_i . n) + C_IP/h g phi_i )
 // with C_IP = 10 p^2 and h = min over the facet's cells of 2 (prod_i |grad xi_i|^-1)^(1/3)
 // (sbm_cell_map.i90:429-461, sbm_facet_integrator.i90:248-264).  Facet geometry per facet
-// Gauss point ((p+1)^2 points): the bilinear map of the smaller cell's face vertices gives x,
-// dx/ds, dx/dt; n = dx/ds x dx/dt, |n| the area element, n/|n| oriented outward of that
-// cell (sbm_facet_map.i90:74-128); each cell evaluates its shapes at its own reference
-// point of the facet point (the other cell through the face's shared corners).  Both cells
-// of a facet compute it in the same frame, each keeps the rows it owns: deterministic, no
-// facet matrices in HBM, no atomics.  The reference sums a diagonal entry's contributions in
-// facet id order, this kernel in local face order: entries agree to rounding.
+// Gauss point ((p+1)^2 points, sbm_facet_map.i90:74-128): |J_F| n is the cofactor row of the cell's
+// Jacobian for the face's direction, outward of the cell; the other cell evaluates its Jacobian
+// at its own reference point of the facet point (through the face's shared corners).  Each cell
+// computes its facets in its own frame and keeps the rows it owns: deterministic, no facet
+// matrices in HBM, no atomics.  The reference sums a diagonal entry's contributions in facet id
+// order, this kernel in local face order: entries agree to rounding.
 #include <cub/cub.cuh>
 
 #include "fg_internal.h"
@@ -209,267 +208,344 @@ __device__ __forceinline__ int64_t dg_vertex(const DgParams& q, int64_t c, int k
   return (ci + (k & 1)) + (nx + 1) * ((cj + ((k >> 1) & 1)) + (ny + 1) * (ck + ((k >> 2) & 1)));
 }
 
-// 1D Lagrange basis of order P on equispaced nodes of [-1,1]: values and derivatives at x
-template <int P>
-__device__ __forceinline__ void lag1d(double x, double* v, double* dv) {
-#pragma unroll
-  for (int j = 0; j <= P; ++j) {
-    const double xj = -1.0 + 2.0 * j / P;
-    double val = 1.0, der = 0.0;
-#pragma unroll
-    for (int k = 0; k <= P; ++k) {
-      if (k == j) continue;
-      const double xk = -1.0 + 2.0 * k / P;
-      const double inv = 1.0 / (xj - xk);
-      der = der * ((x - xk) * inv) + val * inv;
-      val = val * ((x - xk) * inv);
-    }
-    v[j] = val;
-    dv[j] = der;
-  }
-}
-
-// Jacobian of the trilinear map of vertices xv (8 x 3) at reference point xi: inverse (column-major,
-// b[i + 3j] = d xi_i / d x_j), determinant, and h = 2 (prod_i |grad xi_i|^-1)^(1/3)
-__device__ void dg_side_geometry(const double* xv, const double* xi, double* b, double& det, double& h) {
-  double J[9];
-  for (int j = 0; j < 3; ++j) {
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    for (int k = 0; k < 8; ++k) {
-      double g = 1.0;
-      for (int d = 0; d < 3; ++d) {
-        const double s = ((k >> d) & 1) ? 1.0 : -1.0;
-        g *= d == j ? 0.5 * s : 0.5 * (1.0 + s * xi[d]);
-      }
-      a0 = a0 + g * xv[k * 3 + 0];
-      a1 = a1 + g * xv[k * 3 + 1];
-      a2 = a2 + g * xv[k * 3 + 2];
-    }
-    J[0 + 3 * j] = a0; J[1 + 3 * j] = a1; J[2 + 3 * j] = a2;
-  }
-  const double t1 = J[4] * J[8] - J[5] * J[7];
-  const double t2 = -J[1] * J[8] + J[2] * J[7];
-  const double t3 = J[1] * J[5] - J[2] * J[4];
-  det = J[0] * t1 + J[3] * t2 + J[6] * t3;
-  const double dn = 1.0 / det;
-  b[0] = t1 * dn;
-  b[1] = t2 * dn;
-  b[2] = t3 * dn;
-  b[4] = (J[0] * J[8] - J[2] * J[6]) * dn;
-  b[5] = (-J[0] * J[5] + J[3] * J[2]) * dn;
-  b[8] = (J[0] * J[4] - J[1] * J[3]) * dn;
-  b[3] = (-J[3] * J[8] + J[5] * J[6]) * dn;
-  b[6] = (J[3] * J[7] - J[4] * J[6]) * dn;
-  b[7] = (-J[0] * J[7] + J[1] * J[6]) * dn;
-  double ih[3];
-  for (int i = 0; i < 3; ++i) {
-    double s = 0.0;
-    for (int j = 0; j < 3; ++j) s = s + b[i + 3 * j] * b[i + 3 * j];
-    ih[i] = sqrt(s);
-  }
-  const double vh = 1.0 / (ih[0] * ih[1] * ih[2]);
-  h = 2.0 * pow(vh, 1.0 / 3.0);
-}
-
+// A block owns a cell's rows.  The facet terms of its rows, in the cell's own frame of each face
+// (tangential directions 0 and 1, layers l of nodes along the normal):
+//  * on a face a shape function is nonzero only for the face's nodes, where it is the 2D shape
+//    Phi_alpha; its gradient has the tangential parts there too and a normal part
+//    L_l'(+-1) Phi_alpha in every layer;
+//  * with w = w_q |J_F| J^-1 n per side (tangential w_0, w_1, normal w_n) the facet therefore needs
+//    five (p+1)^2 x (p+1)^2 matrices, sums over its Gauss points of Phi_alpha(q) times
+//      N: w_n Phi_beta   M: pen Phi_beta   T: w_0 d_0 Phi_beta + w_1 d_1 Phi_beta
+//    and N, T of the other side (its nodes renumbered into this frame), and every entry of the
+//    diagonal and neighbour blocks is a combination of at most five of their entries.
+// That is ~5 (p+1)^6 FMAs per face where summing all node pairs took 8 (p+1)^8.  The geometry of
+// all 6 (p+1)^2 facet points is computed at once, a thread per point and side (three threads did
+// it point after point: an FP64 warp instruction holds the SM's FP64 pipe for 16 cycles however
+// few lanes are active).  n |J_F| is a cofactor row of J, so no normalisation is needed.
+// FP64-bound; 32^3 Q2: 66.1 -> 3.9 ms.
 template <int P>
 struct DgShape {
-  static constexpr int NP1 = P + 1, NN = NP1 * NP1 * NP1, NQF = NP1 * NP1;
-  static constexpr int WARPS = P == 3 ? 1 : (P == 2 ? 4 : 8);
-  // per warp: D, O (NN*NN), rv (NN), V[2][NN], A[2][NN], xv[3][24], misc[40], 1D tables[2][3][4][2]
-  static constexpr int DOUBLES = 2 * NN * NN + NN + 2 * NN + 2 * NN + 72 + 40 + 48;
-  static constexpr size_t BYTES_WARP = (size_t)DOUBLES * 8;
+  static constexpr int NP1 = P + 1, NN = NP1 * NP1 * NP1, NQF = NP1 * NP1, NF = NQF * NQF, NG = 6 * NQF;
+  static constexpr int NT = P == 1 ? 32 : (P == 2 ? 96 : 256);
+  // table: Phi, d_0 Phi, d_1 Phi [node][point], L'(-1), L'(1)
+  static constexpr int TAB = 3 * NF + 2 * NP1;
+  // D, O, r, vertices and edge differences of 7 cells, per facet point n[3], own w[3], other
+  // w[3], pen, s; five scaled tables
+  static constexpr int DOUBLES = TAB + 2 * NN * NN + NN + 7 * (24 + 36) + 11 * NG + 5 * NF;
+  static constexpr size_t SMEM = sizeof(double) * DOUBLES;
 };
 
+// J of the trilinear map at xi from the 12 edge differences (3 directions x 4 edges), its cofactors
+// C[k][i] = det d xi_k / d x_i and determinant
+__device__ __forceinline__ double dg_cofactors(const double* ed, const double* xi, double (&C)[3][3]) {
+  double J[3][3];  // [d][i] = d x_i / d xi_d
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double a = xi[d == 0 ? 1 : 0], b = xi[d == 2 ? 1 : 2];
+    const double am = 0.125 * (1.0 - a), ap = 0.125 * (1.0 + a), bm = 1.0 - b, bp = 1.0 + b;
+    const double w[4] = {am * bm, ap * bm, am * bp, ap * bp};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      double v = 0.0;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v = fma(w[e], ed[d * 12 + e * 3 + i], v);
+      J[d][i] = v;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int u = (k + 1) % 3, v = (k + 2) % 3;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const int x = (i + 1) % 3, y = (i + 2) % 3;
+      C[k][i] = J[u][x] * J[v][y] - J[u][y] * J[v][x];
+    }
+  }
+  return J[0][0] * C[0][0] + J[0][1] * C[0][1] + J[0][2] * C[0][2];
+}
+// prod_k |grad xi_k|^2
+__device__ __forceinline__ double dg_grad_product(const double (&C)[3][3], double inv) {
+  double s = 1.0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) s *= (C[k][0] * C[k][0] + C[k][1] * C[k][1] + C[k][2] * C[k][2]) * (inv * inv);
+  return s;
+}
+
 template <int P>
-__global__ void __launch_bounds__(DgShape<P>::WARPS * 32)
-    k_dg_rows(int64_t nc, DgParams q, const double* __restrict__ coords, const int32_t* __restrict__ nbr,
-              const int8_t* __restrict__ nbrface, const double* __restrict__ E, const double* __restrict__ EV,
-              const int64_t* __restrict__ rowptr, double* __restrict__ val, float* __restrict__ val32,
-              double* __restrict__ rhs) {
+__global__ void __launch_bounds__(DgShape<P>::NT)
+    k_dg_rows(int64_t nc, DgParams q, const double* __restrict__ table, const double* __restrict__ coords,
+              const int32_t* __restrict__ nbr, const int8_t* __restrict__ nbrface, const double* __restrict__ E,
+              const double* __restrict__ EV, const int64_t* __restrict__ rowptr, double* __restrict__ val,
+              float* __restrict__ val32, double* __restrict__ rhs) {
   using S = DgShape<P>;
-  constexpr int NP1 = S::NP1, NN = S::NN, NQF = S::NQF;
+  constexpr int NP1 = S::NP1, NN = S::NN, NQF = S::NQF, NF = S::NF, NG = S::NG, NT = S::NT;
   extern __shared__ double sm[];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  double* D = sm + (size_t)wib * (S::BYTES_WARP / 8);
+  double* Phi = sm;             // [node][point]
+  double* D0 = Phi + NF;
+  double* D1 = D0 + NF;
+  double* dL = D1 + NF;         // [side][layer]
+  double* D = dL + 2 * NP1;
   double* O = D + NN * NN;
   double* rv = O + NN * NN;
-  double* sval = rv + NN;        // [2][NN] shape values of both sides
-  double* sA = sval + 2 * NN;    // [2][NN] scaled normal derivatives of both sides
-  double* xv = sA + 2 * NN;      // [3][24]: (unused), left cell, right cell
-  double* misc = xv + 72;        // n[0..2], factor[3], g[5], b[2][9] at 6, xi[2][3] at 24, h[2] at 30, det at 32,
-                                 // B n per side at 33..38
-  double* tab = misc + 40;       // [side][dir][j][value, derivative] of the 1D basis
-  const int64_t c = (int64_t)blockIdx.x * S::WARPS + wib;
-  if (c >= nc) return;
-  for (int t = lane; t < NN * NN; t += 32) D[t] = E[(size_t)c * NN * NN + t];
-  for (int t = lane; t < NN; t += 32) rv[t] = EV[c * NN + t];
-  int64_t blk[7];
-  const int nb = dg_blocks(c, nbr, blk);
-  __syncwarp();
-  for (int lf = 0; lf < 6; ++lf) {
+  double* xv = rv + NN;         // [7][24]
+  double* ed = xv + 7 * 24;     // [7][36]
+  double* gn = ed + 7 * 36;     // [NG][3] |J_F| n, outward
+  double* gw = gn + 3 * NG;     // [NG][3] own side: tangential 0, 1, normal
+  double* go = gw + 3 * NG;     // [NG][3] other side in this frame
+  double* gp = go + 3 * NG;     // [NG] pen
+  double* gs = gp + NG;         // [NG] gradient product of the own side; boundary value
+  double* pre = gs + NG;        // [5][node][point]
+  __shared__ int s_o[6], s_ax[6], s_k[6];  // neighbour, packed orientation, block of the neighbour
+  __shared__ int s_nb, s_kc;
+  const int tid = threadIdx.x;
+  const int64_t c = blockIdx.x;
+  for (int i = tid; i < S::TAB; i += NT) sm[i] = table[i];
+  for (int i = tid; i < NN * NN; i += NT) D[i] = E[(size_t)c * NN * NN + i];
+  for (int i = tid; i < NN; i += NT) rv[i] = EV[c * NN + i];
+  // orientation of each neighbour: its face axes in this cell's face frame, through the shared corners
+  if (tid < 6) {
+    const int lf = tid;
     const int64_t o = nbr[c * 6 + lf];
-    const bool boundary = o < 0;
-    const int64_t left = boundary ? c : (o < c ? o : c);
-    const int64_t right = boundary ? -1 : (o < c ? c : o);
-    const int flf = boundary ? lf : (o < c ? nbrface[c * 6 + lf] : lf);  // left cell's local face
-    const int I = (left == c) ? 0 : 1;
-    int ld1, ld2, ldn, la;
-    dg_face(flf, ld1, ld2, ldn, la);
-    // vertex coordinates of the left and right cells
-    for (int t = lane; t < 48; t += 32) {
-      const int side = t / 24, k = (t % 24) / 3, l = t % 3;
-      const int64_t cc = side == 0 ? left : right;
-      if (cc >= 0) xv[24 + t] = coords[dg_vertex(q, cc, k) * 3 + l];
-    }
-    // right cell's face axes in the left face's frame, through the shared corners
-    int raxis[2] = {0, 1}, rflip[2] = {0, 0}, rd[3] = {0, 0, 0}, ra = 0;
-    if (!boundary) {
-      const int rlf = (left == c) ? nbrface[c * 6 + lf] : lf;
-      dg_face(rlf, rd[0], rd[1], rd[2], ra);
-      int M[4];
-      for (int bs = 0; bs < 4; ++bs) {
-        const int64_t gs = dg_vertex(q, right, ra | ((bs & 1) << rd[0]) | (((bs >> 1) & 1) << rd[1]));
+    int packed = 0;
+    if (o >= 0) {
+      int d1, d2, dn, a, r1, r2, rn, ra;
+      dg_face(lf, d1, d2, dn, a);
+      dg_face(nbrface[c * 6 + lf], r1, r2, rn, ra);
+      int M[3];
+      for (int bs = 0; bs < 3; ++bs) {  // corners (0,0), (1,0), (0,1) of the neighbour's face
+        const int64_t gv = dg_vertex(q, o, ra | ((bs & 1) << r1) | ((bs >> 1) << r2));
         M[bs] = 0;
         for (int bl = 0; bl < 4; ++bl)
-          if (dg_vertex(q, left, la | ((bl & 1) << ld1) | (((bl >> 1) & 1) << ld2)) == gs) M[bs] = bl;
+          if (dg_vertex(q, c, a | ((bl & 1) << d1) | ((bl >> 1) << d2)) == gv) M[bs] = bl;
       }
-      for (int k = 0; k < 2; ++k) {
-        const int diff = M[0] ^ M[1 << k];
-        raxis[k] = (diff & 1) ? 0 : 1;
-        rflip[k] = (M[0] >> raxis[k]) & 1;
+      const int ax0 = ((M[0] ^ M[1]) & 1) ? 0 : 1, ax1 = ((M[0] ^ M[2]) & 1) ? 0 : 1;
+      // bits: axis of r1, axis of r2, flips, neighbour's local face
+      packed = ax0 | (ax1 << 1) | (((M[0] >> ax0) & 1) << 2) | (((M[0] >> ax1) & 1) << 3) | (nbrface[c * 6 + lf] << 4);
+    }
+    s_o[lf] = (int)o;
+    s_ax[lf] = packed;
+  }
+  for (int t = tid; t < 7 * 24; t += NT) {
+    const int m = t / 24, k = (t % 24) / 3, l = t % 3;
+    const int64_t cc = m == 0 ? c : nbr[c * 6 + m - 1];
+    xv[t] = cc >= 0 ? coords[dg_vertex(q, cc, k) * 3 + l] : 0.0;
+  }
+  if (tid == 0) {
+    int64_t blk[7];
+    const int nb = dg_blocks(c, nbr, blk);
+    for (int k = 0; k < nb; ++k) {
+      if (blk[k] == c) s_kc = k;
+      for (int lf = 0; lf < 6; ++lf)
+        if (nbr[c * 6 + lf] == blk[k]) s_k[lf] = k;
+    }
+    s_nb = nb;
+  }
+  __syncthreads();
+  for (int t = tid; t < 7 * 36; t += NT) {
+    const int m = t / 36, d = (t % 36) / 12, e = (t % 12) / 3, l = t % 3;
+    const int p1 = d == 0 ? 1 : 0, p2 = d == 2 ? 1 : 2;
+    const int lo = ((e & 1) << p1) | ((e >> 1) << p2);
+    ed[t] = xv[m * 24 + (lo | (1 << d)) * 3 + l] - xv[m * 24 + lo * 3 + l];
+  }
+  __syncthreads();
+  // own side of every facet point
+  for (int t = tid; t < NG; t += NT) {
+    const int lf = t / NQF, qp = t % NQF;
+    int d1, d2, dn, a;
+    dg_face(lf, d1, d2, dn, a);
+    const double u0 = q.x1[qp % NP1], u1 = q.x1[qp / NP1], wq = q.w1[qp % NP1] * q.w1[qp / NP1];
+    const bool side = (a >> dn) & 1, boundary = s_o[lf] < 0;
+    double xi[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) xi[d] = d == d1 ? u0 : (d == d2 ? u1 : (side ? 1.0 : -1.0));
+    double C[3][3];
+    const double det = dg_cofactors(ed, xi, C);
+    const double inv = 1.0 / det;
+    const double sg = side == (det > 0.0) ? 1.0 : -1.0;  // outward
+    double n[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      n[i] = sg * (dn == 0 ? C[0][i] : (dn == 1 ? C[1][i] : C[2][i]));
+      gn[t * 3 + i] = n[i];
+    }
+    const double f = (boundary ? wq : 0.5 * wq) * inv;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double w = f * (C[k][0] * n[0] + C[k][1] * n[1] + C[k][2] * n[2]);
+      gw[t * 3 + (k == d1 ? 0 : (k == d2 ? 1 : 2))] = w;
+    }
+    const double s = dg_grad_product(C, inv);
+    // C_IP / h = C_IP / 2 (prod |grad xi|)^(1/3)
+    if (boundary) {
+      gp[t] = sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]) * wq * (0.5 * q.cip) * cbrt(sqrt(s));
+      double x[3] = {0.0, 0.0, 0.0};
+      for (int k = 0; k < 4; ++k) {
+        const int v = a | ((k & 1) << d1) | ((k >> 1) << d2);
+        const double fs = 0.5 * ((k & 1) ? 1.0 + u0 : 1.0 - u0), ft = 0.5 * ((k & 2) ? 1.0 + u1 : 1.0 - u1);
+        for (int l = 0; l < 3; ++l) x[l] = x[l] + fs * ft * xv[v * 3 + l];
+      }
+      gs[t] = dg_boundary_value(q.bfn, q.prm, x);
+    } else {
+      gs[t] = s;
+    }
+  }
+  __syncthreads();
+  // other side of every interior facet point
+  for (int t = tid; t < NG; t += NT) {
+    const int lf = t / NQF, qp = t % NQF;
+    if (s_o[lf] < 0) continue;
+    const int pk = s_ax[lf], ax0 = pk & 1, ax1 = (pk >> 1) & 1;
+    int r1, r2, rn, ra;
+    dg_face(pk >> 4, r1, r2, rn, ra);
+    const double u[2] = {q.x1[qp % NP1], q.x1[qp / NP1]}, wq = q.w1[qp % NP1] * q.w1[qp / NP1];
+    const double f1 = (pk & 4) ? -1.0 : 1.0, f2 = (pk & 8) ? -1.0 : 1.0;
+    const double v1 = f1 * (ax0 ? u[1] : u[0]), v2 = f2 * (ax1 ? u[1] : u[0]), vn = ((ra >> rn) & 1) ? 1.0 : -1.0;
+    double xi[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) xi[d] = d == r1 ? v1 : (d == r2 ? v2 : vn);
+    double C[3][3];
+    const double det = dg_cofactors(ed + (lf + 1) * 36, xi, C);
+    const double inv = 1.0 / det;
+    const double n0 = gn[t * 3], n1 = gn[t * 3 + 1], n2 = gn[t * 3 + 2];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double w = 0.5 * wq * inv * (C[k][0] * n0 + C[k][1] * n1 + C[k][2] * n2);
+      if (k == r1) go[t * 3 + ax0] = f1 * w;
+      else if (k == r2) go[t * 3 + ax1] = f2 * w;
+      else go[t * 3 + 2] = w;
+    }
+    const double s = fmax(gs[t], dg_grad_product(C, inv));  // h = min over the two cells
+    gp[t] = sqrt(n0 * n0 + n1 * n1 + n2 * n2) * wq * (0.5 * q.cip) * cbrt(sqrt(s));
+  }
+  __syncthreads();
+  const int nb = s_nb;
+  const int64_t row0 = rowptr[c * NN];
+  const int st[3] = {1, NP1, NP1 * NP1};
+  for (int lf = 0; lf < 6; ++lf) {
+    int d1, d2, dn, a;
+    dg_face(lf, d1, d2, dn, a);
+    const int side = (a >> dn) & 1, fl = side ? P : 0;
+    const bool boundary = s_o[lf] < 0;
+    const int g0 = lf * NQF;
+    const int sd1 = st[d1], sd2 = st[d2], sdn = st[dn];
+    // tables scaled by the facet's weights; the neighbour block cleared
+    for (int t = tid; t < NF; t += NT) {
+      const int g = g0 + t % NQF;
+      const double ph = Phi[t], e0 = D0[t], e1 = D1[t];
+      pre[t] = gw[g * 3 + 2] * ph;
+      pre[NF + t] = gp[g] * ph;
+      pre[2 * NF + t] = gw[g * 3] * e0 + gw[g * 3 + 1] * e1;
+      if (!boundary) {
+        pre[3 * NF + t] = go[g * 3 + 2] * ph;
+        pre[4 * NF + t] = go[g * 3] * e0 + go[g * 3 + 1] * e1;
       }
     }
-    for (int t = lane; t < NN * NN; t += 32) O[t] = 0.0;
-    const double sigma = (ld1 == 0 && ld2 == 2) ? -1.0 : 1.0;
-    const double outward = ((la >> ldn) & 1) ? 1.0 : -1.0;
-    double orient = 1.0;
-    __syncwarp();
-    for (int qp = 0; qp < NQF; ++qp) {
-      const double s = q.x1[qp % NP1], tt = q.x1[qp / NP1];
-      // lanes 0/1: the left/right cell's reference point, Jacobian inverse and h; lane 2: facet map
-      if (lane < 2 && (lane == 0 || !boundary)) {
-        double xi[3];
-        if (lane == 0) {
-          xi[ld1] = s; xi[ld2] = tt; xi[ldn] = ((la >> ldn) & 1) ? 1.0 : -1.0;
-        } else {
-          const double u[2] = {s, tt};
-          for (int k = 0; k < 2; ++k) xi[rd[k]] = rflip[k] ? -u[raxis[k]] : u[raxis[k]];
-          xi[rd[2]] = ((ra >> rd[2]) & 1) ? 1.0 : -1.0;
+    if (!boundary)
+      for (int t = tid; t < NN * NN; t += NT) O[t] = 0.0;
+    __syncthreads();
+    if (boundary) {  // right-hand side: -g (grad phi . n) + pen g phi
+      for (int i = tid; i < NN; i += NT) {
+        const int l = (i / sdn) % NP1, al = (i / sd1) % NP1 + NP1 * ((i / sd2) % NP1);
+        double v = 0.0;
+        for (int qp = 0; qp < NQF; ++qp) {
+          double k = dL[side * NP1 + l] * pre[al * NQF + qp];
+          if (l == fl) k += pre[2 * NF + al * NQF + qp] - pre[NF + al * NQF + qp];
+          v = fma(gs[g0 + qp], k, v);
         }
-        double b[9], det, h;
-        dg_side_geometry(xv + 24 + 24 * lane, xi, b, det, h);
-        for (int k = 0; k < 9; ++k) misc[6 + 9 * lane + k] = b[k];
-        for (int k = 0; k < 3; ++k) misc[24 + 3 * lane + k] = xi[k];
-        misc[30 + lane] = h;
-        if (lane == 0) misc[32] = det;
+        rv[i] -= v;
       }
-      if (lane == 2) {
-        double X[4][3];
-        for (int k = 0; k < 4; ++k) {
-          const int v = la | ((k & 1) << ld1) | (((k >> 1) & 1) << ld2);
-          for (int l = 0; l < 3; ++l) X[k][l] = xv[24 + v * 3 + l];
-        }
-        double xq[3] = {0, 0, 0}, js[3] = {0, 0, 0}, jt[3] = {0, 0, 0};
-        for (int k = 0; k < 4; ++k) {
-          const double fs = (k & 1) ? 0.5 * (1.0 + s) : 0.5 * (1.0 - s);
-          const double ft = (k & 2) ? 0.5 * (1.0 + tt) : 0.5 * (1.0 - tt);
-          const double ds = ((k & 1) ? 0.5 : -0.5) * ft, dt = ((k & 2) ? 0.5 : -0.5) * fs;
-          for (int l = 0; l < 3; ++l) {
-            xq[l] = xq[l] + fs * ft * X[k][l];
-            js[l] = js[l] + ds * X[k][l];
-            jt[l] = jt[l] + dt * X[k][l];
-          }
-        }
-        double n[3] = {js[1] * jt[2] - js[2] * jt[1], js[2] * jt[0] - js[0] * jt[2], js[0] * jt[1] - js[1] * jt[0]};
-        const double det = sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
-        for (int l = 0; l < 3; ++l) misc[l] = det != 0.0 ? n[l] / det : 0.0;
-        misc[3] = det * (q.w1[qp % NP1] * q.w1[qp / NP1]);
-        misc[5] = boundary ? dg_boundary_value(q.bfn, q.prm, xq) : 0.0;
-      }
-      __syncwarp();
-      if (qp == 0) orient = sigma * outward * (misc[32] > 0.0 ? 1.0 : -1.0);
-      const double h = boundary ? misc[30] : fmin(misc[30], misc[31]);
-      const double n0 = misc[0] * orient, n1 = misc[1] * orient, n2 = misc[2] * orient;
-      const double factor = misc[3];
-      const double ch = q.cip / h;
-      // 1D basis at both sides' points; J^-1 n per side: grad(phi) . n = grad_ref(phi) . (J^-1 n)
-      if (lane < 6 && (lane < 3 || !boundary)) {
-        const int side = lane / 3, dir = lane % 3;
-        double v[NP1], dv[NP1];
-        lag1d<P>(misc[24 + 3 * side + dir], v, dv);
-        for (int jj = 0; jj < NP1; ++jj) {
-          tab[((side * 3 + dir) * 4 + jj) * 2 + 0] = v[jj];
-          tab[((side * 3 + dir) * 4 + jj) * 2 + 1] = dv[jj];
-        }
-      } else if (lane >= 8 && lane < 14 && (lane < 11 || !boundary)) {
-        const int side = (lane - 8) / 3, jr = (lane - 8) % 3;
-        const double* b = misc + 6 + 9 * side;
-        misc[33 + 3 * side + jr] = b[jr + 0] * n0 + b[jr + 3] * n1 + b[jr + 6] * n2;
-      }
-      __syncwarp();
-      // per node: value and scaled normal derivative (the sign of this cell's side folded in)
-      const double sI = I == 0 ? 1.0 : -1.0;
-      const double ascale = boundary ? factor : 0.5 * factor * sI;
-      for (int t = lane; t < 2 * NN; t += 32) {
-        const int side = t / NN, a = t % NN;
-        if (side == 1 && boundary) continue;
-        const int ai = a % NP1, aj = (a / NP1) % NP1, ak = a / (NP1 * NP1);
-        const double* T0 = tab + ((side * 3 + 0) * 4 + ai) * 2;
-        const double* T1 = tab + ((side * 3 + 1) * 4 + aj) * 2;
-        const double* T2 = tab + ((side * 3 + 2) * 4 + ak) * 2;
-        const double* w = misc + 33 + 3 * side;
-        const double dn = T0[1] * T1[0] * T2[0] * w[0] + T0[0] * T1[1] * T2[0] * w[1] + T0[0] * T1[0] * T2[1] * w[2];
-        sval[side * NN + a] = T0[0] * T1[0] * T2[0];
-        sA[side * NN + a] = ascale * dn;
-      }
-      __syncwarp();
-      if (boundary) {
-        const double g = misc[5];
-        const double pen = factor * ch;
-        for (int t = lane; t < NN * NN; t += 32) {
-          const int i = t / NN, j = t % NN;
-          D[t] = D[t] - (sA[j] * sval[i] + sA[i] * sval[j]) + pen * sval[i] * sval[j];
-        }
-        for (int i = lane; i < NN; i += 32) rv[i] = rv[i] - g * sA[i] + pen * g * sval[i];
-      } else {
-        // n_I . n_J = +-|n|^2; with A = sI w|J_F| (grad phi . n)/2:
-        //   same side:  -(A_j v_i + A_i v_j) + pen v_j v_i
-        //   other side: -A^J_j v_i + A^I_i v^J_j - pen v^J_j v_i
-        const double pen = factor * ch * (n0 * n0 + n1 * n1 + n2 * n2);
-        const int Jo = 1 - I;
-        for (int t = lane; t < NN * NN; t += 32) {
-          const int i = t / NN, j = t % NN;
-          const double vi = sval[I * NN + i], ai = sA[I * NN + i];
-          const double vj = sval[I * NN + j], aj = sA[I * NN + j];
-          const double vo = sval[Jo * NN + j], ao = sA[Jo * NN + j];
-          D[t] = D[t] - (aj * vi + ai * vj) + pen * vj * vi;
-          O[t] = O[t] - ao * vi + ai * vo - pen * vo * vi;
-        }
-      }
-      __syncwarp();
     }
+    double N[(NF + NT - 1) / NT], T[(NF + NT - 1) / NT];
+    int lp = 0, s1 = 0, s2 = 0, sn = 0, side2 = 0, pk = 0;
     if (!boundary) {
-      int k = 0;
-      while (blk[k] != o) ++k;
-      for (int t = lane; t < NN * NN; t += 32) {
-        const int i = t / NN, j = t % NN;
-        const int64_t pos = rowptr[c * NN + i] + (int64_t)k * NN + j;
+      pk = s_ax[lf];
+      int r1, r2, rn, ra;
+      dg_face(pk >> 4, r1, r2, rn, ra);
+      side2 = (ra >> rn) & 1;
+      lp = side2 ? P : 0;
+      s1 = st[r1]; s2 = st[r2]; sn = st[rn];
+    }
+    // node of this frame's tangential index in the neighbour, without its layer
+    auto other = [&](int al) {
+      const int b0 = al % NP1, b1 = al / NP1;
+      const int x = (pk & 1) ? b1 : b0, y = (pk & 2) ? b1 : b0;
+      return ((pk & 4) ? P - x : x) * s1 + ((pk & 8) ? P - y : y) * s2;
+    };
+#pragma unroll
+    for (int r = 0; r < (NF + NT - 1) / NT; ++r) {
+      const int t = tid + r * NT;
+      N[r] = T[r] = 0.0;
+      if (t >= NF) continue;
+      const int x = t / NQF, y = t % NQF;
+      double M = 0.0, NO = 0.0, TO = 0.0;
+      for (int qp = 0; qp < NQF; ++qp) {
+        const double ph = Phi[x * NQF + qp];
+        const double* pr = pre + y * NQF + qp;
+        N[r] = fma(ph, pr[0], N[r]);
+        M = fma(ph, pr[NF], M);
+        T[r] = fma(ph, pr[2 * NF], T[r]);
+        if (!boundary) {
+          NO = fma(ph, pr[3 * NF], NO);
+          TO = fma(ph, pr[4 * NF], TO);
+        }
+      }
+      // rows of face node x, columns of node (l, y)
+      const int ix = fl * sdn + (x % NP1) * sd1 + (x / NP1) * sd2;
+      const int jy = (y % NP1) * sd1 + (y / NP1) * sd2;
+#pragma unroll
+      for (int l = 0; l < NP1; ++l) {
+        double v = dL[side * NP1 + l] * N[r];
+        if (l == fl) v += T[r] - M;
+        D[ix * NN + jy + l * sdn] -= v;
+      }
+      if (!boundary) {
+        const int oy = other(y);
+#pragma unroll
+        for (int l = 0; l < NP1; ++l) {
+          double v = dL[side2 * NP1 + l] * NO;
+          if (l == lp) v += TO + M;
+          O[ix * NN + oy + l * sn] = -v;
+        }
+      }
+    }
+    __syncthreads();
+    // the transposed terms: rows of node (l, y), columns of face node x
+#pragma unroll
+    for (int r = 0; r < (NF + NT - 1) / NT; ++r) {
+      const int t = tid + r * NT;
+      if (t >= NF) continue;
+      const int x = t / NQF, y = t % NQF;
+      const int jx = (x % NP1) * sd1 + (x / NP1) * sd2 + fl * sdn;
+      const int iy = (y % NP1) * sd1 + (y / NP1) * sd2;
+      const int ox = boundary ? 0 : other(x) + lp * sn;
+#pragma unroll
+      for (int l = 0; l < NP1; ++l) {
+        double v = dL[side * NP1 + l] * N[r];
+        if (l == fl) v += T[r];
+        const int i = iy + l * sdn;
+        D[i * NN + jx] -= v;
+        if (!boundary) O[i * NN + ox] = l == fl ? O[i * NN + ox] + v : v;
+      }
+    }
+    __syncthreads();
+    if (!boundary) {
+      const int k = s_k[lf];
+      for (int t = tid; t < NN * NN; t += NT) {
+        const int i = t / NN, j = t - i * NN;
+        const int64_t pos = row0 + ((int64_t)i * nb + k) * NN + j;
         val[pos] = O[t];
         if (val32) val32[pos] = (float)O[t];
       }
+      __syncthreads();
     }
-    __syncwarp();
   }
-  int k = 0;
-  while (blk[k] != c) ++k;
-  for (int t = lane; t < NN * NN; t += 32) {
-    const int i = t / NN, j = t % NN;
-    const int64_t pos = rowptr[c * NN + i] + (int64_t)k * NN + j;
+  for (int t = tid; t < NN * NN; t += NT) {
+    const int i = t / NN, j = t - i * NN;
+    const int64_t pos = row0 + ((int64_t)i * nb + s_kc) * NN + j;
     val[pos] = D[t];
     if (val32) val32[pos] = (float)D[t];
   }
-  for (int i = lane; i < NN; i += 32) rhs[c * NN + i] = rv[i];
-  (void)nb;
+  for (int i = tid; i < NN; i += NT) rhs[c * NN + i] = rv[i];
 }
 
 template <int P>
@@ -486,10 +562,31 @@ static fg_status launch_dg_rows(fg_system* sys) {
   q.cip = 10.0 * P * P;
   q.bfn = sys->integ.boundary_fn;
   for (int i = 0; i < 8; ++i) q.prm[i] = sys->integ.fn_param[i];
-  const size_t smem = S::BYTES_WARP * S::WARPS;
-  FG_CUDA_TRY(cudaFuncSetAttribute((const void*)k_dg_rows<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_dg_rows<P><<<nblk(m->ncells, S::WARPS), S::WARPS * 32, smem, ctx->stream>>>(
-      m->ncells, q, m->d_coords, sp->d_dgnbr, sp->d_dgnbrface, sys->d_elmat, sys->d_elvec, sp->d_rowptr, sys->d_val,
+  if (!sp->d_dgtab) {
+    // 2D shapes of a face and their derivatives at its Gauss points, and L_l'(-1), L_l'(1)
+    std::vector<double> h(S::TAB);
+    double v[4][4], dv[4][4];
+    for (int j = 0; j <= P; ++j)
+      for (int k = 0; k <= P; ++k) lagrange_1d(P, j, q.x1[k], v[j][k], dv[j][k]);
+    for (int al = 0; al < S::NQF; ++al)
+      for (int qp = 0; qp < S::NQF; ++qp) {
+        const int a0 = al % S::NP1, a1 = al / S::NP1, q0 = qp % S::NP1, q1 = qp / S::NP1;
+        h[al * S::NQF + qp] = v[a0][q0] * v[a1][q1];
+        h[S::NF + al * S::NQF + qp] = dv[a0][q0] * v[a1][q1];
+        h[2 * S::NF + al * S::NQF + qp] = v[a0][q0] * dv[a1][q1];
+      }
+    for (int l = 0; l <= P; ++l) {
+      double val;
+      lagrange_1d(P, l, -1.0, val, h[3 * S::NF + l]);
+      lagrange_1d(P, l, 1.0, val, h[3 * S::NF + S::NP1 + l]);
+    }
+    FG_TRY(dev_alloc(ctx, (void**)&sp->d_dgtab, sizeof(double) * h.size()));
+    FG_CUDA_TRY(cudaMemcpyAsync(sp->d_dgtab, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, ctx->stream));
+    FG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  }
+  FG_CUDA_TRY(cudaFuncSetAttribute((const void*)k_dg_rows<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
+  k_dg_rows<P><<<(unsigned)m->ncells, S::NT, S::SMEM, ctx->stream>>>(
+      m->ncells, q, sp->d_dgtab, m->d_coords, sp->d_dgnbr, sp->d_dgnbrface, sys->d_elmat, sys->d_elvec, sp->d_rowptr, sys->d_val,
       sys->d_val32, sys->d_rhs);
   ctx->launches += 1;
   FG_CUDA_TRY(cudaGetLastError());

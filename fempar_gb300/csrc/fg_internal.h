@@ -173,6 +173,7 @@ struct fg_space {
   bool dg = false;
   int32_t* d_dgnbr = nullptr;     // 6*ncells: neighbour across local face lf, -1 on the boundary
   int8_t* d_dgnbrface = nullptr;  // 6*ncells: the neighbour's local face
+  double* d_dgtab = nullptr;      // face shapes and derivatives (fg_dg.cu)
 };
 
 struct fg_system {
