@@ -366,6 +366,7 @@ static void space_free(fg_space* sp) {
   dev_free(ctx, sp->d_dgnbr);
   dev_free(ctx, sp->d_dgnbrface);
   dev_free(ctx, sp->d_dgtab);
+  dev_free(ctx, sp->d_dgblk);
   dev_free(ctx, sp->d_st_cls);
   dev_free(ctx, sp->d_st_off);
   dev_free(ctx, sp->d_st_scls);
@@ -476,7 +477,7 @@ fg_status fg_space_create_dg(fg_mesh* mesh, int order, fg_space** out) {
   if (s == FG_OK) s = dg_space_build(sp);
   sp->layout = FG_LAYOUT_SELL;
   if (s == FG_OK) {
-    s = space_build_sell(sp);
+    s = dg_space_build_layout(sp);
     sp->nvec = sp->nfree;
     sp->d_row2vec = sp->d_iperm;
   }

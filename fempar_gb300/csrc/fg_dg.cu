@@ -178,6 +178,76 @@ fg_status dg_space_build(fg_space* sp) {
   return FG_OK;
 }
 
+// ---- solver layout ------------------------------------------------------------------------
+// Cell blocks: a row holds its 7 blocks (the cell and its neighbours in ascending order, zero
+// blocks on the cell itself where it has fewer) of nn columns, padded to a multiple of 4; rows in
+// natural order, slices of 32, entries 4-wide per lane as in the other layouts.  A block's
+// columns are consecutive, so one first column per cell and block replaces a column index per
+// entry: 4 B per FP32 entry instead of 8 (196 entries per Q2 row against 192), and the rows of a
+// cell gather the same addresses.
+__global__ void k_dg_block_table(int64_t nc, int nn, const int32_t* nbr, int32_t* blk, int32_t* ident) {
+  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (c >= nc) return;
+  int64_t b[7];
+  const int nb = dg_blocks(c, nbr, b);
+  for (int k = 0; k < 8; ++k) blk[c * 8 + k] = (int32_t)((k < nb ? b[k] : c) * nn);
+  for (int a = 0; a < nn; ++a) ident[c * nn + a] = (int32_t)(c * nn + a);
+}
+
+fg_status dg_space_build_layout(fg_space* sp) {
+  fg_ctx* ctx = sp->mesh->ctx;
+  const int64_t nc = sp->mesh->ncells, nn = sp->tab.nn;
+  sp->nslices = (sp->nfree + 31) / 32;
+  sp->sell_nnz = sp->nslices * 32 * 7 * ((nn + 3) / 4 * 4);
+  FG_TRY(dev_alloc(ctx, (void**)&sp->d_dgblk, sizeof(int32_t) * nc * 8));
+  FG_TRY(dev_alloc(ctx, (void**)&sp->d_iperm, sizeof(int32_t) * sp->nfree));
+  k_dg_block_table<<<nblk(nc, 256), 256, 0, ctx->stream>>>(nc, (int)nn, sp->d_dgnbr, sp->d_dgblk, sp->d_iperm);
+  FG_CUDA_TRY(cudaGetLastError());
+  ctx->launches += 1;
+  return FG_OK;
+}
+
+// CSR values -> cell blocks, FP64 and FP32; a block per slice (its CSR rows are one contiguous
+// piece that stays in L1 over the passes)
+__global__ void __launch_bounds__(256)
+    k_dg_vals(int64_t n, int nn, const int64_t* __restrict__ rowptr, const double* __restrict__ val,
+              double* __restrict__ sval, float* __restrict__ sval32) {
+  __shared__ int64_t s_start[32];
+  __shared__ int s_len[32];
+  const int64_t s = blockIdx.x;
+  if (threadIdx.x < 32) {
+    const int64_t r = s * 32 + threadIdx.x;
+    s_start[threadIdx.x] = r < n ? rowptr[r] : 0;
+    s_len[threadIdx.x] = r < n ? (int)(rowptr[r + 1] - rowptr[r]) : 0;
+  }
+  __syncthreads();
+  const int g = (nn + 3) >> 2, total = 7 * g * 32;  // groups of 4 entries
+  for (int e = threadIdx.x; e < total; e += 256) {
+    const int l = e & 31, gr = e >> 5, k = gr / g, b = 4 * (gr - k * g);
+    double v[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const int j = k * nn + b + t;
+      v[t] = b + t < nn && j < s_len[l] ? val[s_start[l] + j] : 0.0;
+    }
+    const int64_t o = (s * total + e) * 4;
+    double2* d = reinterpret_cast<double2*>(sval + o);
+    d[0] = make_double2(v[0], v[1]);
+    d[1] = make_double2(v[2], v[3]);
+    *reinterpret_cast<float4*>(sval32 + o) = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
+  }
+}
+
+fg_status dg_system_fill(fg_system* sys) {
+  fg_space* sp = sys->space;
+  fg_ctx* ctx = sp->mesh->ctx;
+  k_dg_vals<<<(unsigned)sp->nslices, 256, 0, ctx->stream>>>(sp->nfree, sp->tab.nn, sp->d_rowptr, sys->d_val,
+                                                            sys->d_sval, sys->d_sval32);
+  FG_CUDA_TRY(cudaGetLastError());
+  ctx->launches += 1;
+  return FG_OK;
+}
+
 // ---- numeric phase ------------------------------------------------------------------------
 // weak Dirichlet data g at a facet point (the analytic functions of the drivers)
 __device__ double dg_boundary_value(int fn, const double* prm, const double* x) {

@@ -139,7 +139,8 @@ struct fg_space {
   int32_t* d_iperm = nullptr;     // row -> slot
   int64_t* d_sptr = nullptr;      // nslices+1 entry offsets
   int32_t* d_scol = nullptr;      // sell_nnz column slots
-  // solver layout: FG_LAYOUT_STENCIL (lattice-implicit SELL, default) or FG_LAYOUT_SELL
+  // solver layout: FG_LAYOUT_STENCIL (lattice-implicit SELL, default) or FG_LAYOUT_SELL (explicit
+  // columns; dG spaces: the columns follow from d_dgblk, d_sptr and d_scol are null)
   int layout = 0;
   int64_t nvec = 0;               // solver vector length
   int32_t* d_row2vec = nullptr;   // free row -> solver vector index
@@ -173,6 +174,7 @@ struct fg_space {
   bool dg = false;
   int32_t* d_dgnbr = nullptr;     // 6*ncells: neighbour across local face lf, -1 on the boundary
   int8_t* d_dgnbrface = nullptr;  // 6*ncells: the neighbour's local face
+  int32_t* d_dgblk = nullptr;     // 8*ncells: first columns of a cell's 7 blocks (cell-block layout)
   double* d_dgtab = nullptr;      // face shapes and derivatives (fg_dg.cu)
 };
 
@@ -260,6 +262,8 @@ fg_status usystem_scatter(fg_system* sys);
 // fg_dg.cu
 fg_status dg_space_build(fg_space* sp);
 fg_status dg_assemble_rows(fg_system* sys);
+fg_status dg_space_build_layout(fg_space* sp);
+fg_status dg_system_fill(fg_system* sys);
 
 // fg_sell.cu
 fg_status space_build_sell(fg_space* sp);

@@ -155,6 +155,7 @@ fg_status system_fill_sell(fg_system* sys) {
   fg_space* sp = sys->space;
   fg_ctx* ctx = sp->mesh->ctx;
   if (sp->nfree == 0) return FG_OK;
+  if (sp->d_dgblk) return dg_system_fill(sys);
   k_sell_vals<<<nblk(sp->nslices * 32, 256), 256, 0, ctx->stream>>>(sp->nfree, sp->nslices, sp->d_rowptr, sys->d_val,
                                                                      sp->d_perm, sp->d_sptr, sys->d_sval,
                                                                      sys->d_sval32);

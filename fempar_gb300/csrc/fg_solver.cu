@@ -486,7 +486,13 @@ struct MatArgs {
   // explicit columns
   const int64_t* sptr;
   const int32_t* scol;
+  // cell blocks (dG)
+  const int32_t* blk;
+  int nn;
 };
+
+// matrix layout of a kernel: lattice-implicit, explicit columns, cell blocks
+enum { ML_STENCIL = 0, ML_SELL = 1, ML_DG = 2 };
 
 // One arrival of the calling block (its other threads have met at a block barrier) and the
 // bounded wait for all blocks; called by one thread.  False: the wait ran out or another
@@ -661,12 +667,14 @@ __device__ __forceinline__ void ld4k(const double* p, double (&v)[4]) {
 }
 
 // One slice of the matrix as one lane sees it.
-template <typename T, bool STENCIL>
+template <typename T, int ML>
 struct SliceRef {
+  static constexpr bool STENCIL = ML == ML_STENCIL;
   const T* vp;         // the lane's first value
-  const int32_t* cp;   // lattice-implicit: offsets of the class; explicit: the lane's first column
-  int w4;              // groups of 4 entries
-  int32_t base, vec;   // gather base; the row's vector index (-1: no row)
+  const int32_t* cp;   // lattice-implicit: offsets of the class; explicit: the lane's first column;
+                       // cell blocks: first columns of the row's 7 blocks
+  int w4;              // groups of 4 entries (cell blocks: of one block)
+  int32_t base, vec;   // gather base (cell blocks: columns per block); the row's vector index (-1: no row)
   __device__ __forceinline__ void load(const MatArgs<T>& m, int64_t s, int lane, const int32_t* s_off) {
     if (STENCIL) {
       const int k = m.scls[s];
@@ -679,6 +687,13 @@ struct SliceRef {
       w4 = C.Bp >> 2;
       vp = m.val + m.voff[s] + 4 * lane;
       cp = s_off + C.offbase;
+    } else if (ML == ML_DG) {
+      const int64_t slot = s * 32 + lane;
+      w4 = (m.nn + 3) >> 2;
+      vp = m.val + s * (32 * 7 * 4) * w4 + 4 * lane;
+      cp = m.blk + 8 * ((slot < m.n ? slot : m.n - 1) / m.nn);
+      base = m.nn;
+      vec = slot < m.n ? (int32_t)slot : -1;
     } else {
       const int64_t b = m.sptr[s];
       w4 = (int)((m.sptr[s + 1] - b) >> 7);
@@ -696,6 +711,27 @@ struct SliceRef {
     T acc = 0;
     const T* v0 = vp;
     const int32_t* c0 = cp;
+    if (ML == ML_DG) {
+      // the rows of a cell read the same x: a warp's gather is one or two addresses
+#pragma unroll 1
+      for (int k = 0; k < 7; ++k) {
+        const T* xb = x + cp[k];
+#pragma unroll UNROLL
+        for (int j = 0; j < w4; ++j) {
+          if (!KEEP && sizeof(T) == 4 && k * w4 + j + kPrefetch < 7 * w4)  // inside the slice
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(v0 + kPrefetch * 128));
+          T v[4];
+          ld4k<KEEP>(v0, v);
+          const T x0 = xb[4 * j], x1 = xb[4 * j + 1], x2 = xb[4 * j + 2], x3 = xb[min(4 * j + 3, base - 1)];
+          acc = fmaT(v[0], x0, acc);
+          acc = fmaT(v[1], x1, acc);
+          acc = fmaT(v[2], x2, acc);
+          acc = fmaT(v[3], x3, acc);
+          v0 += 128;
+        }
+      }
+      return acc;
+    }
     const T* xb = x + base;
 #pragma unroll UNROLL
     for (int j = 0; j < w4; ++j) {
@@ -720,9 +756,9 @@ struct SliceRef {
 };
 
 // the class offsets in shared memory (lattice-implicit layout)
-template <typename T, bool STENCIL>
+template <typename T, int ML>
 __device__ __forceinline__ const int32_t* stage_offsets(const MatArgs<T>& m, int32_t* s_off) {
-  if (!STENCIL) return nullptr;
+  if (ML != ML_STENCIL) return nullptr;
   for (int i = threadIdx.x; i < m.noff; i += blockDim.x) s_off[i] = m.soff[i];
   __syncthreads();
   return s_off;
@@ -734,7 +770,7 @@ static constexpr int pcg_blocks(int R) { return R > 0 ? 1 : 2; }
 // FP64 CG, the sequence and stopping tests of the reference (cg.f90:101-238, 279-407).
 // idiag null: no preconditioner.  chunk: the polling interval the caller asked for (a
 // non-finite iteration is reported at its end, if the iteration limit lies beyond it).
-template <bool STENCIL, int R>
+template <int ML, int R>
 __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
     k_pcg64(MatArgs<double> m, int64_t nvec, double* x, double* r, double* p, double* Ap,
             const double* __restrict__ idiag, int criterion, double rtol, double atol, int max_launch, int chunk,
@@ -749,7 +785,7 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
   const int64_t warp = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   const int64_t nwarps = (int64_t)(blockDim.x >> 5) * gridDim.x;
   const bool need_pp = criterion == FG_DELTA_RHS || criterion == FG_DELTA_DELTA;
-  const int32_t* s_off = stage_offsets<double, STENCIL>(m, s_off_buf);
+  const int32_t* s_off = stage_offsets<double, ML>(m, s_off_buf);
   const int it0 = I[I_ITER], maxit = I[I_MAXIT];
   if (threadIdx.x == 0) {
     sc[2] = S[S_RZ];
@@ -758,7 +794,7 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
     sc[5] = S[S_RNRMM];
     si[0] = si[1] = 0;
   }
-  SliceRef<double, STENCIL> ref[RR];
+  SliceRef<double, ML> ref[RR];
   double rx[RR], rr_[RR], rp[RR], rd[RR], ra[RR];
   if (R > 0) {
 #pragma unroll
@@ -793,7 +829,7 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
       }
     } else {
       for (int64_t s = warp; s < m.nslices; s += nwarps) {
-        SliceRef<double, STENCIL> q;
+        SliceRef<double, ML> q;
         q.load(m, s, lane, s_off);
         const double a = q.template dot<false, kUnroll>(p);
         if (q.vec >= 0) {
@@ -913,7 +949,7 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
 // A segment end (reliable update, stop check, breakdown, iteration limit) found by an update
 // is taken one iteration later: that iteration's update keeps p, so the host can fold x and
 // restart the recursion from the true residual with the direction kept.
-template <bool STENCIL, int R>
+template <int ML, int R>
 __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
     k_pcg32(MatArgs<float> m, int64_t nvec, float* x, float* r, float* p, float* q, const float* __restrict__ idiag,
             int max_launch, GridSync g, double* S, int* I) {
@@ -927,7 +963,7 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   const int64_t nwarps = (int64_t)(blockDim.x >> 5) * gridDim.x;
-  const int32_t* s_off = stage_offsets<float, STENCIL>(m, s_off_buf);
+  const int32_t* s_off = stage_offsets<float, ML>(m, s_off_buf);
   const int maxit = I[I_MAXIT];
   int it = I[I_ITER];
   if (threadIdx.x == 0) {
@@ -941,7 +977,7 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
     si[1] = I[I_SKIPP];
     si[2] = FLAG_NONE;
   }
-  SliceRef<float, STENCIL> ref[RR];
+  SliceRef<float, ML> ref[RR];
   float rx[RR], rr_[RR], rp[RR], rq[RR];
   if (R > 0) {
 #pragma unroll
@@ -977,7 +1013,7 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
       }
     } else {
       for (int64_t s = warp; s < m.nslices; s += nwarps) {
-        SliceRef<float, STENCIL> w;
+        SliceRef<float, ML> w;
         w.load(m, s, lane, s_off);
         const float a = w.template dot<false, kUnroll>(p);
         if (w.vec >= 0) {
@@ -1133,6 +1169,58 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
   }
 }
 
+// y = A x (MODE 0) or y = b - A x with its norm (MODE 2) in the cell-block layout
+template <typename T, int MODE>
+__global__ void __launch_bounds__(RB)
+    k_dg_spmv(MatArgs<T> m, const T* x, T* __restrict__ y, const double* __restrict__ b, RedBuf rb, double* S) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = ((int64_t)blockIdx.x * RB + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * RB) >> 5;
+  Acc<T> dot;
+  for (int64_t s = warp; s < m.nslices; s += nwarps) {
+    SliceRef<T, ML_DG> r;
+    r.load(m, s, lane, nullptr);
+    const T a = r.template dot<false, kUnroll>(x);
+    if (r.vec < 0) continue;
+    if (MODE == 2) {
+      const T rr = (T)(b[r.vec] - (double)a);
+      y[r.vec] = rr;
+      dot.add(rr, rr);
+    } else {
+      y[r.vec] = a;
+    }
+  }
+  if (MODE == 0) return;
+  double v[1] = {dot.value()}, tot[1];
+  if (block_reduce_last<1>(v, rb, tot) && threadIdx.x == 0) S[S_ERR] = sqrt(tot[0]);
+}
+
+// FP32 copy of S A S in the cell-block layout (padding stays 0)
+__global__ void __launch_bounds__(RB) k_scale_dg32(MatArgs<double> m, const double* __restrict__ sd, float* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = ((int64_t)blockIdx.x * RB + threadIdx.x) >> 5;
+  const int64_t nwarps = ((int64_t)gridDim.x * RB) >> 5;
+  for (int64_t s = warp; s < m.nslices; s += nwarps) {
+    SliceRef<double, ML_DG> r;
+    r.load(m, s, lane, nullptr);
+    const double srow = r.vec >= 0 ? sd[r.vec] : 0.0;
+    const double* v0 = r.vp;
+    for (int k = 0; k < 7; ++k) {
+      const double* sb = sd + r.cp[k];
+      for (int j = 0; j < r.w4; ++j, v0 += 128) {
+        double v[4];
+        ld4(v0, v);
+        float4 f;
+        f.x = (float)(v[0] * (srow * sb[4 * j]));
+        f.y = (float)(v[1] * (srow * sb[4 * j + 1]));
+        f.z = (float)(v[2] * (srow * sb[4 * j + 2]));
+        f.w = (float)(v[3] * (srow * sb[min(4 * j + 3, m.nn - 1)]));
+        *reinterpret_cast<float4*>(out + (v0 - m.val)) = f;
+      }
+    }
+  }
+}
+
 // inverse diagonal in the solver layout (extract_diagonal by binary search,
 // csr_sparse_matrix.f90:4231-4256); entries of non-free vector slots stay 0
 __global__ void k_inv_diag(int64_t n, const int64_t* rp, const int32_t* ci, const double* av, const int32_t* row2vec,
@@ -1264,6 +1352,34 @@ fg_status system_prepare_diag(fg_system* sys) {
   return FG_OK;
 }
 
+static int mat_layout(const fg_space* sp) {
+  return sp->layout == FG_LAYOUT_STENCIL ? ML_STENCIL : (sp->d_dgblk ? ML_DG : ML_SELL);
+}
+
+// matrix arguments of the CG kernels
+template <typename T>
+static MatArgs<T> mat_args(const fg_space* sp, const T* vals) {
+  MatArgs<T> m;
+  const bool stencil = sp->layout == FG_LAYOUT_STENCIL;
+  m.nslices = stencil ? sp->st_nslices : sp->nslices;
+  m.n = sp->nfree;
+  m.val = vals;
+  m.scls = sp->d_st_scls;
+  m.voff = sp->d_st_voff;
+  m.cls = sp->d_st_cls;
+  m.soff = sp->d_st_off;
+  m.st_row = sp->d_st_row;
+  m.ncomp = sp->ncomp;
+  m.noff = 0;
+  if (stencil)
+    for (const StencilClass& C : sp->h_st_cls) m.noff += C.Bp;
+  m.sptr = sp->d_sptr;
+  m.scol = sp->d_scol;
+  m.blk = sp->d_dgblk;
+  m.nn = sp->tab.nn;
+  return m;
+}
+
 // SpMV of the active solver layout on solver-layout vectors
 template <typename T, int MODE>
 static void spmv_k(fg_system* sys, const Work& w, const T* x, T* y, const double* b, cudaStream_t st);
@@ -1276,6 +1392,8 @@ static void spmv_k(fg_system* sys, const Work& w, const T* x, T* y, const double
       launch_kn(k_stencil_spmv<T, MODE>, w, st, sp->st_nslices * 32, sp->st_nslices, (const uint8_t*)sp->d_st_scls,                       \
                (const int64_t*)sp->d_st_voff, (const StencilClass*)sp->d_st_cls, (const int32_t*)sp->d_st_off, (const int32_t*)sp->d_st_row,       \
                (const T*)sys->TVALS, sp->ncomp, x, y, b, w.rb, w.S, (const int*)w.I);                               \
+    else if (sp->d_dgblk)                                                                                           \
+      launch_kn(k_dg_spmv<T, MODE>, w, st, sp->nslices * 32, mat_args<T>(sp, sys->VALS), x, y, b, w.rb, w.S);       \
     else                                                                                                            \
       launch_kn(k_sell_spmv<T, MODE>, w, st, sp->nslices * 32, sp->nslices, sp->nfree, (const int64_t*)sp->d_sptr,                     \
                (const int32_t*)sp->d_scol, (const T*)sys->VALS, x, y, b, w.rb, w.S, (const int*)w.I);              \
@@ -1305,6 +1423,8 @@ static fg_status ensure_scaled(fg_system* sys, const Work& w) {
              (const StencilClass*)sp->d_st_cls,
              (const int32_t*)sp->d_st_off, (const int32_t*)sp->d_st_row, v64, (const double*)sys->d_sdiag, sp->ncomp,
              sys->d_val32s);
+  else if (sp->d_dgblk)
+    launch_k(k_scale_dg32, w, st, mat_args<double>(sp, v64), (const double*)sys->d_sdiag, sys->d_val32s);
   else
     launch_k(k_scale_sell32, w, st, sp->nslices, sp->nfree, (const int64_t*)sp->d_sptr, (const int32_t*)sp->d_scol, v64,
              (const double*)sys->d_sdiag, sys->d_val32s);
@@ -1363,28 +1483,6 @@ fg_status system_spmv_layout_noalloc(fg_system* sys, int precision, const void* 
   else spmv_k<double, 0>(sys, w, (const double*)xvec, (double*)yvec, nullptr, st);
   FG_CUDA_TRY(cudaGetLastError());
   return FG_OK;
-}
-
-// matrix arguments of the CG kernels
-template <typename T>
-static MatArgs<T> mat_args(const fg_space* sp, const T* vals) {
-  MatArgs<T> m;
-  const bool stencil = sp->layout == FG_LAYOUT_STENCIL;
-  m.nslices = stencil ? sp->st_nslices : sp->nslices;
-  m.n = sp->nfree;
-  m.val = vals;
-  m.scls = sp->d_st_scls;
-  m.voff = sp->d_st_voff;
-  m.cls = sp->d_st_cls;
-  m.soff = sp->d_st_off;
-  m.st_row = sp->d_st_row;
-  m.ncomp = sp->ncomp;
-  m.noff = 0;
-  if (stencil)
-    for (const StencilClass& C : sp->h_st_cls) m.noff += C.Bp;
-  m.sptr = sp->d_sptr;
-  m.scol = sp->d_scol;
-  return m;
 }
 
 // Launch shape of the CG kernels.  One block per SM, a slice per warp while the warps suffice
@@ -1458,8 +1556,8 @@ static int64_t solver_entries(const fg_space* sp) {
 static fg_status run_pcg64(fg_system* sys, const Work& w, const fg_solver_params* prm, int criterion, double rtol,
                            double atol, int chunk, SolveState& h, cudaStream_t st) {
   fg_space* sp = sys->space;
-  const bool stencil = sp->layout == FG_LAYOUT_STENCIL;
-  MatArgs<double> m = mat_args<double>(sp, stencil ? sys->d_tval : sys->d_sval);
+  const int ml = mat_layout(sp);
+  MatArgs<double> m = mat_args<double>(sp, ml == ML_STENCIL ? sys->d_tval : sys->d_sval);
   const PcgShape sh = pcg_shape(m.nslices, w.sms);
   int64_t nvec = sp->nvec;
   double *x = w.x, *r = w.r, *p = w.p, *Ap = w.Ap;
@@ -1470,9 +1568,9 @@ static fg_status run_pcg64(fg_system* sys, const Work& w, const fg_solver_params
   int* I = w.I;
   void* args[] = {&m, &nvec, &x, &r, &p, &Ap, &idiag, &criterion, &rtol, &atol, &iters, &chunk, &g, &S, &I};
   for (;;) {
-#define FG_PCG64(L) \
-  (sh.R == 1 ? k_pcg64<L, 1> : sh.R == 2 ? k_pcg64<L, 2> : k_pcg64<L, 0>)
-    FG_TRY(launch_pcg(stencil ? FG_PCG64(true) : FG_PCG64(false), sh, w, m.noff, st, args));
+#define FG_PCG64(L) (sh.R == 1 ? k_pcg64<L, 1> : sh.R == 2 ? k_pcg64<L, 2> : k_pcg64<L, 0>)
+    FG_TRY(launch_pcg(ml == ML_STENCIL ? FG_PCG64(ML_STENCIL) : ml == ML_DG ? FG_PCG64(ML_DG) : FG_PCG64(ML_SELL), sh, w,
+                      m.noff, st, args));
 #undef FG_PCG64
     sp->mesh->ctx->launches += 1;
     FG_TRY(read_state(w, h, st));
@@ -1488,7 +1586,7 @@ static fg_status run_pcg64(fg_system* sys, const Work& w, const fg_solver_params
 static fg_status run_pcg32(fg_system* sys, const Work& w, const fg_solver_params* prm, const float* vals,
                            const float* idiag, SolveState& h, cudaStream_t st) {
   fg_space* sp = sys->space;
-  const bool stencil = sp->layout == FG_LAYOUT_STENCIL;
+  const int ml = mat_layout(sp);
   MatArgs<float> m = mat_args<float>(sp, vals);
   const PcgShape sh = pcg_shape(m.nslices, w.sms);
   int64_t nvec = sp->nvec;
@@ -1499,9 +1597,9 @@ static fg_status run_pcg32(fg_system* sys, const Work& w, const fg_solver_params
   int* I = w.I;
   void* args[] = {&m, &nvec, &x, &r, &p, &q, &idiag, &iters, &g, &S, &I};
   do {
-#define FG_PCG32(L) \
-  (sh.R == 1 ? k_pcg32<L, 1> : sh.R == 2 ? k_pcg32<L, 2> : k_pcg32<L, 0>)
-    FG_TRY(launch_pcg(stencil ? FG_PCG32(true) : FG_PCG32(false), sh, w, m.noff, st, args));
+#define FG_PCG32(L) (sh.R == 1 ? k_pcg32<L, 1> : sh.R == 2 ? k_pcg32<L, 2> : k_pcg32<L, 0>)
+    FG_TRY(launch_pcg(ml == ML_STENCIL ? FG_PCG32(ML_STENCIL) : ml == ML_DG ? FG_PCG32(ML_DG) : FG_PCG32(ML_SELL), sh, w,
+                      m.noff, st, args));
 #undef FG_PCG32
     sp->mesh->ctx->launches += 1;
     FG_TRY(read_state(w, h, st));

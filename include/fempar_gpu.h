@@ -126,7 +126,8 @@ typedef struct {
   int64_t nnz_full, nnz_upper;
   int64_t solver_vec_len;  /* entries of a vector in the solver's own layout (>= num_free) */
   int64_t solver_entries;  /* matrix entries stored by the solver's layout (>= nnz_full: padding) */
-  int32_t solver_layout;   /* 0 = lattice-implicit SELL (no column indices), 1 = explicit-column SELL */
+  int32_t solver_layout;   /* 0 = lattice-implicit SELL (no column indices), 1 = explicit-column SELL
+                              (dG spaces: columns implied by the cell and its neighbours) */
 } fg_space_info;
 
 const char* fg_status_string(fg_status s);

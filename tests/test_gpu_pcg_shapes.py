@@ -86,6 +86,40 @@ def test_pcg_shapes(fg, ctx, n, layout, monkeypatch):
     tri.close()
 
 
+@pytest.mark.parametrize("n,order", [((1, 1, 1), 1), ((5, 3, 2), 2), ((2, 3, 2), 3), ((30, 30, 30), 1), ((34, 34, 34), 1)],
+                         ids=["one_cell", "ragged_slice", "q3", "two_slices_per_warp", "streamed"])
+def test_dg_cell_block_layout(fg, ctx, n, order):
+    """The dG layout whose columns follow from the cell and its neighbours: products with the
+    exported CSR (FP64 and FP32), and solves by their true residual, at the edges of the shapes."""
+    import scipy.sparse as sp
+    import torch
+    rng = np.random.default_rng(order + sum(n))
+    tri = fg.SerialTriangulation(ctx, n)
+    space = fg.SerialFESpace(tri, order=order, dg=True)
+    op = fg.FEAffineOperator(space, fg.PoissonIntegration(source_fn=fg.FG_FN_CONST, fn_param=[1.0],
+                                                          boundary_fn=fg.FG_FN_ZERO)).compute()
+    irp, ja, val = op.get_matrix(symmetric_storage=False, one_based=False)
+    A = sp.csr_matrix((val, ja, irp), shape=(space.num_free_dofs,) * 2)
+    x = rng.standard_normal(space.num_free_dofs)
+    scale = abs(A) @ abs(x)
+    m = np.diff(irp).max()
+    for prec, dt, eps in ((fg.FG_FP64, torch.float64, 2.0 ** -53), (fg.FG_MIXED, torch.float32, 2.0 ** -24)):
+        dx = torch.from_numpy(x).to("cuda", dt)
+        y = op.apply_device(dx, torch.empty_like(dx), prec).double().cpu().numpy()
+        # m products summed, and the roundings of the values and of x to the type
+        assert np.all(np.abs(y - A @ x) <= (m + 3) * eps * scale)
+    b = op.get_translation()
+    for prec in ("fp64", "mixed"):
+        s = fg.IterativeLinearSolver().set_type_from_string("CG").set_operators(op, "jacobi")
+        s.set_parameters_from_pl({"ILS_RTOL": 1e-10, "ILS_MAX_NUM_ITERATIONS": 20000, "PRECISION": prec})
+        x = s.solve()
+        assert s.info()["converged"], prec
+        assert np.linalg.norm(b - A @ x) <= (1e-10 + 1e-12) * np.linalg.norm(b), prec
+    op.close()
+    space.close()
+    tri.close()
+
+
 def test_pcg_bounded_barrier_runs_out_and_context_survives(fg, ctx, monkeypatch):
     """A block that skips its first arrival: the bounded grid barriers run out, the solve reports
     FG_ERR_TIMEOUT and the same system then solves."""
