@@ -1496,9 +1496,13 @@ struct PcgShape {
   int R;
   unsigned blocks, threads;
 };
-static PcgShape pcg_shape(int64_t nslices, int sms) {
+static PcgShape pcg_shape(int64_t nslices, int64_t value_bytes, bool fp32, int sms) {
   const int64_t cap = (int64_t)sms * 32;
-  if (nslices > 2 * cap) return PcgShape{0, (unsigned)(2 * sms), (unsigned)pcg_threads(0)};
+  // FP32 with two slices per warp only while the matrix stays in L2: streaming it wants the 48
+  // warps and the prefetch (dG 20^3 Q2, 169 MB: 38 us per iteration against 64; 19^3 Q3, 150 MB: 45
+  // against 48; 34^3 Q2, 80 MB: 36 against 29).  FP64 is bound by its pipe there (103 against 90).
+  const bool streams = fp32 && nslices > cap && value_bytes > (int64_t)112 << 20;
+  if (nslices > 2 * cap || streams) return PcgShape{0, (unsigned)(2 * sms), (unsigned)pcg_threads(0)};
   const int R = nslices <= cap ? 1 : 2;
   const int64_t warps = std::max<int64_t>(1, (nslices + R - 1) / R);
   const int64_t blocks = warps <= 16 ? 1 : std::min<int64_t>(sms, warps);
@@ -1558,7 +1562,7 @@ static fg_status run_pcg64(fg_system* sys, const Work& w, const fg_solver_params
   fg_space* sp = sys->space;
   const int ml = mat_layout(sp);
   MatArgs<double> m = mat_args<double>(sp, ml == ML_STENCIL ? sys->d_tval : sys->d_sval);
-  const PcgShape sh = pcg_shape(m.nslices, w.sms);
+  const PcgShape sh = pcg_shape(m.nslices, 8 * solver_entries(sp), false, w.sms);
   int64_t nvec = sp->nvec;
   double *x = w.x, *r = w.r, *p = w.p, *Ap = w.Ap;
   const double* idiag = prm->precond == FG_PREC_JACOBI ? sys->d_idiag : nullptr;
@@ -1588,7 +1592,7 @@ static fg_status run_pcg32(fg_system* sys, const Work& w, const fg_solver_params
   fg_space* sp = sys->space;
   const int ml = mat_layout(sp);
   MatArgs<float> m = mat_args<float>(sp, vals);
-  const PcgShape sh = pcg_shape(m.nslices, w.sms);
+  const PcgShape sh = pcg_shape(m.nslices, 4 * solver_entries(sp), true, w.sms);
   int64_t nvec = sp->nvec;
   float *x = w.x32, *r = w.r32, *p = w.p32, *q = w.Ap32;
   int iters = pcg_iters(prm, solver_entries(sp), nvec, 4);
