@@ -150,32 +150,60 @@ struct CholSmem {
   int fail;
 };
 
-// Load the nb x nb diagonal block at j0, factor it in shared memory (warp 0), write it
-// back.  Returns false (to every thread) on a non-positive pivot.
+// s / d from the correctly rounded reciprocal r of d: the quotient with one correction step
+// (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J.
+// Res. Dev. 34, 1990), the rounding of a division in three operations where many values are
+// divided by the same d.
+__device__ __forceinline__ double quotient(double s, double d, double r) {
+  const double q = s * r;
+  return fma(fma(-q, d, s), r, q);
+}
+
+// Load the nb x nb diagonal block at j0, factor it, leave the factor in sm.D and write it back.
+// Returns false (to every thread) on a non-positive pivot.  128 threads work: warp q holds the
+// columns j = 4c + q, lane = row.  A step divides the pivot column by its pivot (its owner), and
+// the warps subtract l_i a_j from their columns; the square roots wait for the end (all columns
+// at once), so the chain from pivot to pivot is one division and one update.  FP64 issues once in
+// 64 cycles per scheduler here, which one warp doing everything spent on ~1500 instructions:
+// a 32 x 32 block 60 -> 33 us.
 __device__ bool chol_diag(double* A, int64_t lda, int j0, int nb, CholSmem& sm) {
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  double(&col)[2][2][32] = *reinterpret_cast<double(*)[2][2][32]>(&sm.Pi[0][0]);  // [buffer][a, l][row]
   for (int t = tid; t < 32 * 32; t += blockDim.x) {
     int i = t & 31, j = t >> 5;
-    sm.D[i][j] = (i < nb && j < nb && i >= j) ? A[(j0 + i) + (int64_t)(j0 + j) * lda] : 0.0;
+    // rows and columns past nb: the unit matrix
+    sm.D[i][j] = (i < nb && j < nb) ? (i >= j ? A[(j0 + i) + (int64_t)(j0 + j) * lda] : 0.0) : (i == j ? 1.0 : 0.0);
   }
   if (tid == 0) sm.fail = 0;
   __syncthreads();
-  if (tid < 32) {
-    const int lane = tid;
-    for (int k = 0; k < nb; ++k) {
-      double piv = sm.D[k][k];
-      if (!(piv > 0.0)) {
-        if (lane == 0) sm.fail = 1;
-        break;
-      }
-      double d = sqrt(piv);
-      __syncwarp();
-      if (lane > k && lane < nb) sm.D[lane][k] /= d;
-      __syncwarp();
-      if (lane == k) sm.D[k][k] = d;
-      for (int j = k + 1; j < nb; ++j)
-        if (lane >= j && lane < nb) sm.D[lane][j] -= sm.D[lane][k] * sm.D[j][k];
-      __syncwarp();
+  double v[8];
+  if (w < 4)
+#pragma unroll
+    for (int c = 0; c < 8; ++c) v[c] = sm.D[lane][4 * c + w];
+#pragma unroll
+  for (int k = 0; k < 32; ++k) {
+    const int b = k & 1;
+    if (w == (k & 3)) {
+      const double piv = __shfl_sync(0xffffffffu, v[k >> 2], k);
+      if (!(piv > 0.0) && lane == 0) sm.fail = 1;
+      col[b][0][lane] = v[k >> 2];
+      col[b][1][lane] = v[k >> 2] / piv;
+    }
+    __syncthreads();
+    if (w < 4) {
+      const double l = col[b][1][lane];
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        if (4 * c + w > k) v[c] = v[c] - l * col[b][0][4 * c + w];
+    }
+  }
+  // column k of the factor: a_k / sqrt(pivot)
+  if (w < 4) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int k = 4 * c + w;
+      const double d = sqrt(__shfl_sync(0xffffffffu, v[c], k));
+      sm.D[lane][k] = lane > k ? v[c] / d : (lane == k ? d : 0.0);
     }
   }
   __syncthreads();
@@ -187,8 +215,10 @@ __device__ bool chol_diag(double* A, int64_t lda, int j0, int nb, CholSmem& sm) 
   return true;
 }
 
-// Row i (>= j0+nb): A[i, j0:j0+nb] <- A[i, j0:j0+nb] D^-T  (D in shared memory)
-__device__ __forceinline__ void chol_trsm_row(double* A, int64_t lda, int j0, int nb, int64_t i, const double (&D)[32][33]) {
+// Row i (>= j0+nb): A[i, j0:j0+nb] <- A[i, j0:j0+nb] D^-T  (D in shared memory, rd the reciprocals
+// of its diagonal)
+__device__ __forceinline__ void chol_trsm_row(double* A, int64_t lda, int j0, int nb, int64_t i, const double (&D)[32][33],
+                                              const double* rd) {
   double x[32];
 #pragma unroll
   for (int k = 0; k < 32; ++k) x[k] = k < nb ? A[i + (int64_t)(j0 + k) * lda] : 0.0;
@@ -198,7 +228,7 @@ __device__ __forceinline__ void chol_trsm_row(double* A, int64_t lda, int j0, in
       double s = x[k];
 #pragma unroll
       for (int l = 0; l < k; ++l) s -= x[l] * D[k][l];
-      x[k] = s / D[k][k];
+      x[k] = quotient(s, D[k][k], rd[k]);
     }
   }
 #pragma unroll
@@ -254,7 +284,10 @@ __device__ bool chol_partial_cta(double* A, int64_t lda, int N, int ncols, CholS
     const int nb = min(32, ncols - j0);
     if (!chol_diag(A, lda, j0, nb, sm)) return false;
     __syncthreads();
-    for (int64_t i = j0 + nb + threadIdx.x; i < N; i += blockDim.x) chol_trsm_row(A, lda, j0, nb, i, sm.D);
+    double* rd = &sm.Pj[0][0];
+    if (threadIdx.x < nb) rd[threadIdx.x] = 1.0 / sm.D[threadIdx.x][threadIdx.x];
+    __syncthreads();
+    for (int64_t i = j0 + nb + threadIdx.x; i < N; i += blockDim.x) chol_trsm_row(A, lda, j0, nb, i, sm.D, rd);
     __syncthreads();
     const int t0 = j0 + nb, tn = N - t0;
     if (tn <= 0) continue;
@@ -394,7 +427,7 @@ __global__ void k_bstep_diag(const BSub* __restrict__ subs, double* __restrict__
 }
 
 __global__ void __launch_bounds__(256) k_bstep_trsm(const BSub* __restrict__ subs, double* __restrict__ A, int j0) {
-  __shared__ double Dsh[32][33];
+  __shared__ double Dsh[32][33], rd[32];
   const BSub S = subs[blockIdx.y];
   if (j0 >= S.nr) return;
   const int nb = min(32, S.nr - j0);
@@ -406,7 +439,9 @@ __global__ void __launch_bounds__(256) k_bstep_trsm(const BSub* __restrict__ sub
     Dsh[r][c] = (r < nb && c < nb && r >= c) ? As[(j0 + r) + (int64_t)(j0 + c) * S.N] : 0.0;
   }
   __syncthreads();
-  if (i < S.N) chol_trsm_row(As, S.N, j0, nb, i, Dsh);
+  if (threadIdx.x < nb) rd[threadIdx.x] = 1.0 / Dsh[threadIdx.x][threadIdx.x];
+  __syncthreads();
+  if (i < S.N) chol_trsm_row(As, S.N, j0, nb, i, Dsh, rd);
 }
 
 __global__ void __launch_bounds__(256) k_bstep_syrk(const BSub* __restrict__ subs, double* __restrict__ A, int j0) {
@@ -424,20 +459,6 @@ __global__ void __launch_bounds__(256) k_bstep_syrk(const BSub* __restrict__ sub
   while ((int64_t)ti * (ti + 1) / 2 > b) --ti;
   const int tj = (int)(b - (int64_t)ti * (ti + 1) / 2);
   chol_syrk_tile(A + S.aoff, S.N, S.N, j0, nb, t0, ti, tj, sm);
-}
-
-// k_bstep_syrk restricted to the columns [j0 + nb, min(cend, nr)) of a wider panel: tiles
-// (ti, tj, subdomain) = blockIdx (x, y, z), ti >= tj.
-__global__ void __launch_bounds__(256) k_bstep_syrk_panel(const BSub* __restrict__ subs, double* __restrict__ A,
-                                                          int j0, int cend) {
-  __shared__ CholSmem sm;
-  const BSub S = subs[blockIdx.z];
-  if (j0 >= S.nr) return;
-  const int nb = min(32, S.nr - j0);
-  const int t0 = j0 + nb, cN = min(cend, S.nr);
-  const int ti = blockIdx.x, tj = blockIdx.y;
-  if (ti < tj || t0 + tj * 64 >= cN || t0 + ti * 64 >= S.N) return;
-  chol_syrk_tile(A + S.aoff, S.N, S.N, j0, nb, t0, ti, tj, sm, cN);
 }
 
 // Local coarse matrix K_Pi (order [V | e]), S_e^-1 and H = S_e^-1 T from the trailing block.
@@ -584,16 +605,21 @@ __global__ void k_chol_diag1(double* A, int64_t lda, int j0, int nb, int* err) {
   }
 }
 
-__global__ void __launch_bounds__(256) k_chol_trsm1(double* A, int64_t lda, int N, int j0, int nb) {
-  __shared__ double Dsh[32][33];
+// 64 rows per block: the row solves are bound by the FP64 pipe, and a coarse panel has too few
+// rows to fill the SMs with 256 (9,492 coarse dofs: 78 -> 53 us; with the divisions by the
+// diagonal as products with its reciprocals and a correction, 27 us)
+__global__ void __launch_bounds__(64) k_chol_trsm1(double* A, int64_t lda, int N, int j0, int nb) {
+  __shared__ double Dsh[32][33], rd[32];
   for (int t = threadIdx.x; t < 32 * 32; t += blockDim.x) {
     int i = t & 31, j = t >> 5;
     Dsh[i][j] = (i < nb && j < nb && i >= j) ? A[(j0 + i) + (int64_t)(j0 + j) * lda] : 0.0;
   }
   __syncthreads();
+  if (threadIdx.x < nb) rd[threadIdx.x] = 1.0 / Dsh[threadIdx.x][threadIdx.x];
+  __syncthreads();
   int64_t i = j0 + nb + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= N) return;
-  chol_trsm_row(A, lda, j0, nb, i, Dsh);
+  chol_trsm_row(A, lda, j0, nb, i, Dsh, rd);
 }
 
 __global__ void __launch_bounds__(256) k_chol_syrk1(double* A, int64_t lda, int N, int j0, int nb, int nt) {
@@ -1732,11 +1758,11 @@ static fg_status chol_partial_grid(fg_ctx* ctx, double* A, int64_t lda, int N, i
     const int J1 = std::min(J0 + NB, ncols);
     for (int j0 = J0; j0 < J1; j0 += 32) {
       const int nb = std::min(32, J1 - j0);
-      k_chol_diag1<<<1, 32, 0, st>>>(A, lda, j0, nb, err);
+      k_chol_diag1<<<1, 128, 0, st>>>(A, lda, j0, nb, err);
       const int Neff = (int)std::min<int64_t>(N, (int64_t)zrow + j0 + nb);
       const int rows = Neff - j0 - nb;
       if (rows > 0) {
-        k_chol_trsm1<<<nblk(rows, 256), 256, 0, st>>>(A, lda, Neff, j0, nb);
+        k_chol_trsm1<<<nblk(rows, 64), 64, 0, st>>>(A, lda, Neff, j0, nb);
         const int nt = (rows + 63) / 64;
         if (work) {
           const int ntc = (J1 - (j0 + nb) + 63) / 64;  // columns left inside the panel
@@ -1803,11 +1829,23 @@ static fg_status bddc_numeric(fg_bddc* B) {
         if (S.N - J1 <= 0) continue;
         double* As = B->dA + S.aoff;
         items.push_back(OzSyrk{As + J1 + (int64_t)J0 * S.N, As + J1 + (int64_t)J1 * S.N, (int64_t)S.N, S.N - J1,
-                               J1 - J0});
+                               J1 - J0, S.N - J1});
       }
       return items;
     };
-    const size_t wbytes = ozaki_syrk_batch_bytes(panel_items(0));
+    // the 32 columns at j0 into the rest of their 128-column panel
+    auto step_items = [&](int j0, int J1) {
+      std::vector<OzSyrk> items;
+      for (const BSub& S : B->subs) {
+        const int j1 = j0 + 32, c1 = std::min(J1, S.nr);
+        if (j1 >= c1) continue;
+        double* As = B->dA + S.aoff;
+        items.push_back(OzSyrk{As + j1 + (int64_t)j0 * S.N, As + j1 + (int64_t)j1 * S.N, (int64_t)S.N, S.N - j1, 32,
+                               c1 - j1});
+      }
+      return items;
+    };
+    const size_t wbytes = std::max(ozaki_syrk_batch_bytes(panel_items(0)), ozaki_syrk_batch_bytes(step_items(0, 128)));
     void* work = nullptr;
     FG_TRY(dev_alloc(ctx, &work, wbytes + sizeof(int)));
     int* oz_err = (int*)((uint8_t*)work + wbytes);
@@ -1815,21 +1853,16 @@ static fg_status bddc_numeric(fg_bddc* B) {
     cudaError_t ce = cudaMemsetAsync(oz_err, 0, sizeof(int), st);
     for (int J0 = 0; J0 < B->maxnr && ls == FG_OK && ce == cudaSuccess; J0 += 128) {
       for (int j0 = J0; j0 < std::min(J0 + 128, B->maxnr); j0 += 32) {
-        k_bstep_diag<<<ns, 32, 0, st>>>(B->d_subs, B->dA, j0, B->dErr);
+        k_bstep_diag<<<ns, 128, 0, st>>>(B->d_subs, B->dA, j0, B->dErr);
         const int rem = B->maxN - j0 - 1;
         if (rem > 0) {
           k_bstep_trsm<<<dim3(nblk(rem, 256), ns), 256, 0, st>>>(B->d_subs, B->dA, j0);
-          const int nt = (rem + 63) / 64;
-          const int ntc = std::max(0, (J0 + 128 - (j0 + 32) + 63) / 64);  // column tiles left in the panel
-          if (ntc > 0) {
-            k_bstep_syrk_panel<<<dim3((unsigned)nt, (unsigned)ntc, ns), 256, 0, st>>>(B->d_subs, B->dA, j0, J0 + 128);
-            ctx->launches += 1;
-          }
+          if (ls == FG_OK) ls = ozaki_syrk_batch(ctx, st, step_items(j0, J0 + 128), work, wbytes, oz_err);
           ctx->launches += 1;
         }
         ctx->launches += 1;
       }
-      ls = ozaki_syrk_batch(ctx, st, panel_items(J0), work, wbytes, oz_err);
+      if (ls == FG_OK) ls = ozaki_syrk_batch(ctx, st, panel_items(J0), work, wbytes, oz_err);
     }
     int h_oz = 0;
     if (ls == FG_OK && ce == cudaSuccess) ce = cudaMemcpyAsync(&h_oz, oz_err, sizeof(int), cudaMemcpyDeviceToHost, st);
@@ -1852,7 +1885,7 @@ static fg_status bddc_numeric(fg_bddc* B) {
     B->local_emulated = true;
   } else if (B->stepped) {
     for (int j0 = 0; j0 < B->maxnr; j0 += 32) {
-      k_bstep_diag<<<ns, 32, 0, st>>>(B->d_subs, B->dA, j0, B->dErr);
+      k_bstep_diag<<<ns, 128, 0, st>>>(B->d_subs, B->dA, j0, B->dErr);
       const int rem = B->maxN - j0 - 1;
       if (rem > 0) {
         k_bstep_trsm<<<dim3(nblk(rem, 256), ns), 256, 0, st>>>(B->d_subs, B->dA, j0);

@@ -556,6 +556,19 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
     const int bmode = g.beta == 0.0 ? 0 : (g.beta == 1.0 ? 1 : 2);
     int gc = 0;
     for (int t = first; t < ntiles; t = next_tile(t)) {
+      if (bmode != 0) {
+        // C is needed after the sums: ask L2 for this thread's elements while the MMAs run
+        const OzItem it = item_of(g, t);
+        int rt, ct;
+        it.locate(t, rt, ct);
+        const int i = rt * OZ_BM + row, c0 = ct * BN + part4 * OZ_EPI_COLS;
+        const double* p = it.c + (int64_t)i * it.c_rs;
+        if (i < it.m)
+#pragma unroll
+          for (int j = 0; j < OZ_EPI_COLS; ++j)
+            if (c0 + j < it.n && !(g.lower && c0 + j > i))
+              asm volatile("prefetch.global.L2 [%0];" ::"l"(p + (int64_t)(c0 + j) * it.c_cs));
+      }
       // per column: sum over K chunks of the chunk's product / 2^(e_i + f_j - 16), in FP64
       double acc[OZ_EPI_COLS];
       bool ok = true;
@@ -766,11 +779,17 @@ fg_status ozaki_gemm_nt(fg_ctx* ctx, cudaStream_t st, int64_t m, int64_t n, int6
                      : oz_launch<OZ_S>(ctx, st, sa, rta + rtb, g, rta * tiles_n);
 }
 
-// Batch of lower updates C_b -= P_b P_b^T, P_b m_b x k_b (k_b <= 128), all column-major.
+// Batch of lower updates C_b -= P_b P_b^T, P_b m_b x k_b (k_b <= 128), all column-major; the first
+// n_b columns of C_b.  All items take the K steps of the longest.
+static int syrk_ksteps(const std::vector<OzSyrk>& b) {
+  int k = 1;
+  for (const auto& x : b) k = std::max(k, x.k);
+  return (k + OZ_BK - 1) / OZ_BK;
+}
 size_t ozaki_syrk_batch_bytes(const std::vector<OzSyrk>& b) {
   int64_t rt = 0;
   for (const auto& x : b) rt += rtiles_of(x.m);
-  return (size_t)rt * (128 / OZ_BK) * oz_a_bytes(OZ_S) + (size_t)rt * OZ_BM * sizeof(int32_t) +
+  return (size_t)rt * syrk_ksteps(b) * oz_a_bytes(OZ_S) + (size_t)rt * OZ_BM * sizeof(int32_t) +
          b.size() * (sizeof(OzSplit) + sizeof(OzItem)) + 512;
 }
 
@@ -785,9 +804,9 @@ fg_status ozaki_syrk_batch(fg_ctx* ctx, cudaStream_t st, const std::vector<OzSyr
       set_error("ozaki_syrk_batch: k = %d > 128", x.k);
       return FG_ERR_UNSUPPORTED;
     }
-    const int64_t tn = (x.m + OZ_BN - 1) / OZ_BN;
+    const int64_t tn = (x.n + OZ_BN - 1) / OZ_BN;
     hs.push_back(OzSplit{x.p, 1, x.ld, x.m, x.k, (int)rt});
-    hi.push_back(OzItem{x.c, 1, x.ld, x.m, x.m, (int)rt, (int)rt, (int)tn, (int)tiles, 0});
+    hi.push_back(OzItem{x.c, 1, x.ld, x.m, x.n, (int)rt, (int)rt, (int)tn, (int)tiles, 0});
     rt += rtiles_of(x.m);
     tiles += rtiles_of(x.m) * tn;
   }
@@ -796,7 +815,7 @@ fg_status ozaki_syrk_batch(fg_ctx* ctx, cudaStream_t st, const std::vector<OzSyr
     set_error("ozaki_syrk_batch: workspace too small or too many tiles");
     return FG_ERR_UNSUPPORTED;
   }
-  const int ksteps = 128 / OZ_BK;
+  const int ksteps = syrk_ksteps(b);
   uint8_t* w = (uint8_t*)work;
   const size_t dig_bytes = (size_t)rt * ksteps * oz_a_bytes(OZ_S);
   int32_t* ex = (int32_t*)(w + dig_bytes);
