@@ -28,11 +28,10 @@
 //     maximum and the error left is that of the dropped pairs, ~50 times smaller than the cut's
 //     at S = 7 (36 pairs instead of 34; a class 7 sum could pass 2^24 by 11 % if every digit were
 //     extreme, and would then round in its last bit, below what the dropped pairs leave out);
-//   * the epilogue converts the 8 class sums to integers, combines them exactly (H 2^-24 +
-//     L 2^-56), turns the chunk's sum into FP64 with one rounding (two exact bit patterns, one
-//     addition), adds the K chunks in FP64, applies the power of two 2^(e_i + f_j - 16) through
-//     the exponent field and updates C: about two FP64 operations per output element and chunk
-//     instead of 128.
+//   * the epilogue converts the 8 class sums to integers and adds them, over all chunks of K,
+//     into one exact 96-bit integer per output element; that becomes FP64 with one rounding, and
+//     the power of two 2^(e_i + f_j - 16) goes into the exponent field, all in integer arithmetic:
+//     one FP64 operation per output element where C is updated, none where it is written.
 //
 // Digit layout in HBM: per operand, blocks of 128 rows x 16 columns (one MMA K step) per
 // digit, 4 KB each, ordered [row tile][K step][digit]; inside a block the rows are in the
@@ -45,19 +44,23 @@
 // round robin).  Every wait is bounded: after ~1 s the CTA records FG_ERR_TIMEOUT, stops, waits
 // (bounded) for its copies and MMAs in flight, frees its tensor memory and returns.
 //
-// What bounds it (4096^3: 13.1 us per chunk of 10 K steps and tile): the MMAs, ~60 cycles each
-// where a 128 x 64 x 16 one runs 32, then ~4.7 k cycles in which the epilogue takes the class
-// sums out of the accumulators (they fill the tensor memory, so the next tile's MMAs wait); the
-// conversion and the update of C (10 k cycles) run beside the next tile's MMAs.  What it took,
-// TFLOP/s at 4096^3 and 8192 x 8192 x 128:
+// What bounds it: at 4096^3 the MMAs (34 digit pairs, 4.7 PFLOP of bf16 in 2.9 ms beside 0.2 ms
+// of cutting: 1.6 PFLOP/s, 85 % of the measured bf16 rate; without any epilogue work the kernel
+// takes as long).  At K = 128 (8192 x 8192: 0.44 ms) the MMAs run 56 % of the time and the epilogue's
+// ~120 instructions per element, a C tile every 8 K steps, are as long.  What it took, TFLOP/s at
+// 4096^3 and 8192 x 8192 x 128:
 //     13.7 / 13.0  eight epilogue warps converting before they release the accumulators, MMAs
 //                  issued by the lane that also feeds the copies
 //     16.8 / 15.2  release first, sixteen warps
 //     26.0 / 23.0  a copy warp, and MMAs issued from warp-uniform code (descriptors in uniform
-//                  registers): 139 -> 78 cycles per MMA
-//     30.5 / 25.6  each A digit block read from shared memory once per K step and held in the
-//                  collector buffer for its run of MMAs: 78 -> 60
-// 128 x 32 tiles with two accumulator sets: 25.9 / 22.9.
+//                  registers)
+//     30.5 / 25.6  each A digit block held in the collector buffer for its run of MMAs
+//     31.8 / 25.3  an A digit against four B digits per MMA (N = 256; no collector needed)
+//     33.3 / 26.2  chunks added as integers instead of in FP64
+//     42.7 / 24.0  the classes in two halves with barriers of their own, so that the epilogue
+//                  empties one half of the tensor memory while the MMAs fill the other
+//     44.0 / 34.5  the conversion to FP64 branch-free (every warp had a lane on the slow side of
+//                  a branch) and the class sums as 64-bit multiply-adds: 150 -> 120 instructions
 
 #include <cuda_runtime.h>
 
@@ -87,7 +90,7 @@ constexpr int OZ_THREADS = (OZ_EPI_WARPS + 2) * 32;        // with the MMA warp 
 constexpr int OZ_BN = 64;
 template <int BN, int S>
 struct OzT {
-  static constexpr int NSET = (int)OZ_TMEM_COLS / (OZ_NACC * BN);
+  static_assert(OZ_NACC * BN == (int)OZ_TMEM_COLS, "the accumulators fill the tensor memory");
   static constexpr int EPI = BN * 4 / OZ_EPI_WARPS;           // columns per epilogue thread
   static constexpr int QB = OZ_BM / BN;                       // B tiles per 128-row digit block
   static constexpr uint32_t B_DIGIT = BN * OZ_BK * 2;         // one digit of a B tile per K step
@@ -95,9 +98,10 @@ struct OzT {
   static constexpr uint32_t STAGE = A_BYTES + S * B_DIGIT;
   static constexpr int NBUF = S == 7 ? 5 : 4;                 // stages: 215040 or 196608 B
   static constexpr uint32_t SMEM = NBUF * STAGE;
-  // kind::f16: FP32 accumulator, bf16 A and B, both K-major, N = BN, M = 128
-  static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
-                                    ((uint32_t)(OZ_BM >> 4) << 24);
+  // kind::f16: FP32 accumulator, bf16 A and B, both K-major, N = nd digits of BN, M = 128
+  static constexpr uint32_t idesc(int nd) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nd * BN >> 3) << 17) | ((uint32_t)(OZ_BM >> 4) << 24);
+  }
 };
 constexpr int OZ_MAXBUF = 5;
 
@@ -139,23 +143,14 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, 128 x BN x 16, bf16 -> FP32.  A run of MMAs on the same A
-// block reads it from shared memory once: the first fills the A collector buffer, the others
-// use it, the last one gives it up.
-enum { COLL_FILL = 0, COLL_USE = 1, COLL_LAST = 2 };
-template <int COLL>
+// D[tmem] (+)= A[smem] * B[smem]^T, 128 x N x 16, bf16 -> FP32
 __device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-#define FG_TC_MMA(C)                                                                   \
-  asm volatile(                                                                        \
-      "{\n\t.reg .pred p;\n\t"                                                         \
-      "setp.ne.b32 p, %4, 0;\n\t"                                                      \
-      "tcgen05.mma.cta_group::1.kind::f16.collector::a::" C " [%0], %1, %2, %3, p;\n\t}" \
-      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc)                                   \
-      : "memory")
-  if (COLL == COLL_FILL) FG_TC_MMA("fill");
-  else if (COLL == COLL_USE) FG_TC_MMA("use");
-  else FG_TC_MMA("lastuse");
-#undef FG_TC_MMA
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(acc)
+      : "memory");
 }
 // arrive on the mbarrier once every tcgen05 operation issued so far by this thread is done
 __device__ __forceinline__ void tc_commit(uint32_t mbar) {
@@ -377,33 +372,33 @@ __device__ __forceinline__ OzItem item_of(const OzGemmArgs& g, int t) {
   return g.items[lo];
 }
 
-// x 2^off as FP64, for |x| < 2^53 (exact) and an exponent that stays normal, by integer
-// operations on the bit pattern (no FP64 operation)
-__device__ __forceinline__ double i64_to_f64(long long x, int off) {
-  if (x == 0) return 0.0;
-  const unsigned long long sgn = x < 0 ? (1ull << 63) : 0ull;
-  const unsigned long long a = x < 0 ? (unsigned long long)(-x) : (unsigned long long)x;
-  const int lz = __clzll((long long)a);
-  const unsigned long long mant = (a << (lz + 1)) >> 12;  // the bits after the leading one
-  return __longlong_as_double((long long)(sgn | ((unsigned long long)(63 - lz + 1023 + off) << 52) | mant));
+// (h 2^32 + l) 2^(off - 72) as FP64, rounded to nearest (ties to even), the sign flipped by flip =
+// 2^31, by integer operations and without a branch (the columns' chains then overlap).  slow: the
+// result is not a normal FP64 number; sum_slow does it.
+__device__ __forceinline__ double sum_f64(long long h, uint32_t l, int off, uint32_t flip, bool& slow) {
+  const uint32_t sgn = (uint32_t)(h >> 63);  // 0 or all ones: |x| = (x ^ sgn) - sgn
+  const unsigned long long lo = (unsigned long long)(l ^ sgn) + (sgn & 1u);
+  const unsigned long long a = ((unsigned long long)h ^ (unsigned long long)(h >> 63)) + (lo >> 32);
+  const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a, al2 = (uint32_t)lo;
+  // the upper word with the leading bit (a2), and the two after it
+  const uint32_t b2 = al ? al : al2, b1 = al ? al2 : 0u;
+  const uint32_t a2 = ah ? ah : b2, a1 = ah ? al : b1, a0 = ah ? al2 : 0u;
+  const int lz = __clz((int)a2);  // 32: the sum is zero
+  const uint32_t n2 = __funnelshift_l(a1, a2, lz), n1 = __funnelshift_l(a0, a1, lz), n0 = a0 << (lz & 31);
+  const int e = off + (1023 + 95 - 72) - (ah ? 0 : (al ? 32 : 64)) - lz;  // biased exponent of the leading bit
+  slow = a2 != 0 && (unsigned)(e - 1) > 2044u;                            // 2046 could round up to infinity
+  const unsigned long long m = ((unsigned long long)n2 << 21) | (n1 >> 11);  // 53 bits, the leading one included
+  // half an ulp is 0x400 of the 11 bits left; the bits below them and an odd m break the tie
+  const uint32_t up = ((n1 & 0x7FFu) * 2 + (n0 != 0 ? 1u : 0u) + ((uint32_t)m & 1u)) > 0x800u ? 1u : 0u;
+  const uint32_t top = a2 != 0 ? ((uint32_t)(e - 1) << 20) + ((sgn ^ flip) & 0x80000000u) : 0u;
+  return __longlong_as_double((long long)(m + up + ((unsigned long long)top << 32)));
 }
 
-// d 2^off by adding off to the exponent field; false if d or the result is not a normal
-// FP64 number (zero passes).
-__device__ __forceinline__ bool scale_f64(double d, int off, double& r) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(d);
-  const int e = (int)((b >> 52) & 0x7FF);
-  if ((b << 1) == 0) {
-    r = d;
-    return true;
-  }
-  if (e == 0 || e == 0x7FF || e + off < 1 || e + off > 2046) return false;
-  r = __longlong_as_double((long long)(b + ((unsigned long long)(long long)off << 52)));
-  return true;
+// the same for any sum (kept out of line: it costs FP64 operations)
+__device__ __noinline__ double sum_slow(long long h, uint32_t l, int off, uint32_t flip) {
+  bool slow;
+  return ldexp(sum_f64(h, l, 0, flip, slow), off);
 }
-
-// out-of-range fallback of scale_f64 (kept out of line: it costs FP64 operations)
-__device__ __noinline__ double scale_slow(double d, int off) { return ldexp(d, off); }
 
 // Persistent: CTA b takes the output tiles b, b + gridDim.x, ... of all items (tiles above
 // the diagonal skipped when lower).  The accumulators are released as soon as the epilogue
@@ -413,7 +408,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
   using T = OzT<BN, S>;
   constexpr int OZ_NBUF = T::NBUF;
   extern __shared__ __align__(1024) uint8_t oz_smem[];
-  __shared__ __align__(8) uint64_t bar_full[OZ_MAXBUF], bar_empty[OZ_MAXBUF], bar_acc_full[2], bar_acc_empty[2];
+  __shared__ __align__(8) uint64_t bar_full[OZ_MAXBUF], bar_empty[OZ_MAXBUF], bar_acc_full[2], bar_acc_empty[2], bar_stop;
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int abort_flag;
 
@@ -446,8 +441,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
       }
       for (int z = 0; z < 2; ++z) {
         mbar_init(smem_u32(&bar_acc_full[z]), 1);
-        mbar_init(smem_u32(&bar_acc_empty[z]), OZ_EPI_WARPS * 32);
+        mbar_init(smem_u32(&bar_acc_empty[z]), OZ_EPI_WARPS);
       }
+      mbar_init(smem_u32(&bar_stop), 1);
       abort_flag = 0;
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -464,49 +460,72 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
     // MMA warp.  The whole warp runs the loop and one elected lane issues: the descriptors then
     // stay in uniform registers.  (Issued from a branch on lane == 0, an MMA cost ~80 cycles
     // of moves to the uniform registers, more than the 32 it runs.)
+    //
+    // An MMA takes an A digit against up to four B digits: digits t, t + 1, .. of the stage are
+    // consecutive rows of one operand and their classes s + t, .. consecutive accumulators.
+    // The K steps of a chunk go in groups of NBUF stages, per group first the classes 0-3 (lo) of
+    // every stage, then the classes 4-7 (hi), each half with its own pair of barriers: the
+    // epilogue takes the lo sums out while the last group's hi MMAs run, and the hi sums while
+    // the next chunk's lo MMAs do.
     bool ok = true;
     int gs = 0, gc = 0;
+    const uint64_t d0 = smem_desc(sbase);
     for (int t = first; t < ntiles && ok; t = next_tile(t)) {
-      for (int ks = 0; ks < KS; ++ks) {
-        const int kin = ks % g.chunk;
-        const int buf = gs % OZ_NBUF;
-        const int z = gc % T::NSET;  // accumulator set of this chunk
-        if (kin == 0 && gc >= T::NSET)
-          ok = mbar_wait(smem_u32(&bar_acc_empty[z]), ((gc / T::NSET) - 1) & 1, &abort_flag, g.err);
-        ok = ok && mbar_wait(smem_u32(&bar_full[buf]), (gs / OZ_NBUF) & 1, &abort_flag, g.err);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t sa = sbase + buf * T::STAGE, sb = sa + T::A_BYTES;
-        const uint64_t da = smem_desc(sa), db = smem_desc(sb);
-        const uint32_t tacc = tmem + z * (OZ_NACC * BN);
-        const bool last = kin == g.chunk - 1 || ks == KS - 1;
-        if (elect_one()) {
-          // A digit by A digit: the digit stays in the collector buffer for its run; the first
-          // pair of a class starts the chunk's sum
+      for (int c0 = 0; c0 < KS && ok; c0 += g.chunk, ++gc) {
+        const int c1 = min(KS, c0 + g.chunk);
+        for (int g0 = c0; g0 < c1 && ok; g0 += OZ_NBUF) {
+          const int ng = min(OZ_NBUF, c1 - g0);
+          const bool last = g0 + ng == c1;
 #pragma unroll
-          for (int s = 0; s < S; ++s)
+          for (int half = 0; half < 2; ++half) {
+            if (g0 == c0 && gc > 0 && ok)
+              ok = mbar_wait(smem_u32(&bar_acc_empty[half]), (gc - 1) & 1, &abort_flag, g.err);
+            for (int q = 0; q < ng; ++q) {
+              const int buf = (gs + q) % OZ_NBUF;
+              if (half == 0) ok = ok && mbar_wait(smem_u32(&bar_full[buf]), ((gs + q) / OZ_NBUF) & 1, &abort_flag, g.err);
+              ok = __all_sync(0xffffffffu, ok);
+              if (!ok) break;
+              tc_fence_after();
+              if (elect_one()) {
+                const uint64_t da = d0 + (uint64_t)((uint32_t)buf * (T::STAGE >> 4)), db = da + (T::A_BYTES >> 4);
+                // the first pair of a class starts the chunk's sum: s = 0, and s = 1 for class 7
+                // of S = 7 (t = 6), which then goes by itself
+                const uint32_t cont = g0 + q > c0 ? 1u : 0u;
+                auto mma = [&](int s, int t0, int nd, uint32_t acc) {
+                  tc_mma(tmem + (s + t0) * BN, da + (uint64_t)(s * (OZ_BLOCK >> 4)),
+                         db + (uint64_t)(t0 * (T::B_DIGIT >> 4)), T::idesc(nd), acc);
+                };
+                if (half == 0) {
 #pragma unroll
-            for (int kk = s; kk < OZ_NACC && kk - s < S; ++kk) {
-              const bool end = kk + 1 == OZ_NACC || kk + 1 - s == S;
-              // start-address field in 16-byte units
-              const uint32_t d = tacc + kk * BN;
-              const uint64_t ad = da + (uint64_t)(s * (OZ_BLOCK >> 4)), bd = db + (uint64_t)((kk - s) * (T::B_DIGIT >> 4));
-              const uint32_t acc = (kin > 0 || s > (kk > S - 1 ? kk - (S - 1) : 0)) ? 1u : 0u;
-              if (kk == s) tc_mma<COLL_FILL>(d, ad, bd, T::IDESC, acc);
-              else if (!end) tc_mma<COLL_USE>(d, ad, bd, T::IDESC, acc);
-              else tc_mma<COLL_LAST>(d, ad, bd, T::IDESC, acc);
+                  for (int s = 0; s < 4; ++s) mma(s, 0, 4 - s, s == 0 ? cont : 1u);
+                } else {
+#pragma unroll
+                  for (int s = 0; s < S; ++s) {
+                    const int t0 = s < 4 ? 4 - s : 0, t1 = 7 - s < S - 1 ? 7 - s : S - 1;
+                    if (S == 7 && s == 1 && cont == 0) {
+                      mma(s, t0, t1 - t0, 1u);
+                      mma(s, t1, 1, 0u);
+                    } else {
+                      mma(s, t0, t1 - t0 + 1, s == 0 ? cont : 1u);
+                    }
+                  }
+                  tc_commit(smem_u32(&bar_empty[buf]));
+                }
+                if (last && q == ng - 1) tc_commit(smem_u32(&bar_acc_full[half]));
+              }
+              __syncwarp();
             }
-          tc_commit(smem_u32(&bar_empty[buf]));
-          if (last) tc_commit(smem_u32(&bar_acc_full[z]));
+          }
+          gs += ng;
         }
-        __syncwarp();
-        if (last) ++gc;
-        ++gs;
       }
     }
     // after an abort: every MMA issued
-    if (!ok && gs > 0) mbar_drain(smem_u32(&bar_empty[(gs - 1) % OZ_NBUF]), ((gs - 1) / OZ_NBUF) & 1);
+    if (!ok) {
+      if (elect_one()) tc_commit(smem_u32(&bar_stop));
+      __syncwarp();
+      mbar_drain(smem_u32(&bar_stop), 0);
+    }
     __syncwarp();
   } else if (warp == OZ_EPI_WARPS + 1) {
     // copy warp: lane 0 streams the stages
@@ -554,6 +573,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
     // much as the element's arithmetic)
     const int amode = g.alpha == -1.0 ? 0 : (g.alpha == 1.0 ? 1 : 2);
     const int bmode = g.beta == 0.0 ? 0 : (g.beta == 1.0 ? 1 : 2);
+    const uint32_t flip = amode == 0 ? 0x80000000u : 0u;
     int gc = 0;
     for (int t = first; t < ntiles; t = next_tile(t)) {
       if (bmode != 0) {
@@ -562,105 +582,106 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
         int rt, ct;
         it.locate(t, rt, ct);
         const int i = rt * OZ_BM + row, c0 = ct * BN + part4 * OZ_EPI_COLS;
-        const double* p = it.c + (int64_t)i * it.c_rs;
-        if (i < it.m)
+        const int nv = i < it.m ? min(it.n - c0, g.lower ? i - c0 + 1 : OZ_EPI_COLS) : 0;
+        const double* p = it.c + (int64_t)i * it.c_rs + (int64_t)c0 * it.c_cs;
 #pragma unroll
-          for (int j = 0; j < OZ_EPI_COLS; ++j)
-            if (c0 + j < it.n && !(g.lower && c0 + j > i))
-              asm volatile("prefetch.global.L2 [%0];" ::"l"(p + (int64_t)(c0 + j) * it.c_cs));
+        for (int j = 0; j < OZ_EPI_COLS; ++j)
+          if (j < nv) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + (int64_t)j * it.c_cs));
       }
-      // per column: sum over K chunks of the chunk's product / 2^(e_i + f_j - 16), in FP64
-      double acc[OZ_EPI_COLS];
+      // per column: the product / 2^(e_i + f_j - 16) as an exact integer H 2^-24 + L 2^-56 over
+      // all K chunks (|H| < 2^44 per chunk, at most 2^16 K steps), three registers
+      long long H[OZ_EPI_COLS];
+      uint32_t L[OZ_EPI_COLS];
+#pragma unroll
+      for (int j = 0; j < OZ_EPI_COLS; ++j) {
+        H[j] = 0;
+        L[j] = 0;
+      }
       bool ok = true;
       for (int chunk = 0; chunk < nchunks; ++chunk, ++gc) {
-        const int z = gc % T::NSET;
-        if (!mbar_wait(smem_u32(&bar_acc_full[z]), (gc / T::NSET) & 1, &abort_flag, g.err)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t trow = trow0 + z * (OZ_NACC * BN);
-        // sum_k v_k 2^(-8k) = H 2^-24 + L 2^-56 exactly (every v_k is an integer below 2^24 held
-        // in FP32): |H| < 2^50 and 0 <= L < 2^32, three registers per column
-        long long H[OZ_EPI_COLS];
-        uint32_t L[OZ_EPI_COLS];
+        // sum_k v_k 2^(-8k), every v_k an integer below 2^24 held in FP32
 #pragma unroll
-        for (int cb = 0; cb < OZ_EPI_COLS / 8; ++cb) {
+        for (int half = 0; half < 2; ++half) {
+          ok = ok && mbar_wait(smem_u32(&bar_acc_full[half]), gc & 1, &abort_flag, g.err);
+          if (!ok) break;
+          tc_fence_after();
 #pragma unroll
-          for (int part = 0; part < 2; ++part) {
+          for (int cb = 0; cb < OZ_EPI_COLS / 8; ++cb) {
             uint32_t v[OZ_NACC / 2][8];
 #pragma unroll
-            for (int q = 0; q < OZ_NACC / 2; ++q) tc_ld8(trow + (part * 4 + q) * BN + cb * 8, v[q]);
+            for (int q = 0; q < OZ_NACC / 2; ++q) tc_ld8(trow0 + (half * 4 + q) * BN + cb * 8, v[q]);
             tc_wait_ld();
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
               int a[OZ_NACC / 2];
 #pragma unroll
               for (int q = 0; q < OZ_NACC / 2; ++q) a[q] = __float2int_rn(__uint_as_float(v[q][j]));
-              if (part == 0) {
-                // |a0| < 2^19.5, |a1| < 2^21.5, |a2| < 2^22.5, |a3| < 2^23: each pair fits 32 bits
-                H[cb * 8 + j] = (long long)(a[0] * 256 + a[1]) * 65536 + (a[2] * 256 + a[3]);
+              // as multiply-adds into 64 bits (|a0| < 2^19.5, |a1| < 2^21.5, |a2| < 2^22.5,
+              // |a3| < 2^23: those two pairs fit 32 bits)
+              long long& h = H[cb * 8 + j];
+              if (half == 0) {
+                h += (long long)(a[0] * 256 + a[1]) * 65536;
+                h += a[2] * 256 + a[3];
               } else {
-                const long long x = ((long long)a[0] * 256 + a[1]) * 65536 + ((long long)a[2] * 256 + a[3]);
-                H[cb * 8 + j] += x >> 32;
+                long long x = (long long)a[0] * 16777216 + (long long)(unsigned long long)L[cb * 8 + j];
+                x += (long long)a[1] * 65536;
+                x += (long long)a[2] * 256;
+                x += a[3];
+                h += x >> 32;
                 L[cb * 8 + j] = (uint32_t)x;
               }
             }
           }
+          tc_fence_before();
+          __syncwarp();
+          // accumulators free: the next MMAs on them may start
+          if (lane == 0) mbar_arrive(smem_u32(&bar_acc_empty[half]));
         }
-        tc_fence_before();
-        mbar_arrive(smem_u32(&bar_acc_empty[z]));  // accumulators free: the next MMAs may start
-        // keeps the conversion below the release (volatile statements stay in order)
-#pragma unroll
-        for (int j = 0; j < OZ_EPI_COLS; ++j) asm volatile("" : "+l"(H[j]), "+r"(L[j]));
-#pragma unroll
-        for (int j = 0; j < OZ_EPI_COLS; ++j) {
-          // xl = 2^-4 + L 2^-56 is a bit pattern (the ulp of 2^-4 is 2^-56); xh takes the 2^-4
-          // (2^20 units of 2^-24) away again, exactly: one FP64 rounding for the chunk
-          const double xl = __hiloint2double(0x3FB00000, (int)L[j]);
-          const double xh = i64_to_f64(H[j] - (1ll << 20), -24);
-          acc[j] = chunk == 0 ? xh + xl : acc[j] + (xh + xl);
-        }
+        if (!ok) break;
       }
+#pragma unroll
+      for (int j = 0; j < OZ_EPI_COLS; ++j)
+        // keeps the update of C below the release (volatile statements stay in order)
+        asm volatile("" : "+l"(H[j]), "+r"(L[j]));
       if (!ok) break;
       const OzItem it = item_of(g, t);
       int rt, ct;
       it.locate(t, rt, ct);
       const int i = rt * OZ_BM + row;
-      const bool row_ok = i < it.m;
-      const int ei = g.ex[(int64_t)(it.arow0 + rt) * OZ_BM + row];
       const int c0 = ct * BN + part4 * OZ_EPI_COLS;
+      const int ei = g.ex[(int64_t)(it.arow0 + rt) * OZ_BM + row];
       // lane j < EPI holds the exponent of column c0 + j (padding rows of the exponents are 0)
       const int ecol = g.ex[(int64_t)(it.brow0 + ct / T::QB) * OZ_BM + (ct % T::QB) * BN + part4 * OZ_EPI_COLS +
                             (lane < OZ_EPI_COLS ? lane : 0)];
-      double* crow = it.c + (int64_t)i * it.c_rs;
+      const int nv = i < it.m ? min(it.n - c0, g.lower ? i - c0 + 1 : OZ_EPI_COLS) : 0;  // columns to write
+      double* crow = it.c + (int64_t)i * it.c_rs + (int64_t)c0 * it.c_cs;
 #pragma unroll
       for (int j0 = 0; j0 < OZ_EPI_COLS; j0 += 8) {
-        // eight columns at a time: their exponents and C values are loaded before any store
-        int off[8];
-        double cv[8];
-        bool w[8];
+        // eight columns at a time: their C values are loaded before any store
+        double cv[8], xs[8];
+        bool any = false;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) cv[j] = (j0 + j < nv && bmode != 0) ? crow[(int64_t)(j0 + j) * it.c_cs] : 0.0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const int col = c0 + j0 + j;
-          w[j] = row_ok && col < it.n && !(g.lower && col > i);
-          off[j] = ei + __shfl_sync(0xffffffffu, ecol, j0 + j);
-          cv[j] = (w[j] && bmode != 0) ? crow[(int64_t)col * it.c_cs] : 0.0;
+          bool slow;  // x = (-)(H 2^(off - 40) + L 2^(off - 72))
+          xs[j] = sum_f64(H[j0 + j], L[j0 + j], ei + __shfl_sync(0xffffffffu, ecol, j0 + j), flip, slow);
+          any |= slow;
         }
+        if (__any_sync(0xffffffffu, any))
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (!w[j]) continue;
-          // product = 2^(e_i + f_j - 16) acc: a power of two, applied to the exponent field
-          double x;
-          if (!scale_f64(acc[j0 + j], off[j] - 16, x)) x = scale_slow(acc[j0 + j], off[j] - 16);
-          double r;
-          if (bmode == 0) {
-            r = amode == 0 ? -x : (amode == 1 ? x : g.alpha * x);
-          } else {
-            const double base = bmode == 1 ? cv[j] : g.beta * cv[j];
-            r = amode == 0 ? base - x : (amode == 1 ? base + x : fma(g.alpha, x, base));
-          }
-          crow[(int64_t)(c0 + j0 + j) * it.c_cs] = r;
+          for (int j = 0; j < 8; ++j)
+            xs[j] = sum_slow(H[j0 + j], L[j0 + j], ei + __shfl_sync(0xffffffffu, ecol, j0 + j), flip);
+        if (amode != 2 && bmode != 2) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (j0 + j < nv) crow[(int64_t)(j0 + j) * it.c_cs] = bmode == 0 ? xs[j] : cv[j] + xs[j];
+        } else {
+          const double alpha = amode == 0 ? 1.0 : g.alpha;  // -1: in the sign already
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (j0 + j < nv)
+              crow[(int64_t)(j0 + j) * it.c_cs] = bmode == 0 ? alpha * xs[j] : fma(alpha, xs[j], bmode == 1 ? cv[j] : g.beta * cv[j]);
         }
       }
     }

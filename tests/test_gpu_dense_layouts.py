@@ -71,3 +71,21 @@ def test_lower(env, m, k):
         low = np.tril(np.ones((m, m), dtype=bool))
         assert np.all(np.abs(got - want)[low] <= tol[low])
         assert np.array_equal(got[~low], C0[~low])
+
+
+@pytest.mark.parametrize("p,q", [(0, 0), (-700, -350), (520, 503), (40, -31)])
+def test_sum_to_fp64(env, p, q):
+    """The integer sum's way to FP64, exactly: sums that cancel down to the last digit, of both
+    signs, zero, and results that are subnormal or close to overflow (rows are cut 56 bits below a
+    power of two above their largest value, so 2^-i for i <= 53 beside 1 is exact)."""
+    ctx, dense, torch = env
+    i = np.arange(54)
+    A = np.zeros((109, 3))
+    A[:54], A[54:108] = [1.0, -1.0, 0.0], [1.0, -1.0, 0.0]
+    A[:54, 2], A[54:108, 2] = np.ldexp(1.0, -i), -np.ldexp(1.0, -i)
+    B = np.ones((65, 3))
+    for sign in (1.0, -1.0):
+        C = dense.gemm_nt(ctx, torch.from_numpy(np.ldexp(A, p)).cuda(), torch.from_numpy(np.ldexp(B, q)).cuda(),
+                          torch.zeros((109, 65), dtype=torch.float64, device="cuda"), alpha=sign)
+        want = sign * np.ldexp(A[:, 2], p + q)
+        assert np.array_equal(C.cpu().numpy(), np.repeat(want[:, None], 65, axis=1))
