@@ -24,8 +24,9 @@
 //    replaces it (reliable update, the direction is kept).
 //  * One persistent cooperative launch.  A host planner orders the problems by estimated
 //    work and gives each a team of co-resident CTAs (one CTA for most problems); team
-//    members synchronise through a counter in global memory with a bounded spin, and sum
-//    their per-CTA partials in rank order (deterministic for a given plan).
+//    members synchronise through a counter in global memory with a bounded spin; one warp sums
+//    the per-CTA partials in a fixed order (deterministic for a given plan) and one thread does
+//    the scalar step (96 problems, n 8-24: 155 -> 99 ms).
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -135,12 +136,6 @@ struct Kf {
   __device__ __forceinline__ double val() const { return (double)s - (double)c; }
 };
 
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
 struct BatchSmem {
   __align__(16) float sh[kMaxBox];
   __align__(16) float sl[kMaxBox];
@@ -148,26 +143,11 @@ struct BatchSmem {
   int blo[kMaxCls][3], bw[kMaxCls][3];
   float dinv[kMaxCls];
   double mw[(kBatchMaxP + 1) * (kBatchMaxP + 1)];
-  double red[32][4];
-  double tot[4];
+  double red[16][2];
+  float alpha, beta;
+  int flag;
   int abort_flag;
 };
-
-// Block sum of nv doubles; result in sm.tot (all threads, after the call).
-__device__ void block_sum(double* v, int nv, BatchSmem& sm) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int k = 0; k < nv; ++k) {
-    double a = warp_sum_d(v[k]);
-    if (lane == 0) sm.red[warp][k] = a;
-  }
-  __syncthreads();
-  if (threadIdx.x < nv) {
-    double s = 0.0;
-    for (int w = 0; w < nw; ++w) s += sm.red[w][threadIdx.x];
-    sm.tot[threadIdx.x] = s;
-  }
-  __syncthreads();
-}
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -181,50 +161,89 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   return v;
 }
 
-// Team reduction of nv values: CTA partials into slot, barrier, ranks summed in order.
-// Returns false if the barrier gave up (status set).
-__device__ bool team_sum(const BatchArgs& a, const BatchProb& P, int prob, int rank, int& phase, double* v, int nv,
-                         BatchSmem& sm, double* out) {
-  block_sum(v, nv, sm);
-  if (P.team == 1) {
-    for (int k = 0; k < nv; ++k) out[k] = sm.tot[k];
-    return true;
-  }
-  double* slot = a.rpool + P.roff + (int64_t)(phase % 3) * P.team * 4;
-  if (threadIdx.x < nv) slot[rank * 4 + threadIdx.x] = sm.tot[threadIdx.x];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    if (!(a.drop_arrival && rank == 1 && phase == 0)) atomicAdd(a.bar + prob, 1u);
-    const unsigned target = (unsigned)(phase + 1) * (unsigned)P.team;
-    const unsigned long long t0 = global_ns();
-    int ok = 1;
-    while (ld_acquire(a.bar + prob) < target) {
-      if (*(volatile int*)a.abort_all || global_ns() - t0 > a.timeout_ns) { ok = 0; break; }
-      __nanosleep(256);
-    }
-    __threadfence();
-    sm.abort_flag = ok ? 0 : 1;
-    if (!ok) {
+// Arrive at the team's barrier and wait for the others (one thread).  False if the wait gave up
+// (status set).
+__device__ bool team_arrive_wait(const BatchArgs& a, const BatchProb& P, int prob, int rank, int phase) {
+  __threadfence();
+  if (!(a.drop_arrival && rank == 1 && phase == 0)) atomicAdd(a.bar + prob, 1u);
+  const unsigned target = (unsigned)(phase + 1) * (unsigned)P.team;
+  const unsigned long long t0 = global_ns();
+  while (ld_acquire(a.bar + prob) < target) {
+    if (*(volatile int*)a.abort_all || global_ns() - t0 > a.timeout_ns) {
       atomicExch(a.status + prob, (int)FG_ERR_TIMEOUT);
       atomicExch(a.abort_all, 1);
+      return false;
+    }
+    __nanosleep(32);
+  }
+  __threadfence();
+  return true;
+}
+
+// Team reduction of NV (1 or 2) values, then post(totals) on thread 0, whose results in shared
+// memory every thread sees after the call.  Returns false if the barrier gave up.
+// FP64 is scarce here (a warp's FP64 instruction holds the SM's pipe 16 cycles), so nothing is
+// summed or divided by more than one warp: two values share a butterfly (lanes 0-15 go on with the
+// first, 16-31 with the second), warp 0 alone adds the warps' sums, writes the CTA's partial,
+// waits, adds the team's partials (16 lanes per value) and thread 0 does the scalar step.  With
+// every thread adding the partials of all ranks, a team of 89 spent ~25 us per reduction.
+template <int NV, class Post>
+__device__ bool team_sum(const BatchArgs& a, const BatchProb& P, int prob, int rank, int& phase, const double* v,
+                         BatchSmem& sm, Post post) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int k = lane >> 4;  // value of this half warp (NV = 2)
+  double x;
+  if (NV == 2) {
+    const double give = k ? v[0] : v[1], keep = k ? v[1] : v[0];
+    x = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+  } else {
+    x = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+  }
+  auto half_sum = [](double y) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+    return y;
+  };
+  x = half_sum(x);
+  if ((lane & 15) == 0 && k < NV) sm.red[warp][k] = x;
+  __syncthreads();
+  if (warp == 0) {
+    x = half_sum((lane & 15) < nw && k < NV ? sm.red[lane & 15][k] : 0.0);
+    bool ok = true;
+    if (P.team > 1) {
+      double* slot = a.rpool + P.roff + (int64_t)(phase % 3) * P.team * 4;
+      if ((lane & 15) == 0 && k < NV) slot[rank * 4 + k] = x;
+      __syncwarp();
+      if (lane == 0) ok = team_arrive_wait(a, P, prob, rank, phase);
+      ok = __shfl_sync(0xffffffffu, ok, 0);
+      x = 0.0;
+      if (ok && k < NV)
+#pragma unroll 4
+        for (int r = lane & 15; r < P.team; r += 16) x += ((volatile double*)slot)[r * 4 + k];
+      x = half_sum(x);
+    }
+    const double y = __shfl_sync(0xffffffffu, x, 16);
+    if (lane == 0) {
+      sm.abort_flag = ok ? 0 : 1;
+      if (ok) post(x, y);
     }
   }
   __syncthreads();
   ++phase;
-  if (sm.abort_flag) return false;
-  for (int k = 0; k < nv; ++k) {
-    double s = 0.0;
-    for (int r = 0; r < P.team; ++r) s += ((volatile double*)slot)[r * 4 + k];
-    out[k] = s;
-  }
-  return true;
+  return !sm.abort_flag;
 }
 
 // Barrier without values (phases shared with team_sum).
 __device__ bool team_sync(const BatchArgs& a, const BatchProb& P, int prob, int rank, int& phase, BatchSmem& sm) {
-  double dummy[1] = {0.0}, o[1];
-  return team_sum(a, P, prob, rank, phase, dummy, 1, sm, o);
+  __syncthreads();
+  if (P.team > 1) {
+    if (threadIdx.x == 0) sm.abort_flag = team_arrive_wait(a, P, prob, rank, phase) ? 0 : 1;
+    __syncthreads();
+  } else if (threadIdx.x == 0) {
+    sm.abort_flag = 0;
+  }
+  ++phase;
+  return P.team == 1 || !sm.abort_flag;
 }
 
 // Cell load vectors E_c[a] = (h/2)^3 sum_q w_q f_q phi_a(q) by sum factorisation, FP64, cells [c0, c1).
@@ -508,14 +527,19 @@ __device__ void solve_problem(const BatchArgs& a, int prob, int rank, BatchSmem&
     loc[0] = bb;
     loc[1] = rz.val();
   }
-  double red[4];
-  if (!team_sum(a, P, prob, rank, phase, loc, 2, sm, red)) return;
-  const double bnorm = sqrt(red[0]);
-  double rzv = red[1];
-  double rtrue2 = red[0];
-  const double tol = a.rtol * bnorm + a.atol;
-  int it = 0, nref = 0, conv = bnorm <= a.atol ? 1 : 0;
-  double relres = 1.0;
+  // the scalars of the iteration live on thread 0; alpha, beta and what to do next go through
+  // shared memory
+  enum { STEP = 0, REFINE = 1, BREAKDOWN = 2, CONVERGED = 3 };
+  double bnorm = 0.0, rzv = 0.0, rtrue2 = 0.0, tol = 0.0, relres = 1.0;
+  if (!team_sum<2>(a, P, prob, rank, phase, loc, sm, [&](double t0, double t1) {
+        bnorm = sqrt(t0);
+        rzv = t1;
+        rtrue2 = t0;
+        tol = a.rtol * bnorm + a.atol;
+        sm.flag = bnorm <= a.atol ? CONVERGED : STEP;
+      }))
+    return;
+  int it = 0, nref = 0, conv = sm.flag == CONVERGED ? 1 : 0;
   const float khf = P.kh_hi;
   while (!conv && it < a.max_iters) {
     ++it;
@@ -542,12 +566,16 @@ __device__ void solve_problem(const BatchArgs& a, int prob, int rank, BatchSmem&
       }
       loc[0] = pq.val();
     }
-    if (!team_sum(a, P, prob, rank, phase, loc, 1, sm, red)) return;
-    if (!(red[0] > 0.0)) {
+    if (!team_sum<1>(a, P, prob, rank, phase, loc, sm, [&](double pq, double) {
+          sm.flag = pq > 0.0 ? STEP : BREAKDOWN;
+          if (pq > 0.0) sm.alpha = (float)(rzv / pq);
+        }))
+      return;
+    if (sm.flag == BREAKDOWN) {
       if (threadIdx.x == 0 && rank == 0) atomicExch(a.status + prob, (int)FG_ERR_NUMERIC);
       break;
     }
-    const float alpha = (float)(rzv / red[0]);
+    const float alpha = sm.alpha;
     {
       Kf rr, rzn;
       for (NodeWalk w((int)u0, (int)u1, F, L); w.ok(); w.next()) {
@@ -563,11 +591,18 @@ __device__ void solve_problem(const BatchArgs& a, int prob, int rank, BatchSmem&
       loc[0] = rr.val();
       loc[1] = rzn.val();
     }
-    if (!team_sum(a, P, prob, rank, phase, loc, 2, sm, red)) return;
-    double rzn = red[1];
-    const double rr = red[0];
-    const bool near = rr <= 0.25 * tol * tol;
-    if (rr <= (double)a.delta * (double)a.delta * rtrue2 || near || it >= a.max_iters) {
+    if (!team_sum<2>(a, P, prob, rank, phase, loc, sm, [&](double rr, double rzn) {
+          const bool near = rr <= 0.25 * tol * tol;
+          if (rr <= (double)a.delta * (double)a.delta * rtrue2 || near || it >= a.max_iters) {
+            sm.flag = REFINE;
+          } else {
+            sm.flag = STEP;
+            sm.beta = (float)(rzn / rzv);
+            rzv = rzn;
+          }
+        }))
+      return;
+    if (sm.flag == REFINE) {
       // reliable update: x += xc (float-float), then r = b - A x in float-float
       for (NodeWalk w((int)u0, (int)u1, F, L); w.ok(); w.next()) {
         const int64_t g = w.g;
@@ -604,18 +639,21 @@ __device__ void solve_problem(const BatchArgs& a, int prob, int rank, BatchSmem&
       }
       loc[0] = rr2.val();
       loc[1] = rz2.val();
-      if (!team_sum(a, P, prob, rank, phase, loc, 2, sm, red)) return;
       ++nref;
-      rtrue2 = red[0];
-      rzn = red[1];
-      relres = bnorm > 0.0 ? sqrt(rtrue2) / bnorm : 0.0;
-      if (sqrt(rtrue2) <= tol) {
+      if (!team_sum<2>(a, P, prob, rank, phase, loc, sm, [&](double rr, double rzn) {
+            rtrue2 = rr;
+            relres = bnorm > 0.0 ? sqrt(rtrue2) / bnorm : 0.0;
+            sm.flag = sqrt(rtrue2) <= tol ? CONVERGED : STEP;
+            sm.beta = (float)(rzn / rzv);
+            rzv = rzn;
+          }))
+        return;
+      if (sm.flag == CONVERGED) {
         conv = 1;
         break;
       }
     }
-    const float beta = (float)(rzn / rzv);
-    rzv = rzn;
+    const float beta = sm.beta;
     for (NodeWalk w((int)u0, (int)u1, F, L); w.ok(); w.next()) {
       const int I = w.I, J = w.J, K = w.K;
       const int64_t g = w.g;
