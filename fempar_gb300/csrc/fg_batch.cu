@@ -13,13 +13,13 @@
 //    (h/2) k (s x m x m + m x s x m + m x m x s) for the 1D Gauss-integrated mass m and
 //    stiffness s of the reference element (the reference's structured-mesh path reuses the
 //    first cell's Jacobian the same way, sbm_cell_map.i90:272-320), so the assembled
-//    operator is a stencil per node class (I mod p, J mod p, K mod p) built from the 1D
-//    assembled matrices: nothing is stored per nonzero.
+//    operator is Sx My Mz + Mx Sy Mz + Mx My Sz in the 1D assembled matrices (rows per node class
+//    I mod p), applied one direction after the other: nothing is stored per nonzero.
 //  * Right-hand side assembled in the kernel: each cell's load vector by sum factorisation
 //    in FP64, gathered per node over its cells in increasing cell order.
 //  * Mixed precision without the FP64 pipe in the loop: the inner CG runs in FP32; the
 //    solution, the right-hand side and the true residual b - A x are kept in float-float
-//    (pairs of FP32, ~2^-48 relative), the stencil applied with error-free FP32 products.
+//    (pairs of FP32, ~2^-48 relative), the operator applied with error-free FP32 products.
 //    Every time the FP32 recursive residual has dropped 10x the float-float true residual
 //    replaces it (reliable update, the direction is kept).
 //  * One persistent cooperative launch.  A host planner orders the problems by estimated
@@ -40,10 +40,8 @@
 namespace fg {
 
 static constexpr int kBatchMaxP = 3;
-// coefficient table: per class, wy*wz rows of the x box padded to a multiple of 4 floats
-// (128-bit shared-memory loads); p = 3: (8 + 4 + 4) * 15 * 15 = 3600 floats
-static constexpr int kMaxBox = 16 * 15 * 15;
 static constexpr int kMaxCls = 27;
+static constexpr int kApplySmem = 32768;  // bytes for the partly summed rows of an operator chunk
 
 struct BatchProb {
   int n, p, L, F;        // cells per direction, order, lattice nodes, interior nodes per direction
@@ -61,11 +59,14 @@ struct BatchJob {
   int prob, rank;
 };
 
-struct OrderTables {    // unit stencil per order (sum over classes of the boxes)
+// 1D assembled rows of mass and stiffness per node class c = I mod p, as float-float: column t is
+// the neighbour I - p + t for class 0 (2p + 1 of them) and I - c + t for the others (p + 1)
+struct LineTables {
+  float m[kBatchMaxP][2 * kBatchMaxP + 1][2], s[kBatchMaxP][2 * kBatchMaxP + 1][2];
+};
+
+struct OrderTables {
   int ncls;
-  int base[kMaxCls], cnt[kMaxCls];
-  int lo[kMaxCls][3], w[kMaxCls][3];
-  float sh[kMaxBox], sl[kMaxBox];
   float dg[kMaxCls];     // centre coefficient (unit) per class
   double mw[(kBatchMaxP + 1) * (kBatchMaxP + 1)];  // w_q phi_a(xi_q), [a][q]
 };
@@ -75,6 +76,7 @@ struct BatchArgs {
   const int* job_ptr;     // per CTA: first job
   const BatchJob* jobs;
   const OrderTables* tabs;  // index p-1
+  LineTables line[kBatchMaxP];
   float* vpool;
   double* epool;
   double* rpool;
@@ -137,10 +139,8 @@ struct Kf {
 };
 
 struct BatchSmem {
-  __align__(16) float sh[kMaxBox];
-  __align__(16) float sl[kMaxBox];
-  int base[kMaxCls], cnt[kMaxCls];
-  int blo[kMaxCls][3], bw[kMaxCls][3];
+  __align__(16) unsigned char rows[kApplySmem];
+  float2 zc[kBatchMaxP][2 * kBatchMaxP + 1][2];  // (mass, stiffness) per class and neighbour: hi, lo
   float dinv[kMaxCls];
   double mw[(kBatchMaxP + 1) * (kBatchMaxP + 1)];
   double red[16][2];
@@ -174,7 +174,7 @@ __device__ bool team_arrive_wait(const BatchArgs& a, const BatchProb& P, int pro
       atomicExch(a.abort_all, 1);
       return false;
     }
-    __nanosleep(32);
+    __nanosleep(20);
   }
   __threadfence();
   return true;
@@ -281,125 +281,152 @@ struct NodeWalk {
   }
 };
 
-// x-periods of the interior: period (m, J, K) holds the nodes I = p m + k, k = 1..p (x classes
-// 1..p-1, then class 0); the class-0 node of the last period of a row is on the boundary.
-// v = m + n ((J-1) + F (K-1)), advanced incrementally.
-struct PeriodWalk {
-  int v, v1, m, J, K, n, F, step, dm, dJ, dK;
-  __device__ __forceinline__ PeriodWalk(int v0_, int v1_, int n_, int F_) : v1(v1_), n(n_), F(F_) {
-    step = blockDim.x;
-    v = v0_ + threadIdx.x;
-    if (F > 0) {
-      m = v % n;
-      J = 1 + (v / n) % F;
-      K = 1 + v / (n * F);
-      dm = step % n;
-      dJ = (step / n) % F;
-      dK = step / (n * F);
-    } else {
-      m = 0;
-      J = K = 1;
-      dm = dJ = dK = 0;
-    }
-  }
-  __device__ __forceinline__ bool ok() const { return v < v1; }
-  __device__ __forceinline__ void next() {
-    v += step;
-    m += dm;
-    int c = m >= n ? 1 : 0;
-    m -= c * n;
-    J += dJ + c;
-    c = J > F ? 1 : 0;
-    J -= c * F;
-    K += dK + c;
-  }
+// Scalars of the operator: FP32, and float-float with error-free products.  Acc is a running sum.
+struct S32 {
+  using V = float;
+  using P2 = float2;  // two values in shared memory
+  static __device__ __forceinline__ V zero() { return 0.f; }
+  static __device__ __forceinline__ V load(const float* h, const float*, int64_t g) { return h[g]; }
+  static __device__ __forceinline__ void fma(const float (&c)[2], V x, V& s) { s = fmaf(c[0], x, s); }
+  static __device__ __forceinline__ void fma(float ch, float, V x, V& s) { s = fmaf(ch, x, s); }
+  static __device__ __forceinline__ void norm(V&) {}
+  static __device__ __forceinline__ P2 pack(V a, V b) { return make_float2(a, b); }
+  static __device__ __forceinline__ V first(P2 p) { return p.x; }
+  static __device__ __forceinline__ V second(P2 p) { return p.y; }
+};
+struct Sff {
+  struct V { float h, l; };
+  using P2 = float4;
+  static __device__ __forceinline__ V zero() { return {0.f, 0.f}; }
+  static __device__ __forceinline__ V load(const float* h, const float* l, int64_t g) { return {h[g], l[g]}; }
+  static __device__ __forceinline__ void fma(const float (&c)[2], V x, V& s) { ff_fma_acc(c[0], c[1], x.h, x.l, s.h, s.l); }
+  static __device__ __forceinline__ void fma(float ch, float cl, V x, V& s) { ff_fma_acc(ch, cl, x.h, x.l, s.h, s.l); }
+  static __device__ __forceinline__ void norm(V& s) { quick_two_sum(s.h, s.l, s.h, s.l); }
+  static __device__ __forceinline__ P2 pack(V a, V b) { return make_float4(a.h, a.l, b.h, b.l); }
+  static __device__ __forceinline__ V first(P2 p) { return {p.x, p.y}; }
+  static __device__ __forceinline__ V second(P2 p) { return {p.z, p.w}; }
 };
 
-// FP32 stencil on one period: acc[0] for the class-0 node I0+p, acc[k] for I0+k.  Each (y,z)
-// box row loads the window x = I0..I0+2p once and serves all p nodes.
+// The unit operator Sx My Mz + Mx Sy Mz + Mx My Sz applied direction by direction, to a row block at
+// a time: NR = p YB rows in y (YB periods: 4, 2, 1 for p = 1, 2, 3) of one plane.
+//   1. thread per x (consecutive lanes read consecutive nodes): the z sums t = Mz v, u = Sz v of the
+//      rows' y window, then a = My t and b = Sy t + My u for the NR rows, into shared memory;
+//   2. thread per x period of a row: Sx a + Mx b for its p nodes, handed to out(node, I, J, K, value).
+// About 50 multiply-adds per node at p = 3 where the assembled stencil has 125 (and read one
+// coefficient from shared memory for each, and its window with stride p).
+// A rank's row blocks [w0, w1) go in chunks of G row blocks (or pieces of one, for rows that do not
+// fit kApplySmem) that fill the block's threads.
+// What bounds it: instruction issue and the latency of phase 1's loads (everything is in L2); the next
+// plane's loads run beside a plane's products.  One CTA of 512 threads alone on an SM, 314 k nodes at
+// p = 3: 5.7 ns per node and CG iteration, everything included; 96 problems, n 8-24: 99 -> 66 ms with
+// this operator, 55 ms with the loads ahead (here and in the vector updates).
 template <int PO>
-__device__ __forceinline__ void period_apply32(const BatchSmem& sm, const float* __restrict__ v, int L, int I0,
-                                               int J, int K, bool full, float (&acc)[PO]) {
-  const int cy = J % PO, cz = K % PO;
-  const int c0 = PO * (cy + PO * cz);
-  const int ly = sm.blo[c0][1], wy = sm.bw[c0][1], lz = sm.blo[c0][2], wz = sm.bw[c0][2];
+struct ApplyShape {
+  static constexpr int YB = PO == 1 ? 4 : (PO == 2 ? 2 : 1);
+  static constexpr int NR = PO * YB;            // rows of a block: J0 + 1 .. J0 + NR
+  static constexpr int NY = PO * (YB + 1) + 1;  // their y window: J0 .. J0 + NY - 1
+};
+template <int PO, class S, class Out>
+__device__ __forceinline__ void apply_rows(const LineTables& T, BatchSmem& sm, const float* vh, const float* vl, int n,
+                                           int F, int L, int w0, int w1, Out out) {
+  using V = typename S::V;
+  using P2 = typename S::P2;
+  constexpr int NR = ApplyShape<PO>::NR, NY = ApplyShape<PO>::NY, YB = ApplyShape<PO>::YB;
+  constexpr int CAP = kApplySmem / (int)sizeof(P2) / NR;  // nodes of x
+  P2* rows = reinterpret_cast<P2*>(sm.rows);
+  const int nyb = (n + YB - 1) / YB;
+  // pieces of a row block: SP periods each, nodes PO m0 .. PO (m0 + SP) + PO
+  const int SP = PO * (n + 1) + 1 <= CAP ? n : (CAP - 1) / PO - 1;
+  const int nseg = (n + SP - 1) / SP, W = PO * (SP + 1) + 1;
+  const int G = max(1, CAP / W);
+  const int q1 = w1 * nseg;
+  for (int q0 = w0 * nseg; q0 < q1; q0 += G) {
+    const int ng = min(G, q1 - q0);
+    for (int t = threadIdx.x; t < ng * W; t += blockDim.x) {
+      const int gi = t / W, i = t - gi * W;
+      const int q = q0 + gi, blk = q / nseg, m0 = (q - blk * nseg) * SP;
+      const int K = 1 + blk / nyb, J0 = (blk - (K - 1) * nyb) * NR, I = PO * m0 + i;
+      V a[NR], b[NR];
 #pragma unroll
-  for (int k = 0; k < PO; ++k) acc[k] = 0.f;
-  for (int zz = 0; zz < wz; ++zz)
-    for (int yy = 0; yy < wy; ++yy) {
-      const int base = I0 + L * ((J + ly + yy) + L * (K + lz + zz));
-      float win[2 * PO + 1];
+      for (int r = 0; r < NR; ++r) a[r] = b[r] = S::zero();
+      if (I >= 1 && I <= F) {
+        V tz[NY], uz[NY];
 #pragma unroll
-      for (int t = 0; t <= PO; ++t) win[t] = v[base + t];
+        for (int y = 0; y < NY; ++y) tz[y] = uz[y] = S::zero();
+        const int cz = K % PO, kz = cz ? cz : PO, nz = cz ? PO + 1 : 2 * PO + 1;
+        const int ny = min(NY, F + 1 - J0);  // rows from the boundary on are zero
+        const int L2 = L * L;
+        int g = I + L * J0 + L2 * (K - kz);
+        V v[NY];
 #pragma unroll
-      for (int t = PO + 1; t <= 2 * PO; ++t) win[t] = full ? v[base + t] : 0.f;
-      const int row = yy + wy * zz;
-      constexpr int R0 = (2 * PO + 1 + 3) & ~3, RK = (PO + 1 + 3) & ~3;
-      {
-        const float4* S0 = reinterpret_cast<const float4*>(sm.sh + sm.base[c0] + R0 * row);
+        for (int y = 0; y < NY; ++y) v[y] = y < ny ? S::load(vh, vl, g + y * L) : S::zero();
+        for (int z = 0; z < nz; ++z) {
+          V nxt[NY];  // the next plane's loads run beside this one's products
+          if (z + 1 < nz) {
+            g += L2;
 #pragma unroll
-        for (int v4 = 0; v4 < R0 / 4; ++v4) {
-          const float4 c = S0[v4];
-          const float cc[4] = {c.x, c.y, c.z, c.w};
+            for (int y = 0; y < NY; ++y) nxt[y] = y < ny ? S::load(vh, vl, g + y * L) : S::zero();
+          }
+          const float2 ch = sm.zc[cz][z][0], cl = sm.zc[cz][z][1];
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
-            if (4 * v4 + e <= 2 * PO) acc[0] = fmaf(cc[e], win[4 * v4 + e], acc[0]);
+          for (int y = 0; y < NY; ++y) {
+            S::fma(ch.x, cl.x, v[y], tz[y]);
+            S::fma(ch.y, cl.y, v[y], uz[y]);
+          }
+#pragma unroll
+          for (int y = 0; y < NY; ++y) v[y] = nxt[y];
+        }
+#pragma unroll
+        for (int y = 0; y < NY; ++y) {
+          S::norm(tz[y]);
+          S::norm(uz[y]);
+        }
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+          // row J0 + 1 + r: class (r + 1) mod p, first neighbour at window row y0
+          constexpr int P = PO;
+          const int c = (r + 1) % P, y0 = c ? r + 1 - c : r + 1 - P, nn = c ? P + 1 : 2 * P + 1;
+#pragma unroll
+          for (int t2 = 0; t2 < 2 * P + 1; ++t2)
+            if (t2 < nn) {
+              S::fma(T.m[c][t2], tz[y0 + t2], a[r]);
+              S::fma(T.s[c][t2], tz[y0 + t2], b[r]);
+              S::fma(T.m[c][t2], uz[y0 + t2], b[r]);
+            }
+          S::norm(a[r]);
+          S::norm(b[r]);
         }
       }
 #pragma unroll
-      for (int k = 1; k < PO; ++k) {
-        const float4* Sk = reinterpret_cast<const float4*>(sm.sh + sm.base[c0 + k] + RK * row);
-#pragma unroll
-        for (int v4 = 0; v4 < RK / 4; ++v4) {
-          const float4 c = Sk[v4];
-          const float cc[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            if (4 * v4 + e <= PO) acc[k] = fmaf(cc[e], win[4 * v4 + e], acc[k]);
-        }
-      }
+      for (int r = 0; r < NR; ++r) rows[(gi * NR + r) * W + i] = S::pack(a[r], b[r]);
     }
-}
-
-// Float-float stencil on one period (error-free products, float-float sums).
-template <int PO>
-__device__ __forceinline__ void period_apply_ff(const BatchSmem& sm, const float* __restrict__ vh,
-                                                const float* __restrict__ vl, int L, int I0, int J, int K, bool full,
-                                                float (&ah)[PO], float (&al)[PO]) {
-  const int cy = J % PO, cz = K % PO;
-  const int c0 = PO * (cy + PO * cz);
-  const int ly = sm.blo[c0][1], wy = sm.bw[c0][1], lz = sm.blo[c0][2], wz = sm.bw[c0][2];
+    __syncthreads();
+    for (int t = threadIdx.x; t < ng * NR * SP; t += blockDim.x) {
+      const int row = t / SP, m = t - row * SP, gi = row / NR;
+      const int q = q0 + gi, blk = q / nseg, m0 = (q - blk * nseg) * SP;
+      const int K = 1 + blk / nyb, J = (blk - (K - 1) * nyb) * NR + 1 + (row - gi * NR);
+      if (J > F || m0 + m >= n) continue;
+      const P2* w = rows + row * W + PO * m;
+      V o[PO];  // o[0]: the class-0 node at the period's end
 #pragma unroll
-  for (int k = 0; k < PO; ++k) {
-    ah[k] = 0.f;
-    al[k] = 0.f;
+      for (int k = 0; k < PO; ++k) o[k] = S::zero();
+#pragma unroll
+      for (int t2 = 0; t2 < 2 * PO + 1; ++t2) {
+        const P2 ab = w[t2];
+#pragma unroll
+        for (int k = 0; k < PO; ++k)
+          if (k == 0 || t2 <= PO) {
+            S::fma(T.s[k][t2], S::first(ab), o[k]);
+            S::fma(T.m[k][t2], S::second(ab), o[k]);
+          }
+      }
+      const int I0 = PO * (m0 + m), g0 = I0 + L * (J + L * K);
+#pragma unroll
+      for (int k = 1; k <= PO; ++k)
+        if (I0 + k <= F) out(g0 + k, I0 + k, J, K, o[k % PO]);
+    }
+    __syncthreads();
   }
-  for (int zz = 0; zz < wz; ++zz)
-    for (int yy = 0; yy < wy; ++yy) {
-      const int base = I0 + L * ((J + ly + yy) + L * (K + lz + zz));
-      float wh[2 * PO + 1], wl[2 * PO + 1];
-#pragma unroll
-      for (int t = 0; t <= PO; ++t) {
-        wh[t] = vh[base + t];
-        wl[t] = vl[base + t];
-      }
-#pragma unroll
-      for (int t = PO + 1; t <= 2 * PO; ++t) {
-        wh[t] = full ? vh[base + t] : 0.f;
-        wl[t] = full ? vl[base + t] : 0.f;
-      }
-      const int row = yy + wy * zz;
-      constexpr int R0 = (2 * PO + 1 + 3) & ~3, RK = (PO + 1 + 3) & ~3;
-      const int b0 = sm.base[c0] + R0 * row;
-#pragma unroll
-      for (int t = 0; t <= 2 * PO; ++t) ff_fma_acc(sm.sh[b0 + t], sm.sl[b0 + t], wh[t], wl[t], ah[0], al[0]);
-#pragma unroll
-      for (int k = 1; k < PO; ++k) {
-        const int bk = sm.base[c0 + k] + RK * row;
-#pragma unroll
-        for (int t = 0; t <= PO; ++t) ff_fma_acc(sm.sh[bk + t], sm.sl[bk + t], wh[t], wl[t], ah[k], al[k]);
-      }
-    }
 }
 
 template <int PO>
@@ -451,21 +478,11 @@ __device__ void solve_problem(const BatchArgs& a, int prob, int rank, BatchSmem&
   constexpr int NP1 = PO + 1, NQ = NP1 * NP1 * NP1;
   const int L = P.L, F = P.F, n = P.n;
   const int64_t L2 = (int64_t)L * L;
-  // tables into shared memory (offsets depend on L)
-  for (int c = threadIdx.x; c < T.ncls; c += blockDim.x) {
-    sm.base[c] = T.base[c];
-    sm.cnt[c] = T.cnt[c];
-    for (int d = 0; d < 3; ++d) {
-      sm.blo[c][d] = T.lo[c][d];
-      sm.bw[c][d] = T.w[c][d];
-    }
-    float d = T.dg[c] * P.kh_hi;
-    sm.dinv[c] = 1.0f / d;
-  }
-  const int tot = T.base[T.ncls - 1] + T.cnt[T.ncls - 1];
-  for (int t = threadIdx.x; t < tot; t += blockDim.x) {
-    sm.sh[t] = T.sh[t];
-    sm.sl[t] = T.sl[t];
+  const LineTables& line = a.line[PO - 1];
+  for (int c = threadIdx.x; c < T.ncls; c += blockDim.x) sm.dinv[c] = 1.0f / (T.dg[c] * P.kh_hi);
+  for (int t = threadIdx.x; t < PO * (2 * PO + 1) * 2; t += blockDim.x) {
+    const int part = t & 1, z = (t >> 1) % (2 * PO + 1), c = (t >> 1) / (2 * PO + 1);
+    sm.zc[c][z][part] = make_float2(line.m[c][z][part], line.s[c][z][part]);
   }
   for (int t = threadIdx.x; t < NP1 * NP1; t += blockDim.x) sm.mw[t] = T.mw[t];
   __syncthreads();
@@ -483,8 +500,9 @@ __device__ void solve_problem(const BatchArgs& a, int prob, int rank, BatchSmem&
   const int64_t ncells = (int64_t)n * n * n, nint = (int64_t)F * F * F;
   const int64_t c0 = ncells * rank / P.team, c1 = ncells * (rank + 1) / P.team;
   const int64_t u0 = nint * rank / P.team, u1 = nint * (rank + 1) / P.team;
-  const int64_t nper = (int64_t)n * F * F;
-  const int v0 = (int)(nper * rank / P.team), v1 = (int)(nper * (rank + 1) / P.team);
+  // row blocks of the operator
+  const int64_t nblk = (int64_t)((n + ApplyShape<PO>::YB - 1) / ApplyShape<PO>::YB) * F;
+  const int w0 = (int)(nblk * rank / P.team), w1 = (int)(nblk * (rank + 1) / P.team);
   // 1. load vectors by sum factorisation (FP64)
   load_vectors<PO>(P, E, c0, c1, sm);
   if (!team_sync(a, P, prob, rank, phase, sm)) return;
@@ -546,24 +564,11 @@ __device__ void solve_problem(const BatchArgs& a, int prob, int rank, BatchSmem&
     // q = A p (FP32), <p, q>
     {
       Kf pq;
-      for (PeriodWalk w(v0, v1, n, F); w.ok(); w.next()) {
-        const int I0 = PO * w.m;
-        const bool full = I0 + PO <= F;
-        float acc[PO];
-        period_apply32<PO>(sm, pp, L, I0, w.J, w.K, full, acc);
-        const int g0 = I0 + L * (w.J + L * w.K);
-#pragma unroll
-        for (int k = 1; k < PO; ++k) {
-          const float y = acc[k] * khf;
-          q[g0 + k] = y;
-          pq.add(y * pp[g0 + k]);
-        }
-        if (full) {
-          const float y = acc[0] * khf;
-          q[g0 + PO] = y;
-          pq.add(y * pp[g0 + PO]);
-        }
-      }
+      apply_rows<PO, S32>(line, sm, pp, nullptr, n, F, L, w0, w1, [&](int g, int, int, int, float o) {
+        const float y = o * khf;
+        q[g] = y;
+        pq.add(y * pp[g]);
+      });
       loc[0] = pq.val();
     }
     if (!team_sum<1>(a, P, prob, rank, phase, loc, sm, [&](double pq, double) {
@@ -578,15 +583,29 @@ __device__ void solve_problem(const BatchArgs& a, int prob, int rank, BatchSmem&
     const float alpha = sm.alpha;
     {
       Kf rr, rzn;
-      for (NodeWalk w((int)u0, (int)u1, F, L); w.ok(); w.next()) {
-        const int I = w.I, J = w.J, K = w.K;
-        const int64_t g = w.g;
-        const int cls = (I % PO) + PO * ((J % PO) + PO * (K % PO));
-        xc[g] = fmaf(alpha, pp[g], xc[g]);
-        float ri = fmaf(-alpha, q[g], r[g]);
-        r[g] = ri;
-        rr.add(ri * ri);
-        rzn.add(ri * (sm.dinv[cls] * ri));
+      for (NodeWalk w((int)u0, (int)u1, F, L); w.ok();) {
+        // four nodes' loads before the first store
+        int g[4];
+        float di[4], pv[4], qv[4], xv[4], rv[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k, w.next()) {
+          g[k] = w.ok() ? w.g : -1;
+          if (g[k] < 0) continue;
+          di[k] = sm.dinv[(w.I % PO) + PO * ((w.J % PO) + PO * (w.K % PO))];
+          pv[k] = pp[g[k]];
+          qv[k] = q[g[k]];
+          xv[k] = xc[g[k]];
+          rv[k] = r[g[k]];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (g[k] < 0) continue;
+          xc[g[k]] = fmaf(alpha, pv[k], xv[k]);
+          const float ri = fmaf(-alpha, qv[k], rv[k]);
+          r[g[k]] = ri;
+          rr.add(ri * ri);
+          rzn.add(ri * (di[k] * ri));
+        }
       }
       loc[0] = rr.val();
       loc[1] = rzn.val();
@@ -614,29 +633,17 @@ __device__ void solve_problem(const BatchArgs& a, int prob, int rank, BatchSmem&
       }
       if (!team_sync(a, P, prob, rank, phase, sm)) return;
       Kf rr2, rz2;
-      for (PeriodWalk w(v0, v1, n, F); w.ok(); w.next()) {
-        const int I0 = PO * w.m;
-        const bool full = I0 + PO <= F;
-        float sh[PO], sl[PO];
-        period_apply_ff<PO>(sm, xh, xl, L, I0, w.J, w.K, full, sh, sl);
-        const int g0 = I0 + L * (w.J + L * w.K);
-        const int cyz = PO * ((w.J % PO) + PO * (w.K % PO));
-#pragma unroll
-        for (int k = 0; k < PO; ++k) {
-          const int xo = k == 0 ? PO : k;  // acc[0]: class-0 node at I0 + PO
-          if (k == 0 && !full) continue;
-          const int g = g0 + xo;
-          float h, l, ah, al;
-          quick_two_sum(sh[k], sl[k], h, l);
-          ff_mul(P.kh_hi, P.kh_lo, h, l, ah, al);
-          float rh, rl;
-          ff_add(bh[g], bl[g], -ah, -al, rh, rl);
-          const float ri = rh + rl;
-          r[g] = ri;
-          rr2.add(ri * ri);
-          rz2.add(ri * (sm.dinv[cyz + (xo % PO)] * ri));
-        }
-      }
+      apply_rows<PO, Sff>(line, sm, xh, xl, n, F, L, w0, w1, [&](int g, int I, int J, int K, Sff::V o) {
+        float h, l, ah, al;
+        quick_two_sum(o.h, o.l, h, l);
+        ff_mul(P.kh_hi, P.kh_lo, h, l, ah, al);
+        float rh, rl;
+        ff_add(bh[g], bl[g], -ah, -al, rh, rl);
+        const float ri = rh + rl;
+        r[g] = ri;
+        rr2.add(ri * ri);
+        rz2.add(ri * (sm.dinv[(I % PO) + PO * ((J % PO) + PO * (K % PO))] * ri));
+      });
       loc[0] = rr2.val();
       loc[1] = rz2.val();
       ++nref;
@@ -654,11 +661,19 @@ __device__ void solve_problem(const BatchArgs& a, int prob, int rank, BatchSmem&
       }
     }
     const float beta = sm.beta;
-    for (NodeWalk w((int)u0, (int)u1, F, L); w.ok(); w.next()) {
-      const int I = w.I, J = w.J, K = w.K;
-      const int64_t g = w.g;
-      const int cls = (I % PO) + PO * ((J % PO) + PO * (K % PO));
-      pp[g] = fmaf(beta, pp[g], sm.dinv[cls] * r[g]);
+    for (NodeWalk w((int)u0, (int)u1, F, L); w.ok();) {
+      int g[4];
+      float pv[4], zv[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k, w.next()) {
+        g[k] = w.ok() ? w.g : -1;
+        if (g[k] < 0) continue;
+        pv[k] = pp[g[k]];
+        zv[k] = sm.dinv[(w.I % PO) + PO * ((w.J % PO) + PO * (w.K % PO))] * r[g[k]];
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (g[k] >= 0) pp[g[k]] = fmaf(beta, pv[k], zv[k]);
     }
     if (!team_sync(a, P, prob, rank, phase, sm)) return;
   }
@@ -702,8 +717,9 @@ __global__ void __launch_bounds__(512, 2) k_batch_solve(BatchArgs a) {
 // ---------------------------------------------------------------------------------------
 // Host
 
-static void build_order_tables(int p, OrderTables& T) {
+static void build_order_tables(int p, OrderTables& T, LineTables& line) {
   std::memset(&T, 0, sizeof(T));
+  std::memset(&line, 0, sizeof(line));
   const int np1 = p + 1;
   double xq[kBatchMaxP + 1], wq[kBatchMaxP + 1];
   gl_rule(np1, xq, wq);
@@ -747,32 +763,21 @@ static void build_order_tables(int p, OrderTables& T) {
     }
   }
   T.ncls = p * p * p;
-  int base = 0;
+  auto split = [](double v, float (&f)[2]) {
+    f[0] = (float)v;
+    f[1] = (float)(v - (double)f[0]);
+  };
+  for (int c = 0; c < p; ++c)
+    for (int t = 0; t < w1[c]; ++t) {
+      split(M1[c][t], line.m[c][t]);
+      split(S1[c][t], line.s[c][t]);
+    }
   for (int cz = 0; cz < p; ++cz)
     for (int cy = 0; cy < p; ++cy)
       for (int cx = 0; cx < p; ++cx) {
-        const int c = cx + p * (cy + p * cz);
-        T.base[c] = base;
-        T.lo[c][0] = lo1[cx];
-        T.lo[c][1] = lo1[cy];
-        T.lo[c][2] = lo1[cz];
-        T.w[c][0] = w1[cx];
-        T.w[c][1] = w1[cy];
-        T.w[c][2] = w1[cz];
-        const int rw = (w1[cx] + 3) & ~3;  // padded row
-        T.cnt[c] = rw * w1[cy] * w1[cz];
-        for (int k = 0; k < w1[cz]; ++k)
-          for (int j = 0; j < w1[cy]; ++j)
-            for (int i = 0; i < w1[cx]; ++i) {
-              double v = S1[cx][i] * M1[cy][j] * M1[cz][k] + M1[cx][i] * S1[cy][j] * M1[cz][k] +
-                         M1[cx][i] * M1[cy][j] * S1[cz][k];
-              float h = (float)v;
-              int t = base + i + rw * (j + w1[cy] * k);
-              T.sh[t] = h;
-              T.sl[t] = (float)(v - (double)h);
-              if (lo1[cx] + i == 0 && lo1[cy] + j == 0 && lo1[cz] + k == 0) T.dg[c] = h;
-            }
-        base += T.cnt[c];
+        const double mx = M1[cx][-lo1[cx]], my = M1[cy][-lo1[cy]], mz = M1[cz][-lo1[cz]];
+        const double sx = S1[cx][-lo1[cx]], sy = S1[cy][-lo1[cy]], sz = S1[cz][-lo1[cz]];
+        T.dg[cx + p * (cy + p * cz)] = (float)(sx * my * mz + mx * sy * mz + mx * my * sz);
       }
 }
 
@@ -790,9 +795,10 @@ struct fg_batch {
   std::vector<fg::BatchProb> probs;       // device-facing descriptors
   std::vector<const double*> user_f;      // caller's source pointers
   std::vector<double*> user_x;            // caller's output pointers
+  fg::LineTables line[fg::kBatchMaxP];
   std::vector<int64_t> nf, nx;            // source / output lengths
   int threads = 0, ctas = 0, max_team = 0, teams_gt1 = 0;
-  // team sizing: a problem gets ceil(work / (team_share * per-CTA share)) CTAs
+  // team sizing: a problem gets at most ceil(work / (team_share * per-CTA share)) CTAs
   // (0.5, or FG_BATCH_TEAM_SHARE when set > 0)
   double team_share = 0.5;
   double predicted_balance = 0.0, autotune_ms = 0.0, run_ms = 0.0;
@@ -829,53 +835,74 @@ static fg_status ba(fg_batch* B, void** p, size_t bytes) {
 static size_t batch_smem() { return sizeof(BatchSmem); }
 
 // Team sizes and the per-CTA job lists (greedy list scheduling, problems by decreasing work).
+// A problem with t CTAs takes its iterations (measured: 3, 8, 20 per cell in a direction at
+// orders 1-3) times its share of the nodes plus what an iteration's reductions and barriers cost:
+// on GB300 12 us with one CTA of 512 threads, ~20 us in a team, against 7.9 ns per node, i.e. 3
+// and 5 nodes per thread.  A problem's team is at most ceil(work / (team_share x a CTA's share));
+// all teams are scaled down together by 1, 1.4, 2, 2.8 and the schedule that ends first by this
+// model is taken (96 problems, n 8-24: 66 ms unscaled, 45 ms at 2).
 static void batch_schedule(fg_batch* B, int G, std::vector<int>& job_ptr, std::vector<BatchJob>& jobs) {
   const int np = B->nprob;
-  std::vector<double> w(np);
+  std::vector<double> nodes(np), its(np), w(np);
   double W = 0.0;
   for (int i = 0; i < np; ++i) {
     const BatchProb& P = B->probs[i];
-    double F3 = (double)P.F * P.F * P.F;
-    w[i] = std::max(1.0, F3) * avg_nnz(P.p) * (3.0 * P.p * P.n + 20.0);
+    nodes[i] = std::max(1.0, (double)P.F * P.F * P.F);
+    its[i] = P.n * (P.p == 1 ? 3.0 : (P.p == 2 ? 8.0 : 20.0));
+    w[i] = its[i] * (nodes[i] + 3.0 * B->threads);
     W += w[i];
   }
   std::vector<int> order(np);
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return w[x] > w[y]; });
   const double target = W / G;
-  std::vector<double> avail(G, 0.0);
-  std::vector<std::vector<BatchJob>> per(G);
-  B->max_team = 1;
-  B->teams_gt1 = 0;
+  double best = -1.0;
+  std::vector<int> team(np), best_team(np);
+  std::vector<std::vector<BatchJob>> per(G), best_per(G);
+  std::vector<double> avail(G);
   std::vector<int> idx(G);
-  for (int i : order) {
-    BatchProb& P = B->probs[i];
-    const int64_t F3 = (int64_t)P.F * P.F * P.F;
-    int t = (int)std::ceil(w[i] / (B->team_share * target));
-    t = std::max(1, std::min(t, G));
-    t = (int)std::min<int64_t>(t, std::max<int64_t>(1, F3 / (4 * B->threads)));
-    P.team = t;
-    B->max_team = std::max(B->max_team, t);
-    if (t > 1) B->teams_gt1++;
-    std::iota(idx.begin(), idx.end(), 0);
-    std::partial_sort(idx.begin(), idx.begin() + t, idx.end(),
-                      [&](int x, int y) { return avail[x] < avail[y] || (avail[x] == avail[y] && x < y); });
-    std::sort(idx.begin(), idx.begin() + t);
-    double start = 0.0;
-    for (int k = 0; k < t; ++k) start = std::max(start, avail[idx[k]]);
-    const double end = start + w[i] / t;
-    for (int k = 0; k < t; ++k) {
-      avail[idx[k]] = end;
-      per[idx[k]].push_back({i, k});
+  for (double scale : {1.0, 1.4, 2.0, 2.8}) {
+    std::fill(avail.begin(), avail.end(), 0.0);
+    for (auto& v : per) v.clear();
+    for (int i : order) {
+      const BatchProb& P = B->probs[i];
+      const int64_t F3 = (int64_t)P.F * P.F * P.F;
+      int t = (int)std::ceil(w[i] / (scale * B->team_share * target));
+      t = std::max(1, std::min(t, G));
+      t = (int)std::min<int64_t>(t, std::max<int64_t>(1, F3 / (4 * B->threads)));
+      team[i] = t;
+      std::iota(idx.begin(), idx.end(), 0);
+      std::partial_sort(idx.begin(), idx.begin() + t, idx.end(),
+                        [&](int x, int y) { return avail[x] < avail[y] || (avail[x] == avail[y] && x < y); });
+      std::sort(idx.begin(), idx.begin() + t);
+      double start = 0.0;
+      for (int k = 0; k < t; ++k) start = std::max(start, avail[idx[k]]);
+      const double end = start + its[i] * (nodes[i] / t + (t > 1 ? 5.0 : 3.0) * B->threads);
+      for (int k = 0; k < t; ++k) {
+        avail[idx[k]] = end;
+        per[idx[k]].push_back({i, k});
+      }
+    }
+    const double mk = *std::max_element(avail.begin(), avail.end());
+    if (best < 0.0 || mk < best) {
+      best = mk;
+      best_team = team;
+      best_per.swap(per);
     }
   }
-  double mk = *std::max_element(avail.begin(), avail.end());
-  B->predicted_balance = mk > 0 ? (W / G) / mk : 1.0;
+  B->max_team = 1;
+  B->teams_gt1 = 0;
+  for (int i = 0; i < np; ++i) {
+    B->probs[i].team = best_team[i];
+    B->max_team = std::max(B->max_team, best_team[i]);
+    if (best_team[i] > 1) B->teams_gt1++;
+  }
+  B->predicted_balance = best > 0 ? std::min(1.0, (W / G) / best) : 1.0;
   job_ptr.assign(G + 1, 0);
   jobs.clear();
   for (int g = 0; g < G; ++g) {
     job_ptr[g] = (int)jobs.size();
-    for (auto& j : per[g]) jobs.push_back(j);
+    for (auto& j : best_per[g]) jobs.push_back(j);
   }
   job_ptr[G] = (int)jobs.size();
 }
@@ -886,6 +913,7 @@ static fg_status batch_launch(fg_batch* B, cudaStream_t st) {
   a.job_ptr = B->d_job_ptr;
   a.jobs = B->d_jobs;
   a.tabs = B->d_tabs;
+  std::memcpy(a.line, B->line, sizeof(a.line));
   a.vpool = B->vpool;
   a.epool = B->epool;
   a.rpool = B->rpool;
@@ -1101,7 +1129,7 @@ fg_status fg_batch_create(fg_ctx* ctx, int32_t nprob, const fg_batch_problem* pr
   // vectors: boundary nodes stay zero for the life of the plan
   cudaError_t e = cudaMemsetAsync(B->vpool, 0, sizeof(float) * std::max<int64_t>(1, voff), ctx->stream);
   OrderTables tabs[kBatchMaxP];
-  for (int p = 1; p <= kBatchMaxP; ++p) build_order_tables(p, tabs[p - 1]);
+  for (int p = 1; p <= kBatchMaxP; ++p) build_order_tables(p, tabs[p - 1], B->line[p - 1]);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(B->d_tabs, tabs, sizeof(tabs), cudaMemcpyHostToDevice, ctx->stream);
   if (e != cudaSuccess) {
