@@ -530,112 +530,119 @@ __device__ __forceinline__ void ff_acc(float& h, float& l, float h2, float l2) {
   h = s;
 }
 
-// Block and grid sums of NV accumulators, then f(totals) on lane 0 of warp 0 (the step's
-// scalars, in shared memory); every thread returns after f.  Threads leave their sums in
-// shared memory and warp 0 alone adds them (NT/32 + 5 additions per value instead of 5 in
-// every warp: the FP64 pipe takes 16 cycles per warp instruction).  FP32 accumulators are
-// added as float-float pairs and become FP64 once per block.  Sums in fixed order:
-// deterministic.  False: the grid barrier gave up.
+// Block and grid sums of NV accumulators, then f(totals) on thread 0 (the step's scalars, in
+// shared memory); every thread returns after f.  Threads leave their sums in shared memory and
+// the first four warps add them: an FP64 warp instruction holds the pipe of its SM quarter 64
+// cycles, so a warp alone pays that for each of its ~NT/32 + 5 dependent additions per value; the
+// four sit in different quarters and take a quarter of the sums each.  The grid's partial sums go
+// to one warp per value.  FP32 accumulators are added as float-float pairs and become FP64 once
+// per block.  Sums in fixed order: deterministic.  False: the grid barrier gave up.
+// (Solve with one warp adding and the scalar steps' square roots and reciprocals on their path, and so:
+// 8^3 Q1 FP64, one block, 0.236 -> 0.201 ms; 24^3 Q2 mixed 17.6 -> 16.1 us per iteration; 384^2 Q2
+// FP64 57.9 -> 55.3.)
 template <typename T>
 struct RedShared;
 template <>
 struct RedShared<double> {
-  double v[3][1024];
+  double v[3][1024], w[4][3], tot[3];
 };
 template <>
 struct RedShared<float> {
-  float2 v[2][1024];
+  float2 v[2][1024], w[4][3];
+  double tot[3];
 };
 
-template <int NV, typename F>
-__device__ __forceinline__ bool grid_reduce(RedShared<double>& sh, const double (&v)[NV], const GridSync& g, int buf,
-                                            unsigned& target, int* s_ok, F&& f) {
-  const int t = threadIdx.x;
+// sums over the warp (lane 0), two FP64 values in one butterfly
+template <int NV>
+__device__ __forceinline__ void warp_sums(double (&s)[NV], int lane) {
+  constexpr int N1 = NV >= 2 ? 2 : 0;  // values summed together
+  if (NV >= 2) {
+    const bool up = lane >= 16;
+    double x = (up ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, up ? s[0] : s[1], 16);
 #pragma unroll
-  for (int k = 0; k < NV; ++k) sh.v[k][t] = v[k];
-  __syncthreads();
-  target += gridDim.x;
-  if (t < 32) {
-    double s[NV];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      s[k] = 0.0;
-      for (int i = t; i < (int)blockDim.x; i += 32) s[k] += sh.v[k][i];
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) s[k] += __shfl_down_sync(0xffffffffu, s[k], off);
-    }
-    bool ok = true;
-    if (gridDim.x > 1) {
-      const int nb = gridDim.x;
-      double* part = g.part + (size_t)buf * 3 * nb;
-      if (t == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) part[k * nb + blockIdx.x] = s[k];
-        ok = grid_wait(g, target);
-      }
-      __syncwarp();
-#pragma unroll
-      for (int k = 0; k < NV; ++k) {
-        s[k] = 0.0;
-        for (int i = t; i < nb; i += 32) s[k] += __ldcg(part + k * nb + i);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) s[k] += __shfl_down_sync(0xffffffffu, s[k], off);
-      }
-    }
-    if (t == 0) {
-      *s_ok = ok ? 1 : 0;
-      if (ok) f(s);
-    }
+    for (int off = 8; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+    s[0] = x;
+    s[1] = __shfl_sync(0xffffffffu, x, 16);
   }
-  __syncthreads();
-  return *s_ok != 0;
+#pragma unroll
+  for (int k = N1; k < NV; ++k)
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], off);
 }
 
-template <int NV, typename F>
-__device__ __forceinline__ bool grid_reduce(RedShared<float>& sh, const float2 (&v)[NV], const GridSync& g, int buf,
+__device__ __forceinline__ void sum_in(double (&s), double v) { s += v; }
+__device__ __forceinline__ void sum_in(float2& s, float2 v) { ff_acc(s.x, s.y, v.x, v.y); }
+__device__ __forceinline__ double shfl_xor(double v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
+__device__ __forceinline__ float2 shfl_xor(float2 v, int m) {
+  return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
+}
+__device__ __forceinline__ double to_f64(double v) { return v; }
+__device__ __forceinline__ double to_f64(float2 v) { return (double)v.x + (double)v.y; }
+template <int NV>
+__device__ __forceinline__ void warp_sums(float2 (&s)[NV], int) {
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum_in(s[k], shfl_xor(s[k], off));
+}
+
+template <int NV, typename T, typename V, typename F>
+__device__ __forceinline__ bool grid_reduce(RedShared<T>& sh, const V (&v)[NV], const GridSync& g, int buf,
                                             unsigned& target, int* s_ok, F&& f) {
-  const int t = threadIdx.x;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
 #pragma unroll
   for (int k = 0; k < NV; ++k) sh.v[k][t] = v[k];
   __syncthreads();
   target += gridDim.x;
-  if (t < 32) {
-    double s[NV];
+  const int nt = blockDim.x < 128 ? blockDim.x : 128;  // the adding threads
+  if (t < nt) {
+    auto meet = [&] {
+      if (nt > 32) asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory");
+      else __syncwarp();
+    };
+    V s[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-      float h = 0.f, l = 0.f;
-      for (int i = t; i < (int)blockDim.x; i += 32) {
-        const float2 w = sh.v[k][i];
-        ff_acc(h, l, w.x, w.y);
-      }
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        const float h2 = __shfl_down_sync(0xffffffffu, h, off), l2 = __shfl_down_sync(0xffffffffu, l, off);
-        ff_acc(h, l, h2, l2);
-      }
-      s[k] = (double)h + (double)l;
+      s[k] = V{};
+      for (int i = t; i < (int)blockDim.x; i += nt) sum_in(s[k], sh.v[k][i]);
     }
-    bool ok = true;
-    if (gridDim.x > 1) {
-      const int nb = gridDim.x;
-      double* part = g.part + (size_t)buf * 3 * nb;
-      if (t == 0) {
+    warp_sums(s, lane);
+    if (lane == 0)
 #pragma unroll
-        for (int k = 0; k < NV; ++k) part[k * nb + blockIdx.x] = s[k];
-        ok = grid_wait(g, target);
+      for (int k = 0; k < NV; ++k) sh.w[warp][k] = s[k];
+    meet();
+    const bool grid = gridDim.x > 1;
+    double* part = g.part + (size_t)buf * 3 * gridDim.x;
+    if (warp == 0) {
+      // lane 4 k + w: value k of warp w
+      V y = lane < 4 * NV && (lane & 3) < (nt >> 5) ? sh.w[lane & 3][lane >> 2] : V{};
+      sum_in(y, shfl_xor(y, 1));
+      sum_in(y, shfl_xor(y, 2));
+      if (lane < 4 * NV && (lane & 3) == 0) {
+        const double d = to_f64(y);
+        if (grid) part[(lane >> 2) * gridDim.x + blockIdx.x] = d;
+        else sh.tot[lane >> 2] = d;
       }
       __syncwarp();
-#pragma unroll
-      for (int k = 0; k < NV; ++k) {
-        s[k] = 0.0;
-        for (int i = t; i < nb; i += 32) s[k] += __ldcg(part + k * nb + i);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) s[k] += __shfl_down_sync(0xffffffffu, s[k], off);
-      }
+      if (lane == 0) *s_ok = !grid || grid_wait(g, target) ? 1 : 0;
+      __syncwarp();
     }
-    if (t == 0) {
-      *s_ok = ok ? 1 : 0;
-      if (ok) f(s);
+    if (grid) {
+      meet();
+      for (int k = warp; k < NV; k += nt >> 5) {
+        double z[1] = {0.0};
+#pragma unroll 4
+        for (int i = lane; i < (int)gridDim.x; i += 32) z[0] += __ldcg(part + (size_t)k * gridDim.x + i);
+        warp_sums(z, lane);
+        if (lane == 0) sh.tot[k] = z[0];
+      }
+      meet();
+    }
+    if (t == 0 && *s_ok) {
+      double tot[NV];
+#pragma unroll
+      for (int k = 0; k < NV; ++k) tot[k] = sh.tot[k];
+      f(tot);
     }
   }
   __syncthreads();
@@ -777,7 +784,7 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
             GridSync g, double* S, int* I) {
   extern __shared__ __align__(16) int32_t s_off_buf[];
   __shared__ RedShared<double> sh;
-  __shared__ double sc[8];  // alpha, beta, rz, err, tol, rnrmm
+  __shared__ double sc[9];  // alpha, beta, rz, err, tol, rnrmm, <r,r>, its bound, 1/rz
   __shared__ int si[4];     // stop (1 done, 2 non-finite), converged, ok
   if (I[I_DONE]) return;
   constexpr int RR = R > 0 ? R : 1;
@@ -785,6 +792,7 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
   const int64_t warp = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   const int64_t nwarps = (int64_t)(blockDim.x >> 5) * gridDim.x;
   const bool need_pp = criterion == FG_DELTA_RHS || criterion == FG_DELTA_DELTA;
+  const bool res = criterion == FG_RES_RES || criterion == FG_RES_RHS;
   const int32_t* s_off = stage_offsets<double, ML>(m, s_off_buf);
   const int it0 = I[I_ITER], maxit = I[I_MAXIT];
   if (threadIdx.x == 0) {
@@ -792,6 +800,9 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
     sc[3] = S[S_ERR];
     sc[4] = S[S_TOL];
     sc[5] = S[S_RNRMM];
+    // <r,r> above this cannot have a root within the tolerance: no square root then
+    const double t2 = sc[4] * sc[4] * (1.0 + 1e-12);
+    sc[7] = t2 > 1e-290 ? t2 : INFINITY;
     si[0] = si[1] = 0;
   }
   SliceRef<double, ML> ref[RR];
@@ -817,8 +828,11 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
   }
   const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
   unsigned target = 0;
+  __syncthreads();  // the scalars
   int it = it0;
   for (int n = 0; n < max_launch; ++n) {
+    // beside the product: 1/rz for beta (a division on thread 0 between two barriers is 0.4 us)
+    if (threadIdx.x == blockDim.x - 32) sc[8] = 1.0 / sc[2];
     // Ap = A p, <Ap,p>
     Acc<double> dot;
     if (R > 0) {
@@ -866,28 +880,27 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
     }
     ++it;
     auto test = [&](double trr, double trz, double tpp) {
-      double err = sc[3];
-      if (it == 1 && need_pp) {
-        err = a * sqrt(tpp);
-        if (criterion == FG_DELTA_DELTA) sc[4] = rtol * err + atol;
+      bool conv = false;
+      if (res) {
+        sc[6] = trr;
+        if (trr <= sc[7]) conv = sqrt(trr) <= sc[4];
+      } else {
+        double err = sc[5];
+        if (need_pp) {
+          err = a * sqrt(tpp);
+          if (it == 1 && criterion == FG_DELTA_DELTA) sc[4] = rtol * err + atol;
+        }
+        sc[3] = err;
+        conv = err <= sc[4];
       }
-      switch (criterion) {
-        case FG_RES_RES: case FG_RES_RHS: err = sqrt(trr); break;
-        case FG_DELTA_RHS: case FG_DELTA_DELTA: if (it != 1) err = a * sqrt(tpp); break;
-        default: err = sc[5]; break;
-      }
-      sc[3] = err;
-      const bool conv = err <= sc[4];
       if (conv || it >= maxit) {
         si[0] = 1;
         si[1] = conv ? 1 : 0;
         return;
       }
-      double beta = 1.0 / sc[2];
       sc[2] = trz;
-      beta = beta * trz;
-      sc[1] = beta;
-      sc[5] = sqrt(trz);
+      sc[1] = sc[8] * trz;
+      if (!res && !need_pp) sc[5] = sqrt(trz);  // the next iteration's estimate
       if (!(isfinite(a) && isfinite(trz)) && (it + chunk - 1) / chunk * chunk < maxit) si[0] = 2;
     };
     bool ok;
@@ -931,7 +944,7 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
     S[S_ALPHA] = sc[0];
     S[S_BETA] = sc[1];
     S[S_RZ] = sc[2];
-    S[S_ERR] = sc[3];
+    S[S_ERR] = res ? sqrt(sc[6]) : sc[3];
     S[S_TOL] = sc[4];
     S[S_RNRMM] = sc[5];
     I[I_ITER] = it;
@@ -955,7 +968,7 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
             int max_launch, GridSync g, double* S, int* I) {
   extern __shared__ __align__(16) int32_t s_off_buf[];
   __shared__ RedShared<float> sh;
-  __shared__ double sd[8];  // rr, rmax, delta, sigma, tol, app
+  __shared__ double sd[9];  // rr, rmax^2, delta^2, (tol/sigma)^2, -, app, alpha, beta, 1/rr
   __shared__ float sf[2];   // alpha, beta
   __shared__ int si[8];     // pend, skip, done flag, ok
   if (I[I_DONE]) return;
@@ -968,10 +981,10 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
   int it = I[I_ITER];
   if (threadIdx.x == 0) {
     sd[0] = S[S_RRH];
-    sd[1] = S[S_RMAX];
-    sd[2] = S[S_DELTA];
-    sd[3] = S[S_SIGMA];
-    sd[4] = S[S_TOL];
+    const double rmax = S[S_RMAX], delta = S[S_DELTA], lim = S[S_TOL] / S[S_SIGMA];
+    sd[1] = rmax * rmax;
+    sd[2] = delta * delta;
+    sd[3] = lim * lim;
     sd[5] = S[S_APP];
     si[0] = I[I_PEND];
     si[1] = I[I_SKIPP];
@@ -999,7 +1012,10 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
   }
   const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
   unsigned target = 0;
+  __syncthreads();  // the scalars
   for (int n = 0; n < max_launch; ++n) {
+    // beside the product: 1/rr for beta (see k_pcg64)
+    if (threadIdx.x == blockDim.x - 32) sd[8] = 1.0 / sd[0];
     Acc<float> pq;
     AccPlain qq;
     if (R > 0) {
@@ -1034,7 +1050,7 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
           } else {
             a = rr / pap;
             const double rrn = a * a * nq - rr;
-            b = rrn / rr;
+            b = rrn * sd[8];
             if (!(rrn > 0.0)) {  // the recurrence lost its digits: end the segment here
               skip = 1;
               if (si[0] == FLAG_NONE) si[0] = FLAG_UPDATE;
@@ -1125,13 +1141,13 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
         return;
       }
       sd[0] = trr;
-      const double rn = sqrt(trr);
+      // norms compared as squares (no square root on the path)
       int pend = FLAG_NONE;
-      if (!(rn <= 1e4 * sd[1])) pend = FLAG_BREAK;  // NaN fails too
-      else if (exact && sqrt(trt) * sd[3] <= sd[4]) pend = FLAG_CHECK;
-      else if (rn < sd[2] * sd[1]) pend = FLAG_UPDATE;
+      if (!(trr <= 1e8 * sd[1])) pend = FLAG_BREAK;  // NaN fails too
+      else if (exact && trt <= sd[3]) pend = FLAG_CHECK;
+      else if (trr < sd[2] * sd[1]) pend = FLAG_UPDATE;
       else if (it + 1 >= maxit) pend = FLAG_MAXIT;
-      if (rn > sd[1]) sd[1] = rn;
+      if (trr > sd[1]) sd[1] = trr;
       si[0] = pend;
     };
     bool ok;
@@ -1157,7 +1173,7 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
     S[S_ALPHA] = sd[6];
     S[S_BETA] = sd[7];
     S[S_RRH] = sd[0];
-    S[S_RMAX] = sd[1];
+    S[S_RMAX] = sqrt(sd[1]);
     S[S_APP] = sd[5];
     I[I_ITER] = it;
     I[I_PEND] = si[0];
