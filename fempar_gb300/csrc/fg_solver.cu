@@ -659,18 +659,17 @@ __device__ __forceinline__ bool grid_barrier(const GridSync& g, unsigned& target
   return *s_ok != 0;
 }
 
-// matrix values of one group: cached (R > 0: the matrix of such a system mostly stays in L2
-// from one iteration to the next) or streamed
+// matrix values of one group: kept in L2 (R > 0: the matrix of such a system mostly stays there
+// from one iteration to the next; not in L1, which is the gathered vector's) or streamed
 template <bool KEEP>
 __device__ __forceinline__ void ld4k(const float* p, float (&v)[4]) {
   if (!KEEP) { ld4(p, v); return; }
-  const float4 t = __ldg(reinterpret_cast<const float4*>(p));
-  v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+  asm("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p));
 }
 template <bool KEEP>
 __device__ __forceinline__ void ld4k(const double* p, double (&v)[4]) {
   if (!KEEP) { ld4(p, v); return; }
-  asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+  asm("ld.global.nc.L1::no_allocate.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
 }
 
 // One slice of the matrix as one lane sees it.
@@ -682,6 +681,69 @@ struct SliceRef {
                        // cell blocks: first columns of the row's 7 blocks
   int w4;              // groups of 4 entries (cell blocks: of one block)
   int32_t base, vec;   // gather base (cell blocks: columns per block); the row's vector index (-1: no row)
+  const float4* sv;    // the lane's values in shared memory (keep), or null
+
+  // 16-byte pieces of a lane's group of 4 entries, and groups of the slice
+  static constexpr int PC = sizeof(T) / 4;
+  __device__ __forceinline__ int groups() const { return ML == ML_DG ? 7 * w4 : w4; }
+  // Copies the slice into shared memory at `dst` (32 PC pieces per group, piece by piece: the warp's
+  // accesses are contiguous).  A lane reads back only what it wrote.
+  __device__ __forceinline__ void keep(float4* dst, int lane) {
+    dst += lane;
+    sv = dst;
+    const float4* src = reinterpret_cast<const float4*>(vp);
+    const int n = groups();
+#pragma unroll 4
+    for (int j = 0; j < n; ++j)
+#pragma unroll
+      for (int q = 0; q < PC; ++q) dst[(j * PC + q) * 32] = __ldcs(src + (size_t)j * 32 * PC + q);
+  }
+  static __device__ __forceinline__ void lds4(const float4* s, float (&v)[4]) {
+    const float4 a = s[0];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+  }
+  static __device__ __forceinline__ void lds4(const float4* s, double (&v)[4]) {
+    const double2 a = *reinterpret_cast<const double2*>(s), b = *reinterpret_cast<const double2*>(s + 32);
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+  }
+  // dot with the values in shared memory: the gathers of four groups are in flight together
+  __device__ __forceinline__ T dot_kept(const T* x) const {
+    T acc = 0;
+    const float4* v0 = sv;
+    if (ML == ML_DG) {
+#pragma unroll 1
+      for (int k = 0; k < 7; ++k) {
+        const T* xb = x + cp[k];
+#pragma unroll 4
+        for (int j = 0; j < w4; ++j, v0 += 32 * PC) {
+          const T x0 = xb[4 * j], x1 = xb[4 * j + 1], x2 = xb[4 * j + 2], x3 = xb[min(4 * j + 3, base - 1)];
+          T v[4];
+          lds4(v0, v);
+          acc = fmaT(v[0], x0, acc);
+          acc = fmaT(v[1], x1, acc);
+          acc = fmaT(v[2], x2, acc);
+          acc = fmaT(v[3], x3, acc);
+        }
+      }
+      return acc;
+    }
+    const T* xb = x + base;
+    const int32_t* c0 = cp;
+#pragma unroll 4
+    for (int j = 0; j < w4; ++j, v0 += 32 * PC) {
+      int4 o;
+      if (STENCIL) o = reinterpret_cast<const int4*>(c0)[j];
+      else o = __ldg(reinterpret_cast<const int4*>(c0 + j * 128));
+      const T x0 = xb[o.x], x1 = xb[o.y], x2 = xb[o.z], x3 = xb[o.w];
+      T v[4];
+      lds4(v0, v);
+      acc = fmaT(v[0], x0, acc);
+      acc = fmaT(v[1], x1, acc);
+      acc = fmaT(v[2], x2, acc);
+      acc = fmaT(v[3], x3, acc);
+    }
+    return acc;
+  }
   __device__ __forceinline__ void load(const MatArgs<T>& m, int64_t s, int lane, const int32_t* s_off) {
     if (STENCIL) {
       const int k = m.scls[s];
@@ -742,8 +804,15 @@ struct SliceRef {
     const T* xb = x + base;
 #pragma unroll UNROLL
     for (int j = 0; j < w4; ++j) {
-      if (!KEEP && STENCIL && sizeof(T) == 4 && j + kPrefetch < w4)
+      // FP32 streams, and FP64 matrices of a few hundred MB (R > 0: 22 warps with two groups in
+      // flight hold too few bytes; 23 x 17 x 21 Q3 70.8 -> 64.2 us per iteration)
+      if (STENCIL && KEEP == (sizeof(T) == 8) && j + kPrefetch < w4)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(v0 + kPrefetch * 128));
+      // explicit columns: both streams, the gathers wait for the columns
+      if (ML == ML_SELL && sizeof(T) == 4 && j + kPrefetch < w4) {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(v0 + kPrefetch * 128));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(c0 + kPrefetch * 128));
+      }
       T v[4];
       ld4k<KEEP>(v0, v);
       int4 o;
@@ -771,17 +840,43 @@ __device__ __forceinline__ const int32_t* stage_offsets(const MatArgs<T>& m, int
   return s_off;
 }
 
-static constexpr int pcg_threads(int R) { return R > 0 ? 1024 : 768; }
+// Keeps as many of the block's slices in shared memory as fit `cap` groups (KBs of matrix that no
+// iteration reads again from L2).  s_cnt: RR x 32 ints of shared memory.
+template <typename T, int ML, int RR>
+__device__ __forceinline__ void keep_slices(SliceRef<T, ML> (&ref)[RR], float4* buf, int cap, int* s_cnt) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < RR; ++k) s_cnt[k * 32 + warp] = ref[k].groups();
+  __syncthreads();
+  int before = 0;  // groups of the slices before mine (k by k, warp by warp)
+#pragma unroll
+  for (int k = 0; k < RR; ++k) {
+    const int mine = lane < nw ? s_cnt[k * 32 + lane] : 0;
+    const int upto = before + (int)__reduce_add_sync(0xffffffffu, lane < warp ? mine : 0);
+    ref[k].sv = nullptr;
+    if (ref[k].groups() > 0 && upto + ref[k].groups() <= cap)
+      ref[k].keep(buf + (size_t)upto * 32 * SliceRef<T, ML>::PC, lane);
+    before += (int)__reduce_add_sync(0xffffffffu, mine);
+  }
+}
+
+// Threads per block.  Streaming kernels: 2 x 16 warps of 64 registers, i.e. more of a slice in flight
+// per warp, rather than 2 x 24 of 40 (96^3 Q2 mixed 370 -> 360 us per iteration, 32^3 Q2 dG mixed 130 ->
+// 124, 384^2 Q2 FP64 55.3 -> 52; 2 x 12 of 80: 377, 130, 57).  FP32 with explicit columns waits for its
+// gathers, each behind a column: 2 x 32 warps (unstructured Q2 40^3 90 -> 67, 48^3 119 -> 110, 64^3
+// 256 -> 234 against 2 x 16, with both streams prefetched).
+static constexpr int pcg_threads(int R, int ML, bool fp32) { return R > 0 || (fp32 && ML == ML_SELL) ? 1024 : 512; }
 static constexpr int pcg_blocks(int R) { return R > 0 ? 1 : 2; }
 
 // FP64 CG, the sequence and stopping tests of the reference (cg.f90:101-238, 279-407).
 // idiag null: no preconditioner.  chunk: the polling interval the caller asked for (a
 // non-finite iteration is reported at its end, if the iteration limit lies beyond it).
 template <int ML, int R>
-__global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
+__global__ void __launch_bounds__(pcg_threads(R, ML, false), pcg_blocks(R))
     k_pcg64(MatArgs<double> m, int64_t nvec, double* x, double* r, double* p, double* Ap,
             const double* __restrict__ idiag, int criterion, double rtol, double atol, int max_launch, int chunk,
-            GridSync g, double* S, int* I) {
+            int keep, GridSync g, double* S, int* I) {
   extern __shared__ __align__(16) int32_t s_off_buf[];
   __shared__ RedShared<double> sh;
   __shared__ double sc[9];  // alpha, beta, rz, err, tol, rnrmm, <r,r>, its bound, 1/rz
@@ -826,6 +921,10 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
       }
     }
   }
+  if (R > 0) {
+    __shared__ int s_cnt[32 * RR];
+    keep_slices(ref, reinterpret_cast<float4*>(s_off_buf + ((m.noff + 3) & ~3)), keep, s_cnt);
+  }
   const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
   unsigned target = 0;
   __syncthreads();  // the scalars
@@ -838,14 +937,14 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
     if (R > 0) {
 #pragma unroll
       for (int k = 0; k < RR; ++k) {
-        ra[k] = ref[k].template dot<true, 2>(p);
+        ra[k] = ref[k].sv ? ref[k].dot_kept(p) : ref[k].template dot<true, 2>(p);
         if (ref[k].vec >= 0) dot.add(ra[k], rp[k]);
       }
     } else {
       for (int64_t s = warp; s < m.nslices; s += nwarps) {
         SliceRef<double, ML> q;
         q.load(m, s, lane, s_off);
-        const double a = q.template dot<false, kUnroll>(p);
+        const double a = q.template dot<false, ML == ML_SELL ? 4 : kUnroll>(p);
         if (q.vec >= 0) {
           Ap[q.vec] = a;
           dot.add(a, p[q.vec]);
@@ -963,9 +1062,9 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
 // is taken one iteration later: that iteration's update keeps p, so the host can fold x and
 // restart the recursion from the true residual with the direction kept.
 template <int ML, int R>
-__global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
+__global__ void __launch_bounds__(pcg_threads(R, ML, true), pcg_blocks(R))
     k_pcg32(MatArgs<float> m, int64_t nvec, float* x, float* r, float* p, float* q, const float* __restrict__ idiag,
-            int max_launch, GridSync g, double* S, int* I) {
+            int max_launch, int keep, GridSync g, double* S, int* I) {
   extern __shared__ __align__(16) int32_t s_off_buf[];
   __shared__ RedShared<float> sh;
   __shared__ double sd[9];  // rr, rmax^2, delta^2, (tol/sigma)^2, -, app, alpha, beta, 1/rr
@@ -1010,6 +1109,10 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
       }
     }
   }
+  if (R > 0) {
+    __shared__ int s_cnt[32 * RR];
+    keep_slices(ref, reinterpret_cast<float4*>(s_off_buf + ((m.noff + 3) & ~3)), keep, s_cnt);
+  }
   const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
   unsigned target = 0;
   __syncthreads();  // the scalars
@@ -1021,7 +1124,7 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
     if (R > 0) {
 #pragma unroll
       for (int k = 0; k < RR; ++k) {
-        rq[k] = ref[k].template dot<true, R == 1 ? 4 : 2>(p);
+        rq[k] = ref[k].sv ? ref[k].dot_kept(p) : ref[k].template dot<true, R == 1 ? 4 : 2>(p);
         if (ref[k].vec >= 0) {
           pq.add(rq[k], rp[k]);
           qq.add(rq[k], rq[k]);
@@ -1031,7 +1134,7 @@ __global__ void __launch_bounds__(pcg_threads(R), pcg_blocks(R))
       for (int64_t s = warp; s < m.nslices; s += nwarps) {
         SliceRef<float, ML> w;
         w.load(m, s, lane, s_off);
-        const float a = w.template dot<false, kUnroll>(p);
+        const float a = w.template dot<false, ML == ML_SELL ? 4 : kUnroll>(p);
         if (w.vec >= 0) {
           q[w.vec] = a;
           pq.add(a, p[w.vec]);
@@ -1505,31 +1608,54 @@ fg_status system_spmv_layout_noalloc(fg_system* sys, int precision, const void* 
 // (32 per SM): its lanes' vector entries stay in registers.  Up to 16 slices fit one block,
 // whose barriers are block barriers (8^3 Q1: 8.7 us per iteration, 11.4 with 4 blocks, 12.9
 // with 11).  Twice the slices take two per warp (23 x 17 x 21 Q3 in FP64: 85 us per iteration
-// against 103 streaming; four per warp 120).  Beyond that two blocks per SM, 48 warps, stream
-// the vectors: four slices per warp were slower there too (unstructured 40^3 Q2, 15.4 k
-// slices: 136-144 us against 92).
+// against 103 streaming; four per warp 120).  Beyond that two blocks per SM stream the vectors:
+// four slices per warp were slower there too (unstructured 40^3 Q2, 15.4 k slices: 136-144 us
+// against 92).
 struct PcgShape {
   int R;
   unsigned blocks, threads;
 };
-static PcgShape pcg_shape(int64_t nslices, int64_t value_bytes, bool fp32, int sms) {
+static PcgShape pcg_shape(int64_t nslices, int64_t value_bytes, bool fp32, int ml, int sms) {
   const int64_t cap = (int64_t)sms * 32;
   // FP32 with two slices per warp only while the matrix stays in L2: streaming it wants the 48
   // warps and the prefetch (dG 20^3 Q2, 169 MB: 38 us per iteration against 64; 19^3 Q3, 150 MB: 45
   // against 48; 34^3 Q2, 80 MB: 36 against 29).  FP64 is bound by its pipe there (103 against 90).
   const bool streams = fp32 && nslices > cap && value_bytes > (int64_t)112 << 20;
-  if (nslices > 2 * cap || streams) return PcgShape{0, (unsigned)(2 * sms), (unsigned)pcg_threads(0)};
+  if (nslices > 2 * cap || streams) return PcgShape{0, (unsigned)(2 * sms), (unsigned)pcg_threads(0, ml, fp32)};
   const int R = nslices <= cap ? 1 : 2;
   const int64_t warps = std::max<int64_t>(1, (nslices + R - 1) / R);
   const int64_t blocks = warps <= 16 ? 1 : std::min<int64_t>(sms, warps);
   return PcgShape{R, (unsigned)blocks, (unsigned)(32 * ((warps + blocks - 1) / blocks))};
 }
 
+// keep: groups of 4 x 32 matrix entries (of `bytes` each) that a block holds in shared memory for the
+// launch: its share of the matrix, or what fits beside the class offsets and the kernel's own
+// (24^3 Q2 mixed 16.1 -> 15.5 us per iteration, 23 x 17 x 21 Q3 FP64 81 -> 73, the widest slices').
+// Not where the vectors are streamed: the gathers want the L1 (unstructured 40^3 Q2 89 -> 112).
 template <typename... KA>
-static fg_status launch_pcg(void (*k)(KA...), const PcgShape& sh, const Work& w, int noff, cudaStream_t st, void** args) {
-  const size_t smem = sizeof(int32_t) * (size_t)noff;
-  if (smem > 16 * 1024)  // static and dynamic shared memory together pass 48 KB
-    FG_CUDA_TRY(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+static fg_status pcg_keep(void (*k)(KA...), const PcgShape& sh, int noff, int64_t entries, int bytes, int* keep,
+                          size_t* smem) {
+  *smem = sizeof(int32_t) * (size_t)((noff + 3) & ~3);
+  cudaFuncAttributes fa;
+  FG_CUDA_TRY(cudaFuncGetAttributes(&fa, (const void*)k));
+  int dev = 0, most = 0;
+  FG_CUDA_TRY(cudaGetDevice(&dev));
+  FG_CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  const int64_t limit = (int64_t)most - (int64_t)fa.sharedSizeBytes;
+  // the same limit on every call: contexts on other threads launch this kernel with other sizes
+  FG_CUDA_TRY(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+  *keep = 0;
+  if (sh.R > 0) {
+    // slices are dealt out block by block; a block may have one more of each kind than another
+    const int64_t share = entries / 128 / sh.blocks * 5 / 4 + 64;
+    *keep = (int)std::max<int64_t>(0, std::min((limit - (int64_t)*smem) / (128 * bytes), share));
+    *smem += (size_t)*keep * 128 * bytes;
+  }
+  return FG_OK;
+}
+
+template <typename... KA>
+static fg_status launch_pcg(void (*k)(KA...), const PcgShape& sh, const Work& w, size_t smem, cudaStream_t st, void** args) {
   FG_CUDA_TRY(cudaMemsetAsync(w.rb.ticket + 1, 0, sizeof(unsigned), st));
   FG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k, dim3(sh.blocks), dim3(sh.threads), args, smem, st));
   return FG_OK;
@@ -1578,7 +1704,7 @@ static fg_status run_pcg64(fg_system* sys, const Work& w, const fg_solver_params
   fg_space* sp = sys->space;
   const int ml = mat_layout(sp);
   MatArgs<double> m = mat_args<double>(sp, ml == ML_STENCIL ? sys->d_tval : sys->d_sval);
-  const PcgShape sh = pcg_shape(m.nslices, 8 * solver_entries(sp), false, w.sms);
+  const PcgShape sh = pcg_shape(m.nslices, 8 * solver_entries(sp), false, ml, w.sms);
   int64_t nvec = sp->nvec;
   double *x = w.x, *r = w.r, *p = w.p, *Ap = w.Ap;
   const double* idiag = prm->precond == FG_PREC_JACOBI ? sys->d_idiag : nullptr;
@@ -1586,12 +1712,15 @@ static fg_status run_pcg64(fg_system* sys, const Work& w, const fg_solver_params
   GridSync g = grid_sync(w);
   double* S = w.S;
   int* I = w.I;
-  void* args[] = {&m, &nvec, &x, &r, &p, &Ap, &idiag, &criterion, &rtol, &atol, &iters, &chunk, &g, &S, &I};
-  for (;;) {
+  int keep = 0;
+  size_t smem = 0;
+  void* args[] = {&m, &nvec, &x, &r, &p, &Ap, &idiag, &criterion, &rtol, &atol, &iters, &chunk, &keep, &g, &S, &I};
 #define FG_PCG64(L) (sh.R == 1 ? k_pcg64<L, 1> : sh.R == 2 ? k_pcg64<L, 2> : k_pcg64<L, 0>)
-    FG_TRY(launch_pcg(ml == ML_STENCIL ? FG_PCG64(ML_STENCIL) : ml == ML_DG ? FG_PCG64(ML_DG) : FG_PCG64(ML_SELL), sh, w,
-                      m.noff, st, args));
+  auto k = ml == ML_STENCIL ? FG_PCG64(ML_STENCIL) : ml == ML_DG ? FG_PCG64(ML_DG) : FG_PCG64(ML_SELL);
 #undef FG_PCG64
+  FG_TRY(pcg_keep(k, sh, m.noff, solver_entries(sp), 8, &keep, &smem));
+  for (;;) {
+    FG_TRY(launch_pcg(k, sh, w, smem, st, args));
     sp->mesh->ctx->launches += 1;
     FG_TRY(read_state(w, h, st));
     if (h.I[I_DONE]) return FG_OK;
@@ -1608,19 +1737,22 @@ static fg_status run_pcg32(fg_system* sys, const Work& w, const fg_solver_params
   fg_space* sp = sys->space;
   const int ml = mat_layout(sp);
   MatArgs<float> m = mat_args<float>(sp, vals);
-  const PcgShape sh = pcg_shape(m.nslices, 4 * solver_entries(sp), true, w.sms);
+  const PcgShape sh = pcg_shape(m.nslices, 4 * solver_entries(sp), true, ml, w.sms);
   int64_t nvec = sp->nvec;
   float *x = w.x32, *r = w.r32, *p = w.p32, *q = w.Ap32;
   int iters = pcg_iters(prm, solver_entries(sp), nvec, 4);
   GridSync g = grid_sync(w);
   double* S = w.S;
   int* I = w.I;
-  void* args[] = {&m, &nvec, &x, &r, &p, &q, &idiag, &iters, &g, &S, &I};
-  do {
+  int keep = 0;
+  size_t smem = 0;
+  void* args[] = {&m, &nvec, &x, &r, &p, &q, &idiag, &iters, &keep, &g, &S, &I};
 #define FG_PCG32(L) (sh.R == 1 ? k_pcg32<L, 1> : sh.R == 2 ? k_pcg32<L, 2> : k_pcg32<L, 0>)
-    FG_TRY(launch_pcg(ml == ML_STENCIL ? FG_PCG32(ML_STENCIL) : ml == ML_DG ? FG_PCG32(ML_DG) : FG_PCG32(ML_SELL), sh, w,
-                      m.noff, st, args));
+  auto k = ml == ML_STENCIL ? FG_PCG32(ML_STENCIL) : ml == ML_DG ? FG_PCG32(ML_DG) : FG_PCG32(ML_SELL);
 #undef FG_PCG32
+  FG_TRY(pcg_keep(k, sh, m.noff, solver_entries(sp), 4, &keep, &smem));
+  do {
+    FG_TRY(launch_pcg(k, sh, w, smem, st, args));
     sp->mesh->ctx->launches += 1;
     FG_TRY(read_state(w, h, st));
   } while (!h.I[I_DONE]);

@@ -139,3 +139,32 @@ def test_pcg_bounded_barrier_runs_out_and_context_survives(fg, ctx, monkeypatch)
         monkeypatch.delenv("FG_PCG_BARRIER_TIMEOUT_MS")
         s.solve()
         assert s.info()["converged"]
+
+
+@pytest.mark.parametrize("n,order,layout", [((5, 4, 3), 3, "stencil"), ((13, 12, 11), 3, "stencil"),
+                                            ((13, 12, 11), 3, "sell"), ((20, 17, 19), 2, "sell")])
+def test_slices_kept_in_shared_memory(fg, ctx, n, order, layout, monkeypatch):
+    """Matrices of which a block holds all its slices in shared memory, or the first ones that fit (42
+    MB of FP64 values on 152 SMs), slices of every width: solves by their true residual."""
+    import scipy.sparse as sp
+    if layout == "sell":
+        monkeypatch.setenv("FG_SOLVER_LAYOUT", "sell")
+    rng = np.random.default_rng(order + sum(n))
+    coef = np.exp(rng.normal(size=n[0] * n[1] * n[2]))
+    tri = fg.SerialTriangulation(ctx, n)
+    space = fg.SerialFESpace(tri, order=order, dirichlet_ids=list(range(1, 27)))
+    op = fg.FEAffineOperator(space, fg.PoissonIntegration(cell_coef=coef, source_fn=fg.FG_FN_CONST,
+                                                          fn_param=[1.0])).compute()
+    irp, ja, val = op.get_matrix(symmetric_storage=False, one_based=False)
+    A = sp.csr_matrix((val, ja, irp), shape=(space.num_free_dofs,) * 2)
+    b = op.get_translation()
+    for prec in ("fp64", "mixed"):
+        s = fg.IterativeLinearSolver().set_type_from_string("CG").set_operators(op, "jacobi")
+        s.set_parameters_from_pl({"ILS_RTOL": 1e-10, "ILS_MAX_NUM_ITERATIONS": 20000, "PRECISION": prec})
+        x = s.solve()
+        assert s.info()["converged"], prec
+        assert np.linalg.norm(b - A @ x) <= (1e-10 + 1e-12) * np.linalg.norm(b), prec
+        assert np.array_equal(x, s.solve()), "not deterministic"
+    op.close()
+    space.close()
+    tri.close()
