@@ -333,18 +333,38 @@ struct OzItem {
   int arow0, brow0;
   int tiles_n;
   int tile0;
-  int tiles_m;  // > 0: tiles numbered down the columns (tiles_m row tiles each)
+  int tiles_m;  // > 0: tiles numbered down the columns (tiles_m row tiles each); -1: along the
+                // rows, only the tiles that reach the lower triangle (row tile r has 2 r + 2 of
+                // them, at most tiles_n).  With the others numbered too and skipped, a round robin
+                // gave one CTA 50 and another 25 tiles of 9492 x 9492 (now 38 and 37: the coarse
+                // updates of 24^3 BDDC 525 -> 405 us)
+  __host__ __device__ int64_t lower_full() const { return (int64_t)(tiles_n / 2) * (tiles_n / 2 + 1); }
   __device__ __forceinline__ void locate(int t, int& rt, int& ct) const {
     const int lt = t - tile0;
     if (tiles_m > 0) {
       ct = lt / tiles_m;
       rt = lt - ct * tiles_m;
-    } else {
+    } else if (tiles_m == 0) {
       rt = lt / tiles_n;
       ct = lt - rt * tiles_n;
+    } else if (lt < lower_full()) {
+      // tiles before row r: r (r + 1)
+      rt = (int)((sqrtf(4.0f * (float)lt + 1.0f) - 1.0f) * 0.5f);
+      while ((int64_t)rt * (rt + 1) > lt) --rt;
+      while ((int64_t)(rt + 1) * (rt + 2) <= lt) ++rt;
+      ct = lt - rt * (rt + 1);
+    } else {
+      const int r = (int)(lt - lower_full());
+      rt = tiles_n / 2 + r / tiles_n;
+      ct = r % tiles_n;
     }
   }
 };
+// output tiles of an m x n product, all or those of the lower triangle
+static int64_t lower_tiles(int64_t tiles_m, int64_t tiles_n) {
+  const int64_t r = std::min(tiles_m, tiles_n / 2);
+  return r * (r + 1) + (tiles_m - r) * tiles_n;
+}
 
 struct OzGemmArgs {
   const uint8_t* dig;    // digit blocks [row tile][K step][digit]
@@ -400,8 +420,8 @@ __device__ __noinline__ double sum_slow(long long h, uint32_t l, int off, uint32
   return ldexp(sum_f64(h, l, 0, flip, slow), off);
 }
 
-// Persistent: CTA b takes the output tiles b, b + gridDim.x, ... of all items (tiles above
-// the diagonal skipped when lower).  The accumulators are released as soon as the epilogue
+// Persistent: CTA b takes the output tiles b, b + gridDim.x, ... of all items (lower: those that reach
+// the triangle).  The accumulators are released as soon as the epilogue
 // has read them, so the next tile's MMAs run while the epilogue writes C.
 template <int BN, int S>
 __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
@@ -414,19 +434,8 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ntiles = g.ntiles;
-  auto valid = [&](int t) {
-    if (!g.lower) return true;
-    const OzItem it = item_of(g, t);
-    int rt, ct;
-    it.locate(t, rt, ct);
-    return ct * BN <= rt * OZ_BM + OZ_BM - 1;
-  };
-  auto next_tile = [&](int t) {
-    for (t += gridDim.x; t < ntiles && !valid(t); t += gridDim.x) {
-    }
-    return t;
-  };
-  const int first = valid(blockIdx.x) ? (int)blockIdx.x : next_tile(blockIdx.x);
+  auto next_tile = [&](int t) { return t + (int)gridDim.x; };
+  const int first = blockIdx.x;
   if (first >= ntiles) return;
 
   if (warp == 0) {
@@ -788,16 +797,17 @@ fg_status ozaki_gemm_nt(fg_ctx* ctx, cudaStream_t st, int64_t m, int64_t n, int6
   // consecutive CTAs walk the shorter side of the tile grid: the longer operand's digits are
   // read from HBM once and shared through L2
   g.one = OzItem{C, c_rs, c_cs, (int)m, (int)n, 0, same ? 0 : (int)rta, (int)tiles_n, 0,
-                 !lower && rta < tiles_n ? (int)rta : 0};
-  g.ntiles = (int)(rta * tiles_n);
+                 lower ? -1 : (rta < tiles_n ? (int)rta : 0)};
+  const int64_t ntiles = lower ? lower_tiles(rta, tiles_n) : rta * tiles_n;
+  g.ntiles = (int)ntiles;
   g.ksteps = (int)ksteps;
   g.chunk = k <= OZ_KEXACT ? (int)ksteps : OZ_CHUNK_STEPS;
   g.alpha = alpha;
   g.beta = beta;
   g.lower = lower ? 1 : 0;
   g.err = d_err;
-  return digits == 8 ? oz_launch<8>(ctx, st, sa, rta + rtb, g, rta * tiles_n)
-                     : oz_launch<OZ_S>(ctx, st, sa, rta + rtb, g, rta * tiles_n);
+  return digits == 8 ? oz_launch<8>(ctx, st, sa, rta + rtb, g, ntiles)
+                     : oz_launch<OZ_S>(ctx, st, sa, rta + rtb, g, ntiles);
 }
 
 // Batch of lower updates C_b -= P_b P_b^T, P_b m_b x k_b (k_b <= 128), all column-major; the first
@@ -827,9 +837,9 @@ fg_status ozaki_syrk_batch(fg_ctx* ctx, cudaStream_t st, const std::vector<OzSyr
     }
     const int64_t tn = (x.n + OZ_BN - 1) / OZ_BN;
     hs.push_back(OzSplit{x.p, 1, x.ld, x.m, x.k, (int)rt});
-    hi.push_back(OzItem{x.c, 1, x.ld, x.m, x.n, (int)rt, (int)rt, (int)tn, (int)tiles, 0});
+    hi.push_back(OzItem{x.c, 1, x.ld, x.m, x.n, (int)rt, (int)rt, (int)tn, (int)tiles, -1});
     rt += rtiles_of(x.m);
-    tiles += rtiles_of(x.m) * tn;
+    tiles += lower_tiles(rtiles_of(x.m), tn);
   }
   if (hs.empty()) return FG_OK;
   if (tiles > (1ll << 31) - 1 || ozaki_syrk_batch_bytes(b) > bytes) {
