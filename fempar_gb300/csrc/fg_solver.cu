@@ -865,8 +865,14 @@ __device__ __forceinline__ void keep_slices(SliceRef<T, ML> (&ref)[RR], float4* 
 // per warp, rather than 2 x 24 of 40 (96^3 Q2 mixed 370 -> 360 us per iteration, 32^3 Q2 dG mixed 130 ->
 // 124, 384^2 Q2 FP64 55.3 -> 52; 2 x 12 of 80: 377, 130, 57).  FP32 with explicit columns waits for its
 // gathers, each behind a column: 2 x 32 warps (unstructured Q2 40^3 90 -> 67, 48^3 119 -> 110, 64^3
-// 256 -> 234 against 2 x 16, with both streams prefetched).
-static constexpr int pcg_threads(int R, int ML, bool fp32) { return R > 0 || (fp32 && ML == ML_SELL) ? 1024 : 512; }
+// 256 -> 234 against 2 x 16, with both streams prefetched).  FP64 with explicit columns from HBM
+// (R = PCG_WIDE): 2 x 24, two groups in flight (quadrilaterals 1024^2 0.289 -> 0.282 ms, 2048^2 1.113 ->
+// 1.056, unstructured 88^3 1.062 -> 0.994; 384^2, whose 127 MB stay in L2, 52.2 -> 55.2 us; 700^2, 420 MB,
+// the same either way).
+static constexpr int PCG_WIDE = -1;
+static constexpr int pcg_threads(int R, int ML, bool fp32) {
+  return R > 0 || (fp32 && ML == ML_SELL) ? 1024 : R == PCG_WIDE ? 768 : 512;
+}
 static constexpr int pcg_blocks(int R) { return R > 0 ? 1 : 2; }
 
 // FP64 CG, the sequence and stopping tests of the reference (cg.f90:101-238, 279-407).
@@ -944,7 +950,7 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, false), pcg_blocks(R))
       for (int64_t s = warp; s < m.nslices; s += nwarps) {
         SliceRef<double, ML> q;
         q.load(m, s, lane, s_off);
-        const double a = q.template dot<false, ML == ML_SELL ? 4 : kUnroll>(p);
+        const double a = q.template dot<false, ML == ML_SELL && R == 0 ? 4 : kUnroll>(p);
         if (q.vec >= 0) {
           Ap[q.vec] = a;
           dot.add(a, p[q.vec]);
@@ -1621,7 +1627,10 @@ static PcgShape pcg_shape(int64_t nslices, int64_t value_bytes, bool fp32, int m
   // warps and the prefetch (dG 20^3 Q2, 169 MB: 38 us per iteration against 64; 19^3 Q3, 150 MB: 45
   // against 48; 34^3 Q2, 80 MB: 36 against 29).  FP64 is bound by its pipe there (103 against 90).
   const bool streams = fp32 && nslices > cap && value_bytes > (int64_t)112 << 20;
-  if (nslices > 2 * cap || streams) return PcgShape{0, (unsigned)(2 * sms), (unsigned)pcg_threads(0, ml, fp32)};
+  if (nslices > 2 * cap || streams) {
+    const int R = !fp32 && ml == ML_SELL && value_bytes > (int64_t)170 << 20 ? PCG_WIDE : 0;  // 1.5 x that with columns
+    return PcgShape{R, (unsigned)(2 * sms), (unsigned)pcg_threads(R, ml, fp32)};
+  }
   const int R = nslices <= cap ? 1 : 2;
   const int64_t warps = std::max<int64_t>(1, (nslices + R - 1) / R);
   const int64_t blocks = warps <= 16 ? 1 : std::min<int64_t>(sms, warps);
@@ -1716,7 +1725,7 @@ static fg_status run_pcg64(fg_system* sys, const Work& w, const fg_solver_params
   size_t smem = 0;
   void* args[] = {&m, &nvec, &x, &r, &p, &Ap, &idiag, &criterion, &rtol, &atol, &iters, &chunk, &keep, &g, &S, &I};
 #define FG_PCG64(L) (sh.R == 1 ? k_pcg64<L, 1> : sh.R == 2 ? k_pcg64<L, 2> : k_pcg64<L, 0>)
-  auto k = ml == ML_STENCIL ? FG_PCG64(ML_STENCIL) : ml == ML_DG ? FG_PCG64(ML_DG) : FG_PCG64(ML_SELL);
+  auto k = ml == ML_STENCIL ? FG_PCG64(ML_STENCIL) : ml == ML_DG ? FG_PCG64(ML_DG) : sh.R == PCG_WIDE ? k_pcg64<ML_SELL, PCG_WIDE> : FG_PCG64(ML_SELL);
 #undef FG_PCG64
   FG_TRY(pcg_keep(k, sh, m.noff, solver_entries(sp), 8, &keep, &smem));
   for (;;) {

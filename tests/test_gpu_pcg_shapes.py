@@ -142,10 +142,12 @@ def test_pcg_bounded_barrier_runs_out_and_context_survives(fg, ctx, monkeypatch)
 
 
 @pytest.mark.parametrize("n,order,layout", [((5, 4, 3), 3, "stencil"), ((13, 12, 11), 3, "stencil"),
-                                            ((13, 12, 11), 3, "sell"), ((20, 17, 19), 2, "sell")])
+                                            ((13, 12, 11), 3, "sell"), ((20, 17, 19), 2, "sell"),
+                                            ((38, 36, 37), 2, "sell")])
 def test_slices_kept_in_shared_memory(fg, ctx, n, order, layout, monkeypatch):
     """Matrices of which a block holds all its slices in shared memory, or the first ones that fit (42
-    MB of FP64 values on 152 SMs), slices of every width: solves by their true residual."""
+    MB of FP64 values on 152 SMs), slices of every width, and one streamed from HBM (203 MB of FP64
+    values with columns beside them): solves by their true residual."""
     import scipy.sparse as sp
     if layout == "sell":
         monkeypatch.setenv("FG_SOLVER_LAYOUT", "sell")
