@@ -2029,9 +2029,16 @@ static fg_status bddc_numeric(fg_bddc* B) {
 
 static size_t smem_for(int n, size_t elem) { return std::max<size_t>(16, (size_t)n * elem); }
 
-template <typename T>
+// Static and dynamic shared memory together pass 48 KB: raise the kernel's limit, always to the same
+// value (contexts on other threads may launch it with other sizes).
 static fg_status set_smem(const void* k, size_t bytes) {
-  if (bytes > 48 * 1024) FG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  if (bytes <= 24 * 1024) return FG_OK;
+  cudaFuncAttributes fa;
+  FG_CUDA_TRY(cudaFuncGetAttributes(&fa, k));
+  int dev = 0, most = 0;
+  FG_CUDA_TRY(cudaGetDevice(&dev));
+  FG_CUDA_TRY(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  FG_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes));
   return FG_OK;
 }
 
@@ -2058,10 +2065,10 @@ static fg_status bddc_apply_layout(fg_bddc* B, const double* r, double* z) {
   const T* Kinv = f32 ? (const T*)B->dKinv32 : (const T*)B->dKinv;
   const int prec = f32 ? FG_MIXED : FG_FP64;
   const size_t smI = smem_for(B->maxnI, sizeof(T)), smR = smem_for(B->maxnr, sizeof(T));
-  FG_TRY(set_smem<T>((const void*)k_bddc_dirichlet<T, 1>, smI));
-  FG_TRY(set_smem<T>((const void*)k_bddc_dirichlet<T, 2>, smI));
-  FG_TRY(set_smem<T>((const void*)k_bddc_neumann_fwd<T>, smR));
-  FG_TRY(set_smem<T>((const void*)k_bddc_neumann_bwd<T>, smR));
+  FG_TRY(set_smem((const void*)k_bddc_dirichlet<T, 1>, smI));
+  FG_TRY(set_smem((const void*)k_bddc_dirichlet<T, 2>, smI));
+  FG_TRY(set_smem((const void*)k_bddc_neumann_fwd<T>, smR));
+  FG_TRY(set_smem((const void*)k_bddc_neumann_bwd<T>, smR));
   // 1. interior correction
   k_bddc_dirichlet<T, 1><<<ns, 256, smI, st>>>(B->d_subs, B->dA, B->dF, B->dLoc, r, (const T*)nullptr, u0, z);
   // 2-3. (A u0) on the interface
