@@ -534,7 +534,7 @@ def main():
         "mixed_vs_fp64": value / v64,
         "e2e": {"value": ve2e, "unit": "DOF/s", "h2d_bytes_per_step": int(coef.nbytes),
                 "d2h_bytes_per_step": int(nfree * 8), "ms_per_step": ms_e2e},
-        "roofline": {"bound": "hbm", "kernel": f"{kname}<float,0> (FP32 SpMV, {layout}; the iteration runs MODE 3, the same "
+        "roofline": {"bound": "hbm", "kernel": f"{kname}<float,0> (FP32 SpMV, {layout}; the CG launch runs the same product, the same "
                                "bytes plus two dot products)",
                      "achieved": ach32, "peak": hbm, "unit": "GB/s", "frac": ach32 / hbm,
                      "peak_source": "of measured" if pk else "of fallback",

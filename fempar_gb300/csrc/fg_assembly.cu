@@ -1601,9 +1601,9 @@ __global__ void __launch_bounds__(ElastShape<P>::WARPS * 32)
 // chunk) and three rows of 3 NQ against the antisymmetric table.  The 2 x 2 minors of B are
 // entries of J over det J, so the second kind of factor is +-w J_nm.  lambda and mu are folded
 // into the factors; unpacking a block entry is at most one addition.  0.92 MFLOP per Q2 cell at
-// the products' ~25 TFLOP/s against 0.18 MFLOP on the FP64 pipe's 1.05 (and the warp-per-cell
+// the products' ~35 TFLOP/s against 0.18 MFLOP on the FP64 pipe's 1.05 (and the warp-per-cell
 // kernel that did that holds 73 KB of shared memory: three warps per SM).
-// 32^3 Q2 element matrices: 10.9 ms -> 2.5 ms (geometry 0.43, digits 0.30, products 1.15, unpacking 0.64).
+// 32^3 Q2 element matrices: 10.9 ms -> 2.2 ms (geometry 0.43, digits 0.27, products 0.90, unpacking 0.64).
 template <int P>
 struct ElastTC {
   static constexpr int NQ = ElastShape<P>::NQ, NN = ElastShape<P>::NN, ND = ElastShape<P>::ND;

@@ -453,9 +453,9 @@ __global__ void __launch_bounds__(RB)
 // instead of two or three kernels.  As separate kernels (a CUDA graph of them) each reduction
 // cost 12-18 us whatever the size: 912-1216 blocks took a ticket on one counter, each warp
 // butterflied its sums on the FP64 pipe (16 cycles per warp instruction), and the last block
-// started from cold.  Solve, before -> after: 8^3 Q1 FP64 1.48 -> 0.28 ms, 32^3 Q1 FP64 3.54 ->
-// 1.42 ms, 24^3 Q2 mixed 10.9 -> 4.9 ms, 23 x 17 x 21 Q3 FP64 65.8 -> 48.1 ms, 384^2 Q2 FP64
-// 253 -> 227 ms, 96^3 Q2 mixed 374 -> 364 ms.  Bound by barriers and FP64 latency where the
+// started from cold.  Solve, as kernels -> here: 8^3 Q1 FP64 1.48 -> 0.20 ms, 32^3 Q1 FP64 3.54 ->
+// 1.28 ms, 24^3 Q2 mixed 10.9 -> 4.2 ms, 23 x 17 x 21 Q3 FP64 65.8 -> 36.7 ms, 384^2 Q2 FP64
+// 253 -> 206 ms, 96^3 Q2 mixed 374 -> 361 ms.  Bound by barriers and FP64 latency where the
 // matrix is small, by the SpMV (FP64 pipe; HBM in FP32) where it is large.
 //
 // Rows: warp w of block b owns the slices w nb + b + k (warps nb), k = 0.. (an SM then holds

@@ -63,9 +63,10 @@ enum {
  * BDDC on such a system return FG_ERR_UNSUPPORTED.  Peak device memory of an assembly drops
  * from elmat + CSR + layout to max(elmat + CSR, CSR + layout). */
 enum { FG_INPUTS_ON_DEVICE = 1, FG_LEAN_SYSTEM = 2, FG_FAST_INTEGRATION = 4 };
-/* Poisson element matrices.  By default those of all cells are one FP64 product, emulated on
- * the tensor cores: the cells' geometric factors times a table shared by all cells.  They
- * match the FP64-pipe integration to ~1e-15 of the row scale, with reference parity.
+/* Element matrices.  By default those of all cells (Poisson, elasticity Q2/Q3, the volume terms of
+ * dG) are one or two FP64 products, emulated on the tensor cores: the cells' geometric factors times
+ * a table shared by all cells.  They match the FP64-pipe integration to ~1e-15 of the row scale, with
+ * reference parity.  Elasticity Q1, and Poisson Q1 up to 4096 cells, are integrated directly.
  * FG_FAST_INTEGRATION asks for float-float accuracy (~2^-44, meant for FG_MIXED solves, whose
  * FP64 copy of the matrix feeds the residual refinement).  Its geometric factors are then
  * computed in float-float on the FP32 pipe (GB300's FP64 rate is ~1/70 of FP32's): ~2e-14 of
