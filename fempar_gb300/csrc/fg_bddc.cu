@@ -609,21 +609,38 @@ __global__ void k_chol_diag1(double* A, int64_t lda, int j0, int nb, int* err) {
   }
 }
 
-// 64 rows per block: the row solves are bound by the FP64 pipe, and a coarse panel has too few
-// rows to fill the SMs with 256 (9,492 coarse dofs: 78 -> 53 us; with the divisions by the
-// diagonal as products with its reciprocals and a correction, 27 us)
-__global__ void __launch_bounds__(64) k_chol_trsm1(double* A, int64_t lda, int N, int j0, int nb) {
+// Row solves of one matrix: two lanes per row (lane & 1: its even or odd columns), 16 rows per warp.
+// They are bound by the FP64 pipe, and a coarse panel's rows, one per thread, give each SM only two
+// warps, so half the SM's quarters idle.  9,492 coarse dofs: 78 us with 256 rows per block, 53 with 64, 27
+// with the divisions by the diagonal as products with its reciprocals and a correction, 22 so.
+__global__ void __launch_bounds__(128) k_chol_trsm1(double* A, int64_t lda, int N, int j0, int nb) {
   __shared__ double Dsh[32][33], rd[32];
+  // rows and columns past nb: the unit matrix
   for (int t = threadIdx.x; t < 32 * 32; t += blockDim.x) {
-    int i = t & 31, j = t >> 5;
-    Dsh[i][j] = (i < nb && j < nb && i >= j) ? A[(j0 + i) + (int64_t)(j0 + j) * lda] : 0.0;
+    const int i = t & 31, j = t >> 5;
+    Dsh[i][j] = (i < nb && j < nb) ? (i >= j ? A[(j0 + i) + (int64_t)(j0 + j) * lda] : 0.0) : (i == j ? 1.0 : 0.0);
   }
   __syncthreads();
-  if (threadIdx.x < nb) rd[threadIdx.x] = 1.0 / Dsh[threadIdx.x][threadIdx.x];
+  if (threadIdx.x < 32) rd[threadIdx.x] = 1.0 / Dsh[threadIdx.x][threadIdx.x];
   __syncthreads();
-  int64_t i = j0 + nb + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  chol_trsm_row(A, lda, j0, nb, i, Dsh, rd);
+  const int lane = threadIdx.x & 31, h = lane & 1;
+  const int64_t i = j0 + nb + (int64_t)blockIdx.x * 64 + (threadIdx.x >> 5) * 16 + (lane >> 1);
+  double* row = A + i + (int64_t)j0 * lda;
+  double x[16];  // columns 2 m + h
+#pragma unroll
+  for (int m = 0; m < 16; ++m) x[m] = i < N && 2 * m + h < nb ? row[(2 * m + h) * lda] : 0.0;
+#pragma unroll
+  for (int k = 0; k < 32; ++k) {
+    const double own = quotient(x[k >> 1], Dsh[k][k], rd[k]);
+    const double xk = __shfl_sync(0xffffffffu, own, (lane & ~1) | (k & 1));
+    if (h == (k & 1)) x[k >> 1] = xk;
+#pragma unroll
+    for (int m = k >> 1; m < 16; ++m)
+      if (2 * m + h > k) x[m] -= xk * Dsh[2 * m + h][k];
+  }
+#pragma unroll
+  for (int m = 0; m < 16; ++m)
+    if (i < N && 2 * m + h < nb) row[(2 * m + h) * lda] = x[m];
 }
 
 __global__ void __launch_bounds__(256) k_chol_syrk1(double* A, int64_t lda, int N, int j0, int nb, int nt) {
@@ -1813,10 +1830,10 @@ static fg_status check_err(fg_bddc* B, const char* what) {
 // column i, so at panel j0 the rows from zrow + j0 + nb on are skipped by the solve and the
 // trailing update (exactly: their contributions are zero).  zrow = N: no unit block.
 // With work (ozaki_workspace_bytes(N, N, 128, true) bytes + an int), the factorisation is
-// blocked by 128 columns: each 128-column panel is factored by 32-column steps whose
-// updates stay inside the panel, and the trailing matrix gets one rank-128 update on the
-// tensor cores (FP64 emulated by digit slicing, fg_ozaki.cu) instead of four rank-32
-// updates on the FP64 pipe.
+// blocked by 128 columns: each 64-column half of a panel is factored by 32-column steps whose
+// updates stay inside the half, the second half gets one rank-64 update and the trailing matrix one
+// rank-128 update on the tensor cores (FP64 emulated by digit slicing, fg_ozaki.cu) instead of
+// rank-32 updates on the FP64 pipe (9,492 coarse dofs: updates inside the panels 11.2 -> 7.0 ms).
 static fg_status chol_partial_grid(fg_ctx* ctx, double* A, int64_t lda, int N, int ncols, int zrow, int* err,
                                    void* work = nullptr) {
   cudaStream_t st = ctx->stream;
@@ -1829,13 +1846,20 @@ static fg_status chol_partial_grid(fg_ctx* ctx, double* A, int64_t lda, int N, i
       const int Neff = (int)std::min<int64_t>(N, (int64_t)zrow + j0 + nb);
       const int rows = Neff - j0 - nb;
       if (rows > 0) {
-        k_chol_trsm1<<<nblk(rows, 64), 64, 0, st>>>(A, lda, Neff, j0, nb);
+        k_chol_trsm1<<<nblk(rows, 64), 128, 0, st>>>(A, lda, Neff, j0, nb);
         const int nt = (rows + 63) / 64;
         if (work) {
-          const int ntc = (J1 - (j0 + nb) + 63) / 64;  // columns left inside the panel
-          if (ntc > 0) {
-            k_chol_syrk_panel<<<dim3((unsigned)nt, (unsigned)ntc), 256, 0, st>>>(A, lda, Neff, j0, nb, J1);
+          // the rest of this 64-column half of the panel; after the first half, the second on the
+          // tensor cores (columns J0 + 64 .. J1 of the rows below them, rank 64)
+          const int h1 = std::min(J1, J0 + ((j0 - J0) / 64 + 1) * 64);
+          if (h1 > j0 + nb) {
+            k_chol_syrk_panel<<<dim3((unsigned)nt, 1), 256, 0, st>>>(A, lda, Neff, j0, nb, h1);
             ctx->launches += 1;
+          } else if (h1 < J1) {
+            double* P = A + h1 + (int64_t)J0 * lda;
+            int* oz_err = (int*)((uint8_t*)work + ozaki_workspace_bytes(N, N, 128, true));
+            FG_TRY(ozaki_gemm_nt(ctx, st, Neff - h1, J1 - h1, h1 - J0, -1.0, P, 1, lda, P, 1, lda, 1.0,
+                                 A + h1 + (int64_t)h1 * lda, 1, lda, true, work, oz_err));
           }
         } else {
           k_chol_syrk1<<<(unsigned)((int64_t)nt * (nt + 1) / 2), 256, 0, st>>>(A, lda, Neff, j0, nb, nt);
