@@ -798,7 +798,7 @@ struct fg_batch {
   fg::LineTables line[fg::kBatchMaxP];
   std::vector<int64_t> nf, nx;            // source / output lengths
   int threads = 0, ctas = 0, max_team = 0, teams_gt1 = 0;
-  // team sizing: a problem gets at most ceil(work / (team_share * per-CTA share)) CTAs
+  // team sizing: a problem gets about ceil(work / (team_share * per-CTA share)) CTAs
   // (0.5, or FG_BATCH_TEAM_SHARE when set > 0)
   double team_share = 0.5;
   double predicted_balance = 0.0, autotune_ms = 0.0, run_ms = 0.0;
@@ -837,10 +837,11 @@ static size_t batch_smem() { return sizeof(BatchSmem); }
 // Team sizes and the per-CTA job lists (greedy list scheduling, problems by decreasing work).
 // A problem with t CTAs takes its iterations (measured: 3, 8, 20 per cell in a direction at
 // orders 1-3) times its share of the nodes plus what an iteration's reductions and barriers cost:
-// on GB300 12 us with one CTA of 512 threads, ~20 us in a team, against 7.9 ns per node, i.e. 3
-// and 5 nodes per thread.  A problem's team is at most ceil(work / (team_share x a CTA's share));
-// all teams are scaled down together by 1, 1.4, 2, 2.8 and the schedule that ends first by this
-// model is taken (96 problems, n 8-24: 66 ms unscaled, 45 ms at 2).
+// on GB300 12 us with one CTA of 512 threads, ~30 us in a large team, against 7.9 ns per node, i.e. 3
+// and 8 nodes per thread.  A problem's team is about ceil(work / (team_share x a CTA's share));
+// all teams are scaled together and the schedule that ends first by this model is taken (96
+// problems, n 8-24: 66 ms unscaled, 44 ms; 200 problems, n 6-30: 130 ms with four scales and 5
+// nodes per thread, 118 ms so).
 static void batch_schedule(fg_batch* B, int G, std::vector<int>& job_ptr, std::vector<BatchJob>& jobs) {
   const int np = B->nprob;
   std::vector<double> nodes(np), its(np), w(np);
@@ -861,7 +862,10 @@ static void batch_schedule(fg_batch* B, int G, std::vector<int>& job_ptr, std::v
   std::vector<std::vector<BatchJob>> per(G), best_per(G);
   std::vector<double> avail(G);
   std::vector<int> idx(G);
-  for (double scale : {1.0, 1.4, 2.0, 2.8}) {
+  // (a schedule of thousands of problems takes the host tens of ms, and its teams are few)
+  const std::vector<double> scales = np <= 1024 ? std::vector<double>{0.7, 0.85, 1.0, 1.2, 1.4, 1.7, 2.0, 2.4, 2.8, 3.4}
+                                                : std::vector<double>{1.0, 1.4, 2.0, 2.8};
+  for (double scale : scales) {
     std::fill(avail.begin(), avail.end(), 0.0);
     for (auto& v : per) v.clear();
     for (int i : order) {
@@ -877,7 +881,7 @@ static void batch_schedule(fg_batch* B, int G, std::vector<int>& job_ptr, std::v
       std::sort(idx.begin(), idx.begin() + t);
       double start = 0.0;
       for (int k = 0; k < t; ++k) start = std::max(start, avail[idx[k]]);
-      const double end = start + its[i] * (nodes[i] / t + (t > 1 ? 5.0 : 3.0) * B->threads);
+      const double end = start + its[i] * (nodes[i] / t + (t > 1 ? 8.0 : 3.0) * B->threads);
       for (int k = 0; k < t; ++k) {
         avail[idx[k]] = end;
         per[idx[k]].push_back({i, k});

@@ -485,9 +485,9 @@ typedef struct {
   double predicted_balance;  /* planner's estimate: mean CTA load / the longest            */
   double run_ms;             /* last fg_batch_run (device events, copies included)         */
   double autotune_ms;
-  double team_share;         /* largest teams considered: a problem gets at most
-                                ceil(work / (team_share x a CTA's share)) CTAs (the planner
-                                may scale all teams down)                                   */
+  double team_share;         /* team sizes the planner starts from: a problem gets about
+                                ceil(work / (team_share x a CTA's share)) CTAs, all teams
+                                scaled together to the schedule that ends first             */
 } fg_batch_info;
 /* flags: FG_INPUTS_ON_DEVICE = qp_source and x are device pointers (read / written in place
  * at every run); otherwise host pointers, copied in and out by every run.  params: rtol,
