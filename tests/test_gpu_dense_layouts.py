@@ -89,3 +89,21 @@ def test_sum_to_fp64(env, p, q):
                           torch.zeros((109, 65), dtype=torch.float64, device="cuda"), alpha=sign)
         want = sign * np.ldexp(A[:, 2], p + q)
         assert np.array_equal(C.cpu().numpy(), np.repeat(want[:, None], 65, axis=1))
+
+
+@pytest.mark.parametrize("m,n,k", [(300, 64, 64), (300, 130, 33), (129, 65, 128), (64, 200, 20), (700, 700, 64)])
+def test_lower_rectangular(env, m, n, k):
+    """The tiles of a triangular update of another shape than square: fewer columns than rows (a panel's),
+    more, and the ragged last row and column of tiles; elements above the diagonal stay as they are."""
+    ctx, dense, torch = env
+    rng = np.random.default_rng(m + n + k)
+    A, B, C0 = rng.standard_normal((m, k)), rng.standard_normal((n, k)), rng.standard_normal((m, n))
+    C = torch.from_numpy(np.ascontiguousarray(C0.T)).cuda().t()
+    dense.gemm_nt(ctx, torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda(), C, alpha=-1.0, beta=1.0, lower=True)
+    got = C.cpu().numpy()
+    ref = A.astype(np.longdouble) @ B.astype(np.longdouble).T
+    scale = np.abs(A).max(1)[:, None] * np.abs(B).max(1)[None, :]
+    tol = k * 2.0 ** -53 * scale + 2.0 ** -52 * (np.abs(ref) + np.abs(C0))
+    lower = np.tril(np.ones((m, n), dtype=bool))
+    assert np.all(np.abs(got - (C0 - ref))[lower] <= tol[lower])
+    assert np.array_equal(got[~lower], C0[~lower])
