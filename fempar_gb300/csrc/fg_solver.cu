@@ -744,6 +744,17 @@ struct SliceRef {
     }
     return acc;
   }
+  // a warp's place without a slice (fewer slices than warps): no groups, no row.  The products still
+  // run over it, so every pointer is a valid one (cell blocks read their first columns before the
+  // loop over the groups)
+  __device__ __forceinline__ void none(const MatArgs<T>& m, const int32_t* s_off) {
+    vp = m.val;
+    cp = STENCIL ? s_off : ML == ML_DG ? m.blk : m.scol;
+    w4 = 0;
+    base = ML == ML_DG ? m.nn : 0;
+    vec = -1;
+    sv = nullptr;
+  }
   __device__ __forceinline__ void load(const MatArgs<T>& m, int64_t s, int lane, const int32_t* s_off) {
     if (STENCIL) {
       const int k = m.scls[s];
@@ -913,9 +924,9 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, false), pcg_blocks(R))
     for (int k = 0; k < RR; ++k) {
       const int64_t s = warp + k * nwarps;
       rx[k] = rr_[k] = rp[k] = rd[k] = 0.0;
-      ref[k].vec = -1;
-      ref[k].w4 = 0;
-      if (s < m.nslices) {
+      if (s >= m.nslices) {
+        ref[k].none(m, s_off);
+      } else {
         ref[k].load(m, s, lane, s_off);
         const int32_t v = ref[k].vec;
         if (v >= 0) {
@@ -1102,9 +1113,9 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, true), pcg_blocks(R))
     for (int k = 0; k < RR; ++k) {
       const int64_t s = warp + k * nwarps;
       rx[k] = rr_[k] = rp[k] = 0.f;
-      ref[k].vec = -1;
-      ref[k].w4 = 0;
-      if (s < m.nslices) {
+      if (s >= m.nslices) {
+        ref[k].none(m, s_off);
+      } else {
         ref[k].load(m, s, lane, s_off);
         const int32_t v = ref[k].vec;
         if (v >= 0) {
