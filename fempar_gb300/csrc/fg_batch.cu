@@ -216,6 +216,7 @@ __device__ bool team_sum(const BatchArgs& a, const BatchProb& P, int prob, int r
       __syncwarp();
       if (lane == 0) ok = team_arrive_wait(a, P, prob, rank, phase);
       ok = __shfl_sync(0xffffffffu, ok, 0);
+      __syncwarp();  // lane 0 acquired the other CTAs' partials (a shuffle orders no memory)
       x = 0.0;
       if (ok && k < NV)
 #pragma unroll 4
