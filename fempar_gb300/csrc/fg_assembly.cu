@@ -653,7 +653,7 @@ __global__ void __launch_bounds__(CellGeo<P>::WARPS * 32)
     if (!act) continue;
     const double d = neg ? fabs(det) : det, w = qw[q];
     if (src.fn != FG_FN_ZERO) {
-      double fq = src.prm[0];
+      double fq = src.fn == FG_FN_CONST ? src.prm[0] : 0.0;
       if (src.fn == FG_FN_QP_VALUES) fq = src.qp[c * NQ + q];
       else if (src.fn == FG_FN_SHARP_WAVE) {
         double x[3] = {0.0, 0.0, 0.0};
