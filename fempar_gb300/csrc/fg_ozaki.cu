@@ -84,6 +84,7 @@ constexpr uint32_t oz_a_bytes(int S) { return S * OZ_BLOCK; }  // a row tile's d
 constexpr uint32_t OZ_TMEM_COLS = 512;                     // all of it
 constexpr long long OZ_WAIT_CYCLES = 1ll << 31;            // ~1 s at 2 GHz
 constexpr int OZ_EPI_WARPS = 16;                           // epilogue warps: 4 per TMEM lane quarter
+constexpr int OZ_NONFINITE = 1 << 28;                      // row exponent of a row with a NaN or an infinity
 constexpr int OZ_THREADS = (OZ_EPI_WARPS + 2) * 32;        // with the MMA warp (0) and the copy warp (17)
 
 // Output tiles of 128 x BN: the 8 accumulators of BN = 64 columns fill the tensor memory.
@@ -244,7 +245,8 @@ __global__ void __launch_bounds__(OZ_BM) k_oz_rowexp(OzSplitArgs a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   auto finish = [&](int local, unsigned long long mx) {
     const int E = (int)(mx >> 52);  // biased exponent of the largest |x| (0: zero/subnormal)
-    a.ex[(int64_t)rtile * OZ_BM + local] = mx == 0 ? 0 : (E == 0 ? 1 : E) - 1020;
+    // a NaN or an infinity in the row: no digits, the epilogue makes its results NaN
+    a.ex[(int64_t)rtile * OZ_BM + local] = E == 0x7FF ? OZ_NONFINITE : mx == 0 ? 0 : (E == 0 ? 1 : E) - 1020;
   };
   auto bits = [&](int64_t r, int64_t l) {
     return (unsigned long long)__double_as_longlong(it.x[r * it.rs + l * it.cs]) & 0x7FFFFFFFFFFFFFFFull;
@@ -416,6 +418,7 @@ __device__ __forceinline__ double sum_f64(long long h, uint32_t l, int off, uint
 
 // the same for any sum (kept out of line: it costs FP64 operations)
 __device__ __noinline__ double sum_slow(long long h, uint32_t l, int off, uint32_t flip) {
+  if (off >= OZ_NONFINITE / 2) return __longlong_as_double(0x7FF8000000000000ll);
   bool slow;
   return ldexp(sum_f64(h, l, 0, flip, slow), off);
 }
@@ -662,13 +665,15 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(OzGemmArgs g) {
       // lane j < EPI holds the exponent of column c0 + j (padding rows of the exponents are 0)
       const int ecol = g.ex[(int64_t)(it.brow0 + ct / T::QB) * OZ_BM + (ct % T::QB) * BN + part4 * OZ_EPI_COLS +
                             (lane < OZ_EPI_COLS ? lane : 0)];
+      // a row of A or B in this warp's part holds a NaN or an infinity
+      const bool nonfinite = __any_sync(0xffffffffu, max(ei, ecol) == OZ_NONFINITE);
       const int nv = i < it.m ? min(it.n - c0, g.lower ? i - c0 + 1 : OZ_EPI_COLS) : 0;  // columns to write
       double* crow = it.c + (int64_t)i * it.c_rs + (int64_t)c0 * it.c_cs;
 #pragma unroll
       for (int j0 = 0; j0 < OZ_EPI_COLS; j0 += 8) {
         // eight columns at a time: their C values are loaded before any store
         double cv[8], xs[8];
-        bool any = false;
+        bool any = nonfinite;
 #pragma unroll
         for (int j = 0; j < 8; ++j) cv[j] = (j0 + j < nv && bmode != 0) ? crow[(int64_t)(j0 + j) * it.c_cs] : 0.0;
 #pragma unroll

@@ -554,7 +554,8 @@ fg_status fg_server_destroy(fg_server* srv);
  * flags: FG_DENSE_LOWER writes only the elements with i >= j.  FP64 is emulated by 7 signed
  * 8-bit digits per value and row (Ozaki scheme) with 56 bits below the row's maximum; the
  * result is within ~k 2^-53 max|A_i.| max|B_j.| of the exact product (the FP64 dot-product
- * bound), plus the FP64 rounding of the update.  No counterpart in the
+ * bound), plus the FP64 rounding of the update.  A NaN or an infinity in a row of A or B makes
+ * that row's or column's products NaN.  No counterpart in the
  * reference (its dense factorisations call MKL / PARDISO); the building block of the BDDC
  * set-up's factorisations.  Returns FG_ERR_TIMEOUT if a bounded device wait ran out. */
 #define FG_DENSE_LOWER 1
