@@ -1706,12 +1706,17 @@ static fg_status read_state(const Work& w, SolveState& h, cudaStream_t st) {
   return FG_OK;
 }
 
-// grid barriers of the CG kernels: bounded at 10 s (FG_PCG_BARRIER_TIMEOUT_MS; read per solve)
+// grid barriers of the CG kernels: bounded at 10 s, or FG_PCG_BARRIER_TIMEOUT_MS (read per solve; a value
+// that is not a positive number of milliseconds changes nothing)
 static GridSync grid_sync(const Work& w) {
-  const char* ms = getenv("FG_PCG_BARRIER_TIMEOUT_MS");
+  unsigned long long ms = 10000;
+  if (const char* e = getenv("FG_PCG_BARRIER_TIMEOUT_MS")) {
+    char* end = nullptr;
+    const long long v = strtoll(e, &end, 10);
+    if (end != e && *end == 0 && v > 0) ms = (unsigned long long)std::min<long long>(v, 86400000);
+  }
   const char* drop = getenv("FG_PCG_TEST_DROP_ARRIVAL");
-  return GridSync{w.rb.part, w.rb.ticket + 1, w.I + I_ABORT, (ms ? (unsigned long long)atoll(ms) : 10000ull) * 1000000ull,
-                  drop ? atoi(drop) : 0};
+  return GridSync{w.rb.part, w.rb.ticket + 1, w.I + I_ABORT, ms * 1000000ull, drop ? atoi(drop) : 0};
 }
 
 static int64_t solver_entries(const fg_space* sp) {

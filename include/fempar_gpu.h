@@ -297,7 +297,10 @@ fg_status fg_system_spmv_solver_layout_device(fg_system* sys, int precision, con
  * initial guess (base_iterative_linear_solver.f90:281-282).  Host pointers.
  * Replaces iterative_linear_solver_t%solve -> cg_t (Sources/Lib/LinearAlgebra/IterativeLinearSolver/
  * iterative_linear_solver.f90:124-131, cg.f90:101-407) with jacobi_preconditioner_t
- * (Sources/Lib/LinearAlgebra/Preconditioner/jacobi_preconditioner.f90:356-412). */
+ * (Sources/Lib/LinearAlgebra/Preconditioner/jacobi_preconditioner.f90:356-412).
+ * The iterations run in cooperative launches whose blocks wait for one another; every wait is
+ * bounded at 10 s (environment variable FG_PCG_BARRIER_TIMEOUT_MS, milliseconds), after which the
+ * solve returns FG_ERR_TIMEOUT and the context stays usable. */
 fg_status fg_solve(fg_system* sys, const fg_solver_params* params, const double* b, const double* x0,
                    double* x, fg_solve_info* info);
 /* Same, device pointers (b may be NULL; x0 NULL = zero guess; x written on the device). */
