@@ -1823,6 +1823,7 @@ static fg_status elasticity_element_matrices_tc(fg_system* sys) {
   const size_t wb = tc_align(std::max(ozaki_workspace_bytes(chunk * 6, T::NPAIR, T::KS, false, 8),
                                       ozaki_workspace_bytes(chunk * 3, T::NPAIR, T::KA, false, 8)));
   const size_t need = gs + ga + cs + ca + wb + 256;
+  if (need > ctx->scratch_limit) return FG_ERR_OOM;
   if (!sys->d_tcbuf || sys->tcbuf_bytes < need) {
     dev_free(ctx, sys->d_tcbuf);
     sys->d_tcbuf = nullptr;

@@ -6,7 +6,10 @@
 // takes the oldest request among the class heads that fits.  While the globally oldest
 // request does not fit, newer requests may still be admitted (backfill) only during its
 // first 2 s of waiting, so a large request is not starved by a stream of small ones.
-// Admitted requests run concurrently: their kernels overlap on the GPU.  Each request
+// The scratch of an elasticity request's tensor-core element matrices is reserved beside its footprint
+// until it is assembled; a request that fits the budget only without it is assembled by the direct
+// kernels (a rule on the whole budget: the path does not depend on what else runs).
+// Admitted requests run concurrently.  Each request
 // builds mesh, space and system on the device, solves (mixed precision by default) and
 // copies its solution to a host buffer, then frees its device memory.
 #include <algorithm>
@@ -34,6 +37,7 @@ struct Request {
   std::vector<double> coef;
   std::vector<int32_t> ids;
   uint64_t bytes = 0;
+  uint64_t scratch = 0;  // of the element matrices; 0: none, or no room for it in the whole budget
   int64_t nfree = 0;
   int cls = 0;
   Clock::time_point t_submit, t_start, t_end;
@@ -127,8 +131,6 @@ static fg_status footprint(const fg_request* q, uint64_t* bytes, int64_t* nfree_
     // packed upper triangles and the digit workspace (7 bf16 digits, K padded to 16)
     const double K = 6.0 * t.nq, npair = nd * (nd + 1) / 2;
     elm += ncells * (K * 8 + npair * 8 + std::ceil(K / 16.0) * 16 * 7 * 2) + npair * K * 8;
-  } else {
-    elm += (double)elasticity_tc_scratch(p, (int64_t)ncells);  // factors, products and digits of a chunk of cells
   }
   const double csr = nnz * (4 + 8) + nfree * 8.0;             // CSR pattern + FP64 values + row pointers
   const double lay = nnz * 1.15 * (8 + 4);                    // solver layout FP64 + FP32 (padding)
@@ -142,7 +144,15 @@ static fg_status footprint(const fg_request* q, uint64_t* bytes, int64_t* nfree_
   return FG_OK;
 }
 
-static void run_request(fg_ctx* ctx, Request* R) {
+// scratch of a request's element matrices on the tensor cores that its footprint does not hold
+static uint64_t element_scratch(const fg_request* q) {
+  return q->kind == FG_ELASTICITY ? elasticity_tc_scratch(q->order, (int64_t)q->n[0] * q->n[1] * q->n[2]) : 0;
+}
+
+// assembled: called once the element matrices are done with their scratch
+template <class F>
+static void run_request(fg_ctx* ctx, Request* R, F assembled) {
+  ctx->scratch_limit = R->scratch;
   fg_status s = FG_OK;
   fg_mesh* mesh = nullptr;
   fg_space* sp = nullptr;
@@ -164,6 +174,7 @@ static void run_request(fg_ctx* ctx, Request* R) {
     s = fg_assemble(sp, &g, &sys);
     if (s == FG_OK) s = fg_space_release_pattern(sp);
   }
+  assembled();
   fg_solve_info info;
   std::memset(&info, 0, sizeof(info));
   if (s == FG_OK) {
@@ -188,13 +199,15 @@ static Request* pick(fg_server* S) {
     if (!kv.second.empty() && (!oldest || kv.second.front()->id < oldest->id)) oldest = kv.second.front();
   if (!oldest) return nullptr;
   const uint64_t room = S->budget - S->reserved;
-  if (oldest->bytes <= room) return oldest;
+  if (oldest->bytes + oldest->scratch <= room) return oldest;
   // backfill with newer requests only during the oldest one's first 2 s of waiting
   if (ms_between(oldest->t_submit, Clock::now()) > 2000.0) return nullptr;
   Request* best = nullptr;
   for (auto& kv : S->queues)
-    if (!kv.second.empty() && kv.second.front()->bytes <= room && (!best || kv.second.front()->id < best->id))
-      best = kv.second.front();
+    if (!kv.second.empty()) {
+      Request* R = kv.second.front();
+      if (R->bytes + R->scratch <= room && (!best || R->id < best->id)) best = R;
+    }
   return best;
 }
 
@@ -210,11 +223,18 @@ static void worker_main(fg_server* S) {
       R = pick(S);
       if (!R) continue;
       S->queues[R->cls].pop_front();
-      S->reserved += R->bytes;
+      S->reserved += R->bytes + R->scratch;
       S->peak = std::max(S->peak, S->reserved);
       R->t_start = Clock::now();
     }
-    run_request(ctx, R);
+    run_request(ctx, R, [&] {
+      if (R->scratch == 0) return;
+      {
+        std::lock_guard<std::mutex> lk(S->mu);
+        S->reserved -= R->scratch;
+      }
+      S->cv_work.notify_all();
+    });
     {
       std::lock_guard<std::mutex> lk(S->mu);
       R->t_end = Clock::now();
@@ -276,6 +296,8 @@ fg_status fg_server_submit(fg_server* S, const fg_request* req, uint64_t* ticket
               (unsigned long long)S->budget);
     return FG_ERR_OOM;
   }
+  R->scratch = element_scratch(req);
+  if (R->bytes + R->scratch > S->budget) R->scratch = 0;
   const int64_t ncells = (int64_t)req->n[0] * req->n[1] * req->n[2];
   if (req->cell_coef) R->coef.assign(req->cell_coef, req->cell_coef + ncells);
   if (req->n_ids > 0) R->ids.assign(req->dirichlet_ids, req->dirichlet_ids + req->n_ids);
