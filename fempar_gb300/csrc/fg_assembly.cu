@@ -1213,6 +1213,14 @@ static int tc_integration_mode() {
 // the product's workspace and its error flag, 256-byte aligned pieces
 static size_t tc_align(size_t b) { return (b + 255) / 256 * 256; }
 
+// Elasticity and dG systems give the scratch back after each assembly (to the context's pool: a few us), so
+// that a budget which the FP64-pipe kernels and a solve fit in stays enough.
+static void release_tc_scratch(fg_system* sys) {
+  dev_free(sys->space->mesh->ctx, sys->d_tcbuf);
+  sys->d_tcbuf = nullptr;
+  sys->tcbuf_bytes = 0;
+}
+
 // tables of CellGeo: edge weights 1/8 (1 +- x)(1 +- y) per line of Gauss points, 1D shape values,
 // quadrature weights
 template <int P>
@@ -1344,6 +1352,7 @@ static fg_status launch_poisson_tc(fg_system* sys) {
   int h_err = 0;
   FG_CUDA_TRY(cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
   FG_CUDA_TRY(cudaStreamSynchronize(st));
+  if (sp->dg) release_tc_scratch(sys);
   if (h_err) {
     set_error("element matrices on the tensor cores: a bounded device wait ran out");
     return (fg_status)h_err;
@@ -1861,6 +1870,7 @@ static fg_status elasticity_element_matrices_tc(fg_system* sys) {
   int h_err = 0;
   FG_CUDA_TRY(cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
   FG_CUDA_TRY(cudaStreamSynchronize(st));
+  release_tc_scratch(sys);
   if (h_err) {
     set_error("element matrices on the tensor cores: a bounded device wait ran out");
     return (fg_status)h_err;
