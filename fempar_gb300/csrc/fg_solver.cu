@@ -886,6 +886,11 @@ static constexpr int pcg_threads(int R, int ML, bool fp32) {
 }
 static constexpr int pcg_blocks(int R) { return R > 0 ? 1 : 2; }
 
+// the polling chunk that iteration `it` lies in ends before the iteration limit
+__host__ __device__ __forceinline__ bool chunk_ends_before(int it, int chunk, int maxit) {
+  return ((int64_t)it + chunk - 1) / chunk * chunk < maxit;
+}
+
 // FP64 CG, the sequence and stopping tests of the reference (cg.f90:101-238, 279-407).
 // idiag null: no preconditioner.  chunk: the polling interval the caller asked for (a
 // non-finite iteration is reported at its end, if the iteration limit lies beyond it).
@@ -1017,7 +1022,7 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, false), pcg_blocks(R))
       sc[2] = trz;
       sc[1] = sc[8] * trz;
       if (!res && !need_pp) sc[5] = sqrt(trz);  // the next iteration's estimate
-      if (!(isfinite(a) && isfinite(trz)) && (it + chunk - 1) / chunk * chunk < maxit) si[0] = 2;
+      if (!(isfinite(a) && isfinite(trz)) && chunk_ends_before(it, chunk, maxit)) si[0] = 2;
     };
     bool ok;
     if (need_pp) {
@@ -1749,7 +1754,9 @@ static fg_status run_pcg64(fg_system* sys, const Work& w, const fg_solver_params
     sp->mesh->ctx->launches += 1;
     FG_TRY(read_state(w, h, st));
     if (h.I[I_DONE]) return FG_OK;
-    if (!std::isfinite(h.S[S_ALPHA]) || !std::isfinite(h.S[S_RZ])) {
+    // (a launch may end inside a chunk)
+    if ((!std::isfinite(h.S[S_ALPHA]) || !std::isfinite(h.S[S_RZ])) &&
+        chunk_ends_before(h.I[I_ITER], chunk, h.I[I_MAXIT])) {
       set_error("non-finite CG scalars");
       return FG_ERR_NUMERIC;
     }
