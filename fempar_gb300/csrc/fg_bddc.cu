@@ -45,6 +45,7 @@
 #include <utility>
 #include <vector>
 
+#include "fg_arith.h"
 #include "fg_internal.h"
 
 namespace fg {
@@ -150,19 +151,6 @@ struct CholSmem {
   int fail;
 };
 
-// s / d from the correctly rounded reciprocal r of d: the quotient with one correction step
-// (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J.
-// Res. Dev. 34, 1990), the rounding of a division in three operations where many values are
-// divided by the same d.
-__device__ __forceinline__ double quotient(double s, double d, double r) {
-  const double q = s * r;
-  return fma(fma(-q, d, s), r, q);
-}
-__device__ __forceinline__ float quotient(float s, float d, float r) {
-  const float q = s * r;
-  return fmaf(fmaf(-q, d, s), r, q);
-}
-
 // Load the nb x nb diagonal block at j0, factor it, leave the factor in sm.D and write it back.
 // Returns false (to every thread) on a non-positive pivot.  128 threads work: warp q holds the
 // columns j = 4c + q, lane = row.  A step divides the pivot column by its pivot (its owner), and
@@ -219,13 +207,24 @@ __device__ bool chol_diag(double* A, int64_t lda, int j0, int nb, CholSmem& sm) 
   return true;
 }
 
-// Row i (>= j0+nb): A[i, j0:j0+nb] <- A[i, j0:j0+nb] D^-T  (D in shared memory, rd the reciprocals
-// of its diagonal)
+// Row i (>= j0+nb): A[i, j0:j0+nb] <- A[i, j0:j0+nb] D^-T (D in shared memory, row length 33), with divisions:
+// for the rare row of which a quotient leaves the range where quotient() rounds like them.
+__device__ __noinline__ void chol_trsm_row_div(double* row, int64_t lda, int nb, const double* D) {
+  for (int k = 0; k < nb; ++k) {
+    double s = row[k * lda];
+    for (int l = 0; l < k; ++l) s -= row[l * lda] * D[k * 33 + l];
+    row[k * lda] = s / D[k * 33 + k];
+  }
+}
+
+// The same by quotients (rd: the reciprocals of D's diagonal)
 __device__ __forceinline__ void chol_trsm_row(double* A, int64_t lda, int j0, int nb, int64_t i, const double (&D)[32][33],
                                               const double* rd) {
   double x[32];
+  double* row = A + i + (int64_t)j0 * lda;
+  bool exact = true;
 #pragma unroll
-  for (int k = 0; k < 32; ++k) x[k] = k < nb ? A[i + (int64_t)(j0 + k) * lda] : 0.0;
+  for (int k = 0; k < 32; ++k) x[k] = k < nb ? row[k * lda] : 0.0;
 #pragma unroll
   for (int k = 0; k < 32; ++k) {
     if (k < nb) {
@@ -233,11 +232,16 @@ __device__ __forceinline__ void chol_trsm_row(double* A, int64_t lda, int j0, in
 #pragma unroll
       for (int l = 0; l < k; ++l) s -= x[l] * D[k][l];
       x[k] = quotient(s, D[k][k], rd[k]);
+      exact &= quotient_exact(x[k], D[k][k]);
     }
+  }
+  if (!exact) {
+    chol_trsm_row_div(row, lda, nb, &D[0][0]);
+    return;
   }
 #pragma unroll
   for (int k = 0; k < 32; ++k)
-    if (k < nb) A[i + (int64_t)(j0 + k) * lda] = x[k];
+    if (k < nb) row[k * lda] = x[k];
 }
 
 // Trailing tile (ti, tj) of 64 x 64 at rows/cols starting t0: A[r, c] -= sum_k A[r, j0+k] A[c, j0+k]
@@ -638,6 +642,13 @@ __global__ void __launch_bounds__(128) k_chol_trsm1(double* A, int64_t lda, int 
     for (int m = k >> 1; m < 16; ++m)
       if (2 * m + h > k) x[m] -= xk * Dsh[2 * m + h][k];
   }
+  bool exact = true;
+#pragma unroll
+  for (int m = 0; m < 16; ++m) exact &= quotient_exact(x[m], Dsh[2 * m + h][2 * m + h]);
+  if (!(exact & __shfl_xor_sync(0xffffffffu, (int)exact, 1))) {
+    if (h == 0 && i < N) chol_trsm_row_div(row, lda, nb, &Dsh[0][0]);
+    return;
+  }
 #pragma unroll
   for (int m = 0; m < 16; ++m)
     if (i < N && 2 * m + h < nb) row[(2 * m + h) * lda] = x[m];
@@ -707,16 +718,30 @@ __device__ __forceinline__ T warp_sum(T v) {
 // solves 2 x 322 -> 199 us, forward 250 -> 152, backward 364 -> 336 (the loads of a step in groups of
 // eight, columns of the transposed product one after another, and solve and update in turn, before).
 
-// x of warp 0's 32 rows for a lower triangle in row[] (row[k]: column k of the lane's row)
+// x of warp 0's 32 rows for a lower triangle at Ld (rows past n: the unit matrix), with divisions: for the
+// rare block of which a quotient leaves the range where quotient() rounds like them
 template <typename T>
-__device__ __forceinline__ T solve_diag(const T (&row)[32], T xv, T dg, int lane) {
+__device__ __noinline__ T solve_diag_div(const T* Ld, int64_t lda, bool in, T xv, T dg, int lane) {
+  for (int k = 0; k < 32; ++k) {
+    const T xk = __shfl_sync(0xffffffffu, xv / dg, k);
+    if (lane == k) xv = xk;
+    if (lane > k) xv -= (in ? Ld[lane + k * lda] : T(0)) * xk;
+  }
+  return xv;
+}
+
+// The same by quotients; row[k]: column k of the lane's row (in: a row of the matrix)
+template <typename T>
+__device__ __forceinline__ T solve_diag(const T* Ld, int64_t lda, bool in, const T (&row)[32], const T x0, T dg, int lane) {
   const T rd = T(1) / dg;
+  T xv = x0;
 #pragma unroll
   for (int k = 0; k < 32; ++k) {
     const T xk = __shfl_sync(0xffffffffu, quotient(xv, dg, rd), k);
     if (lane == k) xv = xk;
     if (lane > k) xv -= row[k] * xk;
   }
+  if (!__all_sync(0xffffffffu, quotient_exact(xv, dg))) xv = solve_diag_div(Ld, lda, in, x0, dg, lane);
   return xv;
 }
 
@@ -737,7 +762,8 @@ __device__ void trsv_lower(const T* __restrict__ L, int64_t lda, int n, int star
   if (warp == 0) {
     T row[32], dg;
     diag(b0, row, dg);
-    const T xv = solve_diag(row, b0 + lane < n ? x[b0 + lane] : T(0), dg, lane);
+    const bool in = b0 + lane < n;
+    const T xv = solve_diag(L + b0 + (int64_t)b0 * lda, lda, in, row, in ? x[b0 + lane] : T(0), dg, lane);
     if (b0 + lane < n) x[b0 + lane] = xv;
   }
   __syncthreads();
@@ -750,7 +776,7 @@ __device__ void trsv_lower(const T* __restrict__ L, int64_t lda, int n, int star
       T acc = T(0);
 #pragma unroll
       for (int k = 0; k < 32; ++k) acc += (i < n ? Lr[k * lda] : T(0)) * x[j0 + k];
-      const T xv = solve_diag(row, i < n ? x[i] - acc : T(0), dg, lane);
+      const T xv = solve_diag(L + (j0 + 32) * (lda + 1), lda, i < n, row, i < n ? x[i] - acc : T(0), dg, lane);
       if (i < n) x[i] = xv;
     } else {
       for (int i = j0 + 32 + tid; i < n; i += blockDim.x - 32) {
@@ -763,6 +789,18 @@ __device__ void trsv_lower(const T* __restrict__ L, int64_t lda, int n, int star
     }
     __syncthreads();
   }
+}
+
+// Upward through the triangle in a tile (row k of the block is column k of the lanes below it), with
+// divisions; as solve_diag_div
+template <typename T>
+__device__ __noinline__ T solve_up_div(const T* column, T xv, T dg, int lane) {
+  for (int k = 31; k >= 0; --k) {
+    const T xk = __shfl_sync(0xffffffffu, xv / dg, k);
+    if (lane == k) xv = xk;
+    if (lane < k) xv -= column[k] * xk;
+  }
+  return xv;
 }
 
 // Solve L^T x = x in place for rows [0, n); blockDim 256.
@@ -794,13 +832,14 @@ __device__ void trsv_upper_t(const T* __restrict__ L, int64_t lda, int n, T* x) 
         if (j0 + 32 + k < n) acc += tile[1][lane][k] * x[j0 + 32 + k];
       xv -= acc;
       // upward: row k of the block is column k of the lanes below it.  Rows past n: the unit matrix
-      const T dg = j0 + lane < n ? tile[0][lane][lane] : T(1), rd = T(1) / dg;
+      const T dg = j0 + lane < n ? tile[0][lane][lane] : T(1), rd = T(1) / dg, x0 = xv;
 #pragma unroll
       for (int k = 31; k >= 0; --k) {
         const T xk = __shfl_sync(0xffffffffu, quotient(xv, dg, rd), k);
         if (lane == k) xv = xk;
         if (lane < k) xv -= tile[0][lane][k] * xk;
       }
+      if (!__all_sync(0xffffffffu, quotient_exact(xv, dg))) xv = solve_up_div(tile[0][lane], x0, dg, lane);
       if (j0 + lane < n) x[j0 + lane] = xv;
     } else if (j0 >= 32) {
       // the next block's columns with the rows from j0 + 32 on, up to five columns per warp
