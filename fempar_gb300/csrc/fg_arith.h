@@ -46,4 +46,26 @@ FG_HD bool quotient_exact(float q, float d) {
                                           (unsigned)(eq + ed + 100) <= 225u;
 }
 
+// s + e = a + b exactly (Knuth's TwoSum)
+FG_HD void two_sum(float a, float b, float& s, float& e) {
+  s = a + b;
+  const float bb = s - a;
+  e = (a - (s - bb)) + (b - bb);
+}
+
+// Sum of FP32 pairs hi + lo (|lo| at most a few last places of hi) in three FP32 words: the first two by
+// exact sums, their errors in the third, so what is lost is ~2^-70 of the sum of magnitudes, less than
+// FP64 additions lose, on the FP32 pipe.
+struct Sum3 {
+  float h = 0.f, m = 0.f, l = 0.f;
+  FG_HD void add(float h2, float m2, float l2) {
+    float e, t, e2, e3;
+    two_sum(h, h2, h, e);
+    two_sum(m, m2, t, e2);
+    two_sum(t, e, m, e3);
+    l += l2 + (e2 + e3);
+  }
+  FG_HD double value() const { return ((double)m + (double)l) + (double)h; }
+};
+
 }  // namespace fg

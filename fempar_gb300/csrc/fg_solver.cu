@@ -24,8 +24,8 @@
 // Inner products.  GB300 runs FP64 FMA and FP32<->FP64 conversion at about 0.5 Tera-op/s,
 // some 70x below FP32.  FP64-path dots accumulate in FP64.  FP32-path dots form each
 // product exactly as an FP32 pair (p = a*b, e = fma(a,b,-p)) and accumulate it with a
-// compensated (double-float) sum; blocks add their threads' pairs in float-float and the grid
-// total is formed in FP64.  Reductions are deterministic: fixed grid, fixed per-thread index
+// compensated (double-float) sum; blocks add their threads' pairs in three FP32 words (more than FP64
+// holds) and the grid total is formed in FP64.  Reductions are deterministic: fixed grid, fixed per-thread index
 // sets, block partials summed in a fixed order.
 #include <algorithm>
 #include <cmath>
@@ -34,6 +34,7 @@
 #include <map>
 #include <mutex>
 
+#include "fg_arith.h"
 #include "fg_internal.h"
 
 namespace fg {
@@ -87,8 +88,9 @@ struct AccPlain {
   __device__ __forceinline__ double value() const { return (double)s; }
 };
 
-// (<q,q> of the mixed iteration.  Measured on GB300 at 128^3 Q2: plain sums 1097 iterations,
-// compensated 1106: a thread sums ~80 positive terms, the grid total is formed in FP64.)
+// (<q,q> of the mixed iteration, all terms positive: a thread's 107 at 128^3 Q2 go to two plain sums in turn,
+// the block's sum and the grid's lose less than FP64.  Compensated sums per thread, with 71 terms in a
+// thread, took 1106 iterations there against 1097, and 0.863 ms each against 0.853.)
 
 // the mixed update sums the unscaled residual norm (the stop estimate) every
 // FG_MIXED_EXACT_EVERY iterations; 8 vs 4: -2 us per iteration at 128^3 Q2
@@ -521,25 +523,16 @@ __device__ __forceinline__ bool grid_wait(const GridSync& g, unsigned target) {
   return true;
 }
 
-// sum of the lanes' float-float values
-__device__ __forceinline__ void ff_acc(float& h, float& l, float h2, float l2) {
-  const float s = __fadd_rn(h, h2);
-  const float bb = __fsub_rn(s, h);
-  const float e = __fadd_rn(__fsub_rn(h, __fsub_rn(s, bb)), __fsub_rn(h2, bb));
-  l = __fadd_rn(l, __fadd_rn(l2, e));
-  h = s;
-}
-
 // Block and grid sums of NV accumulators, then f(totals) on thread 0 (the step's scalars, in
 // shared memory); every thread returns after f.  Threads leave their sums in shared memory and
 // the first four warps add them: an FP64 warp instruction holds the pipe of its SM quarter 64
 // cycles, so a warp alone pays that for each of its ~NT/32 + 5 dependent additions per value; the
 // four sit in different quarters and take a quarter of the sums each.  The grid's partial sums go
-// to one warp per value.  FP32 accumulators are added as float-float pairs and become FP64 once
-// per block.  Sums in fixed order: deterministic.  False: the grid barrier gave up.
+// to one warp per value.  FP32 accumulators (pairs) are added in three FP32 words, which lose less
+// than FP64 additions (Sum3), and become FP64 once per block.  Sums in fixed order: deterministic.
+// False: the grid barrier gave up.
 // (Solve with one warp adding and the scalar steps' square roots and reciprocals on their path, and so:
-// 8^3 Q1 FP64, one block, 0.236 -> 0.201 ms; 24^3 Q2 mixed 17.6 -> 16.1 us per iteration; 384^2 Q2
-// FP64 57.9 -> 55.3.)
+// 8^3 Q1 FP64, one block, 0.236 -> 0.201 ms; 384^2 Q2 FP64 57.9 -> 55.3 us per iteration.)
 template <typename T>
 struct RedShared;
 template <>
@@ -548,7 +541,8 @@ struct RedShared<double> {
 };
 template <>
 struct RedShared<float> {
-  float2 v[2][1024], w[4][3];
+  float2 v[2][1024];
+  Sum3 w[4][3];
   double tot[3];
 };
 
@@ -570,16 +564,28 @@ __device__ __forceinline__ void warp_sums(double (&s)[NV], int lane) {
     for (int off = 16; off > 0; off >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], off);
 }
 
-__device__ __forceinline__ void sum_in(double (&s), double v) { s += v; }
-__device__ __forceinline__ void sum_in(float2& s, float2 v) { ff_acc(s.x, s.y, v.x, v.y); }
+// sums of the values V: FP64, or pairs in three words
+template <typename V>
+struct SumOf;
+template <>
+struct SumOf<double> { using type = double; };
+template <>
+struct SumOf<float2> { using type = Sum3; };
+__device__ __forceinline__ void sum_in(double& s, double v) { s += v; }
+__device__ __forceinline__ void sum_in(Sum3& s, float2 v) { s.add(v.x, v.y, 0.f); }
+__device__ __forceinline__ void sum_in(Sum3& s, const Sum3& v) { s.add(v.h, v.m, v.l); }
 __device__ __forceinline__ double shfl_xor(double v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
-__device__ __forceinline__ float2 shfl_xor(float2 v, int m) {
-  return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
+__device__ __forceinline__ Sum3 shfl_xor(const Sum3& v, int m) {
+  Sum3 o;
+  o.h = __shfl_xor_sync(0xffffffffu, v.h, m);
+  o.m = __shfl_xor_sync(0xffffffffu, v.m, m);
+  o.l = __shfl_xor_sync(0xffffffffu, v.l, m);
+  return o;
 }
 __device__ __forceinline__ double to_f64(double v) { return v; }
-__device__ __forceinline__ double to_f64(float2 v) { return (double)v.x + (double)v.y; }
+__device__ __forceinline__ double to_f64(const Sum3& v) { return v.value(); }
 template <int NV>
-__device__ __forceinline__ void warp_sums(float2 (&s)[NV], int) {
+__device__ __forceinline__ void warp_sums(Sum3 (&s)[NV], int) {
 #pragma unroll
   for (int k = 0; k < NV; ++k)
 #pragma unroll
@@ -600,10 +606,11 @@ __device__ __forceinline__ bool grid_reduce(RedShared<T>& sh, const V (&v)[NV], 
       if (nt > 32) asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory");
       else __syncwarp();
     };
-    V s[NV];
+    using A = typename SumOf<V>::type;
+    A s[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-      s[k] = V{};
+      s[k] = A{};
       for (int i = t; i < (int)blockDim.x; i += nt) sum_in(s[k], sh.v[k][i]);
     }
     warp_sums(s, lane);
@@ -615,7 +622,7 @@ __device__ __forceinline__ bool grid_reduce(RedShared<T>& sh, const V (&v)[NV], 
     double* part = g.part + (size_t)buf * 3 * gridDim.x;
     if (warp == 0) {
       // lane 4 k + w: value k of warp w
-      V y = lane < 4 * NV && (lane & 3) < (nt >> 5) ? sh.w[lane & 3][lane >> 2] : V{};
+      A y = lane < 4 * NV && (lane & 3) < (nt >> 5) ? sh.w[lane & 3][lane >> 2] : A{};
       sum_in(y, shfl_xor(y, 1));
       sum_in(y, shfl_xor(y, 2));
       if (lane < 4 * NV && (lane & 3) == 0) {
@@ -1142,7 +1149,7 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, true), pcg_blocks(R))
     // beside the product: 1/rr for beta (see k_pcg64)
     if (threadIdx.x == blockDim.x - 32) sd[8] = 1.0 / sd[0];
     Acc<float> pq;
-    AccPlain qq;
+    AccPlain qq, qq1;  // <q,q>: the slices' rows alternate between two sums
     if (R > 0) {
 #pragma unroll
       for (int k = 0; k < RR; ++k) {
@@ -1162,9 +1169,13 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, true), pcg_blocks(R))
           pq.add(a, p[w.vec]);
           qq.add(a, a);
         }
+        const float t = qq.s;
+        qq.s = qq1.s;
+        qq1.s = t;
       }
     }
-    const float2 v2[2] = {make_float2(pq.hi, pq.lo), make_float2(qq.s, 0.f)};
+    float2 v2[2] = {make_float2(pq.hi, pq.lo), make_float2(qq.s, 0.f)};
+    if (R == 0) two_sum(qq.s, qq1.s, v2[1].x, v2[1].y);
     if (!grid_reduce<2>(sh, v2, g, 0, target, &si[3], [&](double (&t)[2]) {
           const double pap = t[0], nq = t[1], rr = sd[0];
           int skip = si[0] != FLAG_NONE;
