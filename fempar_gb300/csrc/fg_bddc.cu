@@ -1898,7 +1898,7 @@ static fg_status chol_partial_grid(fg_ctx* ctx, double* A, int64_t lda, int N, i
             double* P = A + h1 + (int64_t)J0 * lda;
             int* oz_err = (int*)((uint8_t*)work + ozaki_workspace_bytes(N, N, 128, true));
             FG_TRY(ozaki_gemm_nt(ctx, st, Neff - h1, J1 - h1, h1 - J0, -1.0, P, 1, lda, P, 1, lda, 1.0,
-                                 A + h1 + (int64_t)h1 * lda, 1, lda, true, work, oz_err));
+                                 A + h1 + (int64_t)h1 * lda, 1, lda, true, work, oz_err, 8));
           }
         } else {
           k_chol_syrk1<<<(unsigned)((int64_t)nt * (nt + 1) / 2), 256, 0, st>>>(A, lda, Neff, j0, nb, nt);
@@ -1963,7 +1963,10 @@ static fg_status bddc_numeric(fg_bddc* B) {
       }
       return items;
     };
-    // the 32 columns at j0 into the rest of their 128-column panel
+    // the 32 columns at j0 into the rest of their 128-column panel, with eight digits: the FP64 pipe did
+    // these updates, and seven leave a factor entry far below its row's largest with fewer bits (componentwise
+    // residual of a panel 1.4e-13 for lognormal Q2 Poisson, 4.5e-15 with eight, 1.2e-15 in FP64; against
+    // sqrt(a_ii a_jj) 7.8e-16 either way and 1.1e-15 in FP64)
     auto step_items = [&](int j0, int J1) {
       std::vector<OzSyrk> items;
       for (const BSub& S : B->subs) {
@@ -1975,7 +1978,7 @@ static fg_status bddc_numeric(fg_bddc* B) {
       }
       return items;
     };
-    const size_t wbytes = std::max(ozaki_syrk_batch_bytes(panel_items(0)), ozaki_syrk_batch_bytes(step_items(0, 128)));
+    const size_t wbytes = std::max(ozaki_syrk_batch_bytes(panel_items(0)), ozaki_syrk_batch_bytes(step_items(0, 128), 8));
     void* work = nullptr;
     FG_TRY(dev_alloc(ctx, &work, wbytes + sizeof(int)));
     int* oz_err = (int*)((uint8_t*)work + wbytes);
@@ -1987,7 +1990,7 @@ static fg_status bddc_numeric(fg_bddc* B) {
         const int rem = B->maxN - j0 - 1;
         if (rem > 0) {
           k_bstep_trsm<<<dim3(nblk(rem, 256), ns), 256, 0, st>>>(B->d_subs, B->dA, j0);
-          if (ls == FG_OK) ls = ozaki_syrk_batch(ctx, st, step_items(j0, J0 + 128), work, wbytes, oz_err);
+          if (ls == FG_OK) ls = ozaki_syrk_batch(ctx, st, step_items(j0, J0 + 128), work, wbytes, oz_err, 8);
           ctx->launches += 1;
         }
         ctx->launches += 1;

@@ -300,15 +300,15 @@ fg_status ozaki_gemm_nt(fg_ctx* ctx, cudaStream_t st, int64_t m, int64_t n, int6
                         int digits = 7);
 // A batch of lower rank-k updates C_b -= P_b P_b^T (k_b <= 128, column-major with leading
 // dimension ld_b; the first n_b <= m_b columns of C_b), in one launch of each kernel; work holds
-// ozaki_syrk_batch_bytes(b) bytes.
+// ozaki_syrk_batch_bytes(b, digits) bytes.
 struct OzSyrk {
   const double* p;
   double* c;
   int64_t ld;
   int m, k, n;
 };
-size_t ozaki_syrk_batch_bytes(const std::vector<OzSyrk>& b);
+size_t ozaki_syrk_batch_bytes(const std::vector<OzSyrk>& b, int digits = 7);
 fg_status ozaki_syrk_batch(fg_ctx* ctx, cudaStream_t st, const std::vector<OzSyrk>& b, void* work, size_t bytes,
-                           int* d_err);
+                           int* d_err, int digits = 7);
 
 }  // namespace fg

@@ -822,15 +822,15 @@ static int syrk_ksteps(const std::vector<OzSyrk>& b) {
   for (const auto& x : b) k = std::max(k, x.k);
   return (k + OZ_BK - 1) / OZ_BK;
 }
-size_t ozaki_syrk_batch_bytes(const std::vector<OzSyrk>& b) {
+size_t ozaki_syrk_batch_bytes(const std::vector<OzSyrk>& b, int digits) {
   int64_t rt = 0;
   for (const auto& x : b) rt += rtiles_of(x.m);
-  return (size_t)rt * syrk_ksteps(b) * oz_a_bytes(OZ_S) + (size_t)rt * OZ_BM * sizeof(int32_t) +
+  return (size_t)rt * syrk_ksteps(b) * oz_a_bytes(digits) + (size_t)rt * OZ_BM * sizeof(int32_t) +
          b.size() * (sizeof(OzSplit) + sizeof(OzItem)) + 512;
 }
 
 fg_status ozaki_syrk_batch(fg_ctx* ctx, cudaStream_t st, const std::vector<OzSyrk>& b, void* work, size_t bytes,
-                           int* d_err) {
+                           int* d_err, int digits) {
   std::vector<OzSplit> hs;
   std::vector<OzItem> hi;
   int64_t rt = 0, tiles = 0;
@@ -847,13 +847,13 @@ fg_status ozaki_syrk_batch(fg_ctx* ctx, cudaStream_t st, const std::vector<OzSyr
     tiles += lower_tiles(rtiles_of(x.m), tn);
   }
   if (hs.empty()) return FG_OK;
-  if (tiles > (1ll << 31) - 1 || ozaki_syrk_batch_bytes(b) > bytes) {
+  if (tiles > (1ll << 31) - 1 || ozaki_syrk_batch_bytes(b, digits) > bytes) {
     set_error("ozaki_syrk_batch: workspace too small or too many tiles");
     return FG_ERR_UNSUPPORTED;
   }
   const int ksteps = syrk_ksteps(b);
   uint8_t* w = (uint8_t*)work;
-  const size_t dig_bytes = (size_t)rt * ksteps * oz_a_bytes(OZ_S);
+  const size_t dig_bytes = (size_t)rt * ksteps * oz_a_bytes(digits);
   int32_t* ex = (int32_t*)(w + dig_bytes);
   uint8_t* tail = (uint8_t*)ex + (size_t)rt * OZ_BM * sizeof(int32_t);
   tail = (uint8_t*)(((uintptr_t)tail + 255) & ~(uintptr_t)255);
@@ -880,7 +880,7 @@ fg_status ozaki_syrk_batch(fg_ctx* ctx, cudaStream_t st, const std::vector<OzSyr
   g.beta = 1.0;
   g.lower = 1;
   g.err = d_err;
-  return oz_launch<OZ_S>(ctx, st, sa, rt, g, tiles);
+  return digits == 8 ? oz_launch<8>(ctx, st, sa, rt, g, tiles) : oz_launch<OZ_S>(ctx, st, sa, rt, g, tiles);
 }
 
 }  // namespace fg
