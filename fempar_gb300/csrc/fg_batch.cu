@@ -33,6 +33,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "fg_internal.h"
@@ -45,7 +46,7 @@ static constexpr int kApplySmem = 32768;  // bytes for the partly summed rows of
 
 struct BatchProb {
   int n, p, L, F;        // cells per direction, order, lattice nodes, interior nodes per direction
-  float kh_hi, kh_lo;    // stencil scale k h / 2 as float-float
+  float kh_hi, kh_lo;    // stencil scale k h / 2 (times the line tables') as float-float
   double h3;             // (h/2)^3, load-vector scale
   const double* f;       // Gauss-point source, n^3 (p+1)^3
   double* x;             // output, F^3 interior nodes
@@ -60,10 +61,23 @@ struct BatchJob {
 };
 
 // 1D assembled rows of mass and stiffness per node class c = I mod p, as float-float: column t is
-// the neighbour I - p + t for class 0 (2p + 1 of them) and I - c + t for the others (p + 1)
+// the neighbour I - p + t for class 0 (2p + 1 of them) and I - c + t for the others (p + 1).  The entries
+// are rational with a common denominator per order and table, so the tables hold small integers (times a
+// power of two), exact in FP32, and kScale goes into each problem's stencil scale.  Rounded entries
+// (1/3, 7/3, ..) made the FP32 operator's <v, A v> for smooth v off by 4e-7 (Q1, 32 nodes in a direction) to
+// 7e-6 (Q3); so it is off by 3e-9 to 1e-7, and the assembled stencil's was by 5e-7 to 9e-6.
 struct LineTables {
   float m[kBatchMaxP][2 * kBatchMaxP + 1][2], s[kBatchMaxP][2 * kBatchMaxP + 1][2];
 };
+
+// mass and stiffness entries times kMass and kStiff are integers (in the tables times 2^-kMassExp and
+// 2^-kStiffExp); index p - 1
+static constexpr double kMass[kBatchMaxP] = {3, 15, 840}, kStiff[kBatchMaxP] = {2, 6, 80};
+static constexpr int kMassExp[kBatchMaxP] = {0, 4, 10}, kStiffExp[kBatchMaxP] = {0, 3, 6};
+// the tables' operator times this is the unit operator
+static double line_scale(int p) {
+  return std::ldexp(1.0, 2 * kMassExp[p - 1] + kStiffExp[p - 1]) / (kMass[p - 1] * kMass[p - 1] * kStiff[p - 1]);
+}
 
 struct OrderTables {
   int ncls;
@@ -334,6 +348,7 @@ __device__ __forceinline__ void apply_rows(const LineTables& T, BatchSmem& sm, c
   using P2 = typename S::P2;
   constexpr int NR = ApplyShape<PO>::NR, NY = ApplyShape<PO>::NY, YB = ApplyShape<PO>::YB;
   constexpr int CAP = kApplySmem / (int)sizeof(P2) / NR;  // nodes of x
+  constexpr bool kDiff = PO == 1 && std::is_same<S, S32>::value;
   P2* rows = reinterpret_cast<P2*>(sm.rows);
   const int nyb = (n + YB - 1) / YB;
   // pieces of a row block: SP periods each, nodes PO m0 .. PO (m0 + SP) + PO
@@ -350,7 +365,31 @@ __device__ __forceinline__ void apply_rows(const LineTables& T, BatchSmem& sm, c
       V a[NR], b[NR];
 #pragma unroll
       for (int r = 0; r < NR; ++r) a[r] = b[r] = S::zero();
-      if (I >= 1 && I <= F) {
+      if (I >= 1 && I <= F && kDiff) {
+        // Q1, FP32: the tables are (-1, 2, -1) and (1, 4, 1), i.e. S w = (w_0 - w_-) + (w_0 - w_+) and M w =
+        // 6 w_0 - S w: differences of close values cost no digits, and a sum is rounded once
+        const int ny = min(NY, F + 1 - J0), L2 = L * L;
+        const int g = I + L * J0 + L2 * K;
+        float v0[NY], vm[NY], vp[NY], tz[NY], uz[NY];
+#pragma unroll
+        for (int y = 0; y < NY; ++y) {
+          v0[y] = y < ny ? vh[g + y * L] : 0.f;
+          vm[y] = y < ny ? vh[g + y * L - L2] : 0.f;
+          vp[y] = y < ny ? vh[g + y * L + L2] : 0.f;
+        }
+#pragma unroll
+        for (int y = 0; y < NY; ++y) {
+          uz[y] = (v0[y] - vm[y]) + (v0[y] - vp[y]);
+          tz[y] = fmaf(6.f, v0[y], -uz[y]);
+        }
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+          const float st = (tz[r + 1] - tz[r]) + (tz[r + 1] - tz[r + 2]);
+          const float su = (uz[r + 1] - uz[r]) + (uz[r + 1] - uz[r + 2]);
+          reinterpret_cast<float*>(a)[r] = fmaf(6.f, tz[r + 1], -st);
+          reinterpret_cast<float*>(b)[r] = fmaf(6.f, uz[r + 1], -su) + st;
+        }
+      } else if (I >= 1 && I <= F) {
         V tz[NY], uz[NY];
 #pragma unroll
         for (int y = 0; y < NY; ++y) tz[y] = uz[y] = S::zero();
@@ -411,6 +450,12 @@ __device__ __forceinline__ void apply_rows(const LineTables& T, BatchSmem& sm, c
       V o[PO];  // o[0]: the class-0 node at the period's end
 #pragma unroll
       for (int k = 0; k < PO; ++k) o[k] = S::zero();
+      if (kDiff) {
+        const float2* wf = reinterpret_cast<const float2*>(w);
+        const float2 m = wf[0], c = wf[1], n1 = wf[2];
+        const float sa = (c.x - m.x) + (c.x - n1.x), sb = (c.y - m.y) + (c.y - n1.y);
+        reinterpret_cast<float*>(o)[0] = fmaf(6.f, c.y, sa) - sb;
+      } else
 #pragma unroll
       for (int t2 = 0; t2 < 2 * PO + 1; ++t2) {
         const P2 ab = w[t2];
@@ -764,6 +809,12 @@ static void build_order_tables(int p, OrderTables& T, LineTables& line) {
     }
   }
   T.ncls = p * p * p;
+  // exact entries: the quadrature's rounding goes, the scale moves to the stencil scale
+  for (int c = 0; c < p; ++c)
+    for (int t = 0; t < w1[c]; ++t) {
+      M1[c][t] = std::ldexp(std::round(M1[c][t] * kMass[p - 1]), -kMassExp[p - 1]);
+      S1[c][t] = std::ldexp(std::round(S1[c][t] * kStiff[p - 1]), -kStiffExp[p - 1]);
+    }
   auto split = [](double v, float (&f)[2]) {
     f[0] = (float)v;
     f[1] = (float)(v - (double)f[0]);
@@ -1079,7 +1130,7 @@ fg_status fg_batch_create(fg_ctx* ctx, int32_t nprob, const fg_batch_problem* pr
     P.p = q.order;
     P.L = q.order * q.n + 1;
     P.F = q.order * q.n - 1;
-    const double kh = q.coef * (0.5 / q.n);
+    const double kh = q.coef * (0.5 / q.n) * line_scale(q.order);
     P.kh_hi = (float)kh;
     P.kh_lo = (float)(kh - (double)P.kh_hi);
     const double hh = 0.5 / q.n;
