@@ -865,13 +865,10 @@ __device__ void trsv_upper_t(const T* __restrict__ L, int64_t lda, int n, T* x) 
   }
 }
 
-// 8^3 subdomains on 152 SMs: four CTAs per SM hold them all at once
-template <typename T>
-static constexpr int apply_blocks() { return sizeof(T) == 4 ? 4 : 2; }
-
+// CTAS: CTAs per SM that the registers must leave room for (many_small).
 // Steps 1 (PHASE 1) and 5 (PHASE 2): interior Dirichlet solves.
-template <typename T, int PHASE>
-__global__ void __launch_bounds__(256, apply_blocks<T>())
+template <typename T, int PHASE, int CTAS>
+__global__ void __launch_bounds__(256, CTAS)
     k_bddc_dirichlet(const BSub* __restrict__ subs, const double* __restrict__ A, const float* __restrict__ F,
                      const int32_t* __restrict__ loc, const double* __restrict__ r, const T* __restrict__ t,
                      T* __restrict__ u0, double* __restrict__ z) {
@@ -899,8 +896,8 @@ __global__ void __launch_bounds__(256, apply_blocks<T>())
 }
 
 // Step 4, before the coarse solve: z = L^-1 [0; g_E], coarse residual f_Pi.
-template <typename T>
-__global__ void __launch_bounds__(256, apply_blocks<T>())
+template <typename T, int CTAS>
+__global__ void __launch_bounds__(256, CTAS)
     k_bddc_neumann_fwd(const BSub* __restrict__ subs, const double* __restrict__ A, const float* __restrict__ F,
                        const T* __restrict__ R, const T* __restrict__ G, const int32_t* __restrict__ loc,
                        const double* __restrict__ w, const double* __restrict__ r, const T* __restrict__ q,
@@ -949,8 +946,8 @@ __global__ void __launch_bounds__(256, apply_blocks<T>())
 }
 
 // Step 4, after the coarse solve: constrained local solution, weighted interface values.
-template <typename T>
-__global__ void __launch_bounds__(256, apply_blocks<T>())
+template <typename T, int CTAS>
+__global__ void __launch_bounds__(256, CTAS)
     k_bddc_neumann_bwd(const BSub* __restrict__ subs, const double* __restrict__ A, const float* __restrict__ F,
                        const T* __restrict__ R, const T* __restrict__ G, const T* __restrict__ Cv,
                        const int32_t* __restrict__ pc, const T* __restrict__ uc, const T* __restrict__ zE,
@@ -2108,8 +2105,18 @@ static fg_status set_smem(const void* k, size_t bytes) {
   return FG_OK;
 }
 
+// FP32 applies: registers for two CTAs per SM keep a step's loads in flight (128 against 64 registers),
+// where four hide the steps' latency behind one another.  The second pays only where there are more subdomains
+// than two per SM and their factors are small.  Per apply, two against four (Q2 elasticity, 152 SMs; 2^3
+// cells: ~350 dofs in a factor, 3^3: ~1,000, 4^3: ~2,200): 2^3 cells, 512 subdomains 450 / 400 us, 729
+// 626 / 613; 3^3 cells, 125 548 / 803, 216 612 / 904, 343 911 / 946, 512 1,102 / 1,118, 729 1,543 / 1,735;
+// 4^3 cells, 8 to 216 914 / 1,462 to 1,769 / 2,728.
+static bool many_small(const fg_bddc* B) {
+  return B->nsub > 2 * B->sys->space->mesh->ctx->sm_count && B->maxnr <= 640;
+}
+
 // z = M^-1 r on solver-layout FP64 vectors (r: nvec, z: nvec; padding of z untouched).
-template <typename T>
+template <typename T, int CTAS>
 static fg_status bddc_apply_layout(fg_bddc* B, const double* r, double* z) {
   fg_system* sys = B->sys;
   fg_space* sp = sys->space;
@@ -2131,36 +2138,37 @@ static fg_status bddc_apply_layout(fg_bddc* B, const double* r, double* z) {
   const T* Kinv = f32 ? (const T*)B->dKinv32 : (const T*)B->dKinv;
   const int prec = f32 ? FG_MIXED : FG_FP64;
   const size_t smI = smem_for(B->maxnI, sizeof(T)), smR = smem_for(B->maxnr, sizeof(T));
-  FG_TRY(set_smem((const void*)k_bddc_dirichlet<T, 1>, smI));
-  FG_TRY(set_smem((const void*)k_bddc_dirichlet<T, 2>, smI));
-  FG_TRY(set_smem((const void*)k_bddc_neumann_fwd<T>, smR));
-  FG_TRY(set_smem((const void*)k_bddc_neumann_bwd<T>, smR));
+  FG_TRY(set_smem((const void*)k_bddc_dirichlet<T, 1, CTAS>, smI));
+  FG_TRY(set_smem((const void*)k_bddc_dirichlet<T, 2, CTAS>, smI));
+  FG_TRY(set_smem((const void*)k_bddc_neumann_fwd<T, CTAS>, smR));
+  FG_TRY(set_smem((const void*)k_bddc_neumann_bwd<T, CTAS>, smR));
   // 1. interior correction
-  k_bddc_dirichlet<T, 1><<<ns, 256, smI, st>>>(B->d_subs, B->dA, B->dF, B->dLoc, r, (const T*)nullptr, u0, z);
+  k_bddc_dirichlet<T, 1, CTAS><<<ns, 256, smI, st>>>(B->d_subs, B->dA, B->dF, B->dLoc, r, (const T*)nullptr, u0, z);
   // 2-3. (A u0) on the interface
   FG_TRY(system_spmv_layout_noalloc(sys, prec, u0, q, st));
   // 4. constrained Neumann (forward), coarse residual, coarse solve, Neumann (backward)
-  k_bddc_neumann_fwd<T><<<ns, 256, smR, st>>>(B->d_subs, B->dA, B->dF, R, G, B->dLoc, B->dW, r, q, zE, fP);
+  k_bddc_neumann_fwd<T, CTAS><<<ns, 256, smR, st>>>(B->d_subs, B->dA, B->dF, R, G, B->dLoc, B->dW, r, q, zE, fP);
   if (B->nC > 0) {
     k_coarse_gather<T><<<nblk(B->nC, 256), 256, 0, st>>>(B->nC, B->dCptr, B->dCsrc, fP, fc);
     k_coarse_gemv<T><<<nblk(B->nC * 32, 256), 256, 0, st>>>(B->nC, Kinv, fc, uc);
     ctx->launches += 2;
   }
   const T* Cv = f32 ? (const T*)B->dCv32 : (const T*)B->dCv;
-  k_bddc_neumann_bwd<T><<<ns, 256, smR, st>>>(B->d_subs, B->dA, B->dF, R, G, Cv, B->dPc, uc, zE, B->dW, B->dRho,
+  k_bddc_neumann_bwd<T, CTAS><<<ns, 256, smR, st>>>(B->d_subs, B->dA, B->dF, R, G, Cv, B->dPc, uc, zE, B->dW, B->dRho,
                                               contrib);
   if (B->nIface > 0)
     k_iface_sum<T><<<nblk(B->nIface, 256), 256, 0, st>>>(B->nIface, B->dIptr, B->dIsrc, B->dIvec, contrib, v, z);
   // 5. harmonic extension
   FG_TRY(system_spmv_layout_noalloc(sys, prec, v, t, st));
-  k_bddc_dirichlet<T, 2><<<ns, 256, smI, st>>>(B->d_subs, B->dA, B->dF, B->dLoc, r, t, u0, z);
+  k_bddc_dirichlet<T, 2, CTAS><<<ns, 256, smI, st>>>(B->d_subs, B->dA, B->dF, B->dLoc, r, t, u0, z);
   ctx->launches += 7;
   FG_CUDA_TRY(cudaGetLastError());
   return FG_OK;
 }
 
 static fg_status bddc_apply(fg_bddc* B, int precision, const double* r, double* z) {
-  return precision == FG_MIXED ? bddc_apply_layout<float>(B, r, z) : bddc_apply_layout<double>(B, r, z);
+  if (precision != FG_MIXED) return bddc_apply_layout<double, 2>(B, r, z);
+  return many_small(B) ? bddc_apply_layout<float, 4>(B, r, z) : bddc_apply_layout<float, 2>(B, r, z);
 }
 
 static fg_status ensure_pcg(fg_bddc* B) {
