@@ -592,58 +592,78 @@ __device__ __forceinline__ void warp_sums(Sum3 (&s)[NV], int) {
     for (int off = 16; off > 0; off >>= 1) sum_in(s[k], shfl_xor(s[k], off));
 }
 
-template <int NV, typename T, typename V, typename F>
-__device__ __forceinline__ bool grid_reduce(RedShared<T>& sh, const V (&v)[NV], const GridSync& g, int buf,
-                                            unsigned& target, int* s_ok, F&& f) {
+// barrier of the first nt threads
+__device__ __forceinline__ void adders_meet(int nt) {
+  if (nt > 32) asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory");
+  else __syncwarp();
+}
+
+// the block's sums as place blk of nblk in part (or, alone, the totals); the values wait in sh.v until the
+// first four warps have added them
+template <int NV, typename T, typename V>
+__device__ __forceinline__ void block_part(RedShared<T>& sh, const V (&v)[NV], double* part, int blk, int nblk) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
 #pragma unroll
   for (int k = 0; k < NV; ++k) sh.v[k][t] = v[k];
   __syncthreads();
-  target += gridDim.x;
   const int nt = blockDim.x < 128 ? blockDim.x : 128;  // the adding threads
+  if (t >= nt) return;
+  using A = typename SumOf<V>::type;
+  A s[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    s[k] = A{};
+    for (int i = t; i < (int)blockDim.x; i += nt) sum_in(s[k], sh.v[k][i]);
+  }
+  warp_sums(s, lane);
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) sh.w[warp][k] = s[k];
+  adders_meet(nt);
+  if (warp == 0) {
+    // lane 4 k + w: value k of warp w
+    A y = lane < 4 * NV && (lane & 3) < (nt >> 5) ? sh.w[lane & 3][lane >> 2] : A{};
+    sum_in(y, shfl_xor(y, 1));
+    sum_in(y, shfl_xor(y, 2));
+    if (lane < 4 * NV && (lane & 3) == 0) {
+      const double d = to_f64(y);
+      if (nblk > 1) part[(lane >> 2) * nblk + blk] = d;
+      else sh.tot[lane >> 2] = d;
+    }
+    __syncwarp();
+  }
+}
+
+// body(b, values): the values of block b of the solve's gridDim.x x vb blocks, which a block of the
+// launch does one after another (PcgShape)
+template <int NV, typename V, typename T, typename B, typename F>
+__device__ __forceinline__ bool grid_reduce(RedShared<T>& sh, const GridSync& g, int buf, unsigned& target, int* s_ok,
+                                            int vb, B&& body, F&& f) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int nblk = (int)gridDim.x * vb;
+  double* part = g.part + (size_t)buf * 3 * nblk;
+  for (int v = 0; v < vb; ++v) {
+    V val[NV];
+    const int blk = blockIdx.x + v * gridDim.x;
+    body(blk, val);
+    if (v > 0) __syncthreads();  // the last one's values have been added
+    block_part<NV>(sh, val, part, blk, nblk);
+  }
+  target += gridDim.x;
+  const int nt = blockDim.x < 128 ? blockDim.x : 128;
   if (t < nt) {
-    auto meet = [&] {
-      if (nt > 32) asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory");
-      else __syncwarp();
-    };
-    using A = typename SumOf<V>::type;
-    A s[NV];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      s[k] = A{};
-      for (int i = t; i < (int)blockDim.x; i += nt) sum_in(s[k], sh.v[k][i]);
-    }
-    warp_sums(s, lane);
-    if (lane == 0)
-#pragma unroll
-      for (int k = 0; k < NV; ++k) sh.w[warp][k] = s[k];
-    meet();
-    const bool grid = gridDim.x > 1;
-    double* part = g.part + (size_t)buf * 3 * gridDim.x;
-    if (warp == 0) {
-      // lane 4 k + w: value k of warp w
-      A y = lane < 4 * NV && (lane & 3) < (nt >> 5) ? sh.w[lane & 3][lane >> 2] : A{};
-      sum_in(y, shfl_xor(y, 1));
-      sum_in(y, shfl_xor(y, 2));
-      if (lane < 4 * NV && (lane & 3) == 0) {
-        const double d = to_f64(y);
-        if (grid) part[(lane >> 2) * gridDim.x + blockIdx.x] = d;
-        else sh.tot[lane >> 2] = d;
-      }
-      __syncwarp();
-      if (lane == 0) *s_ok = !grid || grid_wait(g, target) ? 1 : 0;
-      __syncwarp();
-    }
-    if (grid) {
-      meet();
+    if (t == 0) *s_ok = nblk == 1 || grid_wait(g, target) ? 1 : 0;
+    __syncwarp();
+    if (nblk > 1) {
+      adders_meet(nt);
       for (int k = warp; k < NV; k += nt >> 5) {
         double z[1] = {0.0};
 #pragma unroll 4
-        for (int i = lane; i < (int)gridDim.x; i += 32) z[0] += __ldcg(part + (size_t)k * gridDim.x + i);
+        for (int i = lane; i < nblk; i += 32) z[0] += __ldcg(part + (size_t)k * nblk + i);
         warp_sums(z, lane);
         if (lane == 0) sh.tot[k] = z[0];
       }
-      meet();
+      adders_meet(nt);
     }
     if (t == 0 && *s_ok) {
       double tot[NV];
@@ -905,7 +925,7 @@ template <int ML, int R>
 __global__ void __launch_bounds__(pcg_threads(R, ML, false), pcg_blocks(R))
     k_pcg64(MatArgs<double> m, int64_t nvec, double* x, double* r, double* p, double* Ap,
             const double* __restrict__ idiag, int criterion, double rtol, double atol, int max_launch, int chunk,
-            int keep, GridSync g, double* S, int* I) {
+            int keep, int vblocks, GridSync g, double* S, int* I) {
   extern __shared__ __align__(16) int32_t s_off_buf[];
   __shared__ RedShared<double> sh;
   __shared__ double sc[9];  // alpha, beta, rz, err, tol, rnrmm, <r,r>, its bound, 1/rz
@@ -913,8 +933,9 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, false), pcg_blocks(R))
   if (I[I_DONE]) return;
   constexpr int RR = R > 0 ? R : 1;
   const int lane = threadIdx.x & 31;
-  const int64_t warp = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-  const int64_t nwarps = (int64_t)(blockDim.x >> 5) * gridDim.x;
+  const int vb = R > 0 ? 1 : vblocks, nblk = (int)gridDim.x * vb;
+  const int64_t nwarps = (int64_t)(blockDim.x >> 5) * nblk;
+  auto warp_of = [&](int blk) { return (int64_t)(threadIdx.x >> 5) * nblk + blk; };
   const bool need_pp = criterion == FG_DELTA_RHS || criterion == FG_DELTA_DELTA;
   const bool res = criterion == FG_RES_RES || criterion == FG_RES_RHS;
   const int32_t* s_off = stage_offsets<double, ML>(m, s_off_buf);
@@ -934,7 +955,7 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, false), pcg_blocks(R))
   if (R > 0) {
 #pragma unroll
     for (int k = 0; k < RR; ++k) {
-      const int64_t s = warp + k * nwarps;
+      const int64_t s = warp_of(blockIdx.x) + k * nwarps;
       rx[k] = rr_[k] = rp[k] = rd[k] = 0.0;
       if (s >= m.nslices) {
         ref[k].none(m, s_off);
@@ -954,7 +975,8 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, false), pcg_blocks(R))
     __shared__ int s_cnt[32 * RR];
     keep_slices(ref, reinterpret_cast<float4*>(s_off_buf + ((m.noff + 3) & ~3)), keep, s_cnt);
   }
-  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t stride = (int64_t)nblk * blockDim.x;
+  auto thread_of = [&](int blk) { return (int64_t)blk * blockDim.x + threadIdx.x; };
   unsigned target = 0;
   __syncthreads();  // the scalars
   int it = it0;
@@ -962,50 +984,54 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, false), pcg_blocks(R))
     // beside the product: 1/rz for beta (a division on thread 0 between two barriers is 0.4 us)
     if (threadIdx.x == blockDim.x - 32) sc[8] = 1.0 / sc[2];
     // Ap = A p, <Ap,p>
-    Acc<double> dot;
-    if (R > 0) {
+    auto product = [&](int blk, double (&v)[1]) {
+      Acc<double> dot;
+      if (R > 0) {
 #pragma unroll
-      for (int k = 0; k < RR; ++k) {
-        ra[k] = ref[k].sv ? ref[k].dot_kept(p) : ref[k].template dot<true, 2>(p);
-        if (ref[k].vec >= 0) dot.add(ra[k], rp[k]);
-      }
-    } else {
-      for (int64_t s = warp; s < m.nslices; s += nwarps) {
-        SliceRef<double, ML> q;
-        q.load(m, s, lane, s_off);
-        const double a = q.template dot<false, ML == ML_SELL && R == 0 ? 4 : kUnroll>(p);
-        if (q.vec >= 0) {
-          Ap[q.vec] = a;
-          dot.add(a, p[q.vec]);
+        for (int k = 0; k < RR; ++k) {
+          ra[k] = ref[k].sv ? ref[k].dot_kept(p) : ref[k].template dot<true, 2>(p);
+          if (ref[k].vec >= 0) dot.add(ra[k], rp[k]);
+        }
+      } else {
+        for (int64_t s = warp_of(blk); s < m.nslices; s += nwarps) {
+          SliceRef<double, ML> q;
+          q.load(m, s, lane, s_off);
+          const double a = q.template dot<false, ML == ML_SELL && R == 0 ? 4 : kUnroll>(p);
+          if (q.vec >= 0) {
+            Ap[q.vec] = a;
+            dot.add(a, p[q.vec]);
+          }
         }
       }
-    }
-    double v1[1] = {dot.value()};
-    if (!grid_reduce<1>(sh, v1, g, 0, target, &si[2], [&](double (&t)[1]) { sc[0] = t[0] != 0.0 ? sc[2] / t[0] : 0.0; }))
+      v[0] = dot.value();
+    };
+    if (!grid_reduce<1, double>(sh, g, 0, target, &si[2], vb, product,
+                                [&](double (&t)[1]) { sc[0] = t[0] != 0.0 ? sc[2] / t[0] : 0.0; }))
       return;
     // x += alpha p; r -= alpha Ap; the convergence test; beta
     const double a = sc[0];
-    Acc<double> rr, rz, pp;
-    if (R > 0) {
+    auto update = [&](int blk, Acc<double>& rr, Acc<double>& rz, Acc<double>& pp) {
+      if (R > 0) {
 #pragma unroll
-      for (int k = 0; k < RR; ++k) {
-        rx[k] = fma(a, rp[k], rx[k]);
-        if (ref[k].vec >= 0) rr_[k] = fma(-a, ra[k], rr_[k]);
-        rr.add(rr_[k], rr_[k]);
-        if (idiag) rz.add(rr_[k], rd[k] * rr_[k]);
-        if (need_pp) pp.add(rp[k], rp[k]);
+        for (int k = 0; k < RR; ++k) {
+          rx[k] = fma(a, rp[k], rx[k]);
+          if (ref[k].vec >= 0) rr_[k] = fma(-a, ra[k], rr_[k]);
+          rr.add(rr_[k], rr_[k]);
+          if (idiag) rz.add(rr_[k], rd[k] * rr_[k]);
+          if (need_pp) pp.add(rp[k], rp[k]);
+        }
+      } else {
+        for (int64_t i = thread_of(blk); i < nvec; i += stride) {
+          const double pi = p[i];
+          x[i] = fma(a, pi, x[i]);
+          const double ri = fma(-a, Ap[i], r[i]);
+          r[i] = ri;
+          rr.add(ri, ri);
+          if (idiag) rz.add(ri, idiag[i] * ri);
+          if (need_pp) pp.add(pi, pi);
+        }
       }
-    } else {
-      for (int64_t i = t0; i < nvec; i += stride) {
-        const double pi = p[i];
-        x[i] = fma(a, pi, x[i]);
-        const double ri = fma(-a, Ap[i], r[i]);
-        r[i] = ri;
-        rr.add(ri, ri);
-        if (idiag) rz.add(ri, idiag[i] * ri);
-        if (need_pp) pp.add(pi, pi);
-      }
-    }
+    };
     ++it;
     auto test = [&](double trr, double trz, double tpp) {
       bool conv = false;
@@ -1033,14 +1059,35 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, false), pcg_blocks(R))
     };
     bool ok;
     if (need_pp) {
-      double v3[3] = {rr.value(), idiag ? rz.value() : rr.value(), pp.value()};
-      ok = grid_reduce<3>(sh, v3, g, 1, target, &si[2], [&](double (&t)[3]) { test(t[0], t[1], t[2]); });
+      ok = grid_reduce<3, double>(
+          sh, g, 1, target, &si[2], vb,
+          [&](int blk, double (&v)[3]) {
+            Acc<double> rr, rz, pp;
+            update(blk, rr, rz, pp);
+            v[0] = rr.value();
+            v[1] = idiag ? rz.value() : rr.value();
+            v[2] = pp.value();
+          },
+          [&](double (&t)[3]) { test(t[0], t[1], t[2]); });
     } else if (idiag) {
-      double v2[2] = {rr.value(), rz.value()};
-      ok = grid_reduce<2>(sh, v2, g, 1, target, &si[2], [&](double (&t)[2]) { test(t[0], t[1], 0.0); });
+      ok = grid_reduce<2, double>(
+          sh, g, 1, target, &si[2], vb,
+          [&](int blk, double (&v)[2]) {
+            Acc<double> rr, rz, pp;
+            update(blk, rr, rz, pp);
+            v[0] = rr.value();
+            v[1] = rz.value();
+          },
+          [&](double (&t)[2]) { test(t[0], t[1], 0.0); });
     } else {
-      double v2[1] = {rr.value()};
-      ok = grid_reduce<1>(sh, v2, g, 1, target, &si[2], [&](double (&t)[1]) { test(t[0], t[0], 0.0); });
+      ok = grid_reduce<1, double>(
+          sh, g, 1, target, &si[2], vb,
+          [&](int blk, double (&v)[1]) {
+            Acc<double> rr, rz, pp;
+            update(blk, rr, rz, pp);
+            v[0] = rr.value();
+          },
+          [&](double (&t)[1]) { test(t[0], t[0], 0.0); });
     }
     if (!ok) return;
     if (si[0]) break;
@@ -1053,10 +1100,11 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, false), pcg_blocks(R))
         if (ref[k].vec >= 0) p[ref[k].vec] = rp[k];
       }
     } else {
-      for (int64_t i = t0; i < nvec; i += stride) {
-        const double ri = r[i];
-        p[i] = fma(beta, p[i], idiag ? idiag[i] * ri : ri);
-      }
+      for (int v = 0; v < vb; ++v)
+        for (int64_t i = thread_of(blockIdx.x + v * gridDim.x); i < nvec; i += stride) {
+          const double ri = r[i];
+          p[i] = fma(beta, p[i], idiag ? idiag[i] * ri : ri);
+        }
     }
     if (n + 1 < max_launch && !grid_barrier(g, target, &si[2])) return;
   }
@@ -1093,7 +1141,7 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, false), pcg_blocks(R))
 template <int ML, int R>
 __global__ void __launch_bounds__(pcg_threads(R, ML, true), pcg_blocks(R))
     k_pcg32(MatArgs<float> m, int64_t nvec, float* x, float* r, float* p, float* q, const float* __restrict__ idiag,
-            int max_launch, int keep, GridSync g, double* S, int* I) {
+            int max_launch, int keep, int vblocks, GridSync g, double* S, int* I) {
   extern __shared__ __align__(16) int32_t s_off_buf[];
   __shared__ RedShared<float> sh;
   __shared__ double sd[9];  // rr, rmax^2, delta^2, (tol/sigma)^2, -, app, alpha, beta, 1/rr
@@ -1102,8 +1150,9 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, true), pcg_blocks(R))
   if (I[I_DONE]) return;
   constexpr int RR = R > 0 ? R : 1;
   const int lane = threadIdx.x & 31;
-  const int64_t warp = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-  const int64_t nwarps = (int64_t)(blockDim.x >> 5) * gridDim.x;
+  const int vb = R > 0 ? 1 : vblocks, nblk = (int)gridDim.x * vb;
+  const int64_t nwarps = (int64_t)(blockDim.x >> 5) * nblk;
+  auto warp_of = [&](int blk) { return (int64_t)(threadIdx.x >> 5) * nblk + blk; };
   const int32_t* s_off = stage_offsets<float, ML>(m, s_off_buf);
   const int maxit = I[I_MAXIT];
   int it = I[I_ITER];
@@ -1123,7 +1172,7 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, true), pcg_blocks(R))
   if (R > 0) {
 #pragma unroll
     for (int k = 0; k < RR; ++k) {
-      const int64_t s = warp + k * nwarps;
+      const int64_t s = warp_of(blockIdx.x) + k * nwarps;
       rx[k] = rr_[k] = rp[k] = 0.f;
       if (s >= m.nslices) {
         ref[k].none(m, s_off);
@@ -1142,41 +1191,45 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, true), pcg_blocks(R))
     __shared__ int s_cnt[32 * RR];
     keep_slices(ref, reinterpret_cast<float4*>(s_off_buf + ((m.noff + 3) & ~3)), keep, s_cnt);
   }
-  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t stride = (int64_t)nblk * blockDim.x;
+  auto thread_of = [&](int blk) { return (int64_t)blk * blockDim.x + threadIdx.x; };
   unsigned target = 0;
   __syncthreads();  // the scalars
   for (int n = 0; n < max_launch; ++n) {
     // beside the product: 1/rr for beta (see k_pcg64)
     if (threadIdx.x == blockDim.x - 32) sd[8] = 1.0 / sd[0];
-    Acc<float> pq;
-    AccPlain qq, qq1;  // <q,q>: the slices' rows alternate between two sums
-    if (R > 0) {
+    auto product = [&](int blk, float2 (&v)[2]) {
+      Acc<float> pq;
+      AccPlain qq, qq1;  // <q,q>: the slices' rows alternate between two sums
+      if (R > 0) {
 #pragma unroll
-      for (int k = 0; k < RR; ++k) {
-        rq[k] = ref[k].sv ? ref[k].dot_kept(p) : ref[k].template dot<true, R == 1 ? 4 : 2>(p);
-        if (ref[k].vec >= 0) {
-          pq.add(rq[k], rp[k]);
-          qq.add(rq[k], rq[k]);
+        for (int k = 0; k < RR; ++k) {
+          rq[k] = ref[k].sv ? ref[k].dot_kept(p) : ref[k].template dot<true, R == 1 ? 4 : 2>(p);
+          if (ref[k].vec >= 0) {
+            pq.add(rq[k], rp[k]);
+            qq.add(rq[k], rq[k]);
+          }
+        }
+      } else {
+        for (int64_t s = warp_of(blk); s < m.nslices; s += nwarps) {
+          SliceRef<float, ML> w;
+          w.load(m, s, lane, s_off);
+          const float a = w.template dot<false, ML == ML_SELL ? 4 : kUnroll>(p);
+          if (w.vec >= 0) {
+            q[w.vec] = a;
+            pq.add(a, p[w.vec]);
+            qq.add(a, a);
+          }
+          const float t = qq.s;
+          qq.s = qq1.s;
+          qq1.s = t;
         }
       }
-    } else {
-      for (int64_t s = warp; s < m.nslices; s += nwarps) {
-        SliceRef<float, ML> w;
-        w.load(m, s, lane, s_off);
-        const float a = w.template dot<false, ML == ML_SELL ? 4 : kUnroll>(p);
-        if (w.vec >= 0) {
-          q[w.vec] = a;
-          pq.add(a, p[w.vec]);
-          qq.add(a, a);
-        }
-        const float t = qq.s;
-        qq.s = qq1.s;
-        qq1.s = t;
-      }
-    }
-    float2 v2[2] = {make_float2(pq.hi, pq.lo), make_float2(qq.s, 0.f)};
-    if (R == 0) two_sum(qq.s, qq1.s, v2[1].x, v2[1].y);
-    if (!grid_reduce<2>(sh, v2, g, 0, target, &si[3], [&](double (&t)[2]) {
+      v[0] = make_float2(pq.hi, pq.lo);
+      v[1] = make_float2(qq.s, 0.f);
+      if (R <= 0) two_sum(qq.s, qq1.s, v[1].x, v[1].y);
+    };
+    if (!grid_reduce<2, float2>(sh, g, 0, target, &si[3], vb, product, [&](double (&t)[2]) {
           const double pap = t[0], nq = t[1], rr = sd[0];
           int skip = si[0] != FLAG_NONE;
           double a = 0.0, b = 0.0;
@@ -1202,71 +1255,72 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, true), pcg_blocks(R))
     const float a = sf[0], b = sf[1];
     const bool keep_p = si[1] != 0;
     const bool exact = n % FG_MIXED_EXACT_EVERY == FG_MIXED_EXACT_EVERY - 1 || n == max_launch - 1;
-    Acc<float> rr, rt;
     // unscaled residual entry r^ sqrt(d): r^2 d = r^2 / (1/d); slots that are not free dofs hold
     // r = 0 and 1/d = 0: skipped
-    auto unscaled = [&](float ri, float di) { rt.add(ri, di != 0.f ? ri / di : 0.f); };
-    if (R > 0) {
+    auto unscaled = [](Acc<float>& rt, float ri, float di) { rt.add(ri, di != 0.f ? ri / di : 0.f); };
+    auto update = [&](int blk, Acc<float>& rr, Acc<float>& rt) {
+      if (R > 0) {
 #pragma unroll
-      for (int k = 0; k < RR; ++k) {
-        if (ref[k].vec < 0) continue;
-        rx[k] = fmaf(a, rp[k], rx[k]);
-        rr_[k] = fmaf(-a, rq[k], rr_[k]);
-        if (!keep_p) {
-          rp[k] = fmaf(b, rp[k], rr_[k]);
-          p[ref[k].vec] = rp[k];
+        for (int k = 0; k < RR; ++k) {
+          if (ref[k].vec < 0) continue;
+          rx[k] = fmaf(a, rp[k], rx[k]);
+          rr_[k] = fmaf(-a, rq[k], rr_[k]);
+          if (!keep_p) {
+            rp[k] = fmaf(b, rp[k], rr_[k]);
+            p[ref[k].vec] = rp[k];
+          }
+          rr.add(rr_[k], rr_[k]);
+          if (exact) unscaled(rt, rr_[k], idiag ? idiag[ref[k].vec] : 1.f);
         }
-        rr.add(rr_[k], rr_[k]);
-        if (exact) unscaled(rr_[k], idiag ? idiag[ref[k].vec] : 1.f);
-      }
-    } else {
-      const int64_t n4 = nvec >> 2;
-      float4* x4 = reinterpret_cast<float4*>(x);
-      float4* r4 = reinterpret_cast<float4*>(r);
-      float4* p4 = reinterpret_cast<float4*>(p);
-      const float4* q4 = reinterpret_cast<const float4*>(q);
-      const float4* d4 = reinterpret_cast<const float4*>(idiag);
-      for (int64_t i = t0; i < n4; i += stride) {
-        float4 xi = x4[i], ri = r4[i], pi = p4[i];
-        const float4 qi = q4[i];
-        xi.x = fmaf(a, pi.x, xi.x);
-        xi.y = fmaf(a, pi.y, xi.y);
-        xi.z = fmaf(a, pi.z, xi.z);
-        xi.w = fmaf(a, pi.w, xi.w);
-        ri.x = fmaf(-a, qi.x, ri.x);
-        ri.y = fmaf(-a, qi.y, ri.y);
-        ri.z = fmaf(-a, qi.z, ri.z);
-        ri.w = fmaf(-a, qi.w, ri.w);
-        x4[i] = xi;
-        r4[i] = ri;
-        if (!keep_p) {
-          pi.x = fmaf(b, pi.x, ri.x);
-          pi.y = fmaf(b, pi.y, ri.y);
-          pi.z = fmaf(b, pi.z, ri.z);
-          pi.w = fmaf(b, pi.w, ri.w);
-          p4[i] = pi;
+      } else {
+        const int64_t n4 = nvec >> 2;
+        float4* x4 = reinterpret_cast<float4*>(x);
+        float4* r4 = reinterpret_cast<float4*>(r);
+        float4* p4 = reinterpret_cast<float4*>(p);
+        const float4* q4 = reinterpret_cast<const float4*>(q);
+        const float4* d4 = reinterpret_cast<const float4*>(idiag);
+        for (int64_t i = thread_of(blk); i < n4; i += stride) {
+          float4 xi = x4[i], ri = r4[i], pi = p4[i];
+          const float4 qi = q4[i];
+          xi.x = fmaf(a, pi.x, xi.x);
+          xi.y = fmaf(a, pi.y, xi.y);
+          xi.z = fmaf(a, pi.z, xi.z);
+          xi.w = fmaf(a, pi.w, xi.w);
+          ri.x = fmaf(-a, qi.x, ri.x);
+          ri.y = fmaf(-a, qi.y, ri.y);
+          ri.z = fmaf(-a, qi.z, ri.z);
+          ri.w = fmaf(-a, qi.w, ri.w);
+          x4[i] = xi;
+          r4[i] = ri;
+          if (!keep_p) {
+            pi.x = fmaf(b, pi.x, ri.x);
+            pi.y = fmaf(b, pi.y, ri.y);
+            pi.z = fmaf(b, pi.z, ri.z);
+            pi.w = fmaf(b, pi.w, ri.w);
+            p4[i] = pi;
+          }
+          rr.add(ri.x, ri.x);
+          rr.add(ri.y, ri.y);
+          rr.add(ri.z, ri.z);
+          rr.add(ri.w, ri.w);
+          if (exact) {
+            const float4 di = idiag ? d4[i] : make_float4(1.f, 1.f, 1.f, 1.f);
+            unscaled(rt, ri.x, di.x);
+            unscaled(rt, ri.y, di.y);
+            unscaled(rt, ri.z, di.z);
+            unscaled(rt, ri.w, di.w);
+          }
         }
-        rr.add(ri.x, ri.x);
-        rr.add(ri.y, ri.y);
-        rr.add(ri.z, ri.z);
-        rr.add(ri.w, ri.w);
-        if (exact) {
-          const float4 di = idiag ? d4[i] : make_float4(1.f, 1.f, 1.f, 1.f);
-          unscaled(ri.x, di.x);
-          unscaled(ri.y, di.y);
-          unscaled(ri.z, di.z);
-          unscaled(ri.w, di.w);
+        for (int64_t i = (n4 << 2) + thread_of(blk); i < nvec; i += stride) {
+          x[i] = fmaf(a, p[i], x[i]);
+          const float ri = fmaf(-a, q[i], r[i]);
+          r[i] = ri;
+          if (!keep_p) p[i] = fmaf(b, p[i], ri);
+          rr.add(ri, ri);
+          if (exact) unscaled(rt, ri, idiag ? idiag[i] : 1.f);
         }
       }
-      for (int64_t i = (n4 << 2) + t0; i < nvec; i += stride) {
-        x[i] = fmaf(a, p[i], x[i]);
-        const float ri = fmaf(-a, q[i], r[i]);
-        r[i] = ri;
-        if (!keep_p) p[i] = fmaf(b, p[i], ri);
-        rr.add(ri, ri);
-        if (exact) unscaled(ri, idiag ? idiag[i] : 1.f);
-      }
-    }
+    };
     ++it;
     auto decide = [&](double trr, double trt) {
       if (keep_p) {
@@ -1288,11 +1342,24 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, true), pcg_blocks(R))
     };
     bool ok;
     if (exact) {
-      const float2 v[2] = {make_float2(rr.hi, rr.lo), make_float2(rt.hi, rt.lo)};
-      ok = grid_reduce<2>(sh, v, g, 1, target, &si[3], [&](double (&t)[2]) { decide(t[0], t[1]); });
+      ok = grid_reduce<2, float2>(
+          sh, g, 1, target, &si[3], vb,
+          [&](int blk, float2 (&v)[2]) {
+            Acc<float> rr, rt;
+            update(blk, rr, rt);
+            v[0] = make_float2(rr.hi, rr.lo);
+            v[1] = make_float2(rt.hi, rt.lo);
+          },
+          [&](double (&t)[2]) { decide(t[0], t[1]); });
     } else {
-      const float2 v[1] = {make_float2(rr.hi, rr.lo)};
-      ok = grid_reduce<1>(sh, v, g, 1, target, &si[3], [&](double (&t)[1]) { decide(t[0], 0.0); });
+      ok = grid_reduce<1, float2>(
+          sh, g, 1, target, &si[3], vb,
+          [&](int blk, float2 (&v)[1]) {
+            Acc<float> rr, rt;
+            update(blk, rr, rt);
+            v[0] = make_float2(rr.hi, rr.lo);
+          },
+          [&](double (&t)[1]) { decide(t[0], 0.0); });
     }
     if (!ok) return;
     if (si[2] != FLAG_NONE) break;
@@ -1691,10 +1758,25 @@ static fg_status pcg_keep(void (*k)(KA...), const PcgShape& sh, int noff, int64_
 }
 
 template <typename... KA>
-static fg_status launch_pcg(void (*k)(KA...), const PcgShape& sh, const Work& w, size_t smem, cudaStream_t st, void** args) {
+static fg_status launch_pcg(void (*k)(KA...), const PcgShape& sh, int vblocks, const Work& w, size_t smem, cudaStream_t st,
+                            void** args) {
   FG_CUDA_TRY(cudaMemsetAsync(w.rb.ticket + 1, 0, sizeof(unsigned), st));
-  FG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k, dim3(sh.blocks), dim3(sh.threads), args, smem, st));
+  FG_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k, dim3(sh.blocks / vblocks), dim3(sh.threads), args, smem, st));
   return FG_OK;
+}
+
+// Blocks of a solve per block of the launch.  A streaming solve's 2 x SMs blocks fill the SMs, so those of
+// several contexts would take turns; while other requests of the same server solve, a launch is half as wide
+// and its blocks do two of the solve's each, so that two solves share the SMs and fill one another's waits.
+// The sums are the same blocks' in the same order: the same bits.  Alone, half the warps cost 15-25 %
+// (96^3 Q2 mixed 361 -> 480 us per iteration); two contexts at once solve 24^3 Q2 elasticity 11.9 times a
+// second against 10.0 in turn, 64^3 Q2 Poisson 18.1 against 17.5, 48^3 in FP64 22.5 against 21.5.
+// FG_PCG_TEST_SHARE=1: always (tests).
+static int pcg_vblocks(const fg_ctx* ctx, const PcgShape& sh) {
+  if (sh.R > 0) return 1;
+  const char* e = getenv("FG_PCG_TEST_SHARE");
+  if (e && e[0] == '1') return 2;
+  return ctx->solving && ctx->solving->load(std::memory_order_relaxed) > 1 ? 2 : 1;
 }
 
 // Iterations of one launch: about 5 ms (contexts on other threads get the GPU in between),
@@ -1755,13 +1837,15 @@ static fg_status run_pcg64(fg_system* sys, const Work& w, const fg_solver_params
   int* I = w.I;
   int keep = 0;
   size_t smem = 0;
-  void* args[] = {&m, &nvec, &x, &r, &p, &Ap, &idiag, &criterion, &rtol, &atol, &iters, &chunk, &keep, &g, &S, &I};
+  int vb = 1;
+  void* args[] = {&m, &nvec, &x, &r, &p, &Ap, &idiag, &criterion, &rtol, &atol, &iters, &chunk, &keep, &vb, &g, &S, &I};
 #define FG_PCG64(L) (sh.R == 1 ? k_pcg64<L, 1> : sh.R == 2 ? k_pcg64<L, 2> : k_pcg64<L, 0>)
   auto k = ml == ML_STENCIL ? FG_PCG64(ML_STENCIL) : ml == ML_DG ? FG_PCG64(ML_DG) : sh.R == PCG_WIDE ? k_pcg64<ML_SELL, PCG_WIDE> : FG_PCG64(ML_SELL);
 #undef FG_PCG64
   FG_TRY(pcg_keep(k, sh, m.noff, solver_entries(sp), 8, &keep, &smem));
   for (;;) {
-    FG_TRY(launch_pcg(k, sh, w, smem, st, args));
+    vb = pcg_vblocks(sp->mesh->ctx, sh);
+    FG_TRY(launch_pcg(k, sh, vb, w, smem, st, args));
     sp->mesh->ctx->launches += 1;
     FG_TRY(read_state(w, h, st));
     if (h.I[I_DONE]) return FG_OK;
@@ -1789,13 +1873,15 @@ static fg_status run_pcg32(fg_system* sys, const Work& w, const fg_solver_params
   int* I = w.I;
   int keep = 0;
   size_t smem = 0;
-  void* args[] = {&m, &nvec, &x, &r, &p, &q, &idiag, &iters, &keep, &g, &S, &I};
+  int vb = 1;
+  void* args[] = {&m, &nvec, &x, &r, &p, &q, &idiag, &iters, &keep, &vb, &g, &S, &I};
 #define FG_PCG32(L) (sh.R == 1 ? k_pcg32<L, 1> : sh.R == 2 ? k_pcg32<L, 2> : k_pcg32<L, 0>)
   auto k = ml == ML_STENCIL ? FG_PCG32(ML_STENCIL) : ml == ML_DG ? FG_PCG32(ML_DG) : FG_PCG32(ML_SELL);
 #undef FG_PCG32
   FG_TRY(pcg_keep(k, sh, m.noff, solver_entries(sp), 4, &keep, &smem));
   do {
-    FG_TRY(launch_pcg(k, sh, w, smem, st, args));
+    vb = pcg_vblocks(sp->mesh->ctx, sh);
+    FG_TRY(launch_pcg(k, sh, vb, w, smem, st, args));
     sp->mesh->ctx->launches += 1;
     FG_TRY(read_state(w, h, st));
   } while (!h.I[I_DONE]);
