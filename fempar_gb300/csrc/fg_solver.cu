@@ -41,8 +41,7 @@ namespace fg {
 
 static constexpr int RB = 256;  // threads per block of the vector / SpMV kernels
 
-enum { S_RZ = 0, S_ALPHA, S_BETA, S_ERR, S_TOL, S_APP, S_RNRMM, S_BNRM, S_R0NRM, S_SIGMA, S_RMAX, S_DELTA, S_RNSCALED,
-       S_RRH, S_COUNT = 16 };
+enum { S_RZ = 0, S_ALPHA, S_BETA, S_ERR, S_TOL, S_APP, S_RNRMM, S_BNRM, S_SIGMA, S_RMAX, S_DELTA, S_RRH, S_COUNT = 16 };
 // I_PEND: a segment end decided by the last x/r/p update, taken at the next iteration;
 // I_SKIPP: this iteration's update keeps p (the segment ends after it)
 // I_ABORT: a grid barrier of the CG kernels ran out of time
@@ -273,7 +272,7 @@ template <typename T, int MODE>
 __global__ void __launch_bounds__(RB)
     k_sell_spmv(int64_t nslices, int64_t n, const int64_t* __restrict__ sptr, const int32_t* __restrict__ scol,
                 const T* __restrict__ sval, const T* __restrict__ x, T* __restrict__ y, const double* __restrict__ b,
-                RedBuf rb, double* S, const int* I) {
+                RedBuf rb, double* S) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * RB + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * RB) >> 5;
@@ -335,7 +334,6 @@ __global__ void __launch_bounds__(RB)
     S[S_RZ] = tot[1];
     S[S_RNRMM] = sqrt(tot[1]);
     const double rn = sqrt(tot[0]), bn = sqrt(tot[2]), bnm = sqrt(tot[3]);
-    S[S_R0NRM] = rn;
     S[S_BNRM] = bn;
     double tol = 0.0;
     switch (criterion) {
@@ -395,7 +393,7 @@ __global__ void __launch_bounds__(RB)
                    const StencilClass* __restrict__ cls, const int32_t* __restrict__ soff,
                    const int32_t* __restrict__ st_row, const T* __restrict__ tval,
                    int ncomp, const T* __restrict__ x, T* __restrict__ y, const double* __restrict__ b, RedBuf rb,
-                   double* S, const int* I) {
+                   double* S) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * RB + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * RB) >> 5;
@@ -1144,7 +1142,7 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, true), pcg_blocks(R))
             int max_launch, int keep, int vblocks, GridSync g, double* S, int* I) {
   extern __shared__ __align__(16) int32_t s_off_buf[];
   __shared__ RedShared<float> sh;
-  __shared__ double sd[9];  // rr, rmax^2, delta^2, (tol/sigma)^2, -, app, alpha, beta, 1/rr
+  __shared__ double sd[8];  // rr, rmax^2, delta^2, (tol/sigma)^2, 1/rr, app, alpha, beta
   __shared__ float sf[2];   // alpha, beta
   __shared__ int si[8];     // pend, skip, done flag, ok
   if (I[I_DONE]) return;
@@ -1197,7 +1195,7 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, true), pcg_blocks(R))
   __syncthreads();  // the scalars
   for (int n = 0; n < max_launch; ++n) {
     // beside the product: 1/rr for beta (see k_pcg64)
-    if (threadIdx.x == blockDim.x - 32) sd[8] = 1.0 / sd[0];
+    if (threadIdx.x == blockDim.x - 32) sd[4] = 1.0 / sd[0];
     auto product = [&](int blk, float2 (&v)[2]) {
       Acc<float> pq;
       AccPlain qq, qq1;  // <q,q>: the slices' rows alternate between two sums
@@ -1239,7 +1237,7 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, true), pcg_blocks(R))
           } else {
             a = rr / pap;
             const double rrn = a * a * nq - rr;
-            b = rrn * sd[8];
+            b = rrn * sd[4];
             if (!(rrn > 0.0)) {  // the recurrence lost its digits: end the segment here
               skip = 1;
               if (si[0] == FLAG_NONE) si[0] = FLAG_UPDATE;
@@ -1484,7 +1482,6 @@ static inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / 
 struct Work {
   double *x, *r, *p, *Ap, *b, *t;  // FP64, solver layout
   float *x32, *r32, *p32, *Ap32;
-  double *io;                       // FP64 row-order staging (x0 of spmv)
   double* S;
   int* I;
   RedBuf rb;
@@ -1541,7 +1538,6 @@ static fg_status ensure_work(fg_system* sys, Work& w) {
   }
   w.x = sys->d_work; w.r = w.x + n; w.p = w.r + n; w.Ap = w.p + n; w.b = w.Ap + n; w.t = w.b + n;
   w.x32 = sys->d_work32; w.r32 = w.x32 + n; w.p32 = w.r32 + n; w.Ap32 = w.p32 + n;
-  w.io = nullptr;
   w.S = sys->d_red + 4 * sys->red_blocks;
   w.I = (int*)(w.S + S_COUNT);
   w.rb.part = sys->d_red;
@@ -1610,12 +1606,12 @@ static void spmv_k(fg_system* sys, const Work& w, const T* x, T* y, const double
     if (sp->layout == FG_LAYOUT_STENCIL)                                                                            \
       launch_kn(k_stencil_spmv<T, MODE>, w, st, sp->st_nslices * 32, sp->st_nslices, (const uint8_t*)sp->d_st_scls,                       \
                (const int64_t*)sp->d_st_voff, (const StencilClass*)sp->d_st_cls, (const int32_t*)sp->d_st_off, (const int32_t*)sp->d_st_row,       \
-               (const T*)sys->TVALS, sp->ncomp, x, y, b, w.rb, w.S, (const int*)w.I);                               \
+               (const T*)sys->TVALS, sp->ncomp, x, y, b, w.rb, w.S);                                                \
     else if (sp->d_dgblk)                                                                                           \
       launch_kn(k_dg_spmv<T, MODE>, w, st, sp->nslices * 32, mat_args<T>(sp, sys->VALS), x, y, b, w.rb, w.S);       \
     else                                                                                                            \
       launch_kn(k_sell_spmv<T, MODE>, w, st, sp->nslices * 32, sp->nslices, sp->nfree, (const int64_t*)sp->d_sptr,                     \
-               (const int32_t*)sp->d_scol, (const T*)sys->VALS, x, y, b, w.rb, w.S, (const int*)w.I);              \
+               (const int32_t*)sp->d_scol, (const T*)sys->VALS, x, y, b, w.rb, w.S);                               \
     sp->mesh->ctx->launches += 1;                                                                                   \
   }
 FG_SPMV_IMPL(double, 0, d_sval, d_tval)
