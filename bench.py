@@ -10,7 +10,7 @@ x0 = 0 to ||r|| <= 1e-8 ||r0||.  16,581,375 free dofs.
 A step = numeric assembly (integration + CSR + FP32 copy + Jacobi diagonal) + PCG solve;
 the symbolic phase (dof numbering, sparsity) is built once before timing ("warm" DOF/s).
 value = free dofs / device time of a step (inputs resident in HBM), mixed precision
-(FP32 matrix/SpMV/Jacobi inner PCG, FP64 residual, dots and refinement).  The plain FP64
+(FP32 matrix/SpMV/Jacobi inner PCG, dots in compensated FP32 and FP64, FP64 residual and refinement).  The plain FP64
 drop-in is timed beside it.  e2e = the same through the public API with host buffers:
 per-cell coefficients copied in from pinned host memory and the solution copied out.
 
@@ -247,10 +247,10 @@ def run_reference(args):
     print(json.dumps(line), flush=True)
 
 
-# DRAM bytes per stored byte of the FP32 SpMV launch at 128^3 Q2, one ncu capture of the
-# full-size launch (dram__bytes_read.sum + dram__bytes_write.sum = 4990 MB + 65 MB for 4508.9 MB
-# stored): the values once, the x vector about 7 times (once per node class)
-DRAM_PER_STORED_BYTE_FP32 = 5055.0 / 4508.9
+# DRAM bytes of one iteration of the FP32 CG kernel per byte it stores or updates (k_pcg32 at 64^3 Q2, one
+# ncu capture of a 16-iteration launch: 9138 MB read + 444 MB written, against 16 x 635 MB of values and
+# vectors): the vectors stay in L2 at that size
+DRAM_PER_FORMAT_BYTE_PCG32 = 599.0 / 635.3
 
 
 def replica_aggregate(dist, times_ms, units, device="cpu"):
@@ -473,6 +473,9 @@ def main():
     layout = "lattice-implicit SELL-32x4 (no column indices)" if space.info.solver_layout == 0 else "SELL-32x4-256"
     kname = "k_stencil_spmv" if space.info.solver_layout == 0 else "k_sell_spmv"
     fmt32 = 4 * nent + 8 * nvec + (0 if space.info.solver_layout == 0 else 4 * nent)
+    ms_it = imx[-1]["solve_ms"] / max(1, imx[-1]["iterations"])
+    bit = 4 * nnz + 36 * nfree
+    fmt_it = 4 * nent + 36 * nvec + (0 if space.info.solver_layout == 0 else 4 * nent)
     fmt64 = 8 * nent + 16 * nvec + (0 if space.info.solver_layout == 0 else 4 * nent)
 
     # ---- replicas: slowest rank's time, every rank's dofs ----
@@ -518,7 +521,7 @@ def main():
     line = {
         "metric": METRIC, "value": value, "unit": "DOF/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_mx, "higher_is_better": True, "scaling": "weak",
-        "vs_baseline": None, "dtype": "fp32 matrix/SpMV/Jacobi + fp64 residual/dots/refinement",
+        "vs_baseline": None, "dtype": "fp32 matrix/SpMV/Jacobi, dots in compensated fp32 and fp64, fp64 residual/refinement",
         "data": f"synthetic (PCG64 seed {SEED}): perturbed vertices U(+-0.15h), k=exp(N(0,1)) per cell, f=1",
         "config": workload_config(n, nfree, nnz, space.info.nnz_upper),
         "parallelism": "replicas" if world > 1 else "single", "symbolic_s": t_symbolic,
@@ -534,18 +537,22 @@ def main():
         "mixed_vs_fp64": value / v64,
         "e2e": {"value": ve2e, "unit": "DOF/s", "h2d_bytes_per_step": int(coef.nbytes),
                 "d2h_bytes_per_step": int(nfree * 8), "ms_per_step": ms_e2e},
-        "roofline": {"bound": "hbm", "kernel": f"{kname}<float,0> (FP32 SpMV, {layout}; the CG launch runs the same product, the same "
-                               "bytes plus two dot products)",
-                     "achieved": ach32, "peak": hbm, "unit": "GB/s", "frac": ach32 / hbm,
-                     "peak_source": "of measured" if pk else "of fallback",
-                     "traffic": DRAM_PER_STORED_BYTE_FP32 * fmt32,
-                     "traffic_source": "ncu dram__bytes_read+write of this kernel at 128^3 Q2 (5055 MB = 1.121 x its "
-                                       "stored bytes: values once, x re-read per node class), scaled by the stored bytes",
-                     "bytes_per_launch": b32, "ms_per_launch": ms32,
-                     "bytes_def": "4*nnz + 8*n (values once, x once, y once)",
-                     "format_bytes_per_launch": fmt32, "format_frac": fmt32 / (ms32 * 1e-3) / 1e9 / hbm,
-                     "csr_bytes_per_launch": csr_bytes(nfree, nnz, True),
-                     "csr_equivalent_gbs": csr_bytes(nfree, nnz, True) / (ms32 * 1e-3) / 1e9},
+        "roofline": {"bound": "hbm", "kernel": f"k_pcg32 (the solve's FP32 CG iterations: product, two dots and the three "
+                               f"updates; {layout}), per iteration of the timed steps, FP64 residuals included",
+                     "achieved": bit / (ms_it * 1e-3) / 1e9, "peak": hbm, "unit": "GB/s",
+                     "frac": bit / (ms_it * 1e-3) / 1e9 / hbm, "peak_source": "of measured" if pk else "of fallback",
+                     "traffic": DRAM_PER_FORMAT_BYTE_PCG32 * fmt_it,
+                     "traffic_source": "ncu dram__bytes_read+write of a k_pcg32 launch at 64^3 Q2 per byte of values and "
+                                       "vectors, scaled by those bytes",
+                     "bytes_per_iteration": bit, "ms_per_iteration": ms_it,
+                     "bytes_def": "4*nnz + 36*n (values once; p read, q written; x, r, p, q read, x, r, p written)",
+                     "format_bytes_per_iteration": fmt_it, "format_frac": fmt_it / (ms_it * 1e-3) / 1e9 / hbm},
+        "roofline_spmv": {"kernel": f"{kname}<float,0> (FP32 SpMV alone, {layout}; not launched by the steps)",
+                          "achieved": ach32, "frac": ach32 / hbm, "bytes_per_launch": b32, "ms_per_launch": ms32,
+                          "bytes_def": "4*nnz + 8*n (values once, x once, y once)",
+                          "format_bytes_per_launch": fmt32, "format_frac": fmt32 / (ms32 * 1e-3) / 1e9 / hbm,
+                          "csr_bytes_per_launch": csr_bytes(nfree, nnz, True),
+                          "csr_equivalent_gbs": csr_bytes(nfree, nnz, True) / (ms32 * 1e-3) / 1e9},
         "roofline_fp64": {"kernel": f"{kname}<double,0>", "bound": "fp64 pipe (1 DFMA per stored entry)",
                           "achieved_gbs": ach64, "frac_hbm": ach64 / hbm, "bytes_per_launch": b64,
                           "ms_per_launch": ms64, "dfma_per_s": nent / (ms64 * 1e-3),
