@@ -964,7 +964,7 @@ __global__ void __launch_bounds__(W * 32)
 // out, FP64 and FP32, padding included: no clearing pass and no CSR in between.
 //
 // Bound by load latency and HBM: every element-matrix entry is read once, 216-byte rows for Q2.
-// So eight (row, cell) pairs are loaded before any is summed whatever the class (1, 2, 4 or 8
+// So eight (row, cell) pairs, four for rows of one cell, are loaded before any is summed (1, 2, 4 or 8
 // cells per row: 4, 4, 2 or 1 rows at once) and the slice's row ids come in one load at the
 // block's start.  64^3 Q2 1.80 -> 1.15 ms (2.8 GB read, 1.6 written), 32^3 elasticity Q2 2.78 ->
 // 1.46 ms, 23 x 17 x 21 Q3 0.285 -> 0.245 ms.  Walking the classes together along the mesh, so that
@@ -1201,7 +1201,7 @@ static fg_status poisson_scatter(fg_system* sys, const AsmGeom& g) {
 // FG_TC_INTEGRATION: 0 the FP64-pipe and float-float kernels only; 1 Poisson element
 // matrices on the tensor cores where FP64 integration is asked for; 2 (default) also where
 // float-float is (FG_FAST_INTEGRATION): the tensor-core matrices are FP64-accurate and, on
-// GB300, faster than both (128^3 Q2: 61 / 48 ms per assembly against 186 ms FP64, 84 ms
+// GB300, faster than both (128^3 Q2: 31 / 28 ms per assembly against 177 ms FP64, 75 ms
 // float-float)
 static int tc_integration_mode() {
   const char* e = getenv("FG_TC_INTEGRATION");

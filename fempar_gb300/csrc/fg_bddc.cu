@@ -715,7 +715,7 @@ __device__ __forceinline__ T warp_sum(T v) {
 // date itself and solves them while the other warps apply the last step to the rows beyond; every
 // warp has all loads of its step in flight at once, and a step costs one block barrier.  24^3 Q2
 // elasticity, 512 subdomains of 375 interior and ~950 dofs in all, FP32 factors, one apply: two interior
-// solves 2 x 322 -> 199 us, forward 250 -> 152, backward 364 -> 336 (the loads of a step in groups of
+// solves 322 -> 190 us each, forward 250 -> 150, backward 364 -> 349 (the loads of a step in groups of
 // eight, columns of the transposed product one after another, and solve and update in turn, before).
 
 // x of warp 0's 32 rows for a lower triangle at Ld (rows past n: the unit matrix), with divisions: for the

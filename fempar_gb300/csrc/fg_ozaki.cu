@@ -47,20 +47,10 @@
 // What bounds it: at 4096^3 the MMAs (34 digit pairs, 4.7 PFLOP of bf16 in 2.9 ms beside 0.2 ms
 // of cutting: 1.6 PFLOP/s, 85 % of the measured bf16 rate; without any epilogue work the kernel
 // takes as long).  At K = 128 (8192 x 8192: 0.44 ms) the MMAs run 56 % of the time and the epilogue's
-// ~120 instructions per element, a C tile every 8 K steps, are as long.  What it took, TFLOP/s at
-// 4096^3 and 8192 x 8192 x 128:
-//     13.7 / 13.0  eight epilogue warps converting before they release the accumulators, MMAs
-//                  issued by the lane that also feeds the copies
-//     16.8 / 15.2  release first, sixteen warps
-//     26.0 / 23.0  a copy warp, and MMAs issued from warp-uniform code (descriptors in uniform
-//                  registers)
-//     30.5 / 25.6  each A digit block held in the collector buffer for its run of MMAs
-//     31.8 / 25.3  an A digit against four B digits per MMA (N = 256; no collector needed)
-//     33.3 / 26.2  chunks added as integers instead of in FP64
-//     42.7 / 24.0  the classes in two halves with barriers of their own, so that the epilogue
-//                  empties one half of the tensor memory while the MMAs fill the other
-//     44.0 / 34.5  the conversion to FP64 branch-free (every warp had a lane on the slow side of
-//                  a branch) and the class sums as 64-bit multiply-adds: 150 -> 120 instructions
+// ~120 instructions per element, a C tile every 8 K steps, are as long.  From 13.7 to 44 TFLOP/s at 4096^3 (13 to
+// 33 at K = 128): accumulators released before they are converted, MMAs issued from warp-uniform code,
+// an A digit against four B digits per MMA, chunks of K added as integers, the classes in two halves with barriers
+// of their own, a conversion without branches.
 
 #include <cuda_runtime.h>
 

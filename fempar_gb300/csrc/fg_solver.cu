@@ -450,16 +450,13 @@ __global__ void __launch_bounds__(RB)
 // The CG loop as one cooperative launch.  A launch runs up to max_launch iterations; its
 // blocks are co-resident and meet at grid barriers (one per inner product, and one before
 // the next SpMV gathers the new p; ~1.4 us each), so an iteration costs two or three barriers
-// instead of two or three kernels.  As separate kernels (a CUDA graph of them) each reduction
-// cost 12-18 us whatever the size: 912-1216 blocks took a ticket on one counter, each warp
-// butterflied its sums on the FP64 pipe (16 cycles per warp instruction), and the last block
-// started from cold.  Solve, as kernels -> here: 8^3 Q1 FP64 1.48 -> 0.20 ms, 32^3 Q1 FP64 3.54 ->
-// 1.28 ms, 24^3 Q2 mixed 10.9 -> 4.2 ms, 23 x 17 x 21 Q3 FP64 65.8 -> 36.7 ms, 384^2 Q2 FP64
-// 253 -> 206 ms, 96^3 Q2 mixed 374 -> 361 ms.  Bound by barriers and FP64 latency where the
-// matrix is small, by the SpMV (FP64 pipe; HBM in FP32) where it is large.
+// instead of two or three kernels of a CUDA graph, whose reductions cost 12-18 us each whatever the
+// size (32^3 Q1 FP64 solve 3.54 -> 1.28 ms, 24^3 Q2 mixed 10.9 -> 4.4, 96^3 Q2 mixed 374 -> 358).  Bound by
+// barriers and FP64 latency where the matrix is small, by the SpMV (FP64 pipe; HBM in FP32) where it is
+// large.
 //
-// Rows: warp w of block b owns the slices w nb + b + k (warps nb), k = 0.. (an SM then holds
-// slices of every width).  R > 0: a lane keeps its R rows' x, r, p and 1/d in registers
+// Rows: warp w of the solve's block b (nb of them) owns the slices w nb + b + k (warps nb), k = 0.. (an SM then
+// holds slices of every width).  R > 0: a lane keeps its R rows' x, r, p and 1/d in registers
 // (small and medium systems: at most R slices per warp); only p goes through memory.  R = 0:
 // any size, vectors streamed.
 
@@ -900,7 +897,7 @@ __device__ __forceinline__ void keep_slices(SliceRef<T, ML> (&ref)[RR], float4* 
 // Threads per block.  Streaming kernels: 2 x 16 warps of 64 registers, i.e. more of a slice in flight
 // per warp, rather than 2 x 24 of 40 (96^3 Q2 mixed 370 -> 360 us per iteration, 32^3 Q2 dG mixed 130 ->
 // 124, 384^2 Q2 FP64 55.3 -> 52; 2 x 12 of 80: 377, 130, 57).  FP32 with explicit columns waits for its
-// gathers, each behind a column: 2 x 32 warps (unstructured Q2 40^3 90 -> 67, 48^3 119 -> 110, 64^3
+// gathers, each behind a column: 2 x 32 warps (unstructured Q2 40^3 90 -> 69, 48^3 119 -> 110, 64^3
 // 256 -> 234 against 2 x 16, with both streams prefetched).  FP64 with explicit columns from HBM
 // (R = PCG_WIDE): 2 x 24, two groups in flight (quadrilaterals 1024^2 0.289 -> 0.282 ms, 2048^2 1.113 ->
 // 1.056, unstructured 88^3 1.062 -> 0.994; 384^2, whose 127 MB stay in L2, 52.2 -> 55.2 us; 700^2, 420 MB,
