@@ -92,7 +92,8 @@ struct fg_ctx {
   cudaStream_t stream = nullptr;
   uint64_t budget = 0;
   uint64_t in_use = 0;
-  const std::atomic<int>* solving = nullptr;  // solves running beside this context's (a server's workers)
+  // a server's workers: requests in their solve, and in all (this context's among them)
+  const std::atomic<int>*solving = nullptr, *running = nullptr;
   uint64_t scratch_limit = ~0ull;  // most scratch that elasticity element matrices may take
   int64_t launches = 0;           // kernels launched through this context
   std::map<void*, size_t> allocs;

@@ -75,7 +75,7 @@ struct fg_server {
   std::map<int, std::deque<Request*>> queues;
   std::unordered_map<uint64_t, std::unique_ptr<Request>> reqs;
   std::vector<std::thread> workers;
-  std::atomic<int> solving{0};  // requests in their solve
+  std::atomic<int> solving{0}, running{0};  // requests in their solve, and in all
   bool stop = false;
   uint64_t next_id = 1;
   int64_t completed = 0;
@@ -219,6 +219,7 @@ static void worker_main(fg_server* S) {
   fg_ctx* ctx = nullptr;
   if (fg_ctx_create(S->device, 0, &ctx) != FG_OK) return;
   ctx->solving = &S->solving;
+  ctx->running = &S->running;
   for (;;) {
     Request* R = nullptr;
     {
@@ -232,6 +233,7 @@ static void worker_main(fg_server* S) {
       S->peak = std::max(S->peak, S->reserved);
       R->t_start = Clock::now();
     }
+    ++S->running;
     run_request(ctx, R, S->solving, [&] {
       if (R->scratch == 0) return;
       {
@@ -240,6 +242,7 @@ static void worker_main(fg_server* S) {
       }
       S->cv_work.notify_all();
     });
+    --S->running;
     {
       std::lock_guard<std::mutex> lk(S->mu);
       R->t_end = Clock::now();

@@ -1128,15 +1128,15 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, false), pcg_blocks(R))
 //   q = A^ p, <p,q>, <q,q>; then alpha = |r|^2/<p,q> and, by the recurrence
 //   |r - alpha q|^2 = alpha^2 |q|^2 - |r|^2 (as <r,q> = <p,q> in CG), beta = |r_new|^2/|r|^2;
 //   x += alpha p; r -= alpha q; p = r + beta p; the exact |r_new|^2 for the next alpha, and on
-//   every FG_MIXED_EXACT_EVERY-th iteration sum r^2 D (the unscaled residual, for the stop
-//   estimate).
+//   every FG_MIXED_EXACT_EVERY-th iteration of the segment (phase: those before this launch) sum r^2 D
+//   (the unscaled residual, for the stop estimate), with the caller's polling interval also on its last.
 // A segment end (reliable update, stop check, breakdown, iteration limit) found by an update
 // is taken one iteration later: that iteration's update keeps p, so the host can fold x and
 // restart the recursion from the true residual with the direction kept.
 template <int ML, int R>
 __global__ void __launch_bounds__(pcg_threads(R, ML, true), pcg_blocks(R))
     k_pcg32(MatArgs<float> m, int64_t nvec, float* x, float* r, float* p, float* q, const float* __restrict__ idiag,
-            int max_launch, int keep, int vblocks, GridSync g, double* S, int* I) {
+            int max_launch, int phase, int last_exact, int keep, int vblocks, GridSync g, double* S, int* I) {
   extern __shared__ __align__(16) int32_t s_off_buf[];
   __shared__ RedShared<float> sh;
   __shared__ double sd[8];  // rr, rmax^2, delta^2, (tol/sigma)^2, 1/rr, app, alpha, beta
@@ -1249,7 +1249,7 @@ __global__ void __launch_bounds__(pcg_threads(R, ML, true), pcg_blocks(R))
       return;
     const float a = sf[0], b = sf[1];
     const bool keep_p = si[1] != 0;
-    const bool exact = n % FG_MIXED_EXACT_EVERY == FG_MIXED_EXACT_EVERY - 1 || n == max_launch - 1;
+    const bool exact = (n + phase) % FG_MIXED_EXACT_EVERY == FG_MIXED_EXACT_EVERY - 1 || (last_exact && n == max_launch - 1);
     // unscaled residual entry r^ sqrt(d): r^2 d = r^2 / (1/d); slots that are not free dofs hold
     // r = 0 and 1/d = 0: skipped
     auto unscaled = [](Acc<float>& rt, float ri, float di) { rt.add(ri, di != 0.f ? ri / di : 0.f); };
@@ -1772,13 +1772,19 @@ static int pcg_vblocks(const fg_ctx* ctx, const PcgShape& sh) {
   return ctx->solving && ctx->solving->load(std::memory_order_relaxed) > 1 ? 2 : 1;
 }
 
-// Iterations of one launch: about 5 ms (contexts on other threads get the GPU in between),
-// or the caller's polling interval.
-static int pcg_iters(const fg_solver_params* prm, int64_t entries, int64_t nvec, int width) {
+// Iterations of one launch: the caller's polling interval; or about 5 ms, at least 16 iterations while they
+// stay under 15 ms (a launch costs ~20 us of host time: 0.3 % of a 128^3 Q2 step in launches of 5 ms); or about 1 ms
+// while other requests of the same server run, as a launch holds the SMs and every kernel and host
+// synchronisation of a small request beside it waits for its end.  (Launches of at least 16 iterations, 50 ms at
+// 96^3 Q2 elasticity, gave a server's mix a median latency of 237 ms; kernels in a graph 161; this 97-113.)  The
+// iterates do not depend on it.
+static int pcg_iters(const fg_ctx* ctx, const fg_solver_params* prm, int64_t entries, int64_t nvec, int width) {
   if (prm->check_every > 0) return prm->check_every;
+  if (const char* e = getenv("FG_PCG_TEST_LAUNCH_ITERS")) return std::max(1, atoi(e));  // tests
   const double us = 8.0 + ((double)entries + 10.0 * (double)nvec) * width / 5.5e6;
-  const int n = (int)(5000.0 / us) & ~7;
-  return std::min(1024, std::max(16, n));
+  const bool beside = ctx->running && ctx->running->load(std::memory_order_relaxed) > 1;
+  const double n = beside ? 1000.0 / us : std::max(5000.0 / us, std::min(16.0, 15000.0 / us));
+  return (int)std::min(1024.0, std::max(1.0, n));
 }
 
 // scalars and flags of the solve, copied to the host in one piece
@@ -1824,7 +1830,7 @@ static fg_status run_pcg64(fg_system* sys, const Work& w, const fg_solver_params
   int64_t nvec = sp->nvec;
   double *x = w.x, *r = w.r, *p = w.p, *Ap = w.Ap;
   const double* idiag = prm->precond == FG_PREC_JACOBI ? sys->d_idiag : nullptr;
-  int iters = pcg_iters(prm, solver_entries(sp), nvec, 8);
+  int iters = 0;
   GridSync g = grid_sync(w);
   double* S = w.S;
   int* I = w.I;
@@ -1838,6 +1844,7 @@ static fg_status run_pcg64(fg_system* sys, const Work& w, const fg_solver_params
   FG_TRY(pcg_keep(k, sh, m.noff, solver_entries(sp), 8, &keep, &smem));
   for (;;) {
     vb = pcg_vblocks(sp->mesh->ctx, sh);
+    iters = pcg_iters(sp->mesh->ctx, prm, solver_entries(sp), nvec, 8);
     FG_TRY(launch_pcg(k, sh, vb, w, smem, st, args));
     sp->mesh->ctx->launches += 1;
     FG_TRY(read_state(w, h, st));
@@ -1860,23 +1867,27 @@ static fg_status run_pcg32(fg_system* sys, const Work& w, const fg_solver_params
   const PcgShape sh = pcg_shape(m.nslices, 4 * solver_entries(sp), true, ml, w.sms);
   int64_t nvec = sp->nvec;
   float *x = w.x32, *r = w.r32, *p = w.p32, *q = w.Ap32;
-  int iters = pcg_iters(prm, solver_entries(sp), nvec, 4);
+  // (the first segment of a solve starts with no state on the host)
+  int iters = 0, phase = 0, last_exact = prm->check_every > 0 ? 1 : 0;
+  const int it0 = h.I[I_ITER];
   GridSync g = grid_sync(w);
   double* S = w.S;
   int* I = w.I;
   int keep = 0;
   size_t smem = 0;
   int vb = 1;
-  void* args[] = {&m, &nvec, &x, &r, &p, &q, &idiag, &iters, &keep, &vb, &g, &S, &I};
+  void* args[] = {&m, &nvec, &x, &r, &p, &q, &idiag, &iters, &phase, &last_exact, &keep, &vb, &g, &S, &I};
 #define FG_PCG32(L) (sh.R == 1 ? k_pcg32<L, 1> : sh.R == 2 ? k_pcg32<L, 2> : k_pcg32<L, 0>)
   auto k = ml == ML_STENCIL ? FG_PCG32(ML_STENCIL) : ml == ML_DG ? FG_PCG32(ML_DG) : FG_PCG32(ML_SELL);
 #undef FG_PCG32
   FG_TRY(pcg_keep(k, sh, m.noff, solver_entries(sp), 4, &keep, &smem));
   do {
     vb = pcg_vblocks(sp->mesh->ctx, sh);
+    iters = pcg_iters(sp->mesh->ctx, prm, solver_entries(sp), nvec, 4);
     FG_TRY(launch_pcg(k, sh, vb, w, smem, st, args));
     sp->mesh->ctx->launches += 1;
     FG_TRY(read_state(w, h, st));
+    if (!last_exact) phase = (h.I[I_ITER] - it0) % FG_MIXED_EXACT_EVERY;
   } while (!h.I[I_DONE]);
   return FG_OK;
 }

@@ -74,3 +74,33 @@ def test_server_gives_the_same_bits_alone_and_beside_others(fg):
         out.append(xs)
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("kind,n,order", [("poisson", (9, 8, 7), 2), ("poisson", (26, 24, 25), 2), ("poisson", (40, 36, 38), 2),
+                                          ("elasticity", (19, 19, 19), 2)],
+                         ids=["one_block", "one_slice_per_warp", "two_slices_per_warp", "streamed"])
+def test_bits_do_not_depend_on_the_length_of_launches(fg, monkeypatch, kind, n, order):
+    """Launches of 1, 3, 8 and 21 iterations against the default (~5 ms): the stop estimate of the mixed
+    iteration is taken at the same iterations of a segment whatever launch they are in."""
+    ctx = fg.Context(0)
+    tri = fg.SerialTriangulation(ctx, n)
+    coef = np.exp(np.random.default_rng(1).normal(size=int(np.prod(n))))
+    if kind == "elasticity":
+        space = fg.SerialFESpace(tri, order=order, ncomp=3, dirichlet_ids=[1, 3, 5, 7, 13, 15, 17, 19, 25])
+        integ = fg.ElasticityIntegration(cell_coef=coef, nu=0.3, source_fn=fg.FG_FN_CONST, fn_param=[0.0, 0.0, -1.0])
+    else:
+        space = fg.SerialFESpace(tri, order=order, dirichlet_ids=list(range(1, 27)))
+        integ = fg.PoissonIntegration(cell_coef=coef, source_fn=fg.FG_FN_CONST, fn_param=[1.0])
+    op = fg.FEAffineOperator(space, integ).compute()
+    for prec in ("mixed", "fp64"):
+        s = fg.IterativeLinearSolver().set_type_from_string("CG").set_operators(op, "jacobi")
+        s.set_parameters_from_pl({"ILS_RTOL": 1e-5, "ILS_MAX_NUM_ITERATIONS": 5000, "PRECISION": prec})
+        x, i = s.solve(), s.info()["iterations"]
+        assert s.info()["converged"]
+        for its in ("1", "3", "8", "21"):
+            monkeypatch.setenv("FG_PCG_TEST_LAUNCH_ITERS", its)
+            assert np.array_equal(x, s.solve()) and s.info()["iterations"] == i, (prec, its)
+        monkeypatch.delenv("FG_PCG_TEST_LAUNCH_ITERS")
+    op.close()
+    space.close()
+    tri.close()
