@@ -16,6 +16,11 @@ void set_error(const char* fmt, ...) {
   va_end(ap);
 }
 
+DeviceLoad* device_load(int device) {
+  static DeviceLoad loads[64];
+  return &loads[device & 63];
+}
+
 fg_status dev_alloc(fg_ctx* ctx, void** p, size_t bytes) {
   *p = nullptr;
   if (bytes == 0) bytes = 16;
@@ -60,7 +65,9 @@ using namespace fg;
     }                                     \
   } while (0)
 
-#define FG_DEVICE_GUARD(ctx) FG_CUDA_TRY(cudaSetDevice((ctx)->device))
+#define FG_DEVICE_GUARD(ctx)                     \
+  FG_CUDA_TRY(cudaSetDevice((ctx)->device));     \
+  const CallScope fg_call_scope((ctx)->load)
 
 extern "C" {
 
@@ -115,6 +122,7 @@ fg_status fg_ctx_create(int device, uint64_t hbm_budget_bytes, fg_ctx** out) {
   FG_CUDA_TRY(cudaSetDevice(device));
   fg_ctx* c = new fg_ctx();
   c->device = device;
+  c->load = device_load(device);
   cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {

@@ -1102,6 +1102,7 @@ fg_status fg_batch_create(fg_ctx* ctx, int32_t nprob, const fg_batch_problem* pr
     return FG_ERR_BADARG;
   }
   FG_CUDA_TRY(cudaSetDevice(ctx->device));
+  const CallScope call(ctx->load);
   fg_batch* B = new fg_batch();
   B->ctx = ctx;
   if (const char* env = std::getenv("FG_BATCH_TEAM_SHARE"))
@@ -1276,6 +1277,7 @@ fg_status fg_batch_run(fg_batch* B, fg_batch_result* results) {
   }
   fg_ctx* ctx = B->ctx;
   FG_CUDA_TRY(cudaSetDevice(ctx->device));
+  const CallScope call(ctx->load);
   cudaStream_t st = ctx->stream;
   const bool dev = (B->flags & FG_INPUTS_ON_DEVICE) != 0;
   cudaEvent_t e0, e1;

@@ -2364,6 +2364,7 @@ fg_status fg_bddc_create(fg_system* sys, const fg_bddc_params* prm, fg_bddc** ou
   fg_space* sp = sys->space;
   fg_ctx* ctx = sp->mesh->ctx;
   FG_CUDA_TRY(cudaSetDevice(ctx->device));
+  const CallScope call(ctx->load);
   if (sp->mesh->unst || sp->dg || sp->mesh->dim != 3) {
     set_error("BDDC: box subdomains are built for continuous spaces on structured meshes only");
     return FG_ERR_UNSUPPORTED;
@@ -2434,6 +2435,7 @@ fg_status fg_bddc_create(fg_system* sys, const fg_bddc_params* prm, fg_bddc** ou
 fg_status fg_bddc_numerical_setup(fg_bddc* B) {
   if (!B) return bddc_bad("bddc");
   FG_CUDA_TRY(cudaSetDevice(B->sys->space->mesh->ctx->device));
+  const CallScope call((B->sys->space->mesh->ctx)->load);
   double t0 = now_ms();
   FG_TRY(bddc_numeric(B));
   B->numeric_ms = now_ms() - t0;
@@ -2463,6 +2465,7 @@ fg_status fg_bddc_apply_device(fg_bddc* B, int precision, const double* r_dev, d
   fg_space* sp = B->sys->space;
   fg_ctx* ctx = sp->mesh->ctx;
   FG_CUDA_TRY(cudaSetDevice(ctx->device));
+  const CallScope call(ctx->load);
   FG_TRY(ensure_pcg(B));
   const int64_t n = sp->nfree;
   cudaStream_t st = ctx->stream;
@@ -2490,6 +2493,7 @@ fg_status fg_bddc_solve_device(fg_bddc* B, const fg_solver_params* prm, const do
   if (!B || !x_dev) return bddc_bad("bddc/x");
   FG_TRY(check_solve(prm));
   FG_CUDA_TRY(cudaSetDevice(B->sys->space->mesh->ctx->device));
+  const CallScope call((B->sys->space->mesh->ctx)->load);
   return bddc_pcg(B, prm, b_dev, x0_dev, x_dev, info);
 }
 
@@ -2500,6 +2504,7 @@ fg_status fg_bddc_solve(fg_bddc* B, const fg_solver_params* prm, const double* b
   fg_space* sp = B->sys->space;
   fg_ctx* ctx = sp->mesh->ctx;
   FG_CUDA_TRY(cudaSetDevice(ctx->device));
+  const CallScope call(ctx->load);
   const int64_t n = sp->nfree;
   const size_t bytes = sizeof(double) * (size_t)(n > 0 ? n : 1);
   double *db = nullptr, *dx0 = nullptr, *dx = nullptr;

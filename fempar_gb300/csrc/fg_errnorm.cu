@@ -300,6 +300,7 @@ extern "C" fg_status fg_system_error_norms(fg_system* sys, const double* x, int3
     return FG_ERR_BADARG;
   }
   FG_CUDA_TRY(cudaSetDevice(ctx->device));
+  const CallScope call(ctx->load);
   cudaStream_t st = ctx->stream;
   const int64_t nc = sp->mesh->ncells, n = sp->nfree;
   double *dx = nullptr, *dC = nullptr, *dout = nullptr, *dprm = nullptr, *de = nullptr;

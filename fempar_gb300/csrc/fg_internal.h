@@ -86,14 +86,53 @@ struct DevTables {
 
 }  // namespace fg
 
+namespace fg {
+
+// Calls that the contexts of a device are in, in this process: how CG launches divide the SMs' time
+// (fg_solver.cu).  It decides the width and length of launches only, never a result.
+struct DeviceLoad {
+  std::atomic<int> running{0};  // threads in a call that computes on the device
+  std::atomic<int> solving{0};  // of them in a solve
+};
+DeviceLoad* device_load(int device);
+
+// counts the calling thread while its outermost call lasts
+class CallScope {
+ public:
+  explicit CallScope(DeviceLoad* l) : load_(depth_++ == 0 ? l : nullptr) {
+    if (load_) ++load_->running;
+  }
+  ~CallScope() {
+    --depth_;
+    if (load_) --load_->running;
+  }
+  CallScope(const CallScope&) = delete;
+  CallScope& operator=(const CallScope&) = delete;
+
+ private:
+  static inline thread_local int depth_ = 0;
+  DeviceLoad* load_;
+};
+class SolveScope {
+ public:
+  explicit SolveScope(DeviceLoad* l) : load_(l) { ++load_->solving; }
+  ~SolveScope() { --load_->solving; }
+  SolveScope(const SolveScope&) = delete;
+  SolveScope& operator=(const SolveScope&) = delete;
+
+ private:
+  DeviceLoad* load_;
+};
+
+}  // namespace fg
+
 struct fg_ctx {
   int device = 0;
   int sm_count = 0;
   cudaStream_t stream = nullptr;
   uint64_t budget = 0;
   uint64_t in_use = 0;
-  // a server's workers: requests in their solve, and in all (this context's among them)
-  const std::atomic<int>*solving = nullptr, *running = nullptr;
+  fg::DeviceLoad* load = nullptr; // of the context's device
   uint64_t scratch_limit = ~0ull;  // most scratch that elasticity element matrices may take
   int64_t launches = 0;           // kernels launched through this context
   std::map<void*, size_t> allocs;

@@ -892,6 +892,7 @@ fg_status fg_dense_gemm_nt(fg_ctx* ctx, int64_t m, int64_t n, int64_t k, double 
     return FG_ERR_BADARG;
   }
   FG_CUDA_TRY(cudaSetDevice(ctx->device));
+  const CallScope call(ctx->load);
   if (m == 0 || n == 0) return FG_OK;
   void* work = nullptr;
   FG_TRY(dev_alloc(ctx, &work, ozaki_workspace_bytes(m, n, k, B == nullptr) + 16));

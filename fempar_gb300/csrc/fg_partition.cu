@@ -496,6 +496,7 @@ fg_status fg_partition_create(fg_space* space, const int32_t num_parts_x_dir[3],
   }
   fg_ctx* ctx = space->mesh->ctx;
   FG_CUDA_TRY(cudaSetDevice(ctx->device));
+  const CallScope call(ctx->load);
   fg_partition* P = new fg_partition();
   P->gsp = space;
   for (int d = 0; d < 3; ++d) P->np[d] = num_parts_x_dir[d];
@@ -597,6 +598,7 @@ fg_status fg_partition_assemble(fg_partition* P, const fg_integrand* integrand, 
 fg_status fg_partition_comm_device(fg_partition* P, double* x) {
   if (!P || !x) { set_error("bad argument: partition/x"); return FG_ERR_BADARG; }
   FG_CUDA_TRY(cudaSetDevice(P->gsp->mesh->ctx->device));
+  const CallScope call((P->gsp->mesh->ctx)->load);
   FG_TRY(partition_comm(P, x));
   FG_CUDA_TRY(cudaStreamSynchronize(P->gsp->mesh->ctx->stream));
   return FG_OK;
@@ -613,6 +615,7 @@ fg_status fg_partition_solve(fg_partition* P, fg_system* sub, const fg_solver_pa
   if (!sub->d_val) { set_error("the partitioned system was assembled lean"); return FG_ERR_UNSUPPORTED; }
   fg_ctx* ctx = P->gsp->mesh->ctx;
   FG_CUDA_TRY(cudaSetDevice(ctx->device));
+  const CallScope call(ctx->load);
   const int64_t n = P->nl;
   double* w = nullptr;  // b d x r z p q dinv | partials | scalar
   FG_TRY(dev_alloc(ctx, (void**)&w, sizeof(double) * (8 * (size_t)n + kDotBlocks + 8)));

@@ -13,7 +13,6 @@
 // builds mesh, space and system on the device, solves (mixed precision by default) and
 // copies its solution to a host buffer, then frees its device memory.
 #include <algorithm>
-#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <condition_variable>
@@ -75,7 +74,6 @@ struct fg_server {
   std::map<int, std::deque<Request*>> queues;
   std::unordered_map<uint64_t, std::unique_ptr<Request>> reqs;
   std::vector<std::thread> workers;
-  std::atomic<int> solving{0}, running{0};  // requests in their solve, and in all
   bool stop = false;
   uint64_t next_id = 1;
   int64_t completed = 0;
@@ -153,7 +151,7 @@ static uint64_t element_scratch(const fg_request* q) {
 
 // assembled: called once the element matrices are done with their scratch
 template <class F>
-static void run_request(fg_ctx* ctx, Request* R, std::atomic<int>& solving, F assembled) {
+static void run_request(fg_ctx* ctx, Request* R, F assembled) {
   ctx->scratch_limit = R->scratch;
   fg_status s = FG_OK;
   fg_mesh* mesh = nullptr;
@@ -184,9 +182,7 @@ static void run_request(fg_ctx* ctx, Request* R, std::atomic<int>& solving, F as
     fg_space_get_info(sp, &si);
     R->x.assign(si.num_free, 0.0);
     R->res.num_free = si.num_free;
-    ++solving;
     s = fg_solve(sys, &R->r.solver, nullptr, nullptr, R->x.data(), &info);
-    --solving;
   }
   R->res.status = s;
   R->res.iterations = info.iterations;
@@ -218,8 +214,6 @@ static Request* pick(fg_server* S) {
 static void worker_main(fg_server* S) {
   fg_ctx* ctx = nullptr;
   if (fg_ctx_create(S->device, 0, &ctx) != FG_OK) return;
-  ctx->solving = &S->solving;
-  ctx->running = &S->running;
   for (;;) {
     Request* R = nullptr;
     {
@@ -233,8 +227,7 @@ static void worker_main(fg_server* S) {
       S->peak = std::max(S->peak, S->reserved);
       R->t_start = Clock::now();
     }
-    ++S->running;
-    run_request(ctx, R, S->solving, [&] {
+    run_request(ctx, R, [&] {
       if (R->scratch == 0) return;
       {
         std::lock_guard<std::mutex> lk(S->mu);
@@ -242,7 +235,6 @@ static void worker_main(fg_server* S) {
       }
       S->cv_work.notify_all();
     });
-    --S->running;
     {
       std::lock_guard<std::mutex> lk(S->mu);
       R->t_end = Clock::now();

@@ -1759,7 +1759,7 @@ static fg_status launch_pcg(void (*k)(KA...), const PcgShape& sh, int vblocks, c
 }
 
 // Blocks of a solve per block of the launch.  A streaming solve's 2 x SMs blocks fill the SMs, so those of
-// several contexts would take turns; while other requests of the same server solve, a launch is half as wide
+// several contexts would take turns; while another context of the device solves, a launch is half as wide
 // and its blocks do two of the solve's each, so that two solves share the SMs and fill one another's waits.
 // The sums are the same blocks' in the same order: the same bits.  Alone, half the warps cost 15-25 %
 // (96^3 Q2 mixed 361 -> 480 us per iteration); two contexts at once solve 24^3 Q2 elasticity 11.9 times a
@@ -1769,20 +1769,20 @@ static int pcg_vblocks(const fg_ctx* ctx, const PcgShape& sh) {
   if (sh.R > 0) return 1;
   const char* e = getenv("FG_PCG_TEST_SHARE");
   if (e && e[0] == '1') return 2;
-  return ctx->solving && ctx->solving->load(std::memory_order_relaxed) > 1 ? 2 : 1;
+  return ctx->load->solving.load(std::memory_order_relaxed) > 1 ? 2 : 1;
 }
 
 // Iterations of one launch: the caller's polling interval; or about 5 ms, at least 16 iterations while they
 // stay under 15 ms (a launch costs ~20 us of host time: 0.3 % of a 128^3 Q2 step in launches of 5 ms); or about 1 ms
-// while other requests of the same server run, as a launch holds the SMs and every kernel and host
-// synchronisation of a small request beside it waits for its end.  (Launches of at least 16 iterations, 50 ms at
+// while another thread is in a call on the device, as a launch holds the SMs and every kernel and host
+// synchronisation of a small solve beside it waits for its end.  (Launches of at least 16 iterations, 50 ms at
 // 96^3 Q2 elasticity, gave a server's mix a median latency of 237 ms; kernels in a graph 161; this 97-113.)  The
 // iterates do not depend on it.
 static int pcg_iters(const fg_ctx* ctx, const fg_solver_params* prm, int64_t entries, int64_t nvec, int width) {
   if (prm->check_every > 0) return prm->check_every;
   if (const char* e = getenv("FG_PCG_TEST_LAUNCH_ITERS")) return std::max(1, atoi(e));  // tests
   const double us = 8.0 + ((double)entries + 10.0 * (double)nvec) * width / 5.5e6;
-  const bool beside = ctx->running && ctx->running->load(std::memory_order_relaxed) > 1;
+  const bool beside = ctx->load->running.load(std::memory_order_relaxed) > 1;
   const double n = beside ? 1000.0 / us : std::max(5000.0 / us, std::min(16.0, 15000.0 / us));
   return (int)std::min(1024.0, std::max(1.0, n));
 }
@@ -1896,6 +1896,7 @@ fg_status system_solve(fg_system* sys, const fg_solver_params* prm, const double
                        double* d_x, fg_solve_info* info) {
   fg_space* sp = sys->space;
   fg_ctx* ctx = sp->mesh->ctx;
+  const SolveScope solving(ctx->load);
   cudaStream_t st = ctx->stream;
   const int64_t n = sp->nfree, nv = sp->nvec;
   fg_solve_info out;
